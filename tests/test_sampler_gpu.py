@@ -91,6 +91,34 @@ def test_top_k_path_with_many_equal_logits(gpu, top_k, top_p):
     assert np.array_equal(tok_o, tok_g), f"{(tok_o != tok_g).sum()} of {n} tokens differ"
 
 
+@pytest.mark.parametrize("top_k", [1, 2, 3, 4, 31, 32, 33, 48, 63, 64, 65, 66, 129])
+def test_top_k_heap_sizes_and_row_shapes_are_identical(gpu, top_k):
+    """Heap sizes around the ones whose layout changes (a warp's registers hold 64), rows shorter than a filter round, odd
+    vocabularies (rows that start off a 16-byte boundary), ascending rows, equal values, -0 beside +0, masked rows, and NaN
+    among the first K, where the heap has no order and the elements are taken one by one."""
+    rng = np.random.default_rng(1000 + top_k)
+    for v in (top_k + 1, top_k + 6, 997, 4003, 30011):
+        if v <= top_k:
+            continue
+        x = (rng.standard_normal((10, v)) * 3).astype(np.float32)
+        x[1] = np.round(x[1] * 2) / 2                       # ties, zeros of both signs
+        x[2] = np.sort(x[2])
+        x[3] = np.sort(x[3])[::-1]
+        x[4] = np.round(np.sort(x[4]))
+        x[5, rng.random(v) < 0.97] = -np.inf
+        x[6] = (x[6].view(np.uint32) & 0xffff0000).view(np.float32)   # bf16 values
+        x[7, rng.integers(0, top_k)] = np.nan               # (uniform fallback: the heap order decides the token)
+        x[8, v - 1] = np.nan
+        x[9] = -0.0
+        x[9, ::3] = 0.0
+        for top_p, min_p in ((0.9, 0.0), (1.0, 0.0), (0.97, 0.02)):
+            use = [r for r in range(10) if not (r == 7 and top_p != 1.0)]   # sorting NaN is undefined in the reference
+            rows = H.make_rows(len(use), top_k=top_k, temperature=0.8, top_p=top_p, min_p=min_p, seeds=np.arange(len(use)) + 31 * top_k)
+            tok_o, lp_o, _, tok_g, lp_g, _ = _both(gpu, np.ascontiguousarray(x[use]), rows)
+            assert np.array_equal(tok_o, tok_g), (v, top_p, min_p, tok_o, tok_g)
+            assert np.allclose(lp_o, lp_g, atol=2e-6, rtol=1e-6, equal_nan=True)
+
+
 def test_small_vocab_and_k_not_below_vocab(gpu):
     rng = np.random.default_rng(9)
     x = (rng.standard_normal((5, 40)) * 2).astype(np.float32)
