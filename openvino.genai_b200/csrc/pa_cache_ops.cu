@@ -99,21 +99,25 @@ __device__ void build_decode_plan(const KernelArgs& a) {
             for (int w = tid; w < a.decode_all_workers; w += 256) a.worker_start[w] = WorkerStart{-1, 0, 0, total_tiles, 0, 0, 0, 0};
         }
     }
-    // The prefill kernel hands out (q tile, kv head) items from a counter.  Longest context first keeps
-    // the last items short, so the CTAs finish together; sequence order leaves a long item for the end.
+    // The prefill kernel hands out (q tile, kv head) items from a counter.  Longest context first keeps the last items
+    // short, so the CTAs finish together; sequence order leaves a long item for the end.
     const int total_p = sh_run_p;
     const bool sort_items = a.pitem_order != nullptr && total_p > 1 && total_p <= kPrefillSortCap;
     if (sort_items) {
         __shared__ int sh_cost[kPrefillSortCap];
+        const bool in_shared = B <= kPrefixCap;
         if (tid == 0) a.ptile_prefix[B] = total_p;
         __syncthreads();   // the prefix sums written above are visible to the whole block
+        if (in_shared)
+            for (int s = tid; s <= B; s += 256) sh_prefix[s] = a.ptile_prefix[s];   // (the decode prefix there is no longer needed)
+        __syncthreads();
         for (int t = tid; t < total_p; t += 256) {
             int lo = 0, hi = B;   // ptile_prefix[lo] <= t < ptile_prefix[hi]
             while (hi - lo > 1) {
                 const int mid = (lo + hi) >> 1;
-                if (a.ptile_prefix[mid] <= t) lo = mid; else hi = mid;
+                if ((in_shared ? sh_prefix[mid] : a.ptile_prefix[mid]) <= t) lo = mid; else hi = mid;
             }
-            const int p0 = a.ptile_prefix[lo], np = a.ptile_prefix[lo + 1] - p0;
+            const int p0 = in_shared ? sh_prefix[lo] : a.ptile_prefix[lo], np = (in_shared ? sh_prefix[lo + 1] : a.ptile_prefix[lo + 1]) - p0;
             const int qt = np - 1 - (t - p0);   // the kernel's mapping: late (heavy) q tiles first
             const int n_new = a.subsequence_begins[lo + 1] - a.subsequence_begins[lo];
             const int r_hi = min(n_new * G, (qt + 1) * kPrefillItemRows) - 1;
@@ -140,46 +144,219 @@ __device__ void build_decode_plan(const KernelArgs& a) {
     }
 }
 
-// One warp per (token, kv head).  Lane l owns dims {l + 32*i}.  With PLAN set, the last block of
+// Eight consecutive activations as they lie in memory, and their values.  The loads are apart from the conversions so that
+// those of several pieces are in flight together: with the branch on the type around each load they were not.
+template <bool F32>
+struct RawAct8 {
+    uint4 w[F32 ? 2 : 1];
+    __device__ __forceinline__ void load(const void* p, long long i) {   // 16-byte aligned
+        const uint4* q = reinterpret_cast<const uint4*>((const uint8_t*)p + i * (F32 ? 4 : 2));
+#pragma unroll
+        for (int k = 0; k < (F32 ? 2 : 1); ++k) w[k] = q[k];
+    }
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int k = 0; k < (F32 ? 2 : 1); ++k) w[k] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    __device__ __forceinline__ void values(int act, float (&out)[8]) const {
+        if constexpr (F32) {
+            const uint32_t u[8] = {w[0].x, w[0].y, w[0].z, w[0].w, w[1].x, w[1].y, w[1].z, w[1].w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) out[e] = __uint_as_float(u[e]);
+        } else {
+            const uint32_t u[4] = {w[0].x, w[0].y, w[0].z, w[0].w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const unsigned short b = (unsigned short)(u[e / 2] >> (16 * (e & 1)));
+                out[e] = act == PA_DTYPE_F16 ? __half2float(__ushort_as_half(b)) : __bfloat162float(__ushort_as_bfloat16(b));
+            }
+        }
+    }
+};
+
+// Cache record (byte offset of (block, head 0)) and slot of flattened token t, or false with the status bit set.
+__device__ __forceinline__ bool locate_token(const KernelArgs& a, int t, bool report, long long& rec, int& slot) {
+    const int s = find_sequence(a.subsequence_begins, a.num_sequences, t);
+    SeqView sv;
+    if (!seq_view(a, s, sv)) return false;
+    if (t < sv.t0 || t >= sv.t0 + sv.n) {   // prefix sums that are not monotone, or that leave tokens uncovered
+        if (report) atomicOr(a.status, PA_DEV_BAD_BEGINS);
+        return false;
+    }
+    const int pos = sv.past + (t - sv.t0);
+    const int block = a.block_indices[sv.tb + pos / a.g.bs];
+    if (block < 0 || block >= a.num_blocks) {
+        if (report) atomicOr(a.status, PA_DEV_BAD_BLOCK_INDEX);
+        return false;
+    }
+    slot = pos % a.g.bs;
+    rec = (long long)block * a.g.block_bytes;
+    return true;
+}
+
+// Chunks: one CTA writes kWriteTokens consecutive tokens of one kv head, eight lanes per token.  A token is located once per
+// CTA (a chain of about eight dependent loads) instead of once per head and warp, activations come in 16-byte pieces that
+// are all in flight together, the quantiser's divisions are shared by sixteen elements per lane, and the token-minor value
+// bytes of the u8 cache are turned around in shared memory and leave as words instead of single bytes.  Bound by the chain
+// locate -> load -> quantise -> store and, from some 30 k rows on, by the bytes: 65536 rows (bf16 in, u8 out) 55 -> 26 us.
+constexpr int kWriteTokens = 32;
+constexpr long long kWriteGroupRows = 2048;
+template <int D, bool F32>
+__device__ __forceinline__ void write_group(const KernelArgs& a, int group, int h) {
+    constexpr int NP = D / 64;                      // pieces of eight dims per lane: dims 8 l + 64 p
+    constexpr int kCols = kWriteTokens + 4, kColWords = kCols / 4;
+    __shared__ long long sh_rec[kWriteTokens];      // record of (block, head) or -1
+    __shared__ int sh_slot[kWriteTokens];
+    __shared__ long long sh_word[kColWords];        // where a word of four columns goes in its record's value data, or -1
+    __shared__ __align__(4) uint8_t sh_v[D][kCols]; // value bytes, column = token + slot of the first token mod 4
+    const int tid = threadIdx.x;
+    const int t0 = group * kWriteTokens, n = min(kWriteTokens, a.num_tokens - t0);
+    if (tid < kWriteTokens) {
+        long long rec = -1;
+        int slot = 0;
+        if (tid < n && locate_token(a, t0 + tid, h == 0, rec, slot)) rec += (long long)h * a.g.head_bytes;
+        else rec = -1;
+        sh_rec[tid] = rec;
+        sh_slot[tid] = slot;
+    }
+    const int i = tid >> 3, l = tid & 7;            // token, lane of the token
+    RawAct8<F32> kraw[NP], vraw[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        const long long src = ((long long)(t0 + i) * a.g.Hkv + h) * D + 8 * l + 64 * p;
+        if (i < n) { kraw[p].load(a.key, src); vraw[p].load(a.value, src); }
+        else { kraw[p].zero(); vraw[p].zero(); }
+    }
+    __syncthreads();
+    const long long rec = sh_rec[i];
+    const int slot = sh_slot[i];
+    if (a.g.cache != PA_DTYPE_U8) {
+        if (rec < 0) return;
+        const bool same = !F32 && a.g.act == a.g.cache;   // 16-bit activations of the cache's type go in as they are
+#pragma unroll
+        for (int kv = 0; kv < 2; ++kv) {
+            uint8_t* dst = (uint8_t*)(kv ? a.value_cache : a.key_cache) + rec + (long long)slot * D * 2;
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                const RawAct8<F32>& raw = kv ? vraw[p] : kraw[p];
+                uint4 w = raw.w[0];
+                if (!same) {
+                    float x[8];
+                    raw.values(a.g.act, x);
+                    uint32_t o[4];
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2)
+                        o[e / 2] = a.g.cache == PA_DTYPE_F16
+                                       ? __half_as_ushort(__float2half_rn(x[e])) | (uint32_t)__half_as_ushort(__float2half_rn(x[e + 1])) << 16
+                                       : __bfloat16_as_ushort(__float2bfloat16_rn(x[e])) | (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x[e + 1])) << 16;
+                    w = make_uint4(o[0], o[1], o[2], o[3]);
+                }
+                *reinterpret_cast<uint4*>(dst + (8 * l + 64 * p) * 2) = w;
+            }
+        }
+        return;
+    }
+    const int shift = sh_slot[0] & 3;
+    if (tid < kColWords) {   // a word whose tokens are neighbours in one record is stored as one
+        const int i0 = 4 * tid - shift;
+        bool whole = i0 >= 0 && i0 + 3 < kWriteTokens;
+        if (whole) {
+            whole = sh_rec[i0] >= 0 && (sh_slot[i0] & 3) == 0;
+            for (int u = 1; u < 4; ++u) whole = whole && sh_rec[i0 + u] == sh_rec[i0] && sh_slot[i0 + u] == sh_slot[i0] + u;
+        }
+        sh_word[tid] = whole ? sh_rec[i0] + sh_slot[i0] : -1;
+    }
+#pragma unroll
+    for (int kv = 0; kv < 2; ++kv) {
+        float x[NP][8];
+        float mn = 0.f, mx = 0.f;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            (kv ? vraw[p] : kraw[p]).values(a.g.act, x[p]);
+            if (p == 0) { mn = x[0][0]; mx = x[0][0]; }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) { mn = fminf(mn, x[p][e]); mx = fmaxf(mx, x[p][e]); }
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {   // over the token's lanes
+            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        }
+        float sc, zp, inv;
+        quant_params(mn, mx, sc, zp, inv);
+        uint8_t* data = (uint8_t*)(kv ? a.value_cache : a.key_cache) + (rec < 0 ? 0 : rec);
+        if (rec >= 0 && l == 0) {
+            float* par = (float*)(data + (long long)a.g.bs * D);
+            par[slot] = sc; par[a.g.bs + slot] = zp;
+        }
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            uint32_t q[2] = {0u, 0u};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const uint32_t b = quant_one(x[p][e], inv, zp);
+                if (kv) sh_v[8 * l + 64 * p + e][i + shift] = (uint8_t)b;
+                else q[e >> 2] |= b << (8 * (e & 3));
+            }
+            if (!kv && rec >= 0) *reinterpret_cast<uint2*>(data + (long long)slot * D + 8 * l + 64 * p) = make_uint2(q[0], q[1]);   // key data [bs][D]
+        }
+    }
+    __syncthreads();
+    uint8_t* vc = (uint8_t*)a.value_cache;   // value data [D][bs]
+    for (int w = tid; w < D * kColWords; w += 256) {
+        const int d = w / kColWords, g = w % kColWords;
+        const long long at = sh_word[g];
+        if (at >= 0) {
+            *reinterpret_cast<uint32_t*>(vc + at + (long long)d * a.g.bs) = *reinterpret_cast<const uint32_t*>(&sh_v[d][4 * g]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int j = 4 * g + u - shift;
+                if (j >= 0 && j < kWriteTokens && sh_rec[j] >= 0) vc[sh_rec[j] + (long long)d * a.g.bs + sh_slot[j]] = sh_v[d][4 * g + u];
+            }
+        }
+    }
+}
+
+// One warp per (token, kv head).  Lane l owns dims {l + 32*i}.  With PLAN set, the first block of
 // the grid builds the decode plan instead.
-template <int D, bool PLAN>
+template <int D, bool PLAN, bool GROUPS>
 __global__ void __launch_bounds__(256) write_kv_kernel(KernelArgs a) {
     constexpr int PER = D / 32;
     // No early griddepcontrol.launch_dependents here: decode CTAs placed while blocks of this grid still hold
     // shared memory do not all fit, and the decode kernel's static slices then run in two waves.
+    // The plan blocks come first, so that they run beside the writes of a long chunk and not behind them.
+    int first_block = 0;
     if constexpr (PLAN) {
-        if (blockIdx.x == gridDim.x - 1) {
+        if (blockIdx.x == 0) {
             build_decode_plan(a);
             return;
         }
-        // with a score output the block before the last prepares the score offsets and work list
-        if (a.scores && a.score_aggregation_window && blockIdx.x == gridDim.x - 2) {
-            if (threadIdx.x < 32) build_score_plan(a);
-            return;
+        first_block = 1;
+        if (a.scores && a.score_aggregation_window) {   // with a score output the second block prepares the score offsets and work list
+            if (blockIdx.x == 1) {
+                if (threadIdx.x < 32) build_score_plan(a);
+                return;
+            }
+            first_block = 2;
         }
     }
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if constexpr (GROUPS) {
+        const int i = blockIdx.x - first_block;
+        if (a.g.act == PA_DTYPE_F32) write_group<D, true>(a, i / a.g.Hkv, i % a.g.Hkv);
+        else write_group<D, false>(a, i / a.g.Hkv, i % a.g.Hkv);
+        return;
+    }
+    const int warp = ((blockIdx.x - first_block) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const int total = a.num_tokens * a.g.Hkv;
     if (warp >= total) return;
     const int t = warp / a.g.Hkv, h = warp % a.g.Hkv;
-    const int s = find_sequence(a.subsequence_begins, a.num_sequences, t);
-    SeqView sv;
-    if (!seq_view(a, s, sv)) return;
-    const int t0 = sv.t0, past = sv.past, tb = sv.tb;
-    if (t < t0 || t >= t0 + sv.n) {   // prefix sums that are not monotone, or that leave tokens uncovered
-        if (lane == 0) atomicOr(a.status, PA_DEV_BAD_BEGINS);
-        return;
-    }
-    const int pos = past + (t - t0);
-    const int block = a.block_indices[tb + pos / a.g.bs];
-    if (block < 0 || block >= a.num_blocks) {
-        if (lane == 0) atomicOr(a.status, PA_DEV_BAD_BLOCK_INDEX);
-        return;
-    }
-    const int slot = pos % a.g.bs;
+    long long rec;
+    int slot;
+    if (!locate_token(a, t, lane == 0, rec, slot)) return;
+    rec += (long long)h * a.g.head_bytes;
     const long long src = ((long long)t * a.g.Hkv + h) * D;
-    const long long rec = (long long)block * a.g.block_bytes + (long long)h * a.g.head_bytes;
     float k[PER], v[PER];
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
@@ -371,13 +548,22 @@ __global__ void __launch_bounds__(256) copy_blocks_kernel(uint8_t* key_cache, ui
 cudaError_t launch_write_kv(const KernelArgs& a, cudaStream_t stream, bool with_plan) {
     if (a.num_tokens <= 0 && !with_plan) return cudaSuccess;
     const long long warps = (long long)a.num_tokens * a.g.Hkv;
-    const int grid = (int)((warps * 32 + 255) / 256) + (with_plan ? 1 : 0) + (with_plan && a.scores && a.score_aggregation_window ? 1 : 0);
+    const int plan_blocks = (with_plan ? 1 : 0) + (with_plan && a.scores && a.score_aggregation_window ? 1 : 0);
+    // Chunks go in groups of 32 tokens once there are enough rows to give every SM a few (rows = tokens x kv heads, us; one warp
+    // per row | groups): u8 2048 rows 6.2 | 6.2, 8192 rows 12.4 | 8.2, 65536 rows 55 | 26; bf16 2048 rows 5.2 | 4.0, 65536 rows
+    // 20.5 | 11.8.  Decode rows, each in a block of its own, stay with one warp per row: u8 2048 rows 6.3 | 9.3.
+    // The groups' wider loads need activations on 16-byte boundaries.
+    const bool groups = warps >= kWriteGroupRows && a.num_tokens >= 2LL * a.num_sequences &&
+                        ((reinterpret_cast<uintptr_t>(a.key) | reinterpret_cast<uintptr_t>(a.value)) & 15) == 0;
+    const long long blocks = groups ? (long long)((a.num_tokens + kWriteTokens - 1) / kWriteTokens) * a.g.Hkv : (warps * 32 + 255) / 256;
+    const int grid = (int)blocks + plan_blocks;
+    auto launch = [&](auto kernel) { kernel<<<grid, 256, 0, stream>>>(a); };
     if (a.g.D == 128) {
-        if (with_plan) write_kv_kernel<128, true><<<grid, 256, 0, stream>>>(a);
-        else write_kv_kernel<128, false><<<grid, 256, 0, stream>>>(a);
+        if (with_plan) groups ? launch(write_kv_kernel<128, true, true>) : launch(write_kv_kernel<128, true, false>);
+        else groups ? launch(write_kv_kernel<128, false, true>) : launch(write_kv_kernel<128, false, false>);
     } else {
-        if (with_plan) write_kv_kernel<64, true><<<grid, 256, 0, stream>>>(a);
-        else write_kv_kernel<64, false><<<grid, 256, 0, stream>>>(a);
+        if (with_plan) groups ? launch(write_kv_kernel<64, true, true>) : launch(write_kv_kernel<64, true, false>);
+        else groups ? launch(write_kv_kernel<64, false, true>) : launch(write_kv_kernel<64, false, false>);
     }
     return cudaGetLastError();
 }

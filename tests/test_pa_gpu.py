@@ -79,6 +79,49 @@ def test_prefill_and_mixed_parity(cache, d, bs):
     assert res["prefill_kernel"] == "tcgen05"   # every cache type, both head sizes
 
 
+@pytest.mark.parametrize("cache,act,d,bs", [("u8", torch.bfloat16, 128, 32), ("u8", torch.float32, 128, 16), ("u8", torch.float16, 64, 16),
+                                            ("f16", torch.float16, 128, 32), ("bf16", torch.bfloat16, 64, 32), ("bf16", torch.float32, 128, 16),
+                                            ("f16", torch.bfloat16, 64, 16)])
+def test_chunk_writes_in_token_groups(cache, act, d, bs):
+    """Chunks of more than 2048 (token, kv head) rows are written in groups of 32 tokens: bytes equal to the oracle's where
+    groups straddle sequences, blocks and words, start at any slot, hold decode rows or end short; the same bytes from
+    activations off a 16-byte boundary, which are written row by row; a bad block id in one group leaves the rest alone."""
+    import ctypes as C
+    wl = H.small_workload(hq=6, hkv=2, d=d, bs=bs, act=act, cache=cache, past=[0, 5, 31, 42, 7, 703, 16], new=[701, 33, 1, 67, 2, 301, 1], seed=91)
+    assert wl.num_tokens * 2 >= 2048 and wl.num_tokens % 32 != 0
+    data = H.make_host_data(wl)
+    ref = H.run_oracle(wl, data)
+    got = H.run_gpu(wl, data)
+    assert got["status"] == 0
+    assert np.array_equal(got["kc_gpu"], ref["kc_ref"]) and np.array_equal(got["vc_gpu"], ref["vc_ref"])
+    t = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    def write(offset, table):
+        op = H.make_op(wl)
+        kc, vc = op.allocate_cache(wl.num_blocks, fill=0)
+        def shifted(x):
+            flat = torch.empty(x.numel() + 16, dtype=x.dtype, device="cuda")
+            flat[offset:offset + x.numel()] = x.cuda().view(-1)
+            return flat[offset:offset + x.numel()].view(x.shape)
+        k, v = shifted(data[1]), shifted(data[2])
+        args = op.make_args(k, k, v, k, kc, vc, t(wl.past_lens), t(wl.subsequence_begins), t(table), t(wl.block_indices_begins), wl.scale, wl.max_context_len)
+        op._check(op.lib.pa_b200_write_kv(op._h, C.byref(args)))
+        torch.cuda.synchronize()
+        return kc.cpu().numpy(), vc.cpu().numpy(), op.device_status()
+    whole, odd = write(0, wl.block_indices), write(1, wl.block_indices)
+    assert whole[2] == 0 and odd[2] == 0
+    assert np.array_equal(whole[0], odd[0]) and np.array_equal(whole[1], odd[1])
+    table = wl.block_indices.copy()
+    table[wl.block_indices_begins[5] + 703 // bs + 2] = wl.num_blocks   # a block of the sixth sequence that the chunk writes
+    bad = write(0, table)
+    lost = int(wl.block_indices[wl.block_indices_begins[5] + 703 // bs + 2])
+    assert bad[2] != 0
+    n = H.block_bytes(wl)
+    for got_b, want in ((bad[0], whole[0]), (bad[1], whole[1])):
+        want = want.copy()
+        want[lost * n:(lost + 1) * n] = 0
+        assert np.array_equal(got_b, want)
+
+
 @pytest.mark.parametrize("hq,hkv,bs,past,new", [
     (28, 4, 32, [0, 700, 63, 4000], [256, 256, 130, 64]),     # Qwen2.5-7B group of 7: q tiles straddle tokens
     (32, 8, 16, [1000, 5], [200, 33]),                        # block size 16
