@@ -16,7 +16,7 @@
 //   * a warp that leaves a run adds its partial (m, l, O) to the run's accumulator in shared memory (a ring of kShAcc
 //     accumulators, each behind a lock); the warp whose tiles complete the run takes the result out and either writes the
 //     output (the stream lies in this CTA alone) or publishes the CTA's partial exactly as a worker of decode_kernel does
-//     (slot = stream + CTA), the CTA that completes the stream merging the partials;
+//     (slot = stream + CTA); the CTA that completes the stream merges the partials, a row per warp, when its tiles are done;
 //   * the slices are cut in a sequence in which every stream is followed by a few tiles that do not exist
 //     (KernelArgs::decode_phantom), so that a CTA whose slice holds many streams gets fewer tiles.
 // The order in which partials are added depends on timing, so the last bits of the output differ between launches.
@@ -43,6 +43,7 @@ constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kLazyMax = 8.f;
 constexpr int kFoldEvery = 4;
 constexpr int kShQEntry = 2048 + 64;   // bytes of one staged query entry: 16 registers x 32 lanes in fragment order, then (sum, scale) of 8 rows
+constexpr int kShMerges = 4;   // a slice is contiguous: only its first and its last stream can have tiles in other CTAs
 constexpr int kEndRun = -2;     // descriptor of a stage without a tile: the chapter has no more tiles
 
 struct __align__(16) ShDesc {
@@ -95,6 +96,8 @@ struct ShCtl {
     int more;        // the slice has tiles beyond this chapter
     int cont;        // the chapter's last run goes on in the next chapter
     int bad;         // a block id was out of range
+    int nmerge;      // streams that this CTA's partials completed: merged by all warps at the end
+    int4 merge[kShMerges];   // (first slot, partials, row of the token, kv head)
     // walk
     int r_s, hk, r_tiles, p0, pos, ctx, tb, nb, t0row, g_tile, seq;
 };
@@ -139,60 +142,43 @@ __device__ __forceinline__ void mma_lo(float& c0, float& c1, uint32_t a0, uint32
     (void)t2; (void)t3;
 }
 
-// Reduces `n` partials (m, l, O) of `rt` rows each, laid out [partial][row][D] / [partial][row][2], with a whole
-// warp: lane j owns the columns 4j..4j+3 of every row (D == 128), so a row of a partial is one coalesced 512-byte
-// read, and the per-partial factors 2^(m - max) are computed by lane = partial and handed round by shuffles.
-// `mask` selects partials (bit w, for n <= 32); pass all ones otherwise.  Results: acc[row] (unnormalised), m, l.
+// Reduces row `k` of `n` partials (m, l, O) of `rt` rows each, laid out [partial][row][D] / [partial][row][2], with a whole
+// warp: lane j owns the columns 4j..4j+3 (D == 128), so the row of a partial is one coalesced 512-byte read, eight of
+// them in flight, and the partials' factors 2^(m - max) are computed by lane = partial and handed round by shuffles.
+// Results: the unnormalised row, its m and l.
 template <int D>
-__device__ __forceinline__ void merge_partials(const float* po, const float* pml, int n, unsigned mask, int rt, int lane, float4 (&acc)[8],
-                                               float (&mrow)[8], float (&lrow)[8]) {
+__device__ __forceinline__ void merge_row(const float* po, const float* pml, int n, int rt, int k, int lane, float4& acc, float& m, float& l) {
     static_assert(D == 128, "one float4 per lane and row");
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { acc[k] = make_float4(0.f, 0.f, 0.f, 0.f); mrow[k] = -INFINITY; lrow[k] = 0.f; }
+    acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    m = -INFINITY;
+    l = 0.f;
     for (int c0 = 0; c0 < n; c0 += 32) {
         const int w = c0 + lane;
-        const bool on = w < n && ((mask >> (w & 31)) & 1u);
         const int cnt = min(32, n - c0);
-        float fk[8];   // factor of partial w for each row
+        float2 ml = make_float2(-INFINITY, 0.f);
+        if (w < n) ml = __ldcg(reinterpret_cast<const float2*>(pml + ((long long)w * rt + k) * 2));
+        float mx = ml.x;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            fk[k] = 0.f;
-            if (k < rt) {
-                float2 ml = make_float2(-INFINITY, 0.f);
-                if (on) ml = __ldcg(reinterpret_cast<const float2*>(pml + ((long long)w * rt + k) * 2));
-                float mx = ml.x;
+        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float m_new = fmaxf(m, mx);
+        const float alpha = m == -INFINITY ? 0.f : fast_exp2s(m - m_new);
+        const float f = ml.x != -INFINITY ? fast_exp2s(ml.x - m_new) : 0.f;   // factor of partial w
+        float ls = f * ml.y;
 #pragma unroll
-                for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-                const float m_new = fmaxf(mrow[k], mx);
-                const float alpha = mrow[k] == -INFINITY ? 0.f : fast_exp2s(mrow[k] - m_new);
-                const float f = on && ml.x != -INFINITY ? fast_exp2s(ml.x - m_new) : 0.f;
-                float ls = f * ml.y;
+        for (int o = 16; o; o >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, o);
+        l = l * alpha + ls;
+        acc.x *= alpha; acc.y *= alpha; acc.z *= alpha; acc.w *= alpha;
+        m = m_new;
+        for (int j0 = 0; j0 < cnt; j0 += 8) {
+            float4 v[8];
 #pragma unroll
-                for (int o = 16; o; o >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, o);
-                lrow[k] = lrow[k] * alpha + ls;
-                acc[k].x *= alpha; acc[k].y *= alpha; acc[k].z *= alpha; acc[k].w *= alpha;
-                mrow[k] = m_new;
-                fk[k] = f;
-            }
-        }
-        // O: four partials' rows in flight at a time
-        for (int j0 = 0; j0 < cnt; j0 += 4) {
+            for (int u = 0; u < 8; ++u)
+                v[u] = __ldcg(reinterpret_cast<const float4*>(po + ((long long)(c0 + min(j0 + u, cnt - 1)) * rt + k) * D + 4 * lane));
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (k < rt) {
-                    float4 v[4];
-                    float fw[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int j = j0 + u < cnt ? j0 + u : j0;
-                        fw[u] = j0 + u < cnt ? __shfl_sync(0xffffffffu, fk[k], j) : 0.f;
-                        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (fw[u] != 0.f) v[u] = __ldcg(reinterpret_cast<const float4*>(po + ((long long)(c0 + j) * rt + k) * D + 4 * lane));
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        acc[k].x += fw[u] * v[u].x; acc[k].y += fw[u] * v[u].y; acc[k].z += fw[u] * v[u].z; acc[k].w += fw[u] * v[u].w;
-                    }
+            for (int u = 0; u < 8; ++u) {
+                const float fw = __shfl_sync(0xffffffffu, f, min(j0 + u, 31));
+                if (j0 + u < cnt && fw != 0.f) {
+                    acc.x += fw * v[u].x; acc.y += fw * v[u].y; acc.z += fw * v[u].z; acc.w += fw * v[u].w;
                 }
             }
         }
@@ -259,6 +245,7 @@ __global__ void __launch_bounds__(kShMaxWarps * 32, 1) decode_shared_kernel(Kern
         ctl->abort = 0;
         for (int i = 0; i < kShAcc; ++i) accs[i] = ShAcc{0, i, 0, 0};
         ctl->bad = 0;
+        ctl->nmerge = 0;
         ctl->seq = 0;
         ctl->cont = 0;
         ctl->g_tile = g_tile;
@@ -301,6 +288,15 @@ __global__ void __launch_bounds__(kShMaxWarps * 32, 1) decode_shared_kernel(Kern
 
     const long long part_stride = (long long)RT * D;   // floats of one partial
     uint8_t* cta_q = a.cta_q + (size_t)cta * kShRuns * kShQEntry;
+
+    auto write_row = [&](int t0, int hk, int k, const float4& acc, float m, float l) {
+        const long long row = (long long)t0 * a.g.Hq + hk * RT + k;
+        const float inv = 1.f / l;
+        const long long idx = row * D + 4 * lane;
+        store_pair_s(a.output, idx, a.g.act, acc.x * inv, acc.y * inv);
+        store_pair_s(a.output, idx + 2, a.g.act, acc.z * inv, acc.w * inv);
+        if (lane == 0 && a.lse) a.lse[row] = (m + log2f(l)) * kLn2;
+    };
 
     // Adds this warp's partial of run `seq` to the run's accumulator in shared memory (under the accumulator's lock) and,
     // if that completes the run inside the CTA, publishes (or writes) the result.
@@ -398,22 +394,20 @@ __global__ void __launch_bounds__(kShMaxWarps * 32, 1) decode_shared_kernel(Kern
             int sdone = 0;
             if (lane == 0) sdone = atomicAdd(&a.stream_done[fin.stream], 1) + 1;
             sdone = __shfl_sync(0xffffffffu, sdone, 0);
-            if (sdone != fin.nparts) return;
-            __threadfence();
-            merge_partials<D>(a.part_o + (long long)fin.first_slot * part_stride, a.part_ml + (long long)fin.first_slot * RT * 2, fin.nparts, 0xffffffffu,
-                              RT, lane, acc, mrow, lrow);
+            if (sdone == fin.nparts) {   // the stream is complete: all warps merge it once the CTA has no tiles left
+                __threadfence();
+                if (lane == 0) {
+                    const int i = atomicAdd(&ctl->nmerge, 1);
+                    if (i < kShMerges) ctl->merge[i] = make_int4(fin.first_slot, fin.nparts, fin.t0, fin.hk);
+                }
+            }
+            SPROF(pff += clock64() - pq0;)
+            return;
         }
-        // ---- the stream is complete: normalise and write ------------------------------------------------
+        // ---- the stream lies in this CTA alone: normalise and write ----------------------------------------
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-            if (k < RT) {
-                const long long row = (long long)fin.t0 * a.g.Hq + fin.hk * RT + k;
-                const float inv = 1.f / lrow[k];
-                const long long idx = row * D + 4 * lane;
-                store_pair_s(a.output, idx, a.g.act, acc[k].x * inv, acc[k].y * inv);
-                store_pair_s(a.output, idx + 2, a.g.act, acc[k].z * inv, acc[k].w * inv);
-                if (lane == 0 && a.lse) a.lse[row] = (mrow[k] + log2f(lrow[k])) * kLn2;
-            }
+            if (k < RT) write_row(fin.t0, fin.hk, k, acc[k], mrow[k], lrow[k]);
         SPROF(pff += clock64() - pq0;)
     };
 
@@ -803,6 +797,20 @@ __global__ void __launch_bounds__(kShMaxWarps * 32, 1) decode_shared_kernel(Kern
         ch_started_before = true;
     }
     if (tid == 0 && ctl->bad) atomicOr(a.status, PA_DEV_BAD_BLOCK_INDEX);
+    // ---- merge the streams that this CTA completed, a row per warp --------------------------------------------
+    // (The warp that completed a stream used to do it alone, row behind row, while the others had nothing left to do: one
+    // sequence of 9000 tokens, 37 partials in each of 4 streams, 57 -> 22 us; 64 sequences of 4000 136 -> 131 us.)
+    {
+        const int nm = min(ctl->nmerge, kShMerges);
+        for (int i = warp; i < nm * RT; i += nwarps) {
+            const int4 mg = ctl->merge[i / RT];
+            const int k = i % RT;
+            float4 acc;
+            float m, l;
+            merge_row<D>(a.part_o + (long long)mg.x * part_stride, a.part_ml + (long long)mg.x * RT * 2, mg.y, RT, k, lane, acc, m, l);
+            write_row(mg.z, mg.w, k, acc, m, l);
+        }
+    }
 #ifdef PA_DECODE_PROF
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(pt3));
     const int pwid = cta * nwarps + warp;

@@ -52,6 +52,16 @@ def test_decode_long_context_many_splits(monkeypatch):
     _check(H.run_both(wl), "u8", torch.bfloat16)
 
 
+@pytest.mark.parametrize("cache,d", [("u8", 128), ("f16", 128), ("bf16", 64)])
+@pytest.mark.parametrize("hq,hkv,past", [(1, 1, [20000]), (6, 2, [9001, 37]), (7, 1, [4095]), (32, 4, [4736, 5000, 130]), (12, 1, [6000, 1])])
+def test_decode_streams_cut_into_many_partials(cache, d, hq, hkv, past):
+    """A handful of sequences over the whole chip: every stream is cut into tens of partials (more than a warp's 32 among
+    them), merged row by row by the CTA or warp that publishes the last one."""
+    act = torch.bfloat16 if cache == "bf16" else torch.float16
+    wl = H.small_workload(hq=hq, hkv=hkv, d=d, bs=32, act=act, cache=cache, past=past, new=[1] * len(past), seed=hq + len(past))
+    _check(H.run_both(wl), cache, act)
+
+
 def test_decode_u8_keeps_its_precision_over_a_32k_context():
     """With N(0,1) values the output shrinks like 1/sqrt(context) while the u8 accumulators carry
     1024 + byte per unit of probability: the error must stay at the level of the f16 cache's, far
