@@ -358,10 +358,24 @@ __global__ void __launch_bounds__(256) write_kv_kernel(KernelArgs a) {
     rec += (long long)h * a.g.head_bytes;
     const long long src = ((long long)t * a.g.Hkv + h) * D;
     float k[PER], v[PER];
+    if (a.g.act == PA_DTYPE_F32) {
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        k[i] = load_act(a.key, src + lane + 32 * i, a.g.act);
-        v[i] = load_act(a.value, src + lane + 32 * i, a.g.act);
+        for (int i = 0; i < PER; ++i) {
+            k[i] = ((const float*)a.key)[src + lane + 32 * i];
+            v[i] = ((const float*)a.value)[src + lane + 32 * i];
+        }
+    } else {   // all loads in flight before the first conversion
+        unsigned short kr[PER], vr[PER];
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            kr[i] = ((const unsigned short*)a.key)[src + lane + 32 * i];
+            vr[i] = ((const unsigned short*)a.value)[src + lane + 32 * i];
+        }
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            k[i] = a.g.act == PA_DTYPE_F16 ? __half2float(__ushort_as_half(kr[i])) : __bfloat162float(__ushort_as_bfloat16(kr[i]));
+            v[i] = a.g.act == PA_DTYPE_F16 ? __half2float(__ushort_as_half(vr[i])) : __bfloat162float(__ushort_as_bfloat16(vr[i]));
+        }
     }
     if (a.g.cache == PA_DTYPE_U8) {
         uint8_t* kr = (uint8_t*)a.key_cache + rec;

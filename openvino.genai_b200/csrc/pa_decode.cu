@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, (HI || PA_DECODE_STAGES > 2
     const int HK = a.g.Hkv * gtiles;
     const int RT = a.rows_per_tile;
     const float sm_scale = a.scale != 0.f ? a.scale : rsqrtf((float)D);
+    const bool q_pairs = (reinterpret_cast<uintptr_t>(a.query) & 7) == 0;   // a pair of elements is one aligned load
     bool bad_index = false;
     // everything below reads what the launch before this one wrote (plan, start records, cache)
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -393,14 +394,38 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, (HI || PA_DECODE_STAGES > 2
                 const long long qoff = ((long long)t0 * a.g.Hq + hbase + hrow) * D;
                 float q[D / 4];
                 float amax = 0.f;
+                auto dim = [&](int e) {
+                    if constexpr (U8) return 64 * (e / 16) + 16 * c + (e % 16);
+                    else return 16 * (e / 4) + 2 * c + (e & 1) + 8 * ((e >> 1) & 1);
+                };
+                // The type is looked at once, around all loads, and neighbours come in pairs (e and e + 1 are neighbours for
+                // even e): with the branch around each load a row came one element behind the other, 13 us per run.
 #pragma unroll
-                for (int e = 0; e < D / 4; ++e) {
-                    int dd;
-                    if constexpr (U8) dd = 64 * (e / 16) + 16 * c + (e % 16);
-                    else dd = 16 * (e / 4) + 2 * c + (e & 1) + 8 * ((e >> 1) & 1);
-                    q[e] = live ? load_act(a.query, qoff + dd, a.g.act) : 0.f;
-                    amax = fmaxf(amax, fabsf(q[e]));
+                for (int e = 0; e < D / 4; ++e) q[e] = 0.f;
+                if (live && !q_pairs) {
+#pragma unroll
+                    for (int e = 0; e < D / 4; ++e) q[e] = load_act(a.query, qoff + dim(e), a.g.act);
+                } else if (live && a.g.act == PA_DTYPE_F32) {
+                    const float* src = (const float*)a.query + qoff;
+#pragma unroll
+                    for (int e = 0; e < D / 4; e += 2) {
+                        const float2 v = *reinterpret_cast<const float2*>(src + dim(e));
+                        q[e] = v.x; q[e + 1] = v.y;
+                    }
+                } else if (live) {
+                    const uint16_t* src = (const uint16_t*)a.query + qoff;
+                    uint32_t w[D / 8];
+#pragma unroll
+                    for (int e = 0; e < D / 4; e += 2) w[e / 2] = *reinterpret_cast<const uint32_t*>(src + dim(e));
+#pragma unroll
+                    for (int e = 0; e < D / 4; e += 2) {
+                        const float2 f = a.g.act == PA_DTYPE_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[e / 2]))
+                                                                 : make_float2(__uint_as_float(w[e / 2] << 16), __uint_as_float(w[e / 2] & 0xffff0000u));
+                        q[e] = f.x; q[e + 1] = f.y;
+                    }
                 }
+#pragma unroll
+                for (int e = 0; e < D / 4; ++e) amax = fmaxf(amax, fabsf(q[e]));
                 amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
                 amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
                 float qmul = 1.f;  // exact power-of-two prescale that keeps |q| inside the f16 range
