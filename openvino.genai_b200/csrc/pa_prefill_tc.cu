@@ -383,77 +383,132 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
         uint8_t* const sq = sm.q[X];
         const uint32_t tmem_p = tmem + kTmemP + kPCols * X + lane_base;
         uint32_t n = 0;   // tiles of this half so far, over all items
-        for (uint32_t ik = 0;; ++ik) {
-            Item it;
-            const int item = fetch_item(ik, it);
-            if (item == -2) goto done;
-            if (item < 0) break;
-            if (it.nt[X] == 0) continue;
+        uint32_t ik = 0;
+        Item it;
+        // This thread's row of the item in work; the next item's is staged before this one's epilogue.
+        struct Row {
+            long long off;   // (token, q head) row of query / output
+            int ctx;         // context it sees
+            bool live;
+            float qs;        // softmax scale: the kernel's, divided by the row's prescale
+        } row{0, 0, false, qscale};
+        // The next item with rows in this half: 1, none left: 0, a wait ran out: -1
+        auto next_item = [&]() -> int {
+            for (;;) {
+                const int item = fetch_item(ik, it);
+                if (item == -2) return -1;
+                if (item < 0) return 0;
+                ++ik;
+                if (it.nt[X] != 0) return 1;
+            }
+        };
+        // Q -> swizzled A operand; the row's sum goes into the extra dims.  Every S of this half's previous item has
+        // completed, so the tile is free.  16-bit rows come as sixteen 16-byte loads in flight together (64 registers, free
+        // between items); with a branch on the type around each they came one behind the other, twice.
+        auto stage_q = [&]() {
             const int flat = it.row0 + X * kRows + r;
             const int tok = flat / G, hq = it.hk * G + flat % G;
-            const bool row_live = tok < it.n_new;
-            const int my_ctx = row_live ? it.past + tok + 1 : it.ctx_hi[X];
-            const long long grow_off = ((long long)(it.t0 + (row_live ? tok : 0)) * a.g.Hq + hq);
-
-            // ---- Q -> f16 swizzled A operand; the row's sum goes into the extra dims.  Every S of this
-            // half's previous item has completed, so the tile is free. ------------------------------
-            float qs = qscale;   // the row's softmax scale: the kernel's, divided by the row's prescale
-            {
-                // large queries (bf16 / f32 beyond the f16 range, or f16 rows whose sum would leave it): an exact power-of-two
-                // prescale keeps the packed row and its sum inside the f16 range (the decode kernel does the same), and the
-                // softmax scale of the row takes it back out
-                float qmul = 1.f;
-                if (!BF && row_live) {   // (the bf16 variant runs on bf16 activations only: its rows go in as they are)
+            row.live = tok < it.n_new;
+            row.ctx = row.live ? it.past + tok + 1 : it.ctx_hi[X];
+            row.off = ((long long)(it.t0 + (row.live ? tok : 0)) * a.g.Hq + hq);
+            // large queries (bf16 / f32 beyond the f16 range, or f16 rows whose sum would leave it): an exact power-of-two
+            // prescale keeps the packed row and its sum inside the f16 range (the decode kernel does the same), and the
+            // softmax scale of the row takes it back out
+            float qmul = 1.f, qsum = 0.f;
+            auto prescale = [&](float amax) {
+                if (amax > 256.f && amax < INFINITY) {   // 128 terms of at most 2^8 each keep the row sum below the f16 maximum too
+                    int ex;
+                    frexpf(amax, &ex);
+                    qmul = ldexpf(1.f, 8 - ex);
+                }
+            };
+            auto put = [&](int c, const float (&v)[8]) {
+                uint4 w;
+                w.x = pack_h2(v[0] * qmul, v[1] * qmul); w.y = pack_h2(v[2] * qmul, v[3] * qmul);
+                w.z = pack_h2(v[4] * qmul, v[5] * qmul); w.w = pack_h2(v[6] * qmul, v[7] * qmul);
+                if constexpr (U8) {
+                    const __half2* h = reinterpret_cast<const __half2*>(&w);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) qsum += __low2float(h[e]) + __high2float(h[e]);
+                }
+                *reinterpret_cast<uint4*>(sq + (c / 8) * (kRows * 128) + sw128(r, c % 8)) = w;
+            };
+            if (BF || a.g.act != PA_DTYPE_F32) {
+                uint4 raw[kD / 8];
+                const uint4* src = reinterpret_cast<const uint4*>((const uint16_t*)a.query + row.off * kD);
+#pragma unroll
+                for (int c = 0; c < kD / 8; ++c) raw[c] = row.live ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+                if constexpr (BF) {   // (bf16 activations only: the rows go in as they are)
+#pragma unroll
+                    for (int c = 0; c < kD / 8; ++c) *reinterpret_cast<uint4*>(sq + (c / 8) * (kRows * 128) + sw128(r, c % 8)) = raw[c];
+                } else {
+                    const bool f16 = a.g.act == PA_DTYPE_F16;
+                    auto values = [&](const uint4& q, float (&v)[8]) {
+                        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float2 f = f16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[e]))
+                                                 : make_float2(__uint_as_float(w[e] << 16), __uint_as_float(w[e] & 0xffff0000u));
+                            v[2 * e] = f.x; v[2 * e + 1] = f.y;
+                        }
+                    };
                     float amax = 0.f;
-#pragma unroll 4
+#pragma unroll
                     for (int c = 0; c < kD / 8; ++c) {
                         float v[8];
-                        load_act_vec<8>(a.query, grow_off * kD + 8 * c, a.g.act, v);
+                        values(raw[c], v);
 #pragma unroll
                         for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
                     }
-                    if (amax > 256.f && amax < INFINITY) {   // 128 terms of at most 2^8 each keep the row sum below the f16 maximum too
-                        int ex;
-                        frexpf(amax, &ex);
-                        qmul = ldexpf(1.f, 8 - ex);
+                    prescale(amax);
+#pragma unroll
+                    for (int c = 0; c < kD / 8; ++c) {
+                        float v[8];
+                        values(raw[c], v);
+                        put(c, v);
                     }
                 }
-                qs = qscale / qmul;
-                float qsum = 0.f;
+            } else {
+                float amax = 0.f;
 #pragma unroll 4
                 for (int c = 0; c < kD / 8; ++c) {
                     float v[8];
 #pragma unroll
                     for (int e = 0; e < 8; ++e) v[e] = 0.f;
-                    if (row_live) load_act_vec<8>(a.query, grow_off * kD + 8 * c, a.g.act, v);
+                    if (row.live) load_act_vec<8>(a.query, row.off * kD + 8 * c, a.g.act, v);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] *= qmul;
-                    uint4 w;
-                    if constexpr (BF) {
-                        w.x = pack_bf2(v[0], v[1]); w.y = pack_bf2(v[2], v[3]); w.z = pack_bf2(v[4], v[5]); w.w = pack_bf2(v[6], v[7]);
-                    } else {
-                        w.x = pack_h2(v[0], v[1]); w.y = pack_h2(v[2], v[3]); w.z = pack_h2(v[4], v[5]); w.w = pack_h2(v[6], v[7]);
-                    }
-                    if constexpr (U8) {
-                        const __half2* h = reinterpret_cast<const __half2*>(&w);
+                    for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
+                }
+                prescale(amax);
+#pragma unroll 4
+                for (int c = 0; c < kD / 8; ++c) {
+                    float v[8];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) qsum += __low2float(h[e]) + __high2float(h[e]);
-                    }
-                    *reinterpret_cast<uint4*>(sq + (c / 8) * (kRows * 128) + sw128(r, c % 8)) = w;
+                    for (int e = 0; e < 8; ++e) v[e] = 0.f;
+                    if (row.live) load_act_vec<8>(a.query, row.off * kD + 8 * c, a.g.act, v);
+                    put(c, v);
                 }
-                if constexpr (U8) {
-                    const __half qh = f2h(qsum), ql = f2h(qsum - __half2float(qh));
-                    const __half zero = __ushort_as_half(0);
-                    *reinterpret_cast<uint4*>(sm.qx[X] + plain16(r, 0)) = make_uint4(h2_bits(qh, qh), h2_bits(qh, ql), h2_bits(ql, zero), 0u);
-                    *reinterpret_cast<uint4*>(sm.qx[X] + plain16(r, 1)) = make_uint4(0u, 0u, 0u, 0u);
-                }
-                tc05::fence_proxy_async_smem();
-                warp_arrive(&sm.q_full[X]);
             }
+            row.qs = qscale / qmul;
+            if constexpr (U8) {
+                const __half qh = f2h(qsum), ql = f2h(qsum - __half2float(qh));
+                const __half zero = __ushort_as_half(0);
+                *reinterpret_cast<uint4*>(sm.qx[X] + plain16(r, 0)) = make_uint4(h2_bits(qh, qh), h2_bits(qh, ql), h2_bits(ql, zero), 0u);
+                *reinterpret_cast<uint4*>(sm.qx[X] + plain16(r, 1)) = make_uint4(0u, 0u, 0u, 0u);
+            }
+            tc05::fence_proxy_async_smem();
+            warp_arrive(&sm.q_full[X]);
+        };
+        int have = next_item();
+        if (have < 0) goto done;
+        if (have) stage_q();
+        while (have) {
+            const int nt = it.nt[X], my_ctx = row.ctx;
+            const float qs = row.qs;
 
             float m_run = -INFINITY;   // running maximum of q.k' (before the softmax scale)
             float l_own = 0.f;         // bf16 variant: the row's own sum of probabilities
-            for (int j = 0; j < it.nt[X]; ++j, ++n) {
+            for (int j = 0; j < nt; ++j, ++n) {
                 const int col0 = j * kKv;
                 if (!wait_warp(&sm.s_full[X], n & 1, 0)) goto done;
                 if ((warp & 3) == 0) PA_TRACE(X, 0, n);
@@ -556,6 +611,12 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                 warp_arrive(&sm.p_full[X]);
                 if ((warp & 3) == 0) PA_TRACE(X, 4, n);
             }
+            // ---- the next item's rows, so that its first logits are computed beside this item's last P.V and epilogue (its
+            // first P, which starts a new O, comes after) ---------------------------------------------------
+            const Row cur = row;
+            have = next_item();
+            if (have < 0) goto done;
+            if (have) stage_q();
             // ---- epilogue: out = (O - z) / l; z = the three zero-point columns, l = the all-ones column (u8 cache);
             // the f16 cache has no z and its l is the first column of the 16-column product
             if (!wait_warp(&sm.o_done[X], (n - 1) & 1, 2)) goto done;
@@ -575,17 +636,17 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                     uint32_t t[32];
                     tc05::ld_32x32b_x32(tmem_o + 32 * q4, t);
                     tc05::wait_ld();
-                    if (row_live) {
+                    if (cur.live) {
 #pragma unroll
                         for (int c = 0; c < 32; c += 8) {
                             float v[8];
 #pragma unroll
                             for (int e = 0; e < 8; ++e) v[e] = (__uint_as_float(t[c + e]) - z) * inv;
-                            store_act_vec8(a.output, grow_off * kD + 32 * q4 + c, a.g.act, v);
+                            store_act_vec8(a.output, cur.off * kD + 32 * q4 + c, a.g.act, v);
                         }
                     }
                 }
-                if (row_live && a.lse) a.lse[grow_off] = (m_run * qs + log2f(l_run)) * kLn2P;
+                if (cur.live && a.lse) a.lse[cur.off] = (m_run * cur.qs + log2f(l_run)) * kLn2P;
             }
             tc05::fence_before_thread_sync();
         }
