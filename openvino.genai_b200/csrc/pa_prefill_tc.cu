@@ -57,7 +57,7 @@ constexpr float kLog2eP = 1.4426950408889634f;
 constexpr float kLn2P = 0.6931471805599453f;
 
 constexpr int kSoftmaxWarps = 8, kConvWarps = 4;
-constexpr int kWarpMma = kSoftmaxWarps + kConvWarps, kWarpLoad = kWarpMma + 1;
+constexpr int kWarpMma = kSoftmaxWarps + kConvWarps, kWarpLoad = kWarpMma + 1, kWarpMma2 = kWarpMma + 2;   // the second mma warp: 16-bit caches
 constexpr int kThreads = 512;   // four warpgroups: softmax A, softmax B, converter / copy warps, {mma, loader, two idle warps}
 // Registers per thread after the roles have re-divided the register file among the warpgroups (one warp of each shares a
 // scheduler's 16 K registers: 160 + 160 + 104 + 88 = 512 x 32)
@@ -99,6 +99,7 @@ struct PrefillSmem<BS, PA_DTYPE_U8, D> {
     alignas(128) uint8_t kx[kStages][kKv * kDx * 2];  // unswizzled [64 tokens][16 dims]
     alignas(128) uint8_t raw_k[kStages][NREC * RSTRIDE];
     alignas(128) uint8_t raw_v[kStages][NREC * RSTRIDE];
+    alignas(128) uint8_t out_stage[kSoftmaxWarps][32 * 128];   // 128 bytes of each of a warp's rows on their way to global memory
     alignas(16) uint2 v_tab[kConvWarps][kKv / 2];  // per converter warp: (scale, -1024 * scale) f16 pairs of two tokens
     alignas(8) uint64_t raw_full[kStages];   // loader -> converter (transaction bytes)
     alignas(8) uint64_t raw_free[kStages];   // converter -> loader
@@ -108,6 +109,7 @@ struct PrefillSmem<BS, PA_DTYPE_U8, D> {
     alignas(8) uint64_t v_free[kStages];
     alignas(8) uint64_t q_full[2];           // softmax -> mma, per item
     alignas(8) uint64_t s_full[2];           // mma (commit) -> softmax
+    alignas(8) uint64_t s_read[2];           // softmax -> mma: S is in registers
     alignas(8) uint64_t p_full[2];           // softmax -> mma: P written, O rescaled
     alignas(8) uint64_t o_done[2];           // mma (commit) -> softmax: P.V complete
     alignas(8) uint64_t item_full[kItemSlots];   // loader -> every other warp
@@ -133,6 +135,7 @@ struct PrefillSmem16 {
     alignas(1024) uint8_t q[2][kRows * D * 2];        // per half: D / 64 swizzle atoms of [128 rows][64 dims]
     alignas(1024) uint8_t k[NST][kKv * D * 2];    // D / 64 atoms of [64 tokens][64 dims], K-major
     alignas(1024) uint8_t vt[NST][kKv * D * 2];   // the same image read as an MN-major operand: atoms of 64 dims, 8-token groups 1024 bytes apart
+    alignas(128) uint8_t out_stage[kSoftmaxWarps][32 * 128];
     alignas(128) uint8_t ones[16 * 16 * 2];           // unswizzled K-major [16 rows][16 tokens]: row 0 all ones
     alignas(8) uint64_t k_full[NST];     // copy warps -> mma
     alignas(8) uint64_t v_full[NST];
@@ -140,6 +143,7 @@ struct PrefillSmem16 {
     alignas(8) uint64_t v_free[NST];
     alignas(8) uint64_t q_full[2];
     alignas(8) uint64_t s_full[2];
+    alignas(8) uint64_t s_read[2];
     alignas(8) uint64_t p_full[2];
     alignas(8) uint64_t o_done[2];
     alignas(8) uint64_t item_full[kItemSlots];
@@ -294,20 +298,21 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
             }
             mbar_init(&sm.k_full[i], kConvWarps);
             mbar_init(&sm.v_full[i], kConvWarps);
-            mbar_init(&sm.k_free[i], 1);
-            mbar_init(&sm.v_free[i], 1);
+            mbar_init(&sm.k_free[i], U8 ? 1 : 2);   // one arrival per mma warp
+            mbar_init(&sm.v_free[i], U8 ? 1 : 2);
         }
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             mbar_init(&sm.q_full[x], kRows / 32);
             mbar_init(&sm.s_full[x], 1);
+            mbar_init(&sm.s_read[x], kRows / 32);
             mbar_init(&sm.p_full[x], kRows / 32);
             mbar_init(&sm.o_done[x], 1);
         }
 #pragma unroll
         for (int i = 0; i < kItemSlots; ++i) {
             mbar_init(&sm.item_full[i], 1);
-            mbar_init(&sm.item_free[i], kWarpMma + 1);
+            mbar_init(&sm.item_free[i], kWarpMma + (U8 ? 1 : 2));
         }
         mbar_fence_init();
         sm.abort = 0;
@@ -403,45 +408,63 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
             }
         };
         // Q -> swizzled A operand; the row's sum goes into the extra dims.  Every S of this half's previous item has
-        // completed, so the tile is free.  16-bit rows come as sixteen 16-byte loads in flight together (64 registers, free
-        // between items); with a branch on the type around each they came one behind the other, twice.
+        // completed, so the tile is free.  16-bit rows: kD / 8 lanes take one row in 16-byte chunks, all loads of the warp's 32
+        // rows in flight together (64 registers, free between items; cp.async where the row goes in as it is).  One thread per
+        // row touched 32 lines with every load and, behind a branch on the type, had one load in flight: 10 k cycles an item.
         auto stage_q = [&]() {
+            constexpr int CH = kD / 8, RP = 32 / CH;   // chunks of a row, rows per pass; CH passes
             const int flat = it.row0 + X * kRows + r;
             const int tok = flat / G, hq = it.hk * G + flat % G;
             row.live = tok < it.n_new;
             row.ctx = row.live ? it.past + tok + 1 : it.ctx_hi[X];
             row.off = ((long long)(it.t0 + (row.live ? tok : 0)) * a.g.Hq + hq);
-            // large queries (bf16 / f32 beyond the f16 range, or f16 rows whose sum would leave it): an exact power-of-two
-            // prescale keeps the packed row and its sum inside the f16 range (the decode kernel does the same), and the
-            // softmax scale of the row takes it back out
-            float qmul = 1.f, qsum = 0.f;
-            auto prescale = [&](float amax) {
-                if (amax > 256.f && amax < INFINITY) {   // 128 terms of at most 2^8 each keep the row sum below the f16 maximum too
-                    int ex;
-                    frexpf(amax, &ex);
-                    qmul = ldexpf(1.f, 8 - ex);
+            row.qs = qscale;
+            const int wrow = r & ~31;                                  // the warp's first row
+            const int own = row.live ? (int)row.off : -1;              // (rows fit 31 bits: 2^31 of them exceed the memory)
+            const int ch = lane % CH, sub = lane / CH;
+            uint8_t* const dst = sq + (ch / 8) * (kRows * 128);
+            const uint4* const src = reinterpret_cast<const uint4*>(a.query) + ch;   // 16-bit rows of CH chunks
+            if constexpr (BF) {   // bf16 activations only: the rows go in as they are
+#pragma unroll
+                for (int i = 0; i < CH; ++i) {
+                    const int rr = RP * i + sub, o = __shfl_sync(0xffffffffu, own, rr);
+                    cp_async16_zfill(dst + sw128(wrow + rr, ch & 7), src + (long long)max(o, 0) * CH, o >= 0 ? 16u : 0u);
                 }
-            };
-            auto put = [&](int c, const float (&v)[8]) {
-                uint4 w;
-                w.x = pack_h2(v[0] * qmul, v[1] * qmul); w.y = pack_h2(v[2] * qmul, v[3] * qmul);
-                w.z = pack_h2(v[4] * qmul, v[5] * qmul); w.w = pack_h2(v[6] * qmul, v[7] * qmul);
-                if constexpr (U8) {
+                cp_async_commit();
+                cp_async_wait<0>();
+            } else {
+                // large queries (bf16 / f32 beyond the f16 range, or f16 rows whose sum would leave it): an exact power-of-two
+                // prescale keeps the packed row and its sum inside the f16 range (the decode kernel does the same), and the
+                // softmax scale of the row takes it back out
+                auto prescale = [](float amax) {
+                    float mul = 1.f;
+                    if (amax > 256.f && amax < INFINITY) {   // 128 terms of at most 2^8 each keep the row sum below the f16 maximum too
+                        int ex;
+                        frexpf(amax, &ex);
+                        mul = ldexpf(1.f, 8 - ex);
+                    }
+                    return mul;
+                };
+                auto sum8 = [](const uint4& w) {   // of the f16 values the tensor core will see
                     const __half2* h = reinterpret_cast<const __half2*>(&w);
+                    float s4[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) qsum += __low2float(h[e]) + __high2float(h[e]);
-                }
-                *reinterpret_cast<uint4*>(sq + (c / 8) * (kRows * 128) + sw128(r, c % 8)) = w;
-            };
-            if (BF || a.g.act != PA_DTYPE_F32) {
-                uint4 raw[kD / 8];
-                const uint4* src = reinterpret_cast<const uint4*>((const uint16_t*)a.query + row.off * kD);
+                    for (int e = 0; e < 4; ++e) s4[e] = __low2float(h[e]) + __high2float(h[e]);
+                    return (s4[0] + s4[1]) + (s4[2] + s4[3]);
+                };
+                auto pack8 = [](const float (&v)[8], float mul) {
+                    return make_uint4(pack_h2(v[0] * mul, v[1] * mul), pack_h2(v[2] * mul, v[3] * mul), pack_h2(v[4] * mul, v[5] * mul),
+                                      pack_h2(v[6] * mul, v[7] * mul));
+                };
+                float qsum = 0.f;
+                int sum_row = r;   // the row whose sum this thread ends up with
+                if (a.g.act != PA_DTYPE_F32) {
+                    uint4 raw[CH];
 #pragma unroll
-                for (int c = 0; c < kD / 8; ++c) raw[c] = row.live ? src[c] : make_uint4(0u, 0u, 0u, 0u);
-                if constexpr (BF) {   // (bf16 activations only: the rows go in as they are)
-#pragma unroll
-                    for (int c = 0; c < kD / 8; ++c) *reinterpret_cast<uint4*>(sq + (c / 8) * (kRows * 128) + sw128(r, c % 8)) = raw[c];
-                } else {
+                    for (int i = 0; i < CH; ++i) {
+                        const int o = __shfl_sync(0xffffffffu, own, RP * i + sub);
+                        raw[i] = o >= 0 ? src[(long long)o * CH] : make_uint4(0u, 0u, 0u, 0u);
+                    }
                     const bool f16 = a.g.act == PA_DTYPE_F16;
                     auto values = [&](const uint4& q, float (&v)[8]) {
                         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
@@ -452,49 +475,90 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                             v[2 * e] = f.x; v[2 * e + 1] = f.y;
                         }
                     };
-                    float amax = 0.f;
+                    // largest magnitude by bit pattern: both types order like their bits without the sign (NaN above all)
+                    const uint32_t limit = f16 ? 0x5C00u : 0x4380u;   // 256
+                    uint32_t top = 0u;
 #pragma unroll
-                    for (int c = 0; c < kD / 8; ++c) {
+                    for (int i = 0; i < CH; ++i)
+                        top = __vmaxu2(top, __vmaxu2(__vmaxu2(raw[i].x & 0x7fff7fffu, raw[i].y & 0x7fff7fffu),
+                                                     __vmaxu2(raw[i].z & 0x7fff7fffu, raw[i].w & 0x7fff7fffu)));
+                    const bool large = __any_sync(0xffffffffu, max(top & 0xffffu, top >> 16) > limit);
+                    float sum[CH];
+                    if (!large) {   // the usual case, straight through: nothing to scale
+#pragma unroll
+                        for (int i = 0; i < CH; ++i) {
+                            uint4 w = raw[i];
+                            if (!f16) {
+                                float v[8];
+                                values(raw[i], v);
+                                w = pack8(v, 1.f);
+                            }
+                            *reinterpret_cast<uint4*>(dst + sw128(wrow + RP * i + sub, ch & 7)) = w;
+                            if constexpr (U8) sum[i] = sum8(w);
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < CH; ++i) {
+                            float v[8];
+                            values(raw[i], v);
+                            float m = 0.f;
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) m = fmaxf(m, fabsf(v[e]));
+#pragma unroll
+                            for (int o = CH / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+                            const float mul = prescale(m);
+                            const float mine = __shfl_sync(0xffffffffu, mul, (lane % RP) * CH);   // row RP i + lane % RP
+                            if (lane / RP == i) row.qs = qscale / mine;
+                            const uint4 w = pack8(v, mul);
+                            *reinterpret_cast<uint4*>(dst + sw128(wrow + RP * i + sub, ch & 7)) = w;
+                            if constexpr (U8) sum[i] = sum8(w);
+                        }
+                    }
+                    if constexpr (U8) {
+                        // sums over the CH lanes of every row at once: each step halves the rows a lane carries, and lane
+                        // (sub, ch) is left with row RP ch + sub
+#pragma unroll
+                        for (int o = CH / 2; o > 0; o >>= 1) {
+                            const bool hi = (ch & o) != 0;
+#pragma unroll
+                            for (int k = 0; k < o; ++k) {
+                                const float give = hi ? sum[k] : sum[k + o], keep = hi ? sum[k + o] : sum[k];
+                                sum[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                            }
+                        }
+                        qsum = sum[0];
+                        sum_row = wrow + RP * ch + sub;
+                    }
+                } else {
+                    float amax = 0.f;
+#pragma unroll 4
+                    for (int c = 0; c < CH; ++c) {
                         float v[8];
-                        values(raw[c], v);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+                        if (row.live) load_act_vec<8>(a.query, row.off * kD + 8 * c, a.g.act, v);
 #pragma unroll
                         for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
                     }
-                    prescale(amax);
-#pragma unroll
-                    for (int c = 0; c < kD / 8; ++c) {
+                    const float mul = prescale(amax);
+                    row.qs = qscale / mul;
+#pragma unroll 4
+                    for (int c = 0; c < CH; ++c) {
                         float v[8];
-                        values(raw[c], v);
-                        put(c, v);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+                        if (row.live) load_act_vec<8>(a.query, row.off * kD + 8 * c, a.g.act, v);
+                        const uint4 w = pack8(v, mul);
+                        *reinterpret_cast<uint4*>(sq + (c / 8) * (kRows * 128) + sw128(r, c % 8)) = w;
+                        if constexpr (U8) qsum += sum8(w);
                     }
                 }
-            } else {
-                float amax = 0.f;
-#pragma unroll 4
-                for (int c = 0; c < kD / 8; ++c) {
-                    float v[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = 0.f;
-                    if (row.live) load_act_vec<8>(a.query, row.off * kD + 8 * c, a.g.act, v);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
+                if constexpr (U8) {
+                    const __half qh = f2h(qsum), ql = f2h(qsum - __half2float(qh));
+                    const __half zero = __ushort_as_half(0);
+                    *reinterpret_cast<uint4*>(sm.qx[X] + plain16(sum_row, 0)) = make_uint4(h2_bits(qh, qh), h2_bits(qh, ql), h2_bits(ql, zero), 0u);
+                    *reinterpret_cast<uint4*>(sm.qx[X] + plain16(sum_row, 1)) = make_uint4(0u, 0u, 0u, 0u);
                 }
-                prescale(amax);
-#pragma unroll 4
-                for (int c = 0; c < kD / 8; ++c) {
-                    float v[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = 0.f;
-                    if (row.live) load_act_vec<8>(a.query, row.off * kD + 8 * c, a.g.act, v);
-                    put(c, v);
-                }
-            }
-            row.qs = qscale / qmul;
-            if constexpr (U8) {
-                const __half qh = f2h(qsum), ql = f2h(qsum - __half2float(qh));
-                const __half zero = __ushort_as_half(0);
-                *reinterpret_cast<uint4*>(sm.qx[X] + plain16(r, 0)) = make_uint4(h2_bits(qh, qh), h2_bits(qh, ql), h2_bits(ql, zero), 0u);
-                *reinterpret_cast<uint4*>(sm.qx[X] + plain16(r, 1)) = make_uint4(0u, 0u, 0u, 0u);
             }
             tc05::fence_proxy_async_smem();
             warp_arrive(&sm.q_full[X]);
@@ -521,6 +585,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                     tc05::wait_ld();
 #pragma unroll
                     for (int c = 0; c < 32; ++c) { sv[c] = __uint_as_float(s0[c]); sv[32 + c] = __uint_as_float(s1[c]); }
+                }
+                if constexpr (!U8) {
+                    tc05::fence_before_thread_sync();
+                    warp_arrive(&sm.s_read[X]);
                 }
                 if ((warp & 3) == 0) PA_TRACE(X, 1, n);
 #ifdef PA_EXP_NOSOFTMAX
@@ -631,19 +699,58 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                     l_run = __uint_as_float(zr[U8 ? 3 : 0]);
                 }
                 const float inv = 1.f / l_run;
+                // 128 bytes of every row at a time, turned around in shared memory so that eight lanes store one row's piece (a
+                // thread storing its own row touched 32 lines with every store: 7 k cycles an item)
+                uint8_t* const stg = sm.out_stage[warp];
+                const int own = cur.live ? (int)cur.off : -1;
+                const int c8 = lane & 7;
+                auto put = [&](int c, const uint4& w) { *reinterpret_cast<uint4*>(stg + lane * 128 + ((c ^ (lane & 7)) << 4)) = w; };
+                auto send = [&](int piece, int row_bytes) {   // the piece of every row of the warp
+                    __syncwarp();
 #pragma unroll
-                for (int q4 = 0; q4 < kD / 32; ++q4) {
-                    uint32_t t[32];
-                    tc05::ld_32x32b_x32(tmem_o + 32 * q4, t);
-                    tc05::wait_ld();
-                    if (cur.live) {
+                    for (int i = 0; i < 8; ++i) {
+                        const int rr = 4 * i + (lane >> 3), o = __shfl_sync(0xffffffffu, own, rr);
+                        const uint4 w = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((c8 ^ (rr & 7)) << 4));
+                        if (o >= 0) *reinterpret_cast<uint4*>((uint8_t*)a.output + (long long)o * row_bytes + 128 * piece + 16 * c8) = w;
+                    }
+                    __syncwarp();
+                };
+                if (a.g.act == PA_DTYPE_F32) {
 #pragma unroll
-                        for (int c = 0; c < 32; c += 8) {
-                            float v[8];
+                    for (int q4 = 0; q4 < kD / 32; ++q4) {
+                        uint32_t t[32];
+                        tc05::ld_32x32b_x32(tmem_o + 32 * q4, t);
+                        tc05::wait_ld();
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) v[e] = (__uint_as_float(t[c + e]) - z) * inv;
-                            store_act_vec8(a.output, cur.off * kD + 32 * q4 + c, a.g.act, v);
+                        for (int c = 0; c < 8; ++c) {
+                            uint32_t w[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) w[e] = __float_as_uint((__uint_as_float(t[4 * c + e]) - z) * inv);
+                            put(c, make_uint4(w[0], w[1], w[2], w[3]));
                         }
+                        send(q4, kD * 4);
+                    }
+                } else {
+                    const bool f16 = a.g.act == PA_DTYPE_F16;
+#pragma unroll
+                    for (int q = 0; q < kD / 64; ++q) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t t[32];
+                            tc05::ld_32x32b_x32(tmem_o + 64 * q + 32 * h, t);
+                            tc05::wait_ld();
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) {
+                                uint32_t w[4];
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    const float v0 = (__uint_as_float(t[8 * c + 2 * e]) - z) * inv, v1 = (__uint_as_float(t[8 * c + 2 * e + 1]) - z) * inv;
+                                    w[e] = f16 ? pack_h2(v0, v1) : pack_bf2(v0, v1);
+                                }
+                                put(4 * h + c, make_uint4(w[0], w[1], w[2], w[3]));
+                            }
+                        }
+                        send(q, kD * 2);
                     }
                 }
                 if (cur.live && a.lse) a.lse[cur.off] = (m_run * cur.qs + log2f(l_run)) * kLn2P;
@@ -840,8 +947,13 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
             }
             if (__any_sync(0xffffffffu, bad_index) && lane == 0) atomicOr(a.status, PA_DEV_BAD_BLOCK_INDEX);
         }
-    } else if (warp == kWarpMma) {
+    } else if (warp == kWarpMma || (!U8 && warp == kWarpMma2)) {
         // ======================= mma issue ================================================================
+        // u8 cache: one warp serves both halves in turn, S of tile j + 1 of a half behind P of its tile j.  16-bit caches: one warp
+        // per half, so that neither half's waits hold up the other's instructions, and S of tile j + 1 is issued as soon as
+        // the softmax warps hold S of tile j in registers; nine ragged bf16 prompts 214 -> 202 us.  Over the u8 cache that was
+        // slower (716 -> 765 us on 16 x 512; two warps with the later S 771): both halves then wait for the converter's
+        // tile together and their exponentials, which took turns on the special function unit, meet there.
         // The whole warp runs the loop (uniform control flow keeps the descriptors in uniform registers);
         // one elected lane issues the tensor-core instructions.
         {
@@ -920,57 +1032,99 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                 }
                 __syncwarp();
             };
-            uint32_t t = 0, n[2] = {0, 0}, iq[2] = {0, 0};
-            for (uint32_t ik = 0;; ++ik) {
-                Item it;
-                const int item = fetch_item(ik, it);
-                if (item == -2) goto done;
-                if (item < 0) break;
-                // first S of the item.  The S region of a half is free: its softmax published the last P of
-                // the previous item (waited below) after reading that tile's S.
-#pragma unroll
-                for (int X = 0; X < 2; ++X)
-                    if (it.nt[X] > 0) {
-                        if (!wait_warp(&sm.q_full[X], iq[X] & 1, 0)) goto done;
-                        ++iq[X];
-                    }
-                if (!wait_warp(&sm.k_full[t % NST], (t / NST) & 1, 1)) goto done;
-                tc05::fence_after_thread_sync();
-#pragma unroll
-                for (int X = 0; X < 2; ++X)
-                    if (it.nt[X] > 0) issue_s(X, t % NST);
-                if (tc05::elect_one()) tc05::commit(&sm.k_free[t % NST]);
-                for (int j = 0; j < it.ntiles; ++j, ++t) {
-                    const int st = t % NST, st1 = (t + 1) % NST;
-                    const bool more = j + 1 < it.ntiles;
-                    PA_TRACE(3, 0, t);
-                    // The converter finishes V' of tile j before K' of tile j + 1, so the latter's barrier
-                    // covers both; only the item's last tile waits for its V' directly.
-                    if (more) {
-                        if (!wait_warp(&sm.k_full[st1], ((t + 1) / NST) & 1, 1)) goto done;
-                    } else {
-                        if (!wait_warp(&sm.v_full[st], (t / NST) & 1, 3)) goto done;
-                    }
-                    PA_TRACE(3, 3, t);
+            uint32_t t = 0;   // tiles so far, over all items
+            if constexpr (U8) {
+                uint32_t n[2] = {0, 0}, iq[2] = {0, 0};
+                for (uint32_t ik = 0;; ++ik) {
+                    Item it;
+                    const int item = fetch_item(ik, it);
+                    if (item == -2) goto done;
+                    if (item < 0) break;
+                    // first S of the item.  The S region of a half is free: its softmax published the last P of
+                    // the previous item (waited below) after reading that tile's S.
+                    if (!wait_warp(&sm.k_full[t % NST], (t / NST) & 1, 1)) goto done;
 #pragma unroll
                     for (int X = 0; X < 2; ++X)
-                        if (j < it.nt[X]) {
-                            // P of tile j is in TMEM, so S of tile j has been read: both MMAs may go
-                            if (!wait_warp(&sm.p_full[X], (n[X] + j) & 1, 4)) goto done;
-                            PA_TRACE(3, 4 + 2 * X, t);
+                        if (it.nt[X] > 0) {
+                            if (!wait_warp(&sm.q_full[X], iq[X] & 1, 0)) goto done;
+                            ++iq[X];
                             tc05::fence_after_thread_sync();
-                            // the next logits first: the half's softmax warps wait for them, nobody waits for this P.V yet
-                            if (j + 1 < it.nt[X]) issue_s(X, st1);
-                            issue_pv(X, st, j > 0);
-                            PA_TRACE(3, 5 + 2 * X, t);
+                            issue_s(X, t % NST);
                         }
-                    if (tc05::elect_one()) {
-                        if (more) tc05::commit(&sm.k_free[st1]);
-                        tc05::commit(&sm.v_free[st]);
+                    if (tc05::elect_one()) tc05::commit(&sm.k_free[t % NST]);
+                    for (int j = 0; j < it.ntiles; ++j, ++t) {
+                        const int st = t % NST, st1 = (t + 1) % NST;
+                        const bool more = j + 1 < it.ntiles;
+                        // The converter finishes V' of tile j before K' of tile j + 1, so the latter's barrier
+                        // covers both; only the item's last tile waits for its V' directly.
+                        if (more) {
+                            if (!wait_warp(&sm.k_full[st1], ((t + 1) / NST) & 1, 1)) goto done;
+                        } else {
+                            if (!wait_warp(&sm.v_full[st], (t / NST) & 1, 3)) goto done;
+                        }
+#pragma unroll
+                        for (int X = 0; X < 2; ++X)
+                            if (j < it.nt[X]) {
+                                // P of tile j is in TMEM, so S of tile j has been read: both MMAs may go
+                                if (!wait_warp(&sm.p_full[X], (n[X] + j) & 1, 4)) goto done;
+                                tc05::fence_after_thread_sync();
+                                // the next logits first: the half's softmax warps wait for them, nobody waits for this P.V yet
+                                if (j + 1 < it.nt[X]) issue_s(X, st1);
+                                issue_pv(X, st, j > 0);
+                            }
+                        if (tc05::elect_one()) {
+                            if (more) tc05::commit(&sm.k_free[st1]);
+                            tc05::commit(&sm.v_free[st]);
+                        }
                     }
+                    n[0] += it.nt[0];
+                    n[1] += it.nt[1];
                 }
-                n[0] += it.nt[0];
-                n[1] += it.nt[1];
+            } else {
+                const int X = warp == kWarpMma ? 0 : 1;
+                uint32_t n = 0, iq = 0;   // tiles and items of this half
+                for (uint32_t ik = 0;; ++ik) {
+                    Item it;
+                    const int item = fetch_item(ik, it);
+                    if (item == -2) goto done;
+                    if (item < 0) break;
+                    const int nt = it.nt[X];
+                    // first S of the item.  The S region is free: the half's softmax staged these rows after it had read the last S.
+                    if (nt > 0) {
+                        if (!wait_warp(&sm.q_full[X], iq & 1, 0)) goto done;
+                        ++iq;
+                    }
+                    for (int j = -1; j < it.ntiles; ++j) {
+                        if (j + 1 < it.ntiles) {
+                            const int st1 = (t + j + 1) % NST;
+                            if (!wait_warp(&sm.k_full[st1], ((t + j + 1) / NST) & 1, 1)) goto done;
+                            if (j + 1 < nt) {
+                                if (j >= 0 && !wait_warp(&sm.s_read[X], (n + j) & 1, 2)) goto done;
+                                tc05::fence_after_thread_sync();
+                                issue_s(X, st1);
+                                if (tc05::elect_one()) tc05::commit(&sm.k_free[st1]);
+                                __syncwarp();
+                            } else {
+                                warp_arrive(&sm.k_free[st1]);   // this half has no use for the tile
+                            }
+                        }
+                        if (j >= 0) {
+                            const int st = (t + j) % NST;
+                            if (!wait_warp(&sm.v_full[st], ((t + j) / NST) & 1, 3)) goto done;
+                            if (j < nt) {
+                                if (!wait_warp(&sm.p_full[X], (n + j) & 1, 4)) goto done;
+                                tc05::fence_after_thread_sync();
+                                issue_pv(X, st, j > 0);
+                                if (tc05::elect_one()) tc05::commit(&sm.v_free[st]);
+                                __syncwarp();
+                            } else {
+                                warp_arrive(&sm.v_free[st]);
+                            }
+                        }
+                    }
+                    t += it.ntiles;
+                    n += nt;
+                }
             }
             // every commit has landed before the CTA's shared memory is given up
             if (t > 0) wait_warp(&sm.v_free[(t - 1) % NST], ((t - 1) / NST) & 1, 0);
