@@ -291,14 +291,13 @@ __device__ __forceinline__ void write_group(const KernelArgs& a, int group, int 
         }
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-            uint32_t q[2] = {0u, 0u};
+            if (kv) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const uint32_t b = quant_one(x[p][e], inv, zp);
-                if (kv) sh_v[8 * l + 64 * p + e][i + shift] = (uint8_t)b;
-                else q[e >> 2] |= b << (8 * (e & 3));
+                for (int e = 0; e < 8; ++e) sh_v[8 * l + 64 * p + e][i + shift] = (uint8_t)quant_one(x[p][e], inv, zp);
+            } else if (rec >= 0) {   // key data [bs][D]
+                *reinterpret_cast<uint2*>(data + (long long)slot * D + 8 * l + 64 * p) =
+                    make_uint2(quant_four(x[p][0], x[p][1], x[p][2], x[p][3], inv, zp), quant_four(x[p][4], x[p][5], x[p][6], x[p][7], inv, zp));
             }
-            if (!kv && rec >= 0) *reinterpret_cast<uint2*>(data + (long long)slot * D + 8 * l + 64 * p) = make_uint2(q[0], q[1]);   // key data [bs][D]
         }
     }
     __syncthreads();
@@ -423,20 +422,68 @@ __global__ void __launch_bounds__(256) write_kv_kernel(KernelArgs a) {
 // j in EL*l .. EL*l + EL-1.  k'[j] = fma(-k[j+D/2], s, k[j]*c);  k'[j+D/2] = fma(k[j], s, k[j+D/2]*c)
 // with c = lut[row][j], s = lut[row][D/2 + j].  EL = 8: the three divisions of a token's new scale and
 // zero-point (every lane of the token computes them) are spread over sixteen elements per lane.
-template <int D>
-__global__ void __launch_bounds__(256) rotate_kernel(KernelArgs a) {
+// One CTA per rotated block, 256 / LPT of its (kv head, token) units at a time; a pass's loads are issued before the pass
+// before it is worked on.  Bound by instruction issue (76 % of the slots, 350 instructions per warp and pass): 6200 blocks of
+// 4 heads x 32 tokens (u8) 115 us, 95 without conversion instructions (quant_bits), 78 with the loads ahead, shifts for the
+// divisions by the block size and three-way minima; the keys' bytes, once in and once out, take 33.
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float y;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float y;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
+template <bool U8>
+struct RotateRaw {   // a lane's EL elements of both halves, as they lie in memory
+    uint2 l, h;
+    float sc, zp;
+};
+template <>
+struct RotateRaw<false> {
+    uint4 l, h;
+};
+template <int D, bool U8>
+__global__ void __launch_bounds__(256, 4) rotate_kernel(KernelArgs a) {
     constexpr int HALF = D / 2;
     constexpr int EL = 8;                  // pairs per lane: an 8-byte (u8) or 16-byte (f16 / bf16) vector per half
     constexpr int LPT = HALF / EL;         // lanes per token: 8 (D = 128) or 4 (D = 64)
-    // One CTA per rotated block; its sub-warps walk the block's (kv head, token) units.
+    constexpr int UPP = 256 / LPT;         // units per pass
     const int l = threadIdx.x % LPT;
     const int r = blockIdx.x;
     const int units = a.g.Hkv * a.g.bs;
     const int block = a.rotated_block_indices[r];
     const int row = a.rotation_deltas[r];
-    const bool bad = block < 0 || block >= a.num_blocks || row < 0 || row >= a.rotation_lut_rows;
-    if (bad && threadIdx.x == 0) atomicOr(a.status, PA_DEV_BAD_ROTATION);
-    const float* lut = a.rotation_trig_lut + (long long)(bad ? 0 : row) * D;
+    if (block < 0 || block >= a.num_blocks || row < 0 || row >= a.rotation_lut_rows) {   // the same for the whole CTA
+        if (threadIdx.x == 0) atomicOr(a.status, PA_DEV_BAD_ROTATION);
+        return;
+    }
+    uint8_t* const base = (uint8_t*)a.key_cache + (long long)block * a.g.block_bytes;
+    const int bs_log2 = 31 - __clz(a.g.bs);   // 16 or 32 tokens
+    auto record = [&](int unit, int& tok) {
+        tok = unit & (a.g.bs - 1);
+        return base + (unsigned)(unit >> bs_log2) * (unsigned)a.g.head_bytes;   // (inside one block: 32 bits)
+    };
+    auto load = [&](int unit) {
+        RotateRaw<U8> x;
+        int tok;
+        const uint8_t* rec = record(min(unit, units - 1), tok);
+        if constexpr (U8) {
+            const float* params = (const float*)(rec + (long long)a.g.bs * D);
+            x.sc = params[tok]; x.zp = params[a.g.bs + tok];
+            x.l = *reinterpret_cast<const uint2*>(rec + (long long)tok * D + EL * l);
+            x.h = *reinterpret_cast<const uint2*>(rec + (long long)tok * D + HALF + EL * l);
+        } else {
+            const uint16_t* p = (const uint16_t*)rec + (long long)tok * D;
+            x.l = *reinterpret_cast<const uint4*>(p + EL * l);
+            x.h = *reinterpret_cast<const uint4*>(p + HALF + EL * l);
+        }
+        return x;
+    };
+    RotateRaw<U8> next = load(threadIdx.x / LPT);
+    const float* lut = a.rotation_trig_lut + (long long)row * D;
     float cv[EL], sv[EL];
 #pragma unroll
     for (int i = 0; i < EL; i += 4) {
@@ -444,96 +491,76 @@ __global__ void __launch_bounds__(256) rotate_kernel(KernelArgs a) {
         cv[i] = c4.x; cv[i + 1] = c4.y; cv[i + 2] = c4.z; cv[i + 3] = c4.w;
         sv[i] = s4.x; sv[i + 1] = s4.y; sv[i + 2] = s4.z; sv[i + 3] = s4.w;
     }
-    for (int base = 0; base < units; base += blockDim.x / LPT) {   // warp-uniform trip count
-    const int unit = base + threadIdx.x / LPT;
-    const bool live = unit < units;
-    const int uu = live ? unit : units - 1;
-    const int tok = uu % a.g.bs, h = uu / a.g.bs;
-    const bool work = live && !bad;
-    uint8_t* rec = (uint8_t*)a.key_cache + (long long)(bad ? 0 : block) * a.g.block_bytes + (long long)h * a.g.head_bytes;
-    float* params = (float*)(rec + (long long)a.g.bs * D);
-    float lo[EL], hi[EL];
-#pragma unroll
-    for (int i = 0; i < EL; ++i) { lo[i] = 0.f; hi[i] = 0.f; }
-    if (work) {
-        if (a.g.cache == PA_DTYPE_U8) {
-            const float sc = params[tok], zp = params[a.g.bs + tok];
-            const uint2 wl = *reinterpret_cast<const uint2*>(rec + (long long)tok * D + EL * l);
-            const uint2 wh = *reinterpret_cast<const uint2*>(rec + (long long)tok * D + HALF + EL * l);
-            const uint32_t wlv[2] = {wl.x, wl.y}, whv[2] = {wh.x, wh.y};
+    for (int unit = threadIdx.x / LPT; unit - (int)(threadIdx.x / LPT) < units; unit += UPP) {   // the same number of passes for every thread
+        const RotateRaw<U8> x = next;
+        if (unit - (int)(threadIdx.x / LPT) + UPP < units) next = load(unit + UPP);
+        const bool live = unit < units;
+        int tok;
+        uint8_t* rec = record(min(unit, units - 1), tok);
+        float lo[EL], hi[EL], nlo[EL], nhi[EL];
+        if constexpr (U8) {
+            const uint32_t wl[2] = {x.l.x, x.l.y}, wh[2] = {x.h.x, x.h.y};
 #pragma unroll
             for (int i = 0; i < EL; ++i) {
-                lo[i] = dequant_one((wlv[i >> 2] >> (8 * (i & 3))) & 0xffu, sc, zp);
-                hi[i] = dequant_one((whv[i >> 2] >> (8 * (i & 3))) & 0xffu, sc, zp);
+                lo[i] = dequant_byte(wl[i >> 2], i & 3, x.sc, x.zp);
+                hi[i] = dequant_byte(wh[i >> 2], i & 3, x.sc, x.zp);
             }
         } else {
-            const uint16_t* p = (const uint16_t*)rec + (long long)tok * D;
-            const uint4 wl = *reinterpret_cast<const uint4*>(p + EL * l), wh = *reinterpret_cast<const uint4*>(p + HALF + EL * l);
-            const uint32_t wlv[4] = {wl.x, wl.y, wl.z, wl.w}, whv[4] = {wh.x, wh.y, wh.z, wh.w};
+            const uint32_t wl[4] = {x.l.x, x.l.y, x.l.z, x.l.w}, wh[4] = {x.h.x, x.h.y, x.h.z, x.h.w};
 #pragma unroll
             for (int i = 0; i < EL; ++i) {
-                const unsigned short el = (unsigned short)(wlv[i >> 1] >> (16 * (i & 1))), eh = (unsigned short)(whv[i >> 1] >> (16 * (i & 1)));
-                if (a.g.cache == PA_DTYPE_F16) {
-                    lo[i] = __half2float(__ushort_as_half(el));
-                    hi[i] = __half2float(__ushort_as_half(eh));
-                } else {
-                    lo[i] = __bfloat162float(__ushort_as_bfloat16(el));
-                    hi[i] = __bfloat162float(__ushort_as_bfloat16(eh));
-                }
+                const unsigned short el = (unsigned short)(wl[i >> 1] >> (16 * (i & 1))), eh = (unsigned short)(wh[i >> 1] >> (16 * (i & 1)));
+                lo[i] = a.g.cache == PA_DTYPE_F16 ? __half2float(__ushort_as_half(el)) : __bfloat162float(__ushort_as_bfloat16(el));
+                hi[i] = a.g.cache == PA_DTYPE_F16 ? __half2float(__ushort_as_half(eh)) : __bfloat162float(__ushort_as_bfloat16(eh));
             }
         }
-    }
-    float nlo[EL], nhi[EL];
-#pragma unroll
-    for (int i = 0; i < EL; ++i) {
-        nlo[i] = __fmaf_rn(-hi[i], sv[i], __fmul_rn(lo[i], cv[i]));
-        nhi[i] = __fmaf_rn(lo[i], sv[i], __fmul_rn(hi[i], cv[i]));
-    }
-    if (a.g.cache == PA_DTYPE_U8) {
-        float mn = fminf(nlo[0], nhi[0]), mx = fmaxf(nlo[0], nhi[0]);
-#pragma unroll
-        for (int i = 1; i < EL; ++i) {
-            mn = fminf(mn, fminf(nlo[i], nhi[i]));
-            mx = fmaxf(mx, fmaxf(nlo[i], nhi[i]));
-        }
-#pragma unroll
-        for (int o = LPT / 2; o > 0; o >>= 1) {   // over the token's lanes (every lane of the warp takes part)
-            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        }
-        float sc, zp, inv;
-        quant_params(mn, mx, sc, zp, inv);
-        __syncwarp();   // every lane has read the old parameters
-        if (work) {
-            if (l == 0) { params[tok] = sc; params[a.g.bs + tok] = zp; }
-            uint32_t wlv[2] = {0, 0}, whv[2] = {0, 0};
-#pragma unroll
-            for (int i = 0; i < EL; ++i) {
-                wlv[i >> 2] |= quant_one(nlo[i], inv, zp) << (8 * (i & 3));
-                whv[i >> 2] |= quant_one(nhi[i], inv, zp) << (8 * (i & 3));
-            }
-            *reinterpret_cast<uint2*>(rec + (long long)tok * D + EL * l) = make_uint2(wlv[0], wlv[1]);
-            *reinterpret_cast<uint2*>(rec + (long long)tok * D + HALF + EL * l) = make_uint2(whv[0], whv[1]);
-        }
-    } else if (work) {
-        uint16_t* p = (uint16_t*)rec + (long long)tok * D;
-        uint32_t wlv[4] = {0, 0, 0, 0}, whv[4] = {0, 0, 0, 0};
 #pragma unroll
         for (int i = 0; i < EL; ++i) {
-            unsigned short el, eh;
-            if (a.g.cache == PA_DTYPE_F16) {
-                el = __half_as_ushort(__float2half_rn(nlo[i]));
-                eh = __half_as_ushort(__float2half_rn(nhi[i]));
-            } else {
-                el = __bfloat16_as_ushort(__float2bfloat16_rn(nlo[i]));
-                eh = __bfloat16_as_ushort(__float2bfloat16_rn(nhi[i]));
-            }
-            wlv[i >> 1] |= (uint32_t)el << (16 * (i & 1));
-            whv[i >> 1] |= (uint32_t)eh << (16 * (i & 1));
+            nlo[i] = __fmaf_rn(-hi[i], sv[i], __fmul_rn(lo[i], cv[i]));
+            nhi[i] = __fmaf_rn(lo[i], sv[i], __fmul_rn(hi[i], cv[i]));
         }
-        *reinterpret_cast<uint4*>(p + EL * l) = make_uint4(wlv[0], wlv[1], wlv[2], wlv[3]);
-        *reinterpret_cast<uint4*>(p + HALF + EL * l) = make_uint4(whv[0], whv[1], whv[2], whv[3]);
-    }
+        if constexpr (U8) {
+            float mn = fminf(nlo[0], nhi[0]), mx = fmaxf(nlo[0], nhi[0]);
+#pragma unroll
+            for (int i = 1; i < EL; ++i) {
+                mn = min3(mn, nlo[i], nhi[i]);
+                mx = max3(mx, nlo[i], nhi[i]);
+            }
+#pragma unroll
+            for (int o = LPT / 2; o > 0; o >>= 1) {   // over the token's lanes (every lane of the warp takes part)
+                mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            }
+            float sc, zp, inv;
+            quant_params(mn, mx, sc, zp, inv);
+            if (live) {
+                if (l == 0) {   // (the token's lanes read its parameters one pass ago at the latest)
+                    float* params = (float*)(rec + (long long)a.g.bs * D);
+                    params[tok] = sc; params[a.g.bs + tok] = zp;
+                }
+                uint32_t wl[2], wh[2];
+#pragma unroll
+                for (int i = 0; i < EL; i += 4) {
+                    wl[i >> 2] = quant_four(nlo[i], nlo[i + 1], nlo[i + 2], nlo[i + 3], inv, zp);
+                    wh[i >> 2] = quant_four(nhi[i], nhi[i + 1], nhi[i + 2], nhi[i + 3], inv, zp);
+                }
+                *reinterpret_cast<uint2*>(rec + (long long)tok * D + EL * l) = make_uint2(wl[0], wl[1]);
+                *reinterpret_cast<uint2*>(rec + (long long)tok * D + HALF + EL * l) = make_uint2(wh[0], wh[1]);
+            }
+        } else if (live) {
+            uint16_t* p = (uint16_t*)rec + (long long)tok * D;
+            uint32_t wl[4] = {0, 0, 0, 0}, wh[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int i = 0; i < EL; ++i) {
+                const bool f16 = a.g.cache == PA_DTYPE_F16;
+                const unsigned short el = f16 ? __half_as_ushort(__float2half_rn(nlo[i])) : __bfloat16_as_ushort(__float2bfloat16_rn(nlo[i]));
+                const unsigned short eh = f16 ? __half_as_ushort(__float2half_rn(nhi[i])) : __bfloat16_as_ushort(__float2bfloat16_rn(nhi[i]));
+                wl[i >> 1] |= (uint32_t)el << (16 * (i & 1));
+                wh[i >> 1] |= (uint32_t)eh << (16 * (i & 1));
+            }
+            *reinterpret_cast<uint4*>(p + EL * l) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+            *reinterpret_cast<uint4*>(p + HALF + EL * l) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+        }
     }
 }
 
@@ -585,8 +612,10 @@ cudaError_t launch_write_kv(const KernelArgs& a, cudaStream_t stream, bool with_
 cudaError_t launch_rotate(const KernelArgs& a, cudaStream_t stream) {
     if (a.num_rotated_blocks <= 0) return cudaSuccess;
     const int grid = a.num_rotated_blocks;
-    if (a.g.D == 128) rotate_kernel<128><<<grid, 256, 0, stream>>>(a);
-    else rotate_kernel<64><<<grid, 256, 0, stream>>>(a);
+    const bool u8 = a.g.cache == PA_DTYPE_U8;
+    auto launch = [&](auto kernel) { kernel<<<grid, 256, 0, stream>>>(a); };
+    if (a.g.D == 128) u8 ? launch(rotate_kernel<128, true>) : launch(rotate_kernel<128, false>);
+    else u8 ? launch(rotate_kernel<64, true>) : launch(rotate_kernel<64, false>);
     return cudaGetLastError();
 }
 

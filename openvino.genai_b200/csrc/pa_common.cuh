@@ -130,10 +130,26 @@ __device__ __forceinline__ void quant_params(float mn, float mx, float& scale, f
     inv = __fdiv_rn(1.0f, s);
 }
 
-__device__ __forceinline__ unsigned quant_one(float x, float inv, float zp) {
-    float q = rintf(__fmaf_rn(x, inv, zp));
-    q = fminf(255.0f, fmaxf(0.0f, q));
-    return (unsigned)q;
+// clamp(rint(fma(x, inv, zp)), 0, 255).  Clamped first (the bounds are integers and rint is monotone, NaN goes to 0 either
+// way) and rounded by adding 2^23, where a float's ulp is one and the addition rounds halves to even: the byte is the low
+// byte of the bits.  No conversion instruction: those run at a quarter of the rate and, three per element, were what
+// the rotation of u8 blocks waited for.
+__device__ __forceinline__ unsigned quant_bits(float x, float inv, float zp) {   // the byte under 0x4B000000
+    const float q = fminf(255.0f, fmaxf(0.0f, __fmaf_rn(x, inv, zp)));
+    return __float_as_uint(__fadd_rn(q, 8388608.0f));
+}
+__device__ __forceinline__ unsigned quant_one(float x, float inv, float zp) { return quant_bits(x, inv, zp) & 0xffu; }
+// Four bytes in memory order.
+__device__ __forceinline__ uint32_t quant_four(float x0, float x1, float x2, float x3, float inv, float zp) {
+    const uint32_t lo = __byte_perm(quant_bits(x0, inv, zp), quant_bits(x1, inv, zp), 0x0040);
+    const uint32_t hi = __byte_perm(quant_bits(x2, inv, zp), quant_bits(x3, inv, zp), 0x0040);
+    return __byte_perm(lo, hi, 0x5410);
+}
+
+// (byte i of w - zp) * scale; the byte becomes a float as 2^23 + byte - 2^23, exactly.
+__device__ __forceinline__ float dequant_byte(uint32_t w, int i, float scale, float zp) {
+    const float q = __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | (unsigned)i)), 8388608.0f);
+    return __fmul_rn(__fsub_rn(q, zp), scale);
 }
 
 __device__ __forceinline__ float dequant_one(unsigned q, float scale, float zp) {
