@@ -46,9 +46,15 @@ struct __align__(8) Cand {
     int idx;
 };
 
-__device__ __forceinline__ void named_sync(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+// The aligned forms of the barrier instructions ask for a converged warp; the callers come from loops and branches whose
+// trip counts and conditions differ between lanes, so the warp is brought together first.
+__device__ __forceinline__ void named_sync(int id, int count) {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
 __device__ __forceinline__ int named_count(int id, int count, bool pred) {   // barrier that returns how many threads' pred holds
     int n;
+    __syncwarp();
     asm volatile("{ .reg .pred p; setp.ne.s32 p, %3, 0; barrier.cta.red.popc.aligned.u32 %0, %1, %2, p; }" : "=r"(n) : "r"(id), "r"(count), "r"((int)pred) : "memory");
     return n;
 }
