@@ -725,6 +725,16 @@ __device__ void draw_top_k(const Cand* v, const TopKDist& d, const float* ex, fl
     *out_idx = v[pick].idx;
 }
 
+// The ring's counts in shared memory: what a thread wrote before it stored a count is visible to whoever loads that count.
+__device__ __forceinline__ int load_acquire(const int* p) {
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void store_release(int* p, int v) {
+    asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v) : "memory");
+}
+
 // ---- the filter and the ring between it and the replay ------------------------------------------------------
 // Warps 1..15 read the row in rounds of kChunk elements, keep what exceeds a lower bound of the heap minimum, and append it
 // in index order to a ring in shared memory that warp 0 empties.  The bound is the consumer's minimum as last published or
@@ -736,8 +746,6 @@ __device__ void draw_top_k(const Cand* v, const TopKDist& d, const float* ex, fl
 template <class Load>
 __device__ __forceinline__ void produce_candidates(Shared& sh, int K, long long V, long long start, int rounds, float (&x)[kPerThread],
                                                    float (&xn)[kPerThread], Load&& load_round, int ptid, int pwarp, int lane) {
-    volatile int* v_head = &sh.head;
-    volatile int* v_tail = &sh.tail;
     volatile int* v_give_up = &sh.give_up;
     float bound = -CUDART_INF_F, top = -CUDART_INF_F;   // top: the thread's maximum so far
     int head = 0;
@@ -763,11 +771,11 @@ __device__ __forceinline__ void produce_candidates(Shared& sh, int K, long long 
         }
         if (lane == 31) sh.warp_cnt[step & 1][pwarp] = incl;
         named_sync(5, kProducerThreads);
-        if (step > 0 && ptid == 0) { __threadfence_block(); *v_head = head; }   // the entries of the steps before this one
+        if (step > 0 && ptid == 0) store_release(&sh.head, head);   // the entries of the steps before this one
         const int cnt = lane < kProducerWarps ? sh.warp_cnt[step & 1][lane] : 0;
         const int total = __reduce_add_sync(0xffffffffu, cnt), before = __reduce_add_sync(0xffffffffu, lane < pwarp ? cnt : 0);
         if (total > 0) {
-            for (int polls = 0; head + total - *v_tail > kRing && *v_give_up == 0;)
+            for (int polls = 0; head + total - load_acquire(&sh.tail) > kRing && *v_give_up == 0;)
                 if (++polls > kWaitPolls) *v_give_up = 1;
             const long long base = start + (long long)c * kChunk + (long long)ptid * kPerThread;
             int pos = head + before + incl - mine;
@@ -786,7 +794,7 @@ __device__ __forceinline__ void produce_candidates(Shared& sh, int K, long long 
                 const uint32_t mid = lo + span;
                 const int n = named_count(6, kProducerThreads, mid > lo && key >= mid);
                 if (n >= K) lo = mid;
-                if (it == 0 && ptid == 0) { __threadfence_block(); *v_head = head; }
+                if (it == 0 && ptid == 0) store_release(&sh.head, head);
             }
             bound = __uint_as_float((lo & 0x80000000u) ? lo & 0x7fffffffu : ~lo);   // float_key's inverse
         }
@@ -797,10 +805,8 @@ __device__ __forceinline__ void produce_candidates(Shared& sh, int K, long long 
     }
     if (rounds > 0) named_sync(5, kProducerThreads);
     if (ptid == 0) {
-        __threadfence_block();
-        *v_head = head;
-        __threadfence_block();
-        *reinterpret_cast<volatile int*>(&sh.done) = 1;
+        store_release(&sh.head, head);
+        store_release(&sh.done, 1);
     }
 }
 
@@ -812,11 +818,10 @@ __device__ __forceinline__ bool consume_candidates(Shared& sh, int lane, Take&& 
     for (;;) {
         int head = 0, done = 0;
         if (lane == 0) {
-            done = *reinterpret_cast<volatile int*>(&sh.done);
-            __threadfence_block();
-            head = *reinterpret_cast<volatile int*>(&sh.head);
-            __threadfence_block();
+            done = load_acquire(&sh.done);   // before the head: no entry is published after it
+            head = load_acquire(&sh.head);
         }
+        __syncwarp();   // what lane 0 has acquired, the whole warp may read
         head = __shfl_sync(0xffffffffu, head, 0);
         done = __shfl_sync(0xffffffffu, done, 0);
         if (head == tail) {
@@ -837,7 +842,7 @@ __device__ __forceinline__ bool consume_candidates(Shared& sh, int lane, Take&& 
             __syncwarp();
             if (lane == 0) {
                 *reinterpret_cast<volatile float*>(&sh.tau) = heap_min;
-                *reinterpret_cast<volatile int*>(&sh.tail) = tail;
+                store_release(&sh.tail, tail);   // the warp has read these entries: their places may be written again
             }
         }
     }

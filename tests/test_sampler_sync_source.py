@@ -29,3 +29,16 @@ def test_aligned_barriers_are_reached_by_converged_warps():
     for name in helpers:
         rest = rest.replace(_function(name), "")
     assert not re.search(r'"[^"\n]*\b(bar|barrier)\.[a-z]', rest), "a barrier instruction outside the two helpers"
+
+
+def test_ring_entries_are_read_and_overwritten_behind_an_acquired_count():
+    """The consumer's lane 0 acquires the counts and the warp synchronises before any lane reads an entry; the producers
+    acquire the consumer's count before they write to a place again; counts are stored with release."""
+    consume, produce = _function("consume_candidates"), _function("produce_candidates")
+    acquire, read = consume.index("load_acquire(&sh.head)"), consume.index("sh.ring[")
+    assert acquire < read and "__syncwarp()" in consume[acquire:read]
+    taken, freed = read, consume.index("store_release(&sh.tail")
+    assert taken < freed and "__syncwarp()" in consume[taken:freed]
+    assert produce.index("load_acquire(&sh.tail)") < produce.index("sh.ring[")
+    for body in (consume, produce):
+        assert not re.search(r"volatile[^;]*&sh\.(head|tail|done)\b", body), "a count of the ring without its ordering"
