@@ -38,7 +38,6 @@ constexpr int kChunk = kProducerThreads * kPerThread; // elements per filter rou
 constexpr int kMaxTopK = 1024;                        // heap capacity in shared memory
 constexpr int kRegTopK = 64;                          // heaps up to here live in the registers of warp 0
 constexpr int kRing = 8192;                           // candidates between producers and consumer; a power of two, at least kChunk
-constexpr int kWaitPolls = 1 << 22;                   // polls of a wait between the warps of a CTA before it is given up
 static_assert(kRing >= kChunk && (kRing & (kRing - 1)) == 0, "a round must fit the ring");
 
 struct __align__(8) Cand {
@@ -745,7 +744,7 @@ __device__ __forceinline__ void store_release(int* p, int v) {
 // before are written, and the count is published.
 template <class Load>
 __device__ __forceinline__ void produce_candidates(Shared& sh, int K, long long V, long long start, int rounds, float (&x)[kPerThread],
-                                                   float (&xn)[kPerThread], Load&& load_round, int ptid, int pwarp, int lane) {
+                                                   float (&xn)[kPerThread], Load&& load_round, int wait_polls, int ptid, int pwarp, int lane) {
     volatile int* v_give_up = &sh.give_up;
     float bound = -CUDART_INF_F, top = -CUDART_INF_F;   // top: the thread's maximum so far
     int head = 0;
@@ -776,7 +775,7 @@ __device__ __forceinline__ void produce_candidates(Shared& sh, int K, long long 
         const int total = __reduce_add_sync(0xffffffffu, cnt), before = __reduce_add_sync(0xffffffffu, lane < pwarp ? cnt : 0);
         if (total > 0) {
             for (int polls = 0; head + total - load_acquire(&sh.tail) > kRing && *v_give_up == 0;)
-                if (++polls > kWaitPolls) *v_give_up = 1;
+                if (++polls > wait_polls) *v_give_up = 1;
             const long long base = start + (long long)c * kChunk + (long long)ptid * kPerThread;
             int pos = head + before + incl - mine;
             if (mine) {
@@ -813,7 +812,7 @@ __device__ __forceinline__ void produce_candidates(Shared& sh, int K, long long 
 // Warp 0: hands the ring's entries to `take` (32 at a time in index order, the first in the highest lane) until the
 // producers are done; `take` returns the heap minimum.  False when a wait ran out.
 template <class Take>
-__device__ __forceinline__ bool consume_candidates(Shared& sh, int lane, Take&& take) {
+__device__ __forceinline__ bool consume_candidates(Shared& sh, int wait_polls, int lane, Take&& take) {
     int tail = 0, polls = 0;
     for (;;) {
         int head = 0, done = 0;
@@ -826,7 +825,7 @@ __device__ __forceinline__ bool consume_candidates(Shared& sh, int lane, Take&& 
         done = __shfl_sync(0xffffffffu, done, 0);
         if (head == tail) {
             if (done) break;
-            if (++polls > kWaitPolls) {
+            if (++polls > wait_polls) {
                 *reinterpret_cast<volatile int*>(&sh.give_up) = 1;
                 break;
             }
@@ -996,7 +995,7 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
         const bool nan_heap = __syncthreads_or(nan_here) != 0;
         if (warp > 0) {
             if (nan_heap) return;
-            produce_candidates(sh, K, V, start, rounds, x, xn, load_round, ptid, pwarp, lane);
+            produce_candidates(sh, K, V, start, rounds, x, xn, load_round, a.wait_polls, ptid, pwarp, lane);
             return;
         }
         const uint32_t heap_addr = (uint32_t)__cvta_generic_to_shared(sh.heap);
@@ -1052,16 +1051,16 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
                     return order_value(heap.root);
                 };
                 take(x0, K + l0, true);
-                ok = consume_candidates(sh, lane, take);
+                ok = consume_candidates(sh, a.wait_polls, lane, take);
                 lh.store(heap, sh.heap);
             } else {
                 take_shared(x0, K + l0, true);
-                ok = consume_candidates(sh, lane, take_shared);
+                ok = consume_candidates(sh, a.wait_polls, lane, take_shared);
             }
             __syncwarp();
             if (!ok) {   // a wait between the warps ran out
                 if (lane == 0) {
-                    atomicOr(a.status, 16u); a.out_token[r] = -1; a.out_log_prob[r] = 0.f;
+                    atomicOr(a.status, 32u); a.out_token[r] = -1; a.out_log_prob[r] = 0.f;
                     if (a.extra_offsets)
                         for (long long k = a.extra_offsets[r]; k < a.extra_offsets[r + 1]; ++k) { a.extra_out_token[k] = -1; a.extra_out_log_prob[k] = 0.f; }
                 }

@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <string>
 
@@ -40,6 +41,7 @@ struct sampler_handle {
     size_t exact_bytes = 0;
     int exact_ctas = 0;               // persistent grid of that kernel: two CTAs per SM
     int64_t launches = 0;
+    int wait_polls = sampler::kSamplerWaitPolls;   // env SAMPLER_B200_TEST_WAIT_POLLS: a limit that the bounded waits of the top-k path reach
 };
 
 namespace {
@@ -119,6 +121,7 @@ sampler::StepArgs kernel_args(sampler_handle* h, const sampler_step_args* a) {
     k.token_bitmasks = masks ? a->token_bitmasks : nullptr;
     k.bitmask_index = masks ? a->bitmask_index : nullptr;
     k.bitmask_words = masks ? a->bitmask_words : 0;
+    k.wait_polls = h->wait_polls;
     return k;
 }
 
@@ -146,6 +149,7 @@ int sampler_b200_create(int device, int32_t max_rows, int64_t max_vocab, sampler
         delete h;
         return sfail(SAMPLER_ERR_CUDA, std::string("sampler_b200_create: ") + cudaGetErrorString(e));
     }
+    if (const char* polls = std::getenv("SAMPLER_B200_TEST_WAIT_POLLS")) h->wait_polls = std::max(0, std::atoi(polls));
     h->exact_ctas = 2 * prop.multiProcessorCount;
     if (max_rows > 0 && max_vocab > 0) {   // otherwise sized on first use
         const int rc = ensure_exact_scratch(h, max_rows, max_vocab);
@@ -268,7 +272,7 @@ int sampler_b200_step_host(sampler_handle* h, const sampler_step_args* a, int co
     S_CUDA(cudaStreamSynchronize(stream));
     if (bits) {
         S_CUDA(cudaMemsetAsync(h->status, 0, 4, stream));
-        const int code = (bits & 1u) ? SAMPLER_ERR_BAD_TOKEN_ID : (bits & 8u) ? SAMPLER_ERR_UNSUPPORTED : (bits & 16u) ? SAMPLER_ERR_CUDA : SAMPLER_ERR_INVALID_ARG;
+        const int code = (bits & 1u) ? SAMPLER_ERR_BAD_TOKEN_ID : (bits & 8u) ? SAMPLER_ERR_UNSUPPORTED : (bits & (16u | 32u)) ? SAMPLER_ERR_CUDA : SAMPLER_ERR_INVALID_ARG;
         return sfail(code, "device status word " + std::to_string(bits));
     }
     return SAMPLER_OK;

@@ -21,7 +21,8 @@ struct StepArgs {
     int64_t* out_token;
     float* out_log_prob;
     uint32_t* status;  // bit 0: history id out of range, bit 1: logits_row out of range, bit 2: raw log-prob without scratch,
-                       // bit 3: top_k above the heap capacity (and below the vocabulary), bit 4: the sorted walk did not end
+                       // bit 3: top_k above the heap capacity (and below the vocabulary), bit 4: the sorted walk did not end,
+                       // bit 5: a wait between the warps of a top-k row ran out
     float* hist_raw;   // raw logits of the history entries (rows that report raw log-probabilities), may be null
     // further draws of a row (all null: none): CSR offsets, their uniform numbers, their outputs
     const int64_t* extra_offsets;
@@ -32,7 +33,9 @@ struct StepArgs {
     const int32_t* token_bitmasks;
     const int32_t* bitmask_index;
     long long bitmask_words;
+    int wait_polls;    // polls of a wait between the warps of a top-k row before it is given up
 };
+constexpr int kSamplerWaitPolls = 1 << 22;   // a quarter of a second or so
 
 cudaError_t launch_sampler(const StepArgs& a, cudaStream_t stream);
 size_t sampler_smem_bytes();

@@ -119,6 +119,44 @@ def test_top_k_heap_sizes_and_row_shapes_are_identical(gpu, top_k):
             assert np.allclose(lp_o, lp_g, atol=2e-6, rtol=1e-6, equal_nan=True)
 
 
+@pytest.mark.parametrize("top_k,polls,order", [(50, 0, -1), (50, 16, 1), (1024, 64, 1)])
+def test_waits_of_the_top_k_path_that_run_out_are_reported(gpu, monkeypatch, top_k, polls, order):
+    """The warp that replays the heap waits for candidates and the filtering warps for room in the ring, both for a bounded
+    number of polls.  A descending row has no candidates after its first round: the replay finds none and gives up at once.
+    All elements of an ascending row enter the heap: the ring is full long before the replay has made room.  The row then
+    has token -1 (its further draws too) and a status bit of its own; the other rows of the step and later steps are right."""
+    v = 151936
+    x = np.tile(np.linspace(-order, order, v, dtype=np.float32), (4, 1))
+    rows = H.make_rows(4, top_k=top_k, temperature=0.9, top_p=0.9)
+    rows["do_sample"][1] = 0
+    _, tok_o, _, _ = H.run_oracle(x, rows)
+    monkeypatch.setenv("SAMPLER_B200_TEST_WAIT_POLLS", str(polls))
+    limited = H.GpuSampler()
+    monkeypatch.delenv("SAMPLER_B200_TEST_WAIT_POLLS")
+    logits = torch.from_numpy(x).cuda()
+    offs = torch.tensor([0, 2, 2, 2, 3], dtype=torch.int64, device="cuda")
+    u = torch.full((3,), 0.5, device="cuda")
+    xt, xl = torch.full((3,), 7, dtype=torch.int64, device="cuda"), torch.full((3,), 7.0, device="cuda")
+    staged = limited.stage(rows, None, logits.device)
+    a = H.step_args(logits, staged["rows"], None, staged["tok"], staged["lp"], ptr=lambda t: t.data_ptr())
+    a.num_rows, (a.num_logit_rows, a.vocab) = 4, logits.shape
+    a.extra_offsets, a.extra_rand_u, a.extra_out_token, a.extra_out_log_prob = (t.data_ptr() for t in (offs, u, xt, xl))
+    a.stream = torch.cuda.current_stream().cuda_stream or 1
+    assert limited.lib.sampler_b200_step(limited.h, C.byref(a)) == 0
+    torch.cuda.synchronize()
+    bits = C.c_uint32()
+    assert limited.lib.sampler_b200_last_device_status(limited.h, C.byref(bits)) == 0 and bits.value == 32
+    tok = staged["tok"].cpu().numpy()
+    assert list(tok[[0, 2, 3]]) == [-1, -1, -1] and tok[1] == tok_o[1]
+    assert xt.tolist() == [-1, -1, -1] and xl.tolist() == [0.0, 0.0, 0.0]
+    rc, tok, _, _ = limited.step_host(x, rows)
+    assert rc == 3 and tok[0] == -1     # SAMPLER_ERR_CUDA
+    greedy = H.make_rows(4, do_sample=0)
+    assert limited.step_host(x, greedy)[0] == 0
+    rc, tok, _, _ = gpu.step_host(x, rows)
+    assert rc == 0 and np.array_equal(tok, tok_o)
+
+
 def test_small_vocab_and_k_not_below_vocab(gpu):
     rng = np.random.default_rng(9)
     x = (rng.standard_normal((5, 40)) * 2).astype(np.float32)
