@@ -342,7 +342,11 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
 #ifdef PA_PREFILL_PROF
     long long prof[5] = {0, 0, 0, 0, 0};
     const long long prof_begin = clock64();
-    __shared__ long long trace[5][8][4];   // role, event, tile 64..67 of this CTA
+    // role (0, 1 softmax A, B; 2 converter; 3 mma; 4 loader; 5 second mma warp), event, tile 64..67 of this CTA; 0: not met
+    constexpr int kTraceRoles = 6;
+    __shared__ long long trace[kTraceRoles][8][4];
+    for (int i = tid; i < kTraceRoles * 8 * 4; i += kThreads) (&trace[0][0][0])[i] = 0;
+    __syncthreads();
 #define PA_TRACE(role, ev, tile) do { if (lane == 0 && (tile) >= 64 && (tile) < 68) trace[role][ev][(tile) - 64] = clock64(); } while (0)
 #else
 #define PA_TRACE(role, ev, tile) do { } while (0)
@@ -1055,6 +1059,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                     for (int j = 0; j < it.ntiles; ++j, ++t) {
                         const int st = t % NST, st1 = (t + 1) % NST;
                         const bool more = j + 1 < it.ntiles;
+                        PA_TRACE(3, 0, t);
                         // The converter finishes V' of tile j before K' of tile j + 1, so the latter's barrier
                         // covers both; only the item's last tile waits for its V' directly.
                         if (more) {
@@ -1062,15 +1067,18 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                         } else {
                             if (!wait_warp(&sm.v_full[st], (t / NST) & 1, 3)) goto done;
                         }
+                        PA_TRACE(3, 3, t);
 #pragma unroll
                         for (int X = 0; X < 2; ++X)
                             if (j < it.nt[X]) {
                                 // P of tile j is in TMEM, so S of tile j has been read: both MMAs may go
                                 if (!wait_warp(&sm.p_full[X], (n[X] + j) & 1, 4)) goto done;
+                                PA_TRACE(3, 4 + 2 * X, t);
                                 tc05::fence_after_thread_sync();
                                 // the next logits first: the half's softmax warps wait for them, nobody waits for this P.V yet
                                 if (j + 1 < it.nt[X]) issue_s(X, st1);
                                 issue_pv(X, st, j > 0);
+                                PA_TRACE(3, 5 + 2 * X, t);
                             }
                         if (tc05::elect_one()) {
                             if (more) tc05::commit(&sm.k_free[st1]);
@@ -1095,6 +1103,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                         ++iq;
                     }
                     for (int j = -1; j < it.ntiles; ++j) {
+                        if (j >= 0) PA_TRACE(3 + 2 * X, 0, t + j);
                         if (j + 1 < it.ntiles) {
                             const int st1 = (t + j + 1) % NST;
                             if (!wait_warp(&sm.k_full[st1], ((t + j + 1) / NST) & 1, 1)) goto done;
@@ -1104,6 +1113,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                                 issue_s(X, st1);
                                 if (tc05::elect_one()) tc05::commit(&sm.k_free[st1]);
                                 __syncwarp();
+                                if (j >= 0) PA_TRACE(3 + 2 * X, 1, t + j);
                             } else {
                                 warp_arrive(&sm.k_free[st1]);   // this half has no use for the tile
                             }
@@ -1111,12 +1121,15 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                         if (j >= 0) {
                             const int st = (t + j) % NST;
                             if (!wait_warp(&sm.v_full[st], ((t + j) / NST) & 1, 3)) goto done;
+                            PA_TRACE(3 + 2 * X, 3, t + j);
                             if (j < nt) {
                                 if (!wait_warp(&sm.p_full[X], (n + j) & 1, 4)) goto done;
+                                PA_TRACE(3 + 2 * X, 4, t + j);
                                 tc05::fence_after_thread_sync();
                                 issue_pv(X, st, j > 0);
                                 if (tc05::elect_one()) tc05::commit(&sm.v_free[st]);
                                 __syncwarp();
+                                PA_TRACE(3 + 2 * X, 5, t + j);
                             } else {
                                 warp_arrive(&sm.v_free[st]);
                             }
@@ -1195,12 +1208,12 @@ done:
 #ifdef PA_PREFILL_PROF
     __syncthreads();
     if (blockIdx.x == 0 && tid == 0) {
-        const long long base = trace[3][0][0];
-        for (int role = 0; role < 5; ++role)
+        const long long base = trace[3][0][0];   // the first mma warp takes up tile 64
+        auto at = [&](int role, int ev, int tl) { return trace[role][ev][tl] ? trace[role][ev][tl] - base : 0; };
+        for (int role = 0; role < kTraceRoles && base; ++role)
             for (int tl = 0; tl < 4; ++tl)
-                printf("trace role %d tile %d: %lld %lld %lld %lld %lld %lld %lld %lld\n", role, 64 + tl, trace[role][0][tl] - base, trace[role][1][tl] - base,
-                       trace[role][2][tl] - base, trace[role][3][tl] - base, trace[role][4][tl] - base, trace[role][5][tl] - base, trace[role][6][tl] - base,
-                       trace[role][7][tl] - base);
+                printf("trace role %d tile %d: %lld %lld %lld %lld %lld %lld %lld %lld\n", role, 64 + tl, at(role, 0, tl), at(role, 1, tl), at(role, 2, tl),
+                       at(role, 3, tl), at(role, 4, tl), at(role, 5, tl), at(role, 6, tl), at(role, 7, tl));
     }
     if (blockIdx.x == 0 && lane == 0 && (warp == 0 || warp == 4 || warp == kSoftmaxWarps || warp >= kWarpMma))
         printf("prefill prof warp %d total %lld waits %lld %lld %lld %lld %lld\n", warp, clock64() - prof_begin, prof[0], prof[1], prof[2], prof[3], prof[4]);
