@@ -595,14 +595,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                     warp_arrive(&sm.s_read[X]);
                 }
                 if ((warp & 3) == 0) PA_TRACE(X, 1, n);
-#ifdef PA_EXP_NOSOFTMAX
-                float alpha = 1.f;
-                bool rescale = false;
-                uint32_t pw[kKv / 2];
-#pragma unroll
-                for (int c = 0; c < kKv; c += 2) pw[c >> 1] = __float_as_uint(sv[c]) ^ __float_as_uint(sv[c + 1]);
-                m_run = 0.f;
-#else
                 if (col0 + kKv > my_ctx) {     // diagonal tile: hide what this row cannot see
                     const int nvis = my_ctx - col0;   // may be <= 0
 #pragma unroll
@@ -628,11 +620,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                 uint32_t pl[BF ? kKv / 2 : 1];   // bf16 variant: the low pieces, p = high + low up to 2^-17 p
 #pragma unroll
                 for (int c = 0; c < kKv; c += 2) {
-#if defined(PA_EXP_NOEXP)
-                    pw[c >> 1] = __byte_perm(__float_as_uint(fmaf(sv[c], qs, -mq)), __float_as_uint(fmaf(sv[c + 1], qs, -mq)), 0x7632);
-#elif defined(PA_EXP_NOCVT)
-                    pw[c >> 1] = ex2_h2(__byte_perm(__float_as_uint(fmaf(sv[c], qs, -mq)), __float_as_uint(fmaf(sv[c + 1], qs, -mq)), 0x7632));
-#else
                     // the packed f16 exponential is good to 2^-9.9 relative: inside the u8 cache's error bound, not inside the
                     // f16 cache's, whose P goes through the f32 exponential and is rounded once
                     if constexpr (U8) {
@@ -646,9 +633,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                     } else {
                         pw[c >> 1] = pack_h2(ex2(fmaf(sv[c], qs, -mq)), ex2(fmaf(sv[c + 1], qs, -mq)));
                     }
-#endif
                 }
-#endif
                 // P.V of the previous tile of this half still reads the P tile and writes O
                 if ((warp & 3) == 0) PA_TRACE(X, 2, n);
                 if (n > 0) {
@@ -784,7 +769,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                 if (use > 0 && !wait_warp(&sm.k_free[st], (use - 1) & 1, 1)) goto done;
                 if (cwarp == 0) PA_TRACE(2, 1, t);
                 // K' = byte * f16(k scale): unit u = 16 dims of one token
-#ifndef PA_EXP_NOCONV
 #pragma unroll
                 for (int i = 0; i < kD / 32; ++i) {
                     const int u = ctid + 128 * i;
@@ -800,7 +784,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                     *reinterpret_cast<uint4*>(atom + sw128(token, (2 * seg) & 7)) = lo4;
                     *reinterpret_cast<uint4*>(atom + sw128(token, (2 * seg + 1) & 7)) = hi4;
                 }
-#endif
                 if (ctid < kKv) {
                     const int token = ctid;
                     const bool ok = token < live_tokens;
@@ -840,7 +823,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                     tab[k + 1] = make_uint2(t4.z, t4.w);
                 }
                 constexpr int UPR = BS / 16;   // 16-token units per record
-#ifndef PA_EXP_NOCONV
 #pragma unroll
                 for (int i = 0; i < kD / 32; ++i) {
                     const int d = (ctid >> 2) + 32 * i;
@@ -857,7 +839,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                     *reinterpret_cast<uint4*>(sm.vt[st] + sw128(d, 2 * tg)) = make_uint4(w[0], w[1], w[2], w[3]);
                     *reinterpret_cast<uint4*>(sm.vt[st] + sw128(d, 2 * tg + 1)) = make_uint4(w[4], w[5], w[6], w[7]);
                 }
-#endif
                 if (ctid < kKv) {
                     const int token = ctid;
                     const bool ok = token < live_tokens;
@@ -915,9 +896,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
 #pragma unroll
                     for (int u = 0; u < NU; ++u) {
                         const bool ok = off[u] >= 0;
-#ifndef PA_EXP_NOCOPY16
                         cp_async16_zfill(sm.k[st] + dst0 + sw128(trow + TP * u, ch & 7), kc + (ok ? off[u] : 0), ok ? 16u : 0u);
-#endif
                     }
                     cp_async_commit();
                     if (t > 0) {
@@ -929,9 +908,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
 #pragma unroll
                     for (int u = 0; u < NU; ++u) {
                         const bool ok = off[u] >= 0;
-#ifndef PA_EXP_NOCOPY16
                         cp_async16_zfill(sm.vt[st] + dst0 + sw128(trow + TP * u, ch & 7), vc + (ok ? off[u] : 0), ok ? 16u : 0u);
-#endif
                     }
                     cp_async_commit();
                     if (t > 0) {
@@ -1015,14 +992,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                     for (int kk = 0; kk < kKv / 16; ++kk) tc05::mma_ts<1>(d, pa + kKv / 2 + 8 * kk, db0 + 128 * kk, idesc_o);
                 } else {
                     // 16 tokens further along K = 16 rows of 128 bytes; the denominators go to the 16 columns after O
-#ifdef PA_EXP_NOONES
-                    if (acc) { tc05::mma_ts<1>(d, pa, db0, idesc_o); }
-                    else { tc05::mma_ts<0>(d, pa, db0, idesc_o); }
-#pragma unroll
-                    for (int kk = 1; kk < kKv / 16; ++kk) {
-                        tc05::mma_ts<1>(d, pa + 8 * kk, db0 + 128 * kk, idesc_o);
-                    }
-#else
                     if (acc) { tc05::mma_ts<1>(d, pa, db0, idesc_o); tc05::mma_ts<1>(d + kD, pa, dones, idesc_l); }
                     else { tc05::mma_ts<0>(d, pa, db0, idesc_o); tc05::mma_ts<0>(d + kD, pa, dones, idesc_l); }
 #pragma unroll
@@ -1030,7 +999,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                         tc05::mma_ts<1>(d, pa + 8 * kk, db0 + 128 * kk, idesc_o);
                         tc05::mma_ts<1>(d + kD, pa + 8 * kk, dones, idesc_l);
                     }
-#endif
                 }
                 tc05::commit(&sm.o_done[X]);
                 }
@@ -1188,13 +1156,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
                         }
                         blocks[r] = blk;
                     }
-#ifdef PA_EXP_NOLOAD
-                    bytes = 0;
-#endif
                     mbar_expect_tx(&sm.raw_full[st], bytes);
 #pragma unroll
                     for (int r = 0; r < Smem::NREC; ++r)
-                        if (blocks[r] >= 0 && bytes) {
+                        if (blocks[r] >= 0) {
                             bulk_g2s(sm.raw_k[st] + r * Smem::RSTRIDE, kc + (long long)blocks[r] * a.g.block_bytes, Smem::REC, &sm.raw_full[st]);
                             bulk_g2s(sm.raw_v[st] + r * Smem::RSTRIDE, vc + (long long)blocks[r] * a.g.block_bytes, Smem::REC, &sm.raw_full[st]);
                         }
