@@ -33,7 +33,7 @@ struct StepArgs {
     const int32_t* token_bitmasks;
     const int32_t* bitmask_index;
     long long bitmask_words;
-    int wait_polls;    // polls of a wait between the warps of a top-k row before it is given up
+    int wait_polls;    // polls without progress of the other side before a wait between the warps of a top-k row is given up
 };
 constexpr int kSamplerWaitPolls = 1 << 22;   // a quarter of a second or so
 

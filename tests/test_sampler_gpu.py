@@ -122,7 +122,7 @@ def test_top_k_heap_sizes_and_row_shapes_are_identical(gpu, top_k):
 @pytest.mark.parametrize("top_k,polls,order", [(50, 0, -1), (50, 16, 1), (1024, 64, 1)])
 def test_waits_of_the_top_k_path_that_run_out_are_reported(gpu, monkeypatch, top_k, polls, order):
     """The warp that replays the heap waits for candidates and the filtering warps for room in the ring, both for a bounded
-    number of polls.  A descending row has no candidates after its first round: the replay finds none and gives up at once.
+    number of polls without progress of the other side.  A descending row has no candidates after its first round: the replay finds none and gives up at once.
     All elements of an ascending row enter the heap: the ring is full long before the replay has made room.  The row then
     has token -1 (its further draws too) and a status bit of its own; the other rows of the step and later steps are right."""
     v = 151936
@@ -154,6 +154,19 @@ def test_waits_of_the_top_k_path_that_run_out_are_reported(gpu, monkeypatch, top
     greedy = H.make_rows(4, do_sample=0)
     assert limited.step_host(x, greedy)[0] == 0
     rc, tok, _, _ = gpu.step_host(x, rows)
+    assert rc == 0 and np.array_equal(tok, tok_o)
+
+
+def test_waits_of_the_top_k_path_end_with_progress_not_with_time(gpu, monkeypatch):
+    """A descending row of eight million elements: after the first round the replay has nothing to do for two thousand rounds,
+    far longer than its limit of polls, but each round comes well inside it."""
+    x = np.linspace(8, -8, 1 << 23, dtype=np.float32)[None, :].copy()
+    rows = H.make_rows(1, top_k=50, temperature=0.9)
+    monkeypatch.setenv("SAMPLER_B200_TEST_WAIT_POLLS", "8192")
+    patient = H.GpuSampler()
+    monkeypatch.delenv("SAMPLER_B200_TEST_WAIT_POLLS")
+    _, tok_o, _, _ = H.run_oracle(x, rows)
+    rc, tok, _, _ = patient.step_host(x, rows)
     assert rc == 0 and np.array_equal(tok, tok_o)
 
 
