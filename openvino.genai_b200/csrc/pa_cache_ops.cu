@@ -1,7 +1,8 @@
 // Cache maintenance kernels of the PagedAttention operator: writing a chunk's new keys / values
 // into their paged slots (with by-token u8 quantisation), re-rotating the keys of listed blocks,
-// and block copies for copy-on-write.  All three are HBM-bound byte movers; one warp owns one
-// (token, kv head) row so the min/max for the quantiser is a warp shuffle.
+// and block copies for copy-on-write.  All three are byte movers; one warp, or eight lanes where chunks
+// are written in groups of tokens, own one (token, kv head) row, so the min/max for the quantiser is a
+// handful of shuffles.
 #include "pa_common.cuh"
 #include "pa_kernels.h"
 
@@ -593,9 +594,10 @@ cudaError_t launch_write_kv(const KernelArgs& a, cudaStream_t stream, bool with_
     // Chunks go in groups of 32 tokens once there are enough rows to give every SM a few (rows = tokens x kv heads, us; one warp
     // per row | groups): u8 2048 rows 6.2 | 6.2, 8192 rows 12.4 | 8.2, 65536 rows 55 | 26; bf16 2048 rows 5.2 | 4.0, 65536 rows
     // 20.5 | 11.8.  Decode rows, each in a block of its own, stay with one warp per row: u8 2048 rows 6.3 | 9.3.
-    // The groups' wider loads need activations on 16-byte boundaries.
+    // The groups' wider loads and stores need activations and caches on 16-byte boundaries.
     const bool groups = warps >= kWriteGroupRows && a.num_tokens >= 2LL * a.num_sequences &&
-                        ((reinterpret_cast<uintptr_t>(a.key) | reinterpret_cast<uintptr_t>(a.value)) & 15) == 0;
+                        ((reinterpret_cast<uintptr_t>(a.key) | reinterpret_cast<uintptr_t>(a.value) | reinterpret_cast<uintptr_t>(a.key_cache) |
+                          reinterpret_cast<uintptr_t>(a.value_cache)) & 15) == 0;
     const long long blocks = groups ? (long long)((a.num_tokens + kWriteTokens - 1) / kWriteTokens) * a.g.Hkv : (warps * 32 + 255) / 256;
     const int grid = (int)blocks + plan_blocks;
     auto launch = [&](auto kernel) { kernel<<<grid, 256, 0, stream>>>(a); };

@@ -1,6 +1,8 @@
 """Forms of the PagedAttention inputs that decide which branch of a kernel runs, against the CPU oracle: head sizes, block sizes
-and head counts of the rotation, query rows that are scaled before they are packed beside rows that are not, and a query that
-does not start on a boundary of the wide loads."""
+and head counts of the rotation, query rows that are scaled before they are packed beside rows that are not, and a query and
+caches that do not start on a boundary of the wide loads and stores."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -76,3 +78,31 @@ def test_decode_query_off_a_pair_boundary(act, cache, d):
     assert H.rel_err(ref["out_gpu"], want["out_ref"]) < 1e-2
     # the order in which partials are added may differ: one rounding of the output
     assert H.rel_err(out.float().cpu().numpy(), ref["out_gpu"]) < (2 ** -7 if act == torch.bfloat16 else 2 ** -10)
+
+
+@pytest.mark.parametrize("cache,act,shift", [("u8", torch.bfloat16, 4), ("f16", torch.float16, 2), ("bf16", torch.float32, 8)])
+def test_chunk_writes_into_caches_off_a_16_byte_boundary(cache, act, shift):
+    """Enough rows for groups of tokens, whose stores are up to 16 bytes wide: caches that start elsewhere get the same bytes
+    row by row (and nothing around them is touched)."""
+    wl = H.small_workload(hq=8, hkv=4, d=128, bs=32, act=act, cache=cache, past=[0, 5, 31], new=[701, 33, 1], seed=19)
+    assert wl.num_tokens * 4 >= 2048
+    _, k, v, _, _, _ = H.make_host_data(wl)
+    op = H.make_op(wl)
+    t = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    kd, vd = k.cuda(), v.cuda()
+    n = wl.num_blocks * H.block_bytes(wl)
+    def write(off):
+        flat = [torch.full((n + 64,), 0xA5, dtype=torch.uint8, device="cuda") for _ in range(2)]
+        for x in flat:
+            x[off:off + n] = 0
+        kc, vc = (x[off:off + n] for x in flat)
+        args = op.make_args(kd, kd, vd, kd, kc, vc, t(wl.past_lens), t(wl.subsequence_begins), t(wl.block_indices), t(wl.block_indices_begins),
+                            wl.scale, wl.max_context_len)
+        op._check(op.lib.pa_b200_write_kv(op._h, C.byref(args)))
+        torch.cuda.synchronize()
+        assert op.device_status() == 0
+        for x in flat:
+            assert bool((x[:off] == 0xA5).all()) and bool((x[off + n:] == 0xA5).all())
+        return kc.cpu().numpy(), vc.cpu().numpy()
+    want, got = write(0), write(shift)
+    assert want[0].any() and np.array_equal(want[0], got[0]) and np.array_equal(want[1], got[1])
