@@ -37,7 +37,9 @@ constexpr int kPerThread = 8;                         // elements a producer thr
 constexpr int kChunk = kProducerThreads * kPerThread; // elements per filter round
 constexpr int kMaxTopK = 1024;                        // heap capacity in shared memory
 constexpr int kRegTopK = 64;                          // heaps up to here live in the registers of warp 0
-constexpr int kRing = 8192;                           // candidates between producers and consumer; a power of two, at least kChunk
+constexpr int kRing = 4096;                           // candidates between producers and consumer; a power of two, at least kChunk:
+                                                      // 8192 gave top-k rows nothing (90.7 | 90.6 us) and cost the others their L1
+                                                      // (256 greedy rows 31.9 -> 31.5 us a step)
 static_assert(kRing >= kChunk && (kRing & (kRing - 1)) == 0, "a round must fit the ring");
 
 struct __align__(8) Cand {
@@ -929,14 +931,18 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
         ArgMax best{-CUDART_INF_F, 0x7fffffff};
         long long done = 0;
         if ((V & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
-            // 16-byte loads, four in flight per thread; indices ascend per thread so the first maximum is kept
+            // 16-byte loads, four in flight per thread; indices ascend per thread so the first maximum is kept.  The last, partial
+            // four too: one behind the other they were up to three more round trips, most of what a row of 32 k waits for
+            // (1 row 10.4 -> 10.2 us a step, 256 rows x 151936 32.9 -> 31.9).
             const float4* row4 = reinterpret_cast<const float4*>(row);
             const long long n4 = V >> 2;
-            long long i = tid;
-            for (; i + 3 * kThreads < n4; i += 4 * kThreads) {
+            for (long long i = tid; i < n4; i += 4 * kThreads) {
                 float4 q[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) q[u] = __ldcs(row4 + i + u * kThreads);
+                for (int u = 0; u < 4; ++u) {   // beyond the row: above nothing
+                    q[u] = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+                    if (i + u * kThreads < n4) q[u] = __ldcs(row4 + i + u * kThreads);
+                }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int b = (int)((i + u * kThreads) << 2);
@@ -945,14 +951,6 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
                     if (q[u].z > best.v) { best.v = q[u].z; best.i = b + 2; }
                     if (q[u].w > best.v) { best.v = q[u].w; best.i = b + 3; }
                 }
-            }
-            for (; i < n4; i += kThreads) {
-                const float4 q = __ldcs(row4 + i);
-                const int b = (int)(i << 2);
-                if (q.x > best.v) { best.v = q.x; best.i = b; }
-                if (q.y > best.v) { best.v = q.y; best.i = b + 1; }
-                if (q.z > best.v) { best.v = q.z; best.i = b + 2; }
-                if (q.w > best.v) { best.v = q.w; best.i = b + 3; }
             }
             done = V;
         }

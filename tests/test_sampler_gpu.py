@@ -44,6 +44,24 @@ def test_greedy_with_penalties_is_bit_exact(gpu):
     assert np.all(lp_g == 0)
 
 
+@pytest.mark.parametrize("v", [4, 2044, 2048, 2052, 6148, 8188, 8192, 8196, 14340, 32000])
+def test_greedy_rows_around_a_full_group_of_loads(gpu, v):
+    """A CTA reads 8192 elements at a time, 2048 per load of its threads: the maximum in the last element, the first element of
+    the last load, twice (the first counts), among -inf only, and a row whose values are all the lowest float."""
+    rng = np.random.default_rng(v)
+    x = rng.standard_normal((6, v)).astype(np.float32)
+    x[0, v - 1] = 9.0
+    x[1, (v - 1) // 2048 * 2048] = 9.0
+    x[2, [v // 2, v - 1]] = 9.0
+    x[3, :] = -np.inf
+    x[3, v - 2] = np.finfo(np.float32).min
+    x[4, :] = np.finfo(np.float32).min
+    x[5, :] = -np.inf
+    tok_o, _, _, tok_g, _, _ = _both(gpu, x, H.make_rows(6, do_sample=0))
+    assert np.array_equal(tok_o, tok_g)
+    assert list(tok_g) == [v - 1, (v - 1) // 2048 * 2048, v // 2, v - 2, 0, 0]
+
+
 def test_greedy_ties_nan_and_all_masked(gpu):
     x = np.zeros((3, 1000), np.float32)
     x[0, [10, 500, 999]] = 7.0
