@@ -3,6 +3,8 @@
 // and block copies for copy-on-write.  All three are byte movers; one warp, or eight lanes where chunks
 // are written in groups of tokens, own one (token, kv head) row, so the min/max for the quantiser is a
 // handful of shuffles.
+#include <algorithm>
+
 #include "pa_common.cuh"
 #include "pa_kernels.h"
 
@@ -201,7 +203,7 @@ __device__ __forceinline__ bool locate_token(const KernelArgs& a, int t, bool re
 // bytes of the u8 cache are turned around in shared memory and leave as words instead of single bytes.  Bound by the chain
 // locate -> load -> quantise -> store and, from some 30 k rows on, by the bytes: 65536 rows (bf16 in, u8 out) 55 -> 26 us.
 constexpr int kWriteTokens = 32;
-constexpr long long kWriteGroupRows = 2048;
+constexpr long long kWriteLightRows = 2048, kWriteChunkRows = 3072;
 template <int D, bool F32>
 __device__ __forceinline__ void write_group(const KernelArgs& a, int group, int h) {
     constexpr int NP = D / 64;                      // pieces of eight dims per lane: dims 8 l + 64 p
@@ -591,11 +593,17 @@ cudaError_t launch_write_kv(const KernelArgs& a, cudaStream_t stream, bool with_
     if (a.num_tokens <= 0 && !with_plan) return cudaSuccess;
     const long long warps = (long long)a.num_tokens * a.g.Hkv;
     const int plan_blocks = (with_plan ? 1 : 0) + (with_plan && a.scores && a.score_aggregation_window ? 1 : 0);
-    // Chunks go in groups of 32 tokens once there are enough rows to give every SM a few (rows = tokens x kv heads, us; one warp
-    // per row | groups): u8 2048 rows 6.2 | 6.2, 8192 rows 12.4 | 8.2, 65536 rows 55 | 26; bf16 2048 rows 5.2 | 4.0, 65536 rows
-    // 20.5 | 11.8.  Decode rows, each in a block of its own, stay with one warp per row: u8 2048 rows 6.3 | 9.3.
+    // Chunks go in groups of 32 tokens once they have enough rows (tokens x kv heads) to give every SM a few.  Decode rows, each in a
+    // block of its own, are better off with a warp per row: their u8 value bytes are scattered one by one, 4096 of them by one CTA
+    // instead of four.  The line lies where the chunks' gain pays for that (us, warp per row | groups; a 600-token chunk is "600"):
+    // u8, 8 kv heads x 128: 2048 18.5 | 10.2, 512 8.4 | 6.2, 250 decode + 1100 16.5 | 12.4, 1000 + 1010 20.6 | 18.6, but 500 + 520
+    // 12.4 | 12.8 and 128 + 130 6.6 | 8.3; 4 x 64: 64 + 4 x 256 8.3 | 7.3, but 256 + 280 6.3 | 8.3 and 120 + 2 x 300 6.3 | 7.3.  f32 activations, which every cache type converts, lie the same way (f16 cache, 8 x 128: 250 + 1100 8.3 | 6.3,
+    // 128 + 130 4.5 | 5.3).  16-bit activations into 16-bit caches gain from 2048 rows on, decode rows or not (bf16, 8 x 128:
+    // 128 + 130 4.9 | 4.5, 1000 + 1010 10.4 | 6.3).
     // The groups' wider loads and stores need activations and caches on 16-byte boundaries.
-    const bool groups = warps >= kWriteGroupRows && a.num_tokens >= 2LL * a.num_sequences &&
+    const long long chunk_rows = std::max(0LL, (long long)a.num_tokens - a.num_sequences) * a.g.Hkv, decode_rows = (long long)a.num_sequences * a.g.Hkv;
+    const bool light = a.g.cache != PA_DTYPE_U8 && a.g.act != PA_DTYPE_F32;
+    const bool groups = a.num_tokens >= 2LL * a.num_sequences && (light ? warps >= kWriteLightRows : chunk_rows >= kWriteChunkRows + decode_rows / 2) &&
                         ((reinterpret_cast<uintptr_t>(a.key) | reinterpret_cast<uintptr_t>(a.value) | reinterpret_cast<uintptr_t>(a.key_cache) |
                           reinterpret_cast<uintptr_t>(a.value_cache)) & 15) == 0;
     const long long blocks = groups ? (long long)((a.num_tokens + kWriteTokens - 1) / kWriteTokens) * a.g.Hkv : (warps * 32 + 255) / 256;

@@ -84,8 +84,8 @@ def test_decode_query_off_a_pair_boundary(act, cache, d):
 def test_chunk_writes_into_caches_off_a_16_byte_boundary(cache, act, shift):
     """Enough rows for groups of tokens, whose stores are up to 16 bytes wide: caches that start elsewhere get the same bytes
     row by row (and nothing around them is touched)."""
-    wl = H.small_workload(hq=8, hkv=4, d=128, bs=32, act=act, cache=cache, past=[0, 5, 31], new=[701, 33, 1], seed=19)
-    assert wl.num_tokens * 4 >= 2048
+    wl = H.small_workload(hq=10, hkv=5, d=128, bs=32, act=act, cache=cache, past=[0, 5, 31], new=[701, 33, 1], seed=19)
+    assert (wl.num_tokens - 3) * 5 >= 3072 + 3 * 5 // 2
     _, k, v, _, _, _ = H.make_host_data(wl)
     op = H.make_op(wl)
     t = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()

@@ -92,13 +92,15 @@ def test_prefill_and_mixed_parity(cache, d, bs):
 @pytest.mark.parametrize("cache,act,d,bs", [("u8", torch.bfloat16, 128, 32), ("u8", torch.float32, 128, 16), ("u8", torch.float16, 64, 16),
                                             ("f16", torch.float16, 128, 32), ("bf16", torch.bfloat16, 64, 32), ("bf16", torch.float32, 128, 16),
                                             ("f16", torch.bfloat16, 64, 16)])
-def test_chunk_writes_in_token_groups(cache, act, d, bs):
-    """Chunks of more than 2048 (token, kv head) rows are written in groups of 32 tokens: bytes equal to the oracle's where
+@pytest.mark.parametrize("hkv", [2, 3])
+def test_chunk_writes_in_token_groups(cache, act, d, bs, hkv):
+    """Chunks of more than 2048 (16-bit activations and caches) or 3072 (token, kv head) rows are written in groups of 32 tokens,
+    shorter ones row by row: bytes equal to the oracle's where
     groups straddle sequences, blocks and words, start at any slot, hold decode rows or end short; the same bytes from
     activations off a 16-byte boundary, which are written row by row; a bad block id in one group leaves the rest alone."""
     import ctypes as C
-    wl = H.small_workload(hq=6, hkv=2, d=d, bs=bs, act=act, cache=cache, past=[0, 5, 31, 42, 7, 703, 16], new=[701, 33, 1, 67, 2, 301, 1], seed=91)
-    assert wl.num_tokens * 2 >= 2048 and wl.num_tokens % 32 != 0
+    wl = H.small_workload(hq=3 * hkv, hkv=hkv, d=d, bs=bs, act=act, cache=cache, past=[0, 5, 31, 42, 7, 703, 16], new=[701, 33, 1, 67, 2, 301, 1], seed=91)
+    assert wl.num_tokens * 2 >= 2048 and (wl.num_tokens - 7) * 3 >= 3072 + 7 * 3 // 2 and wl.num_tokens % 32 != 0
     data = H.make_host_data(wl)
     ref = H.run_oracle(wl, data)
     got = H.run_gpu(wl, data)
