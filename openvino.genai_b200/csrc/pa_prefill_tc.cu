@@ -1,5 +1,5 @@
-// Prefill-chunk attention on the 5th-generation tensor cores (tcgen05 + TMEM) for the u8 and the f16
-// cache, head sizes 128 and 64.
+// Prefill-chunk attention on the 5th-generation tensor cores (tcgen05 + TMEM) for the u8, f16 and (under bf16 activations)
+// bf16 cache, head sizes 128 and 64.
 //
 // A work item is a q tile of 256 rows = (new token, q head of one GQA group) pairs of one
 // (sequence, kv head), so a K/V byte is read once for the whole group.  The item is split into two
@@ -11,10 +11,11 @@
 //                          K' = byte * f16(k scale) as [64 tokens][128 dims], V'^T = byte *
 //                          f16(v scale) as [128 dims][64 tokens] (the cache keeps value bytes
 //                          token-minor, so both are K-major operands), two stages each;
-//   mma       (1 warp, one elected lane issues) tcgen05.mma: S_X = Q_X.K'^T into TMEM, O_X += P_X.V' in
-//                          TMEM, for X = A, B; as soon as half X has published P of tile j the S of tile
-//                          j + 1 and then its P.V are queued, so the tensor core works on one half while the
-//                          other half's softmax runs;
+//   mma       (one elected lane of a warp issues) tcgen05.mma: S_X = Q_X.K'^T into TMEM, O_X += P_X.V' in TMEM, for
+//                          X = A, B.  u8 cache: one warp for both halves; as soon as half X has published P of tile j
+//                          the S of tile j + 1 and then its P.V are queued, so the tensor core works on one half
+//                          while the other half's softmax runs.  16-bit caches: a warp per half, S of tile j + 1
+//                          queued as soon as the softmax warps hold S of tile j;
 //   softmax   (2 x 4 warps) thread r owns row r of its half: reads S from TMEM, masks (diagonal
 //                          tiles only), keeps a lazy running maximum, writes P = 2^(scale*(s-m)) as
 //                          f16 into TMEM (the A operand of P.V); rescales O in TMEM only when a row maximum
@@ -29,7 +30,7 @@
 // with the same shared-memory image; the softmax denominator comes from a second, 16-column P.V
 // product against a constant tile whose first row is all ones.  The raw ring, the extra dims and
 // the loader's copies do not exist in that variant.
-// The CTA has four warpgroups (softmax A, softmax B, converter / copy, {mma, loader, two idle warps}) that re-divide the
+// The CTA has four warpgroups (softmax A, softmax B, converter / copy, {mma, loader, second mma or idle, idle}) that re-divide the
 // register file with setmaxnreg once their roles start: 160 registers per softmax thread, 104 per converter thread, 88 for
 // the rest (one warp of each warpgroup shares a scheduler's 16 K registers).
 // Every wait is bounded; a wait that runs out raises a flag that all roles poll.
@@ -58,7 +59,7 @@ constexpr float kLn2P = 0.6931471805599453f;
 
 constexpr int kSoftmaxWarps = 8, kConvWarps = 4;
 constexpr int kWarpMma = kSoftmaxWarps + kConvWarps, kWarpLoad = kWarpMma + 1, kWarpMma2 = kWarpMma + 2;   // the second mma warp: 16-bit caches
-constexpr int kThreads = 512;   // four warpgroups: softmax A, softmax B, converter / copy warps, {mma, loader, two idle warps}
+constexpr int kThreads = 512;   // four warpgroups: softmax A, softmax B, converter / copy warps, {mma, loader, second mma (16-bit caches) or idle, idle}
 // Registers per thread after the roles have re-divided the register file among the warpgroups (one warp of each shares a
 // scheduler's 16 K registers: 160 + 160 + 104 + 88 = 512 x 32)
 #ifndef PA_TC_REG_SOFTMAX
@@ -272,6 +273,13 @@ __device__ __forceinline__ Item locate_item(const KernelArgs& a, int item, int G
     return it;
 }
 
+#ifdef PA_PREFILL_PROF
+// role (0, 1 softmax A, B; 2 converter; 3 mma; 4 loader; 5 second mma warp), event, tile 64..67 of CTA 0; 0: not met.  (In global
+// memory: the 16-bit variants use all shared memory there is.)
+constexpr int kTraceRoles = 6;
+__device__ long long trace[kTraceRoles][8][4];
+#endif
+
 template <int BS, int CT, int D>
 __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
     using Smem = PrefillSmem<BS, CT, D>;
@@ -342,12 +350,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
 #ifdef PA_PREFILL_PROF
     long long prof[5] = {0, 0, 0, 0, 0};
     const long long prof_begin = clock64();
-    // role (0, 1 softmax A, B; 2 converter; 3 mma; 4 loader; 5 second mma warp), event, tile 64..67 of this CTA; 0: not met
-    constexpr int kTraceRoles = 6;
-    __shared__ long long trace[kTraceRoles][8][4];
-    for (int i = tid; i < kTraceRoles * 8 * 4; i += kThreads) (&trace[0][0][0])[i] = 0;
+    if (blockIdx.x == 0)
+        for (int i = tid; i < kTraceRoles * 8 * 4; i += kThreads) (&trace[0][0][0])[i] = 0;
     __syncthreads();
-#define PA_TRACE(role, ev, tile) do { if (lane == 0 && (tile) >= 64 && (tile) < 68) trace[role][ev][(tile) - 64] = clock64(); } while (0)
+#define PA_TRACE(role, ev, tile) do { if (lane == 0 && blockIdx.x == 0 && (tile) >= 64 && (tile) < 68) trace[role][ev][(tile) - 64] = clock64(); } while (0)
 #else
 #define PA_TRACE(role, ev, tile) do { } while (0)
 #endif
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
         return item;
     };
 
-    if (warp >= kWarpMma) reg_dec<PA_TC_REG_MISC>();   // the fourth warpgroup: mma, loader and two warps that only keep it whole
+    if (warp >= kWarpMma) reg_dec<PA_TC_REG_MISC>();   // the fourth warpgroup: mma, loader, second mma; what is left over keeps it whole
     if (warp < kSoftmaxWarps) {
         // ======================= softmax + epilogue of half X ==========================================
         reg_inc<PA_TC_REG_SOFTMAX>();

@@ -14,3 +14,9 @@ def test_every_printed_role_of_the_prefill_trace_is_recorded():
     assert recorded == set(range(roles))
     base = re.search(r"base = trace\[(\d+)\]\[(\d+)\]\[0\]", SOURCE)
     assert re.search(r"PA_TRACE\(%s(?: \+ 2 \* X)?, %s," % base.groups(), SOURCE), "nothing records the trace's origin"
+
+
+def test_the_prefill_trace_takes_no_shared_memory():
+    """The 16-bit variants use every byte of shared memory that a CTA can have: with a record of their own there the build with
+    the trace could not be launched."""
+    assert not re.search(r"__shared__[^;]*\btrace\b", SOURCE)
