@@ -462,7 +462,7 @@ struct Shared {
     Cand heap[kMaxTopK];
     Cand ring[kRing];          // survivors of the filter, in index order
     int head, tail;            // entries published / taken (running counts)
-    int step;                  // the producers' step: shows that they are at work where nothing passes the filter
+    int idle;                  // the consumer's empty polls since the producers' last step
     int done;                  // every round is published
     int give_up;               // a wait ran out
     float tau;                 // consumer's heap minimum as the producers see it (may lag, never leads)
@@ -773,7 +773,7 @@ __device__ __forceinline__ void produce_candidates(Shared& sh, int K, long long 
         }
         if (lane == 31) sh.warp_cnt[step & 1][pwarp] = incl;
         named_sync(5, kProducerThreads);
-        if (ptid == 0) *reinterpret_cast<volatile int*>(&sh.step) = step;
+        if (ptid == 0) *reinterpret_cast<volatile int*>(&sh.idle) = 0;
         if (step > 0 && ptid == 0) store_release(&sh.head, head);   // the entries of the steps before this one
         const int cnt = lane < kProducerWarps ? sh.warp_cnt[step & 1][lane] : 0;
         const int total = __reduce_add_sync(0xffffffffu, cnt), before = __reduce_add_sync(0xffffffffu, lane < pwarp ? cnt : 0);
@@ -819,11 +819,10 @@ __device__ __forceinline__ void produce_candidates(Shared& sh, int K, long long 
 // producers are done; `take` returns the heap minimum.  False when a wait ran out.
 template <class Take>
 __device__ __forceinline__ bool consume_candidates(Shared& sh, int wait_polls, int lane, Take&& take) {
-    int tail = 0, polls = 0, seen = 0;
+    int tail = 0;
     for (;;) {
-        int head = 0, done = 0, step = 0;
+        int head = 0, done = 0;
         if (lane == 0) {
-            step = *reinterpret_cast<volatile int*>(&sh.step);
             done = load_acquire(&sh.done);   // before the head: no entry is published after it
             head = load_acquire(&sh.head);
         }
@@ -832,16 +831,17 @@ __device__ __forceinline__ bool consume_candidates(Shared& sh, int wait_polls, i
         done = __shfl_sync(0xffffffffu, done, 0);
         if (head == tail) {
             if (done) break;
-            step = __shfl_sync(0xffffffffu, step, 0);
-            polls = step == seen ? polls + 1 : 0;   // polls without progress of the producers
-            seen = step;
-            if (polls > wait_polls) {
+            int polls = 0;
+            if (lane == 0) {   // (counted where the producers reset it: no register of the replay's)
+                polls = *reinterpret_cast<volatile int*>(&sh.idle) + 1;
+                *reinterpret_cast<volatile int*>(&sh.idle) = polls;
+            }
+            if (__shfl_sync(0xffffffffu, polls, 0) > wait_polls) {
                 *reinterpret_cast<volatile int*>(&sh.give_up) = 1;
                 break;
             }
             continue;
         }
-        polls = 0;
         while (tail < head) {
             const int i = tail + 31 - lane;
             const bool valid = i < head;
@@ -996,7 +996,7 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
             sh.heap[i] = Cand{h, i};
             nan_here |= h != h;
         }
-        if (tid == 0) { sh.head = 0; sh.tail = 0; sh.step = 0; sh.done = 0; sh.give_up = 0; sh.tau = -CUDART_INF_F; }
+        if (tid == 0) { sh.head = 0; sh.tail = 0; sh.idle = 0; sh.done = 0; sh.give_up = 0; sh.tau = -CUDART_INF_F; }
         // NaN among the first K: the heap's comparisons are then those of no order, and the elements are taken one by one
         const bool nan_heap = __syncthreads_or(nan_here) != 0;
         if (warp > 0) {
