@@ -859,6 +859,59 @@ __device__ __forceinline__ bool consume_candidates(Shared& sh, int wait_polls, i
     return *reinterpret_cast<volatile int*>(&sh.give_up) == 0;
 }
 
+// A heap with NaN among its first K elements: the comparisons are those of no order, its root may fall as well as rise, and no
+// bound holds.  Warps 1..15 bring the row into the ring's place, kFeed elements at a time, the next ones in flight while warp 0
+// takes them one by one.  64 rows x 151936, K 50: 312 us; 473 with warp 0 reading the row by itself, 278 through a filter with
+// bounds.
+// Out of line: these registers are not the filter's.
+constexpr int kFeedLoads = 16, kFeed = kFeedLoads * kProducerThreads;
+static_assert(kRing * sizeof(Cand) >= kFeed * sizeof(float), "the elements take the ring's place");
+__device__ __noinline__ void feed_unordered(Shared& sh, const float* row, long long V, int K) {
+    const int ptid = threadIdx.x - 32;
+    float* const buf = reinterpret_cast<float*>(sh.ring);
+    float v[kFeedLoads];
+    auto load = [&](long long base) {
+#pragma unroll
+        for (int u = 0; u < kFeedLoads; ++u) { const long long i = base + kProducerThreads * u + ptid; v[u] = i < V ? row[i] : CUDART_NAN_F; }
+    };
+    load(K);
+    for (long long base = K; base < V; base += kFeed) {
+        named_sync(7, kThreads);   // warp 0 is done with the elements before these
+#pragma unroll
+        for (int u = 0; u < kFeedLoads; ++u) buf[kProducerThreads * u + ptid] = v[u];
+        named_sync(7, kThreads);
+        load(base + kFeed);
+    }
+}
+__device__ __noinline__ void replay_unordered(Shared& sh, long long V, int K) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t heap_addr = (uint32_t)__cvta_generic_to_shared(sh.heap);
+    const float* const buf = reinterpret_cast<const float*>(sh.ring);
+    if (lane == 0) make_heap(sh.heap, K);
+    for (long long base = K; base < V; base += kFeed) {
+        named_sync(7, kThreads);
+        named_sync(7, kThreads);
+        for (int at = 0; at < kFeed; at += 8 * 32) {
+            float w[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) w[u] = buf[at + 32 * u + lane];
+            // the first element after the last one that entered, of those the root lets in now
+            for (int last = -1;;) {
+                const float root = sh.heap[0].v;
+                int first = 8 * 32;
+#pragma unroll
+                for (int u = 7; u >= 0; --u)
+                    if (w[u] > root && 32 * u + lane > last) first = 32 * u + lane;   // (nothing is greater than NaN, nor NaN than anything)
+                first = __reduce_min_sync(0xffffffffu, first);
+                if (first == 8 * 32) break;
+                if (lane == 0) replace_min_shared(heap_addr, K, buf[at + first], (int)(base + at + first));
+                __syncwarp();
+                last = first;
+            }
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
@@ -1000,7 +1053,10 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
         // NaN among the first K: the heap's comparisons are then those of no order, and the elements are taken one by one
         const bool nan_heap = __syncthreads_or(nan_here) != 0;
         if (warp > 0) {
-            if (nan_heap) return;
+            if (nan_heap) {
+                feed_unordered(sh, row, V, K);
+                return;
+            }
             produce_candidates(sh, K, V, start, rounds, x, xn, load_round, a.wait_polls, ptid, pwarp, lane);
             return;
         }
@@ -1023,15 +1079,7 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
         const Cand* kept = sh.heap;
         TopKDist dist;
         if (nan_heap) {
-            if (lane == 0) make_heap(sh.heap, K);
-            __syncwarp();
-            for (long long base = K; base < V; base += 8 * 32) {
-                float v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) { const long long i = base + 32 * u + 31 - lane; v[u] = i < V ? row[i] : CUDART_NAN_F; }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) take_shared(v[u], (int)(base + 32 * u + 31 - lane), true);
-            }
+            replay_unordered(sh, V, K);
             if (lane == 0) dist = build_top_k_dist(sh.heap, sh.prob, K, p);
         } else {
             make_heap_warp(sh.heap, K, lane);
