@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(256) write_kv_kernel(KernelArgs a) {
 // with c = lut[row][j], s = lut[row][D/2 + j].  EL = 8: the three divisions of a token's new scale and
 // zero-point (every lane of the token computes them) are spread over sixteen elements per lane.
 // One CTA per rotated block, 256 / LPT of its (kv head, token) units at a time; a pass's loads are issued before the pass
-// before it is worked on.  Bound by instruction issue (76 % of the slots, 350 instructions per warp and pass): 6200 blocks of
+// before it is worked on.  Bound by instruction issue (81 % of the slots, 332 instructions per warp and pass): 6200 blocks of
 // 4 heads x 32 tokens (u8) 115 us, 95 without conversion instructions (quant_bits), 78 with the loads ahead, shifts for the
 // divisions by the block size and three-way minima; the keys' bytes, once in and once out, take 33.
 __device__ __forceinline__ float min3(float a, float b, float c) {
@@ -597,9 +597,10 @@ cudaError_t launch_write_kv(const KernelArgs& a, cudaStream_t stream, bool with_
     // block of its own, are better off with a warp per row: their u8 value bytes are scattered one by one, 4096 of them by one CTA
     // instead of four.  The line lies where the chunks' gain pays for that (us, warp per row | groups; a 600-token chunk is "600"):
     // u8, 8 kv heads x 128: 2048 18.5 | 10.2, 512 8.4 | 6.2, 250 decode + 1100 16.5 | 12.4, 1000 + 1010 20.6 | 18.6, but 500 + 520
-    // 12.4 | 12.8 and 128 + 130 6.6 | 8.3; 4 x 64: 64 + 4 x 256 8.3 | 7.3, but 256 + 280 6.3 | 8.3 and 120 + 2 x 300 6.3 | 7.3.  f32 activations, which every cache type converts, lie the same way (f16 cache, 8 x 128: 250 + 1100 8.3 | 6.3,
-    // 128 + 130 4.5 | 5.3).  16-bit activations into 16-bit caches gain from 2048 rows on, decode rows or not (bf16, 8 x 128:
-    // 128 + 130 4.9 | 4.5, 1000 + 1010 10.4 | 6.3).
+    // 12.4 | 12.8 and 128 + 130 6.6 | 8.3; 4 x 64: 64 + 4 x 256 8.3 | 7.3, but 256 + 280 6.3 | 8.3 and 120 + 2 x 300 6.3 | 7.3.  f32 activations,
+    // which every cache type converts, lie the same way (f16 cache, 8 x 128: 250 + 1100 8.3 | 6.3, 128 + 130 4.5 | 5.3).  16-bit
+    // activations into 16-bit caches gain from 2048 rows on, decode rows or not (bf16, 8 x 128: 128 + 130 4.9 | 4.5, 1000 + 1010
+    // 10.4 | 6.3).
     // The groups' wider loads and stores need activations and caches on 16-byte boundaries.
     const long long chunk_rows = std::max(0LL, (long long)a.num_tokens - a.num_sequences) * a.g.Hkv, decode_rows = (long long)a.num_sequences * a.g.Hkv;
     const bool light = a.g.cache != PA_DTYPE_U8 && a.g.act != PA_DTYPE_F32;

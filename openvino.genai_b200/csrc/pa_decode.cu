@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, (HI || PA_DECODE_STAGES > 2
                     else return 16 * (e / 4) + 2 * c + (e & 1) + 8 * ((e >> 1) & 1);
                 };
                 // The type is looked at once, around all loads, and neighbours come in pairs (e and e + 1 are neighbours for
-                // even e): with the branch around each load a row came one element behind the other, 13 us per run.
+                // even e): with the branch around each load a row came one element behind the other and a run's start took 13 us, most of it this.
 #pragma unroll
                 for (int e = 0; e < D / 4; ++e) q[e] = 0.f;
                 if (live && !q_pairs) {

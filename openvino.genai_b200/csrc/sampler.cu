@@ -11,13 +11,14 @@
 //      warp 0 replays libstdc++'s pop_heap / push_heap on the few hundred that really enter, with
 //      the heap spread over its registers (K <= 64) or by one lane over shared memory.  Softmax,
 //      min-p, top-p and the draw then run over <= K elements in the same warp, in the reference's
-//      order of operations.  256 rows x 151936, K 50: 289 -> 78 us (the serial replay, about 400
-//      replacements of 250 cycles with two rows per SM, is what a row waits for; reading the rows
-//      takes 24 us); 5 rows x 32000: 209 -> 43 us;
+//      order of operations.  A step (both launches, no penalties, logits in place) of 256 rows x
+//      151936, K 50: 301 -> 91 us (the serial replay, about 400 replacements of 250 cycles with two
+//      rows per SM, is what a row waits for; reading the rows takes 24 us); 5 rows x 32000: 215 -> 50 us;
 //   4. multinomial rows over the full vocabulary get their penalties here and are finished by
 //      sampler_exact_kernel (sampler_exact.cu), which reproduces the reference's index-order and
 //      sorted-order float sums exactly.
-// HBM-bound: the row is read once.
+// Greedy rows are bound by reading the row once (HBM from some 100 rows on, latency below); top-k rows by the serial replay;
+// what the whole-vocabulary rows wait for is said in sampler_exact.cu.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
@@ -743,8 +744,10 @@ __device__ __forceinline__ void store_release(int* p, int v) {
 // the K-th largest of the threads' own maxima so far (K distinct elements of the prefix; taken after every round whose
 // number is a power of two), whichever is larger; so the filter does not wait for the replay, only for room.  The first
 // round is filtered in three parts of 60, 180 and 240 threads with a bound after each: 4 k candidates of a 150 k row
-// became about 1 k, 400 of which enter.  One barrier among the producers per step: passing it, all entries of the steps
-// before are written, and the count is published.
+// became about 1 k, 400 of which enter.  A part with T threads bounds heaps of up to T entries (its K-th largest maximum
+// exists): 60 threads serve the usual K of 20 to 50 after their 480 elements, which all pass; heaps of 61 to 240 entries
+// take their first bound from the second part, larger ones from the third.  One barrier among the producers per step: passing
+// it, all entries of the steps before are written, and the count is published.
 template <class Load>
 __device__ __forceinline__ void produce_candidates(Shared& sh, int K, long long V, long long start, int rounds, float (&x)[kPerThread],
                                                    float (&xn)[kPerThread], Load&& load_round, int wait_polls, int ptid, int pwarp, int lane) {
@@ -862,8 +865,7 @@ __device__ __forceinline__ bool consume_candidates(Shared& sh, int wait_polls, i
 // A heap with NaN among its first K elements: the comparisons are those of no order, its root may fall as well as rise, and no
 // bound holds.  Warps 1..15 bring the row into the ring's place, kFeed elements at a time, the next ones in flight while warp 0
 // takes them one by one.  64 rows x 151936, K 50: 312 us; 473 with warp 0 reading the row by itself, 278 through a filter with
-// bounds.
-// Out of line: these registers are not the filter's.
+// bounds.  Out of line: these registers are not the filter's.
 constexpr int kFeedLoads = 16, kFeed = kFeedLoads * kProducerThreads;
 static_assert(kRing * sizeof(Cand) >= kFeed * sizeof(float), "the elements take the ring's place");
 __device__ __noinline__ void feed_unordered(Shared& sh, const float* row, long long V, int K) {
