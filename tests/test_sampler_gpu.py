@@ -188,6 +188,29 @@ def test_waits_of_the_top_k_path_end_with_progress_not_with_time(gpu, monkeypatc
     assert rc == 0 and np.array_equal(tok, tok_o)
 
 
+@pytest.mark.parametrize("rest", [1, 255, 256, 257, 7679, 7680, 7681, 15360, 15373])
+@pytest.mark.parametrize("top_k", [5, 50, 200])
+def test_top_k_rows_with_nan_in_the_first_elements(gpu, top_k, rest):
+    """A heap without an order: the elements after the first K come in portions of 7680 and are looked at 256 at a time.  NaN at
+    several places (with one at the root nothing enters), random, ascending and descending rows, NaN and -inf among the rest."""
+    rng = np.random.default_rng(top_k * 100003 + rest)
+    v = top_k + rest
+    x = (rng.standard_normal((8, v)) * 3).astype(np.float32)
+    for r, at in enumerate((0, 1, 2, top_k - 1, top_k // 2, 0, 3, 4)):
+        if r in (4, 5):
+            x[r] = np.sort(x[r])
+        if r == 6:
+            x[r] = np.sort(x[r])[::-1]
+        x[r, at] = np.nan
+    x[7, rng.random(v) < 0.3] = np.nan
+    x[7, rng.random(v) < 0.3] = -np.inf
+    x[7, top_k - 1] = np.nan
+    rows = H.make_rows(8, top_k=top_k, temperature=0.8, seeds=np.arange(8) + 13 * top_k)
+    tok_o, lp_o, _, tok_g, lp_g, _ = _both(gpu, x, rows)
+    assert np.array_equal(tok_o, tok_g), (tok_o, tok_g)
+    assert np.allclose(lp_o, lp_g, atol=2e-6, rtol=1e-6, equal_nan=True)
+
+
 def test_small_vocab_and_k_not_below_vocab(gpu):
     rng = np.random.default_rng(9)
     x = (rng.standard_normal((5, 40)) * 2).astype(np.float32)
