@@ -215,8 +215,9 @@ int run_forward(pa_handle* h, const pa_forward_args* a, cudaStream_t stream) {
     if (rc != PA_OK) return rc;
     pa::KernelArgs k = make_kernel_args(h, a, p);
     k.test_drop_copy = h->test_drop_copy ? 1 : 0;
-    // SM-shared kernel while a CTA's slice fits a few of its chapters (four unless the environment says otherwise); longer slices go to the warp-per-slice kernel, whose
-    // fixed slices cost nothing per chapter and balance well when every warp has hundreds of tiles
+    // SM-shared kernel while a CTA's slice fits a few of its chapters (four unless the environment says otherwise); longer slices
+    // go to the warp-per-slice kernel, whose fixed slices cost nothing per chapter and balance well when every warp has hundreds of
+    // tiles
     const bool shared_decode = pa::decode_shared_supported(h->g) && k.max_tiles <= (long long)h->sm_count * pa::decode_shared_chapter_tiles(h->g) * pa::decode_shared_max_chapters();
     if (shared_decode) {   // one CTA per SM is the worker; its warps share the slice
         k.decode_phantom = pa::decode_shared_phantom();
