@@ -327,6 +327,32 @@ static void test_sampler_gpu(const char* oracle_lib) {
     CHECK(want.ids[4].size() <= 7 && want.ids[4].size() >= 3);
 }
 
+// A top-k row whose wait inside the kernel runs out (a descending row: no candidates after its first round, and a limit of no polls)
+// ends the step with an exception on both entry points, and no token -1 reaches the request.
+static void test_sampler_reports_waits_that_ran_out() {
+    const int64_t vocab = 151936;
+    GenerationConfig c;
+    c.max_new_tokens = 4; c.do_sample = true; c.top_k = 20; c.temperature = 0.8f; c.rng_seed = 3;
+    std::vector<float> logits(vocab);
+    for (int64_t i = 0; i < vocab; ++i) logits[i] = 1.f - 2.f * (float)i / (float)vocab;
+    setenv("SAMPLER_B200_TEST_WAIT_POLLS", "0", 1);
+    Sampler impatient(0);
+    unsetenv("SAMPLER_B200_TEST_WAIT_POLLS");
+    float* dev = nullptr;
+    if (cudaMalloc(&dev, vocab * 4) != cudaSuccess) { CHECK(false); return; }
+    cudaMemcpy(dev, logits.data(), vocab * 4, cudaMemcpyHostToDevice);
+    SequenceGroup g = make_group(7, c, {1, 2, 3}, 0), h = make_group(8, c, {1, 2, 3}, 0), k = make_group(9, c, {1, 2, 3}, 0);
+    std::vector<SequenceGroup*> pg{&g}, ph{&h}, pk{&k};
+    CHECK(throws([&] { impatient.sample_device(pg, dev, 1, vocab, nullptr); }));
+    CHECK(g.generated_ids.empty());
+    CHECK(throws([&] { impatient.sample(ph, logits.data(), 1, vocab); }));
+    CHECK(h.generated_ids.empty());
+    Sampler patient(0);
+    patient.sample_device(pk, dev, 1, vocab, nullptr);
+    CHECK(k.generated_ids.size() == 1 && k.generated_ids[0] >= 0 && k.generated_ids[0] < 20);
+    cudaFree(dev);
+}
+
 int main(int argc, char** argv) {
     if (argc < 3) { std::printf("usage: host_layer_test cpu <rotation fixture> | gpu <oracle library>\n"); return 2; }
     const std::string mode = argv[1];
@@ -339,6 +365,7 @@ int main(int argc, char** argv) {
             test_sampler_pack();
             std::printf("pack: %d checks, %d failed\n", g_checks, g_failed);
             test_sampler_gpu(argv[2]);
+            test_sampler_reports_waits_that_ran_out();
         } else {
             return 2;
         }
