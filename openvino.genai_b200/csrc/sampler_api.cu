@@ -37,9 +37,9 @@ struct sampler_handle {
     uint8_t* stage_dev = nullptr;
     uint8_t* stage_host = nullptr;  // pinned
     size_t stage_bytes = 0;
-    float* exact_scratch = nullptr;   // one row of probabilities per CTA of the full-vocabulary kernel
+    float* exact_scratch = nullptr;   // two rows per CTA of the full-vocabulary kernel
     size_t exact_bytes = 0;
-    int exact_ctas = 0;               // persistent grid of that kernel: two CTAs per SM
+    int exact_ctas = 0;               // persistent grid of that kernel: one CTA per SM
     int64_t launches = 0;
     int wait_polls = sampler::kSamplerWaitPolls;   // env SAMPLER_B200_TEST_WAIT_POLLS: a limit that the bounded waits of the top-k path reach
 };
@@ -150,7 +150,7 @@ int sampler_b200_create(int device, int32_t max_rows, int64_t max_vocab, sampler
         return sfail(SAMPLER_ERR_CUDA, std::string("sampler_b200_create: ") + cudaGetErrorString(e));
     }
     if (const char* polls = std::getenv("SAMPLER_B200_TEST_WAIT_POLLS")) h->wait_polls = std::max(0, std::atoi(polls));
-    h->exact_ctas = 2 * prop.multiProcessorCount;
+    h->exact_ctas = prop.multiProcessorCount;
     if (max_rows > 0 && max_vocab > 0) {   // otherwise sized on first use
         const int rc = ensure_exact_scratch(h, max_rows, max_vocab);
         if (rc != SAMPLER_OK) { sampler_b200_destroy(h); return rc; }

@@ -6,17 +6,31 @@
 //   TopPFilter                  logit_transformers.hpp:94-139    (sort descending, add until the float sum > top_p)
 //   Sampler::_multinomial_sample  src/cpp/src/sampling/sampler.cpp:1036-1089
 //       total = sum of the kept probabilities in their order, r = total * u, first running sum > r
-// Every float the reference produces on the way is reproduced: expf with the host libm's bits and
-// the sequential sums through the step algebra of fsum_exact.cuh, so token ids agree with the
+// Every float the reference produces on the way is reproduced: expf with the host libm's bits and the
+// sequential float sums through the step algebra of fsum_exact.cuh, so token ids agree with the
 // reference except where several kept elements have exactly the same probability and the draw falls
-// among them (their relative order after std::sort is not defined; the lowest index is taken here).
+// among them (their relative order after std::sort is not defined; the lowest index comes first here).
 //
-// One CTA works on one row at a time (persistent grid, rows dealt round robin).  Passes over a row:
-//   1. maximum;  2. expf and the index-order sum (tile by tile, a block scan of steps per tile), the
-//   exponentials parked in a per-CTA scratch row;  3. division by the sum, probabilities back to the
-//   scratch row, and either the index-order total (no top-p) or the first level's bin counts;
-//   then, without top-p, one more partial pass that stops at the drawn element; with top-p the
-//   walk of fsum_exact.cuh: a few passes that sum whole bins as translations and list the rest.
+// One CTA of 1024 threads per SM works on one row at a time:
+//   1. maximum;
+//   2. exponentials into a scratch row, with the mass of every 256 elements and, for top-p, the counts of 2048 bins of their
+//      bit patterns (128 per binade);
+//   3. the index-order sum of the exponentials (ordered_sum);
+//   4. without top-p the same for the probabilities, the exact sum before every 256 elements kept for the draws;
+//      with top-p the elements of the highest bins are brought into shared memory bin by bin (one atomic gives a place)
+//      and ordered_sum runs over them in segments of whole bins until the sum exceeds top_p;
+//   5. a draw looks its segment up in the recorded sums and adds that segment's elements one by one.
+//
+// ordered_sum: while a float sum s stays in one binade, adding x to it is adding a whole number of ulps that depends on s
+// through its parity only, and not even on that unless x lies half-way between two.  So a lane adds its eight elements with
+// real float additions to the two sums 2^e and 2^e + ulp, which gives its amounts for an even and an odd s for two
+// additions per element; without a half-way case the amounts of a segment add up as integers in any order - the
+// elements of a bin need not be sorted -, with one the segment is sorted and its lanes' amounts are composed in order.  The
+// binade of every segment is guessed from the masses and checked by the walk of one warp over the segments; those in
+// which the sum changes binade, or whose guess was wrong, are added one by one.
+//
+// What it replaced: one thread walked the bins and lists of sorted elements (most of the 400 - 500 k cycles of a top-p row's
+// sorted part), and the CTA rescanned spans with half-way cases (100 k of the index-order sum).
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
@@ -28,29 +42,1386 @@
 
 namespace sampler {
 
-// Two CTA sizes: 512 threads with two CTAs per SM while there are more rows than SMs (two rows share an SM and fill each
-// other's sequential phases), 1024 threads with one CTA per SM for small batches (a row's passes take about half as long).
 namespace {
-namespace sx512 {
-#define SX_THREADS 512
-#define SX_CTAS_PER_SM 2
-#include "sampler_exact_impl.cuh"
-#undef SX_THREADS
-#undef SX_CTAS_PER_SM
-}  // namespace sx512
-namespace sx1024 {
-#define SX_THREADS 1024
-#define SX_CTAS_PER_SM 1
-#include "sampler_exact_impl.cuh"
-#undef SX_THREADS
-#undef SX_CTAS_PER_SM
-}  // namespace sx1024
+
+constexpr int kThreads = 1024;
+constexpr int kWarps = kThreads / 32;
+constexpr int kBlock = 256;           // consecutive elements a warp takes at a time, eight per lane
+constexpr int kMaxSegs = 640;         // segments of a row in index order; longer rows have segments of several blocks
+constexpr int kBigSegs = 4;           // a bin of so many segments' elements is a segment by itself
+constexpr int kSegCap = kMaxSegs + 2 * kMaxSegs / kBigSegs + 192;   // in descending order: those, two boundaries per such bin, some per level
+constexpr int kBins = 2048;
+constexpr int kBinsPerThread = kBins / kThreads;
+constexpr int kTopShift = 16;         // first level: 2^16 bit patterns per bin, 128 bins per binade, 16 binades
+constexpr int kFinerBy = 5;           // bits a level is cut finer by where a bin is too full to be sorted
+constexpr int kCap = 47104;           // elements of a chunk in shared memory
+constexpr int kSlots = 32;            // segments with the amounts of their lanes at hand, for those in which the sum may change binade
+constexpr int kMaxMisses = 24;        // segments added one by one before the guesses of those behind are made anew
+constexpr float kMargin = 1.0f / 1024, kDrawMargin = 1.0f / 256;   // around the sums at which a segment is sorted ahead
+constexpr uint32_t kOneBits = 0x3f800000u;
+constexpr uint32_t kNoGuess = 0, kEmpty = 255;
+
+// -DSAMPLER_EXACT_PROF: cycles per part of a row, printed by some of the CTAs
+enum { kProfMax, kProfExp, kProfGuess, kProfSteps, kProfWalk, kProfMisses, kProfRank, kProfGather, kProfSame, kProfPlace, kProfMass, kProfFind, kProfIndex, kProfIndex2, kProfOther, kProfTile, kProfTiles, kProfSlot, kProfSlots, kProfSerial, kProfN };
+#ifdef SAMPLER_EXACT_PROF
+#define PROF_BEGIN long long prof_t0 = clock64()
+#define PROF_END(slot) do { if (threadIdx.x == 0) sh.prof[slot] += clock64() - prof_t0; prof_t0 = clock64(); } while (0)
+#define PROF_COUNT(slot) do { if (threadIdx.x == 0) ++sh.prof[slot]; } while (0)
+#else
+#define PROF_BEGIN
+#define PROF_END(slot)
+#define PROF_COUNT(slot)
+#endif
+
+struct ExactShared {
+    alignas(16) float keys[kCap];        // a chunk's probabilities, bin by bin
+    alignas(16) uint32_t bins[kBins];    // counts, then the rank of a bin's first element in its level, then (taken bins) of its end
+    uint32_t start[kSegCap + 1];         // first element of a segment; the next one's start is its end
+    float cum[kSegCap + 1];              // approximate sum before a segment
+    float state[kSegCap];                // exact sum before a segment
+    uint32_t step[kSegCap];              // amounts of a segment's elements for an even and an odd sum (pack_amounts)
+    uint8_t E[kSegCap];                  // binade the sum is taken to lie in
+    uint8_t sorted[kSegCap];             // 1: the elements are in descending order, 2: they are to be brought into it
+    uint8_t slot[kSegCap];               // 1 + its place in `upto` and `from`; 0: none
+    uint16_t bin[kSegCap + 1];           // the segment's first bin
+    uint32_t upto[kSlots][32];           // amounts of the segment's lanes up to this one under E (pack_amounts)
+    uint32_t from[kSlots][32];           // ... from this one on under E + 1
+    int slots;
+    alignas(16) float serial[kBlock];    // elements the walking warp adds one by one
+    uint32_t queue[kWarps];              // rows of this CTA among the kThreads rows looked at, a bit each
+    int stop;                            // first segment of a chunk that is too large to be sorted
+    int count;
+    uint32_t scan_u[kWarps];
+    float scan_f[kWarps];
+    int red_i[kWarps];
+    // results of the walking warp
+    float bc_s;
+    int bc_seg;
+    long long bc_hit;
+    float bc_p;
+#ifdef SAMPLER_EXACT_PROF
+    long long prof[kProfN];
+#endif
+};
+static_assert(sizeof(ExactShared) <= 232448, "shared memory of a CTA");
+extern __shared__ __align__(16) uint8_t sx_smem[];
+// (by its name and not by an argument: the compiler then knows that it is shared memory)
+__device__ __forceinline__ ExactShared& shared_memory() { return *reinterpret_cast<ExactShared*>(sx_smem); }
+
+// ---- reductions and scans over the CTA ------------------------------------------------------------------
+template <class T, class Op>
+__device__ T block_reduce(T v, Op op, T* buf) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncthreads();
+    if (lane == 0) buf[w] = v;
+    __syncthreads();
+    v = buf[lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+template <class T>
+__device__ T block_sum(T v, T* buf) { return block_reduce(v, [](T a, T b) { return a + b; }, buf); }
+
+// combination of the earlier threads' values (of the identity T(0) for the first); *total: of all
+template <class T, class Op>
+__device__ T block_scan_exclusive(T v, T* buf, T* total, Op op) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    T incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl = op(up, incl);
+    }
+    __syncthreads();
+    if (lane == 31) buf[w] = incl;
+    __syncthreads();
+    T t = buf[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T up = __shfl_up_sync(0xffffffffu, t, o);
+        if (lane >= o) t = op(up, t);
+    }
+    if (total) *total = __shfl_sync(0xffffffffu, t, 31);
+    const T before = __shfl_sync(0xffffffffu, t, w > 0 ? w - 1 : 0);
+    const T own = __shfl_up_sync(0xffffffffu, incl, 1);
+    return op(w > 0 ? before : T(0), lane > 0 ? own : T(0));
+}
+template <class T>
+__device__ T block_scan_exclusive(T v, T* buf, T* total) { return block_scan_exclusive(v, buf, total, [](T a, T b) { return a + b; }); }
+
+// ---- sums in a fixed order ---------------------------------------------------------------------------------
+struct Segs {
+    int shift;   // 2^shift elements per segment, kBlock at least
+    int count;   // segments of the row in index order
+    __device__ uint32_t len() const { return 1u << shift; }
+};
+__device__ __forceinline__ Segs segments_of(long long V) {
+    int shift = 8;
+    while (((V - 1) >> shift) >= kMaxSegs) ++shift;
+    return Segs{shift, (int)((V + (1ll << shift) - 1) >> shift)};
+}
+
+// Eight elements from i on (a multiple of eight), those outside lo .. hi - 1 as zero, which leaves a sum as it is.
+__device__ __forceinline__ void load8(const float* v, uint32_t i, uint32_t lo, uint32_t hi, float (&x)[8]) {
+    if (i >= lo && i + 8 <= hi) {
+        const float4 a = *reinterpret_cast<const float4*>(v + i), b = *reinterpret_cast<const float4*>(v + i + 4);
+        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+        x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = i + e >= lo && i + e < hi ? v[i + e] : 0.f;
+    }
+}
+
+// The probability of an exponential (norm > 0): logit_transformers.hpp:357-359
+__device__ __forceinline__ float probability(float e, float norm, float inv_norm) { return e == 0.f ? 0.f : fsx::div_shared(e, norm, inv_norm); }
+
+// What is added: element `i` of the row is v[i - off]; elements that are not in the sum count as zero.
+struct Exponentials {
+    const float* v;
+    uint32_t off;
+    static constexpr bool kSortable = false;
+    __device__ __forceinline__ const float* data() const { return v; }
+    __device__ __forceinline__ void prepare(float (&x)[8]) const {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = fmaxf(x[e], 0.f);   // NaN: not in the sum
+    }
+};
+struct Probabilities {
+    const float* v;
+    uint32_t off;
+    float norm, inv_norm, min_thr;
+    static constexpr bool kSortable = false;
+    __device__ __forceinline__ const float* data() const { return v; }
+    __device__ __forceinline__ void prepare(float (&x)[8]) const {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float p = probability(x[e], norm, inv_norm);
+            x[e] = p >= min_thr ? p : 0.f;
+        }
+    }
+};
+struct Chunk {   // probabilities in shared memory (keys), and the row that they also are in
+    uint32_t off;
+    float* out;
+    static constexpr bool kSortable = true;
+    __device__ __forceinline__ const float* data() const { return shared_memory().keys; }
+    __device__ __forceinline__ void prepare(float (&)[8]) const {}
+};
+struct Sorted {
+    const float* v;
+    uint32_t off;
+    static constexpr bool kSortable = false;
+    __device__ __forceinline__ const float* data() const { return v; }
+    __device__ __forceinline__ void prepare(float (&)[8]) const {}
+};
+
+// Masses in cum[0 .. n - 1] -> sums before the segments.
+__device__ void masses_to_sums(int n) {
+    ExactShared& sh = shared_memory();
+    constexpr int kPer = (kMaxSegs + kThreads - 1) / kThreads;
+    const int j0 = (int)threadIdx.x * kPer;
+    __syncthreads();
+    float m[kPer], sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        m[k] = j0 + k < n ? sh.cum[j0 + k] : 0.f;
+        sum += m[k];
+    }
+    float all, before = block_scan_exclusive(sum, sh.scan_f, &all);
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        if (j0 + k < n) sh.cum[j0 + k] = before;
+        before += m[k];
+    }
+    if (threadIdx.x == 0) sh.cum[n] = all;
+    __syncthreads();
+}
+
+// Sorts a[0 .. n) in descending order (one warp; no value is negative): bitonic merges in the form whose comparators all point the
+// same way.  Up to 512 values lie in registers, sixteen consecutive ones per lane; longer segments are sorted in place, entries
+// beyond n left out.
+__device__ __forceinline__ void order(float& x, float& y) {
+    const float a = x, b = y;
+    x = fmaxf(a, b);
+    y = fminf(a, b);
+}
+__device__ __noinline__ void sort_segment(float* a, int n) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    if (n <= 512) {
+        float v[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) v[r] = 16 * lane + r < n ? a[16 * lane + r] : -1.f;
+#pragma unroll
+        for (int k = 1; k <= 4; ++k) {   // within a lane
+#pragma unroll
+            for (int r = 0; r < 16; ++r)
+                if ((r ^ ((1 << k) - 1)) > r) order(v[r], v[r ^ ((1 << k) - 1)]);
+#pragma unroll
+            for (int j = k - 2; j >= 0; --j)
+#pragma unroll
+                for (int r = 0; r < 16; ++r)
+                    if ((r ^ (1 << j)) > r) order(v[r], v[r ^ (1 << j)]);
+        }
+#pragma unroll 1
+        for (int k = 5; k <= 9; ++k) {
+            const int mask = (1 << (k - 4)) - 1;
+            bool upper = (lane >> (k - 5)) & 1;
+            float w[16];
+#pragma unroll
+            for (int r = 0; r < 16; ++r) w[r] = __shfl_xor_sync(0xffffffffu, v[15 - r], mask);
+#pragma unroll
+            for (int r = 0; r < 16; ++r) v[r] = upper ? fminf(v[r], w[r]) : fmaxf(v[r], w[r]);
+#pragma unroll 1
+            for (int j = k - 6; j >= 0; --j) {
+                upper = (lane >> j) & 1;
+#pragma unroll
+                for (int r = 0; r < 16; ++r) {
+                    const float u = __shfl_xor_sync(0xffffffffu, v[r], 1 << j);
+                    v[r] = upper ? fminf(v[r], u) : fmaxf(v[r], u);
+                }
+            }
+#pragma unroll
+            for (int j = 3; j >= 0; --j)
+#pragma unroll
+                for (int r = 0; r < 16; ++r)
+                    if ((r ^ (1 << j)) > r) order(v[r], v[r ^ (1 << j)]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 16; ++r)
+            if (16 * lane + r < n) a[16 * lane + r] = v[r];
+        __syncwarp();
+        return;
+    }
+    int bits = 1;
+    while ((1 << bits) < n) ++bits;
+    const int half = 1 << (bits - 1);
+    auto exchange = [&](int i, int l) {
+        if (l >= n) return;
+        const float x = a[i], y = a[l];
+        if (x < y) { a[i] = y; a[l] = x; }
+    };
+    for (int k = 1; k <= bits; ++k) {
+        for (int t = lane; t < half; t += 32) {
+            const int block = (t >> (k - 1)) << k, at = t & ((1 << (k - 1)) - 1);
+            exchange(block + at, block + (1 << k) - 1 - at);
+        }
+        __syncwarp();
+        for (int j = k - 2; j >= 0; --j) {
+            for (int t = lane; t < half; t += 32) {
+                const int i = ((t >> j) << (j + 1)) + (t & ((1 << j) - 1));
+                exchange(i, i + (1 << j));
+            }
+            __syncwarp();
+        }
+    }
+}
+// Segment j of a chunk in shared memory, there and in the row in descending order (one warp).
+__device__ __forceinline__ void sort_in_chunk(Chunk src, int j) {
+    ExactShared& sh = shared_memory();
+    const int lane = threadIdx.x & 31;
+    const uint32_t lo = sh.start[j] - src.off, hi = sh.start[j + 1] - src.off;
+    sort_segment(sh.keys + lo, (int)(hi - lo));
+    for (uint32_t i = lo + lane; i < hi; i += 32) src.out[src.off + i] = sh.keys[i];
+    __syncwarp();
+    if (lane == 0) sh.sorted[j] = 1;
+    __syncwarp();
+}
+
+// Guesses the binade of the sum at the segments c .. c1 - 1 from the approximate sums and the exact one, s, before c.  Where the sum
+// may change binade the segment gets a slot.  Segments of unsorted elements in which the order will matter are marked:
+// those, and where the sum may pass one of two thresholds.
+__device__ void guess_binades(int c, int c1, float s, float thr, float thr2) {
+    ExactShared& sh = shared_memory();
+    __syncthreads();
+    if (threadIdx.x == 0) sh.slots = 0;
+    __syncthreads();
+    const float shift = s - sh.cum[c];
+    for (int j = c + (int)threadIdx.x; j < c1; j += kThreads) {
+        const float lo = j == c ? s : sh.cum[j] + shift, hi = sh.cum[j + 1] + shift;
+        const float l = lo * (1.f - kMargin), h = hi * (1.f + kMargin);
+        const uint32_t El = fsx::state_exp(l), Eh = fsx::state_exp(h);
+        uint32_t E = fsx::state_exp(lo);
+        uint8_t slot = 0;
+        const bool empty = sh.start[j] == sh.start[j + 1], usable = lo > 0.f && El >= 24u && Eh < 253u;
+        if (!empty && usable && Eh == El + 1u) {
+            const int at = atomicAdd(&sh.slots, 1);
+            if (at < kSlots) { slot = (uint8_t)(at + 1); E = El; }
+        }
+        sh.slot[j] = slot;
+        sh.E[j] = (uint8_t)(empty ? kEmpty : usable ? E : kNoGuess);
+        if (sh.sorted[j] == 0 && (j == 0 || El != Eh || (l <= thr && thr <= h) || (lo * (1.f - kDrawMargin) <= thr2 && thr2 <= hi * (1.f + kDrawMargin))))
+            sh.sorted[j] = 2;
+    }
+    __syncthreads();
+}
+
+// The amounts for an even and an odd sum differ by one at most: two neighbouring sums stay neighbours or meet.
+__device__ __forceinline__ uint32_t pack_amounts(fsx::Step st) { return st.a << 2 | (st.b - st.a + 1u); }
+__device__ __forceinline__ fsx::Step unpack_amounts(uint32_t w) { return fsx::Step{w >> 2, (w >> 2) + (w & 3u) - 1u}; }
+
+// The amounts of a warp's 256 elements under binade E; *tie: they depend on the order.
+__device__ __forceinline__ fsx::Step block_step(const float (&x)[8], uint32_t E, bool in_order, bool* tie) {
+    const uint32_t even = E << 23, odd = even + 1;
+    float s0 = __uint_as_float(even), s1 = __uint_as_float(odd);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        s0 = __fadd_rn(s0, x[e]);
+        s1 = __fadd_rn(s1, x[e]);
+    }
+    const uint32_t b0 = __float_as_uint(s0), b1 = __float_as_uint(s1);
+    fsx::Step st{b0 - even, b1 - odd};
+    if (b1 >= even + (1u << 23)) st = fsx::Step{fsx::kSat, fsx::kSat};   // the lane's own sum leaves the binade
+    *tie = __any_sync(0xffffffffu, st.a != st.b);
+    if (!*tie) {
+        st.a = st.b = min(__reduce_add_sync(0xffffffffu, st.a), fsx::kSat);   // 32 x kSat at most
+    } else if (in_order) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {   // lane 0: all lanes in order
+            const fsx::Step next{__shfl_down_sync(0xffffffffu, st.a, o), __shfl_down_sync(0xffffffffu, st.b, o)};
+            st = fsx::then(st, next);
+        }
+    }
+    return st;
+}
+
+// A segment with a slot: the amounts of its lanes, each of which takes m * 8 consecutive elements, under E up to every lane and under
+// E + 1 from every lane on.  Elements of rows in memory stay at hand in `keys`, which nothing else uses then (m = 1).
+template <class Src>
+__device__ __forceinline__ void lane_steps(Src src, int j) {
+    ExactShared& sh = shared_memory();
+    const int lane = threadIdx.x & 31, slot = sh.slot[j] - 1;
+    const uint32_t lo = sh.start[j] - src.off, hi = sh.start[j + 1] - src.off, lo8 = lo & ~7u, m = (hi - lo8 + kBlock - 1) / kBlock;
+    const uint32_t even = (uint32_t)sh.E[j] << 23, up = 1u << 23;
+    float s[4] = {__uint_as_float(even), __uint_as_float(even + 1), __uint_as_float(even + up), __uint_as_float(even + up + 1)};
+    for (uint32_t t = 0; t < m; ++t) {
+        float x[8];
+        load8(src.data(), lo8 + 8 * (lane * m + t), lo, hi, x);
+        src.prepare(x);
+        if (!Src::kSortable && m == 1) {
+            *reinterpret_cast<float4*>(sh.keys + slot * kBlock + 8 * lane) = make_float4(x[0], x[1], x[2], x[3]);
+            *reinterpret_cast<float4*>(sh.keys + slot * kBlock + 8 * lane + 4) = make_float4(x[4], x[5], x[6], x[7]);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s[k] = __fadd_rn(s[k], x[e]);
+    }
+    auto amounts = [&](int k, uint32_t base) {
+        const uint32_t b0 = __float_as_uint(s[k]), b1 = __float_as_uint(s[k + 1]);
+        return b1 >= base + up ? fsx::Step{fsx::kSat, fsx::kSat} : fsx::Step{b0 - base, b1 - base - 1};
+    };
+    fsx::Step p = amounts(0, even), q = amounts(2, even + up);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const fsx::Step pu{__shfl_up_sync(0xffffffffu, p.a, o), __shfl_up_sync(0xffffffffu, p.b, o)};
+        const fsx::Step qd{__shfl_down_sync(0xffffffffu, q.a, o), __shfl_down_sync(0xffffffffu, q.b, o)};
+        if (lane >= o) p = fsx::then(pu, p);
+        if (lane + o < 32) q = fsx::then(q, qd);
+    }
+    sh.upto[slot][lane] = pack_amounts(p);
+    sh.from[slot][lane] = pack_amounts(q);
+}
+
+// Amounts of the segments' elements under the guesses: rows in memory, a block of each of four segments at a time (a warp's loads are
+// what it waits for: one block at a time 23 k cycles for 152 k elements).
+template <class Src>
+__device__ __forceinline__ void segment_steps(Src src, int c, int c1) {
+    ExactShared& sh = shared_memory();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kAtOnce = 4;
+    for (int j = c + warp; j < c1; j += kAtOnce * kWarps) {
+        uint32_t lo[kAtOnce], hi[kAtOnce];
+        fsx::Step total[kAtOnce];
+        bool more = false;
+#pragma unroll
+        for (int u = 0; u < kAtOnce; ++u) {
+            const bool in = j + u * kWarps < c1;
+            lo[u] = in ? sh.start[j + u * kWarps] - src.off : 0u;
+            hi[u] = in ? sh.start[j + u * kWarps + 1] - src.off : 0u;
+            total[u] = fsx::step_identity();
+            more |= lo[u] < hi[u];
+        }
+        for (uint32_t at = 0; more; at += kBlock) {
+            float x[kAtOnce][8];
+            more = false;
+#pragma unroll
+            for (int u = 0; u < kAtOnce; ++u) {
+                const uint32_t i = (lo[u] & ~7u) + at;
+                load8(src.data(), i + 8 * lane, lo[u], hi[u], x[u]);
+                more |= i + kBlock < hi[u];
+            }
+#pragma unroll
+            for (int u = 0; u < kAtOnce; ++u) {
+                const uint32_t E = j + u * kWarps < c1 ? sh.E[j + u * kWarps] : kNoGuess;
+                if (E == kNoGuess || E == kEmpty) continue;
+                src.prepare(x[u]);
+                bool tie;
+                total[u] = fsx::then(total[u], block_step(x[u], E, true, &tie));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kAtOnce; ++u)
+            if (j + u * kWarps < c1) {
+                if (lane == 0) sh.step[j + u * kWarps] = pack_amounts(total[u]);
+                if (sh.slot[j + u * kWarps]) lane_steps(src, j + u * kWarps);
+            }
+    }
+    __syncthreads();
+}
+// A chunk in shared memory: a segment is sorted only where the order matters.
+__device__ void segment_steps(Chunk src, int c, int c1) {
+    ExactShared& sh = shared_memory();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int j = c + warp; j < c1; j += kWarps) {
+        const uint32_t E = sh.E[j];
+        if (sh.sorted[j] == 2) sort_in_chunk(src, j);
+        if (E == kNoGuess || E == kEmpty) continue;
+        if (sh.slot[j]) { lane_steps(src, j); continue; }   // (sorted now)
+        const uint32_t lo = sh.start[j] - src.off, hi = sh.start[j + 1] - src.off;
+        for (bool again = true; again;) {
+            const bool in_order = sh.sorted[j] == 1;
+            fsx::Step total = fsx::step_identity();
+            again = false;
+            for (uint32_t i = lo & ~7u; i < hi && !again; i += kBlock) {
+                float x[8];
+                load8(src.data(), i + 8 * lane, lo, hi, x);
+                bool tie;
+                total = fsx::then(total, block_step(x, E, in_order, &tie));
+                again = tie && !in_order;
+            }
+            if (again) sort_in_chunk(src, j);
+            else if (lane == 0) sh.step[j] = pack_amounts(total);
+        }
+    }
+    __syncthreads();
+}
+
+// Adds segment j to s element by element (one warp).  It stops at the first running sum above thr and returns that
+// element (its value in p), else -1.
+template <class Src>
+__device__ __forceinline__ long long add_segment(Src src, int j, float& s, float thr, float& p) {
+    ExactShared& sh = shared_memory();
+    const int lane = threadIdx.x & 31;
+    const uint32_t lo = sh.start[j] - src.off, hi = sh.start[j + 1] - src.off;
+    float4* buf = reinterpret_cast<float4*>(sh.serial);
+    for (uint32_t i = lo & ~7u; i < hi; i += kBlock) {
+        float x[8];
+        load8(src.data(), i + 8 * lane, lo, hi, x);
+        src.prepare(x);
+        __syncwarp();
+        buf[2 * lane] = make_float4(x[0], x[1], x[2], x[3]);
+        buf[2 * lane + 1] = make_float4(x[4], x[5], x[6], x[7]);
+        __syncwarp();
+        for (int q = 0; q < kBlock / 4; q += 4) {   // every lane adds the same
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = buf[q + u];
+            const float before = s;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                s = __fadd_rn(s, v[u].x);
+                s = __fadd_rn(s, v[u].y);
+                s = __fadd_rn(s, v[u].z);
+                s = __fadd_rn(s, v[u].w);
+            }
+            if (s > thr) {   // sums only grow: the end of the sixteen tells
+                s = before;
+                for (int e = 0; e < 16; ++e) {
+                    p = sh.serial[4 * q + e];
+                    s = __fadd_rn(s, p);
+                    if (s > thr) return (long long)src.off + i + 4 * q + e;
+                }
+            }
+        }
+    }
+    return -1;
+}
+
+// Walks the segments from c on (warp 0): whole ones while the guesses hold, one by one elsewhere.  Leaves the sum, the segment
+// it came to and the element whose running sum is the first above thr (-1: none) in shared memory.
+template <class Src>
+__device__ void walk_segments(Src src, int c, int c1, float s, float thr) {
+    ExactShared& sh = shared_memory();
+    const int lane = threadIdx.x & 31;
+    uint32_t E = fsx::state_exp(s), S = fsx::state_sig(s);
+    int misses = 0;
+    long long hit = -1;
+    PROF_BEGIN;
+    while (c < c1) {
+        PROF_END(kProfOther);
+        PROF_COUNT(kProfTiles);
+        const int n = min(32, c1 - c), my = c + lane;
+        fsx::Step st = fsx::step_identity();
+        bool good = true;
+        if (lane < n) {
+            const uint32_t Eg = sh.E[my];
+            good = Eg == kEmpty || (Eg == E && S >= 0x800000u && sh.slot[my] == 0);
+            if (!good) st = fsx::Step{fsx::kSat, fsx::kSat};
+            else if (Eg != kEmpty) st = unpack_amounts(sh.step[my]);
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const fsx::Step up{__shfl_up_sync(0xffffffffu, st.a, o), __shfl_up_sync(0xffffffffu, st.b, o)};
+            if (lane >= o) st = fsx::then(up, st);
+        }
+        const uint32_t after = fsx::apply(st, S);
+        const uint32_t up = __shfl_up_sync(0xffffffffu, after, 1);
+        const uint32_t before = lane > 0 ? up : S;
+        const bool bad = !good || after >= fsx::kOne24 || fsx::state_float(E, after) > thr;
+        const uint32_t mask = __ballot_sync(0xffffffffu, bad);
+        const int first = mask ? __ffs(mask) - 1 : 32;   // below n where any
+        if (lane < n && lane <= first) sh.state[my] = fsx::state_float(E, before);
+        if (first >= n) {
+            S = __shfl_sync(0xffffffffu, after, 31);   // (lanes from n on add nothing)
+            c += n;
+            PROF_END(kProfTile);
+            continue;
+        }
+        S = __shfl_sync(0xffffffffu, before, first);
+        c += first;
+        PROF_END(kProfTile);
+        if (sh.slot[c] && S >= 0x800000u) {   // the sum may change binade in this one: its lanes' amounts are at hand
+            const int slot = sh.slot[c] - 1;
+            const uint32_t Eg = sh.E[c];
+            uint32_t E2 = E, S2 = fsx::kOne24;
+            if (E == Eg + 1u) {
+                S2 = fsx::apply(unpack_amounts(sh.from[slot][0]), S);
+            } else if (E == Eg) {
+                const uint32_t upto = fsx::apply(unpack_amounts(sh.upto[slot][lane]), S);
+                const uint32_t over = __ballot_sync(0xffffffffu, upto >= fsx::kOne24);
+                if (!over) {
+                    S2 = __shfl_sync(0xffffffffu, upto, 31);
+                } else {
+                    const int l = __ffs(over) - 1;   // this lane's elements take it into the next binade
+                    const uint32_t below = __shfl_sync(0xffffffffu, upto, l > 0 ? l - 1 : 0);
+                    float t = fsx::state_float(E, l > 0 ? below : S);
+                    const uint32_t lo = sh.start[c] - src.off, hi = sh.start[c + 1] - src.off, lo8 = lo & ~7u, m = (hi - lo8 + kBlock - 1) / kBlock;
+                    for (uint32_t q = 0; q < m; ++q) {
+                        float x[8];
+                        if (!Src::kSortable && m == 1) {
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) x[e] = sh.keys[slot * kBlock + 8 * l + e];
+                        } else {
+                            load8(src.data(), lo8 + 8 * (l * m + q), lo, hi, x);
+                            src.prepare(x);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) t = __fadd_rn(t, x[e]);
+                    }
+                    E2 = fsx::state_exp(t);
+                    if (E2 == E + 1u && !(t > thr)) S2 = l < 31 ? fsx::apply(unpack_amounts(sh.from[slot][l < 31 ? l + 1 : 31]), fsx::state_sig(t)) : fsx::state_sig(t);
+                }
+            }
+            if (S2 < fsx::kOne24 && !(fsx::state_float(E2, S2) > thr)) {
+                E = E2; S = S2;
+                ++c;
+                PROF_END(kProfSlot);
+                PROF_COUNT(kProfSlots);
+                continue;
+            }
+        }
+        if (++misses > kMaxMisses && c1 - c > 32) break;
+        PROF_COUNT(kProfMisses);
+        if constexpr (Src::kSortable) {
+            if (sh.sorted[c] != 1) sort_in_chunk(src, c);
+        }
+        s = fsx::state_float(E, S);
+        float p;
+        hit = add_segment(src, c, s, thr, p);
+        E = fsx::state_exp(s); S = fsx::state_sig(s);
+        PROF_END(kProfSerial);
+        if (hit >= 0) break;
+        ++c;
+    }
+    if (lane == 0) { sh.bc_s = fsx::state_float(E, S); sh.bc_seg = c; sh.bc_hit = hit; }
+}
+
+// Adds the segments c .. c1 - 1 to s in order, exactly as `s += x[i]` does, from the approximate sums in sh.cum.  It stops at the
+// first running sum above thr and returns that element, else -1.  sh.state: the sum before every segment it came to.
+template <class Src>
+__device__ __noinline__ long long ordered_sum(Src src, int c, int c1, float& s, float thr, float thr2) {
+    ExactShared& sh = shared_memory();
+    PROF_BEGIN;
+    for (;;) {
+        guess_binades(c, c1, s, thr, thr2);
+        PROF_END(kProfGuess);
+        segment_steps(src, c, c1);
+        PROF_END(kProfSteps);
+        if (threadIdx.x < 32) walk_segments(src, c, c1, s, thr);
+        __syncthreads();
+        PROF_END(kProfWalk);
+        s = sh.bc_s; c = sh.bc_seg;
+        const long long hit = sh.bc_hit;
+        __syncthreads();
+        if (hit >= 0 || c >= c1) return hit;
+    }
+}
+// The same over a whole row in index order, from the approximate sums before its segments.
+template <class Src>
+__device__ __noinline__ float index_order_sum(Src src, Segs g, uint32_t V) {
+    ExactShared& sh = shared_memory();
+    for (int j = threadIdx.x; j <= g.count; j += kThreads) {
+        sh.start[j] = min(V, (uint32_t)j << g.shift);
+        if (j < g.count) sh.sorted[j] = 1;
+    }
+    float s = 0.f;
+    ordered_sum(src, 0, g.count, s, CUDART_INF_F, -1.f);
+    return s;
+}
+
+// ---- descending order --------------------------------------------------------------------------------------
+// Keys are the bit patterns of the exponentials.  A level cuts the keys below F into bins of 2^shift, highest first; what lies
+// below the last bin is the level's rest.
+struct Level {
+    uint32_t F;
+    int shift;
+    uint32_t total;   // elements in its bins
+    bool rest;
+};
+__device__ __forceinline__ uint32_t bin_of(const Level& L, uint32_t key) { return (L.F - 1u - key) >> L.shift; }
+
+// Adds one to a word of shared memory where x < end, without a branch; take_below returns what was there, put_below stores.
+__device__ __forceinline__ void count_below(uint32_t addr, uint32_t x, uint32_t end) {
+    asm volatile("{ .reg .pred p; setp.lt.u32 p, %1, %2; @p red.shared.add.u32 [%0], 1; }" ::"r"(addr), "r"(x), "r"(end) : "memory");
+}
+__device__ __forceinline__ uint32_t take_below(uint32_t addr, uint32_t x, uint32_t end) {
+    uint32_t old = 0;
+    asm volatile("{ .reg .pred p; setp.lt.u32 p, %2, %3; @p atom.shared.add.u32 %0, [%1], 1; }" : "+r"(old) : "r"(addr), "r"(x), "r"(end) : "memory");
+    return old;
+}
+__device__ __forceinline__ void put_below(uint32_t addr, float v, uint32_t x, uint32_t end) {
+    asm volatile("{ .reg .pred p; setp.lt.u32 p, %2, %3; @p st.shared.f32 [%0], %1; }" ::"r"(addr), "f"(v), "r"(x), "r"(end) : "memory");
+}
+
+// Calls fn(four elements) for the row's exponentials, 16-byte loads, four in flight per thread; zeros beyond the row.
+template <class F>
+__device__ __forceinline__ void for_exponentials(const float* ex, uint32_t V, F&& fn) {
+    const float4* e4 = reinterpret_cast<const float4*>(ex);
+    const uint32_t n4 = V >> 2;
+    for (uint32_t i = threadIdx.x; i < n4; i += 4 * kThreads) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = i + u * kThreads < n4 ? e4[i + u * kThreads] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) fn(v[u]);
+    }
+    if (threadIdx.x == 0 && (V & 3)) {
+        float t[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+            if (4 * n4 + e < V) t[e] = ex[4 * n4 + e];
+        fn(make_float4(t[0], t[1], t[2], 0.f));
+    }
+}
+
+__device__ __noinline__ void count_level(Level& L, const float* ex, uint32_t V) {
+    ExactShared& sh = shared_memory();
+    __syncthreads();
+    for (int j = threadIdx.x; j < kBins; j += kThreads) sh.bins[j] = 0;
+    __syncthreads();
+    bool rest = false;
+    const uint32_t bins = (uint32_t)__cvta_generic_to_shared(sh.bins);
+    for_exponentials(ex, V, [&](float4 v) {
+        const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t key = __float_as_uint(e[u]), b = bin_of(L, key);
+            const bool in = key - 1u < L.F - 1u;   // zeros are left to the end; NaN and what an earlier level has taken
+            count_below(bins + 4 * b, in ? b : 0xffffffffu, (uint32_t)kBins);
+            rest |= in && b >= (uint32_t)kBins;
+        }
+    });
+    L.rest = __syncthreads_or(rest) != 0;
+}
+
+// Counts -> ranks of the bins' first elements, and the level's segments from number c on: whole bins, one beginning with the first
+// bin at or after every multiple of the segment length, bins of kBigSegs times that by themselves.  `placed` elements come
+// before the level, `sum` is their sum.  Returns the number after the level's last segment; *reach: the first segment that begins
+// above target as far as the bins tell (that number: none).
+__device__ __noinline__ int rank_bins(Level& L, Segs g, int c, uint32_t placed, float inv_norm, float sum, float target, int* reach) {
+    ExactShared& sh = shared_memory();
+    const int tid = threadIdx.x, j0 = tid * kBinsPerThread;
+    __syncthreads();
+    uint32_t n[kBinsPerThread];
+#pragma unroll
+    for (int k = 0; k < kBinsPerThread; ++k) n[k] = sh.bins[j0 + k];
+    const uint32_t big = (uint32_t)kBigSegs << g.shift;
+    float value[kBinsPerThread], mass = 0.f;
+    uint32_t count = 0, own_last = 0;
+#pragma unroll
+    for (int k = 0; k < kBinsPerThread; ++k) {   // the middle of the bin
+        const uint32_t down = ((uint32_t)(j0 + k) << L.shift) + ((1u << L.shift) >> 1) + 1u;
+        value[k] = n[k] && down < L.F ? (float)n[k] * (__uint_as_float(L.F - down) * inv_norm) : 0.f;
+        mass += value[k];
+        count += n[k];
+        own_last = n[k] ? n[k] : own_last;
+    }
+    const uint32_t first = block_scan_exclusive(count, sh.scan_u, &L.total);
+    float cum = sum + block_scan_exclusive(mass, sh.scan_f, (float*)nullptr);
+    // does a segment begin with the bin?  The last bin before that is not empty tells
+    const uint32_t n_before = block_scan_exclusive(own_last, sh.scan_u, (uint32_t*)nullptr, [](uint32_t a, uint32_t b) { return b ? b : a; });
+    bool begins[kBinsPerThread];
+    uint32_t at = first, before = n_before, marks = 0;
+#pragma unroll
+    for (int k = 0; k < kBinsPerThread; ++k) {
+        begins[k] = n[k] && (at == 0 || (at >> g.shift) != ((at - before) >> g.shift) || n[k] >= big || before >= big);
+        marks += begins[k] ? 1u : 0u;
+        at += n[k];
+        if (n[k]) before = n[k];
+    }
+    uint32_t total;
+    uint32_t no = c + block_scan_exclusive(marks, sh.scan_u, &total);
+    at = first;
+    int far = 0x7fffffff;
+#pragma unroll
+    for (int k = 0; k < kBinsPerThread; ++k) {
+        sh.bins[j0 + k] = at;
+        if (begins[k]) {
+            if (no < (uint32_t)kSegCap) {
+                sh.start[no] = placed + at; sh.bin[no] = (uint16_t)(j0 + k); sh.cum[no] = cum;
+                sh.sorted[no] = L.shift == 0 ? 1 : 0;   // bins of one value
+                if (cum > target) far = min(far, (int)no);
+            }
+            ++no;
+        }
+        at += n[k];
+        cum += value[k];
+    }
+    const int end = min(c + (int)total, kSegCap);
+    if (tid == kThreads - 1) { sh.start[end] = placed + L.total; sh.bin[end] = (uint16_t)kBins; sh.cum[end] = cum; }
+    far = block_reduce(far, [](int a, int b) { return min(a, b); }, sh.red_i);   // (its barriers cover the tables)
+    *reach = min(far, end);
+    return end;
+}
+
+struct Row {
+    const float* ex;    // exponentials in index order
+    float* sorted;      // the largest probabilities, as far as they were needed: segment by segment in descending order, those within
+                        // a segment only where it mattered
+    uint32_t V;
+    float norm, inv_norm, min_thr;
+};
+
+// Brings the segments c .. c1 - 1 (whole bins, at most kCap elements) into shared memory and the row, up to sh.stop, the first one that is
+// too large to be sorted and not all the same; elements below the min-p threshold as zeros.  Returns how many are not.
+__device__ __noinline__ uint32_t place_chunk(Row row, Level L, Segs g, int c, int c1, uint32_t placed) {
+    ExactShared& sh = shared_memory();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    PROF_BEGIN;
+    const int j0 = sh.bin[c], j1 = sh.bin[c1];
+    const uint32_t off = sh.start[c];
+    if (tid == 0) sh.stop = c1;
+    __syncthreads();
+    const uint32_t high = L.F - ((uint32_t)j0 << L.shift);   // keys from low to high - 1
+    const long long below = (long long)L.F - ((long long)j1 << L.shift);
+    const uint32_t low = below > 1 ? (uint32_t)below : 1u;
+    const uint32_t bins = (uint32_t)__cvta_generic_to_shared(sh.bins), keys = (uint32_t)__cvta_generic_to_shared(sh.keys) - 4 * (off - placed);
+    for_exponentials(row.ex, row.V, [&](float4 v) {
+        const float e[4] = {v.x, v.y, v.z, v.w};
+        uint32_t pos[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {   // (as many as were counted: a place is within the chunk)
+            const uint32_t key = __float_as_uint(e[u]);
+            pos[u] = take_below(bins + 4 * bin_of(L, key), key - low, high - low);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) put_below(keys + 4 * pos[u], e[u], __float_as_uint(e[u]) - low, high - low);
+    });
+    __syncthreads();
+    PROF_END(kProfGather);
+    const uint32_t big = (uint32_t)kBigSegs << g.shift;
+    for (int j = c + warp; j < c1; j += kWarps) {
+        const uint32_t a = sh.start[j] - off, z = sh.start[j + 1] - off;
+        if (z - a < big || sh.sorted[j] == 1) continue;
+        bool same = true;
+        const float first = sh.keys[a];
+        for (uint32_t i = a + lane; i < z; i += 32) same &= sh.keys[i] == first;
+        same = __all_sync(0xffffffffu, same);
+        if (lane == 0) {
+            if (same) sh.sorted[j] = 1;
+            else if (z - a >= 2 * big) atomicMin(&sh.stop, j);
+        }
+    }
+    __syncthreads();
+    PROF_END(kProfSame);
+    uint32_t valid = 0;
+    float* out = row.sorted + off;
+    const uint32_t n = sh.start[sh.stop] - off;
+    for (uint32_t i = tid; i < n; i += 4 * kThreads) {
+        float p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) p[u] = i + u * kThreads < n ? sh.keys[i + u * kThreads] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            p[u] = probability(p[u], row.norm, row.inv_norm);
+            const bool in = i + u * kThreads < n, keep = p[u] >= row.min_thr;
+            valid += in && keep ? 1u : 0u;
+            if (in) {
+                sh.keys[i + u * kThreads] = keep ? p[u] : 0.f;
+                out[i + u * kThreads] = keep ? p[u] : 0.f;
+            }
+        }
+    }
+    valid = block_sum(valid, sh.scan_u);
+    PROF_END(kProfPlace);
+    return valid;
+}
+
+struct Kept {
+    uint32_t n;        // elements kept, zeros included
+    uint32_t placed;   // of them in row.sorted
+    int segs;          // segments with a recorded sum
+    float total;
+};
+
+// Makes one of every two of the segments 0 .. c - 1.
+__device__ __noinline__ int merge_segments(int c) {
+    ExactShared& sh = shared_memory();
+    constexpr int kPer = (kSegCap / 2 + kThreads - 1) / kThreads + 1;
+    const int half = (c + 1) / 2;
+    uint32_t start[kPer];
+    float state[kPer];
+    uint8_t sorted[kPer];
+    __syncthreads();
+    const uint32_t end = sh.start[c];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int j = 2 * ((int)threadIdx.x + k * kThreads);
+        if (j >= c) continue;
+        start[k] = sh.start[j];
+        state[k] = sh.state[j];
+        sorted[k] = sh.sorted[j] == 1 && (j + 1 >= c || sh.sorted[j + 1] == 1) ? 1 : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int j = (int)threadIdx.x + k * kThreads;
+        if (2 * j >= c) continue;
+        sh.start[j] = start[k]; sh.state[j] = state[k]; sh.sorted[j] = sorted[k];
+    }
+    if (threadIdx.x == 0) sh.start[half] = end;
+    __syncthreads();
+    return half;
+}
+
+// TopPFilter: descending order, until the float sum exceeds top_p.  The first level's bins are counted already.  `u`: the number of
+// the row's own draw.
+__device__ __noinline__ Kept keep_top_p(Row row, Segs g, Level L, float top_p, float u) {
+    ExactShared& sh = shared_memory();
+    const int tid = threadIdx.x;
+    uint32_t placed = 0;       // elements before segment c, and their sum
+    int c = 0;
+    float s = 0.f;
+    int next_shift = kTopShift;
+    bool last = false;
+    while (!last) {
+        PROF_BEGIN;
+        // room for the segments of all that is left (a row of many levels: one or two extra for each)
+        const uint32_t most = (row.V - placed) >> g.shift;
+        while (c > 1 && (uint32_t)c + most + 2 * (most / kBigSegs) + 4 > (uint32_t)kSegCap) c = merge_segments(c);
+        int reach;
+        const int end = rank_bins(L, g, c, placed, row.inv_norm, s, top_p * (1.0f + 1.0f / 1024), &reach);
+        PROF_END(kProfRank);
+        const uint32_t level_at = placed;
+        bool again = false;    // another level takes over before this one's end
+        while (c < end && !last && !again) {
+            // the most segments that fit and may be needed
+            int c1 = c, hi = c < reach ? reach : end;
+            while (c1 < hi) {
+                const int mid = (c1 + hi + 1) >> 1;
+                if (sh.start[mid] - sh.start[c] <= (uint32_t)kCap) c1 = mid; else hi = mid - 1;
+            }
+            const uint32_t key_below = L.F - ((uint32_t)sh.bin[c] << L.shift);   // keys of this segment and those behind are below
+            long long hit = -1;
+            if (c1 > c) {
+                const uint32_t valid = place_chunk(row, L, g, c, c1, level_at);
+                const int stop = sh.stop;
+                const uint32_t n = sh.start[stop] - placed;
+                hit = ordered_sum(Chunk{placed, row.sorted}, c, stop, s, top_p, top_p * u);
+                if (hit >= 0) return Kept{(uint32_t)hit + 1, sh.start[sh.bc_seg + 1], sh.bc_seg + 1, s};
+                last = valid < n;   // below the min-p threshold from here on
+                placed += valid;
+                c = stop;
+                if (stop < c1 && !last) {
+                    L = Level{L.F - ((uint32_t)sh.bin[stop] << L.shift), max(0, L.shift - kFinerBy), 0, false};
+                    next_shift = L.shift;
+                    again = true;
+                }
+            } else if (L.shift > 0) {   // one bin with more than fits
+                L = Level{key_below, max(0, L.shift - kFinerBy), 0, false};
+                next_shift = L.shift;
+                again = true;
+            } else {                    // one value: its segments are made here, those of the level are made anew behind it
+                const uint32_t n = sh.start[c + 1] - sh.start[c];
+                const float p = probability(__uint_as_float(key_below - 1u), row.norm, row.inv_norm);
+                __syncthreads();
+                if (p >= row.min_thr) {
+                    for (uint32_t i = tid; i < n; i += kThreads) row.sorted[placed + i] = p;
+                    const int segs = min((int)((n + g.len() - 1) >> g.shift), kSegCap - c);
+                    for (int j = tid; j <= segs; j += kThreads) {
+                        sh.start[c + j] = placed + min(n, (uint32_t)j << g.shift);
+                        sh.cum[c + j] = s + p * (float)min(n, (uint32_t)j << g.shift);
+                        if (j < segs) sh.sorted[c + j] = 1;
+                    }
+                    __syncthreads();
+                    hit = ordered_sum(Sorted{row.sorted, 0}, c, c + segs, s, top_p, -1.f);
+                    if (hit >= 0) return Kept{(uint32_t)hit + 1, placed + n, sh.bc_seg + 1, s};
+                    placed += n;
+                    c += segs;
+                    L = Level{key_below - 1u, next_shift, 0, true};
+                    again = true;
+                } else {
+                    last = true;
+                }
+            }
+            if (c >= reach) reach = end;
+        }
+        if (last) break;
+        if (!again) {
+            const unsigned long long span = (unsigned long long)kBins << L.shift;
+            if (!L.rest || span >= L.F) break;
+            if (L.total < 4096u) next_shift = min(kTopShift, next_shift + kFinerBy);
+            L = Level{(uint32_t)(L.F - span), next_shift, 0, false};
+        }
+        if (L.F <= 1u) break;
+        count_level(L, row.ex, row.V);
+    }
+    // every candidate is in the sum; without a min-p threshold the zeros are candidates too
+    uint32_t zeros = 0;
+    if (!last && 0.f >= row.min_thr) {
+        for (uint32_t i = tid; i < row.V; i += kThreads) zeros += row.ex[i] == 0.f ? 1u : 0u;
+        zeros = block_sum(zeros, sh.scan_u);
+    }
+    while (c > 0 && sh.start[c - 1] >= placed) --c;   // segments of nothing but zeros
+    return Kept{placed + zeros, placed, c, s};
+}
+
+// The vocabulary index of the element of rank `rank` in descending order, whose probability is p: among equal ones the lowest
+// index comes first.  (Of more than 4096 equal ones the first is taken.)
+__device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p) {
+    ExactShared& sh = shared_memory();
+    constexpr uint32_t kMostEqual = 4096;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    PROF_BEGIN;
+    // the exponentials with this probability are neighbours: a look around p * norm finds the first and the last of them
+    uint32_t key_lo = 0, key_hi = 0;   // zero: they are compared by their probabilities
+    {
+        const int mid = (int)__float_as_uint(p * row.norm), cand = mid - 16 + lane;
+        const bool in = p > 0.f && cand > 0 && cand <= (int)kOneBits && probability(__uint_as_float((uint32_t)cand), row.norm, row.inv_norm) == p;
+        const uint32_t m = __ballot_sync(0xffffffffu, in);
+        if (m && !(m & 0x80000001u)) {
+            key_lo = (uint32_t)(mid - 16 + __ffs(m) - 1);
+            key_hi = (uint32_t)(mid - 16 + 31 - __clz(m));
+        }
+    }
+    auto equal = [&](float e) {
+        if (key_lo) return __float_as_uint(e) - key_lo <= key_hi - key_lo;
+        return probability(e, row.norm, row.inv_norm) == p;
+    };
+    uint32_t same = 0, lowest = 0xffffffffu;
+    const float4* e4 = reinterpret_cast<const float4*>(row.ex);
+    const uint32_t n4 = (row.V + 3) >> 2;   // (the row's pitch is a multiple of four; what lies beyond the row is not counted)
+    const uint32_t span = key_lo ? key_hi - key_lo : 0xffffffffu;
+    for (uint32_t i0 = threadIdx.x; i0 < n4; i0 += 4 * kThreads) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = i0 + u * kThreads < n4 ? e4[i0 + u * kThreads] : make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F);
+        uint32_t nearest = 0xffffffffu;   // two instructions for an element that is not one of them
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            nearest = min(nearest, min(__float_as_uint(v[u].x) - key_lo, __float_as_uint(v[u].y) - key_lo));
+            nearest = min(nearest, min(__float_as_uint(v[u].z) - key_lo, __float_as_uint(v[u].w) - key_lo));
+        }
+        if (nearest > span) continue;
+#pragma unroll 1
+        for (int u = 0; u < 16; ++u) {
+            const uint32_t i = 4 * (i0 + (u >> 2) * kThreads) + (u & 3);
+            if (i < row.V && equal(row.ex[i])) { ++same; lowest = min(lowest, i); }
+        }
+    }
+    __syncthreads();
+    same = block_sum(same, sh.scan_u);
+    lowest = block_reduce(lowest, [](uint32_t a, uint32_t b) { return min(a, b); }, sh.scan_u);
+    PROF_END(kProfIndex);
+    if (same <= 1 || same > kMostEqual) return lowest == 0xffffffffu ? 0 : (long long)lowest;
+    // several: the rank among them
+    const uint32_t blocks = (row.V + kBlock - 1) / kBlock, per = (blocks + kWarps - 1) / kWarps;
+    const uint32_t b0 = min(blocks, warp * per), b1 = min(blocks, b0 + per);
+    uint32_t greater = 0;
+    same = 0;
+    for (uint32_t b = b0; b < b1; ++b) {
+        const uint32_t i = b * kBlock + 8 * lane;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (i + e < row.V) {
+                const float q = probability(row.ex[i + e], row.norm, row.inv_norm);
+                same += q == p ? 1u : 0u;
+                greater += q > p ? 1u : 0u;
+            }
+    }
+    same = __reduce_add_sync(0xffffffffu, same);
+    greater = block_sum(greater, sh.scan_u);
+    const uint32_t scanned = block_scan_exclusive(lane == 0 ? same : 0u, sh.scan_u, (uint32_t*)nullptr);
+    const uint32_t before = __shfl_sync(0xffffffffu, scanned, 0);
+    const uint32_t want = rank < greater ? 0u : rank - greater;
+    if (threadIdx.x == 0) sh.bc_hit = lowest;
+    __syncthreads();
+    if (want >= before && want < before + same) {   // one warp
+        uint32_t seen = before;
+        for (uint32_t b = b0; b < b1; ++b) {
+            const uint32_t i = b * kBlock + 8 * lane;
+            uint32_t mine = 0;   // a bit per element
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (i + e < row.V && probability(row.ex[i + e], row.norm, row.inv_norm) == p) mine |= 1u << e;
+            uint32_t incl = __popc(mine);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += up;
+            }
+            uint32_t at = seen + incl - __popc(mine);
+            for (; mine; mine &= mine - 1, ++at)
+                if (at == want) sh.bc_hit = (long long)i + __ffs(mine) - 1;
+            seen += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    __syncthreads();
+    const long long idx = sh.bc_hit;
+    __syncthreads();
+    PROF_END(kProfIndex2);
+    return idx;
+}
+
+// First element of src, of those below n, whose running sum exceeds r (-1: none), from the sums recorded before the segments
+// 0 .. segs - 1.  `unsorted`: the row in memory whose segment may have to be sorted first.
+template <class Src>
+__device__ __noinline__ long long find_draw(Src src, int segs, uint32_t n, float* unsorted, float r, float& p) {
+    ExactShared& sh = shared_memory();
+    PROF_BEGIN;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int lo = 0, hi = segs - 1;   // the last segment with a sum not above r (the first has none)
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (!(sh.state[mid] > r)) lo = mid; else hi = mid - 1;
+        }
+        float s = segs > 0 ? sh.state[lo] : 0.f, q = 0.f;
+        long long hit = -1;
+        for (int j = lo; j < segs && hit < 0; ++j) {
+            if (unsorted && sh.sorted[j] != 1) {
+                const uint32_t a = sh.start[j], len = sh.start[j + 1] - a;
+                if (len <= (uint32_t)kCap) {
+                    for (uint32_t i = lane; i < len; i += 32) sh.keys[i] = unsorted[a + i];
+                    sort_segment(sh.keys, (int)len);
+                    for (uint32_t i = lane; i < len; i += 32) unsorted[a + i] = sh.keys[i];
+                } else {
+                    sort_segment(unsorted + a, (int)len);   // (merged segments of a very long row)
+                }
+                __syncwarp();
+                if (lane == 0) sh.sorted[j] = 1;
+                __syncwarp();
+            }
+            hit = add_segment(src, j, s, r, q);
+        }
+        if (hit >= (long long)n) hit = -1;
+        if (lane == 0) { sh.bc_hit = hit; sh.bc_p = q; }
+    }
+    __syncthreads();
+    const long long hit = sh.bc_hit;
+    p = sh.bc_p;
+    __syncthreads();
+    PROF_END(kProfFind);
+    return hit;
+}
+
+// expf with the host libm's bits (fsx::expf_libm), the table of 2^(i / 32) in the lanes' registers: in shared memory, 32
+// different entries of eight bytes cost a warp six to seven passes, two shuffles cost two.
+__device__ __forceinline__ float expf_lanes(float x, uint32_t tab_lo, uint32_t tab_hi) {
+    const double kInvLn2N = 0x1.71547652b82fep+0 * 32.0;
+    const double kShift = 0x1.8p+52;
+    const double kC0 = 0x1.c6af84b912394p-5 / 32768.0, kC1 = 0x1.ebfce50fac4f3p-3 / 1024.0, kC2 = 0x1.62e42ff0c52d6p-1 / 32.0;
+    const bool in = x >= -103.972076f && !(x > 88.72283f);
+    const double xd = (double)(in ? x : 0.f);
+    double kd = __fma_rn(kInvLn2N, xd, kShift);
+    const uint64_t ki = (uint64_t)__double_as_longlong(kd);
+    kd = __dadd_rn(kd, -kShift);
+    const double r = __fma_rn(kInvLn2N, xd, -kd);
+    const uint32_t lo = __shfl_sync(0xffffffffu, tab_lo, (int)(ki & 31)), hi = __shfl_sync(0xffffffffu, tab_hi, (int)(ki & 31));
+    const double s = __longlong_as_double((long long)((((uint64_t)hi << 32) | lo) + (ki << 47)));
+    const double z = __fma_rn(kC0, r, kC1);
+    const double r2 = __dmul_rn(r, r);
+    double y = __fma_rn(kC2, r, 1.0);
+    y = __fma_rn(z, r2, y);
+    y = __dmul_rn(y, s);
+    const float f = (float)y;
+    return in ? f : x > 0.f ? CUDART_INF_F : x != x ? x : 0.f;
+}
+
+// The same for arguments from -inf to 0, without the selections: below -104.5 the result is zero as it is at -104.5.
+__device__ __forceinline__ float expf_lanes_nonpositive(float x, uint32_t tab_lo, uint32_t tab_hi) {
+    const double kInvLn2N = 0x1.71547652b82fep+0 * 32.0;
+    const double kShift = 0x1.8p+52;
+    const double kC0 = 0x1.c6af84b912394p-5 / 32768.0, kC1 = 0x1.ebfce50fac4f3p-3 / 1024.0, kC2 = 0x1.62e42ff0c52d6p-1 / 32.0;
+    // the conversion to double in integers, for x <= 0 (zeros and denormals as some other number that small): four instructions instead
+    // of one at a quarter of their sixteenth of a warp's lanes per cycle
+    const uint32_t b = __float_as_uint(fmaxf(x, -104.5f));
+    const double xd = __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + 0xb8000000u), (int)(b << 29));
+    double kd = __fma_rn(kInvLn2N, xd, kShift);
+    const uint32_t ki = (uint32_t)__double2loint(kd);
+    kd = __dadd_rn(kd, -kShift);
+    const double r = __fma_rn(kInvLn2N, xd, -kd);
+    const uint32_t lo = __shfl_sync(0xffffffffu, tab_lo, (int)ki), hi = __shfl_sync(0xffffffffu, tab_hi, (int)ki);   // (lane ki mod 32)
+    const double s = __hiloint2double((int)(hi + (ki << 15)), (int)lo);
+    const double z = __fma_rn(kC0, r, kC1);
+    const double r2 = __dmul_rn(r, r);
+    double y = __fma_rn(kC2, r, 1.0);
+    y = __fma_rn(z, r2, y);
+    return (float)__dmul_rn(y, s);
+}
+
+__device__ float row_maximum(const float* row, uint32_t V, bool vec_ok, bool* has_nan) {
+    ExactShared& sh = shared_memory();
+    float mx = -CUDART_INF_F;
+    bool bad = false;
+    auto take = [&](float x) { mx = fmaxf(mx, x); bad |= x != x; };
+    if (vec_ok) {
+        const float4* r4 = reinterpret_cast<const float4*>(row);
+        const uint32_t n4 = V >> 2;
+        for (uint32_t i = threadIdx.x; i < n4; i += 8 * kThreads) {
+            float4 q[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) q[u] = i + u * kThreads < n4 ? r4[i + u * kThreads] : make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) { take(q[u].x); take(q[u].y); take(q[u].z); take(q[u].w); }
+        }
+        for (uint32_t j = 4 * n4 + threadIdx.x; j < V; j += kThreads) take(row[j]);
+    } else {
+        for (uint32_t i = threadIdx.x; i < V; i += kThreads) take(row[i]);
+    }
+    *has_nan = __syncthreads_or(bad) != 0;
+    return block_reduce(mx, [](float a, float b) { return fmaxf(a, b); }, sh.scan_f);
+}
+
+// Exponentials of the row into ex[], the masses of the segments into sh.cum, and with kCount the counts of the first level's bins.
+// Bound by instruction issue (some 30 per element, eight of them in double precision).
+template <bool kCount>
+__device__ __noinline__ void exponentials(const float* row, uint32_t V, bool vec_ok, bool plain, Segs g, float mx, float inv_T, float* ex, Level& level) {
+    ExactShared& sh = shared_memory();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t tab = fsx::kExp2TabDev[lane];
+    const uint32_t tab_lo = (uint32_t)tab, tab_hi = (uint32_t)(tab >> 32);
+    const uint32_t bins = (uint32_t)__cvta_generic_to_shared(sh.bins);
+    for (int j = tid; j < g.count; j += kThreads) sh.cum[j] = 0.f;
+    if (kCount)
+        for (int j = tid; j < kBins; j += kThreads) sh.bins[j] = 0;
+    __syncthreads();
+    bool rest = false;
+    const uint32_t blocks = (V + kBlock - 1) / kBlock;
+    for (uint32_t b = 2 * warp; b < blocks; b += 2 * kWarps) {   // two blocks: four 16-byte loads in flight per lane
+        float mass[2] = {0.f, 0.f};
+        if (plain && vec_ok && (b + 2) * kBlock <= V) {
+            float4 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = *reinterpret_cast<const float4*>(row + b * kBlock + u * 128 + 4 * lane);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                float y[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) y[e] = expf_lanes_nonpositive(__fmul_rn(__fsub_rn(y[e], mx), inv_T), tab_lo, tab_hi);   // (inv_T 1: as it is)
+                mass[u >> 1] += (y[0] + y[1]) + (y[2] + y[3]);
+                if (kCount) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const uint32_t bin = (kOneBits - __float_as_uint(y[e])) >> kTopShift;
+                        count_below(bins + 4 * bin, bin, (uint32_t)kBins);
+                        rest |= bin >= (uint32_t)kBins;   // (zeros too: the next level's counts tell)
+                    }
+                }
+                *reinterpret_cast<float4*>(ex + b * kBlock + u * 128 + 4 * lane) = make_float4(y[0], y[1], y[2], y[3]);
+            }
+        } else {
+            for (int u = 0; u < 16; ++u) {
+                const uint32_t i = b * kBlock + u * 32 + lane;
+                const float d = i < V ? __fsub_rn(row[i], mx) : -CUDART_INF_F;
+                const float y = expf_lanes(__fmul_rn(d, inv_T), tab_lo, tab_hi);
+                if (i < V) {
+                    if (y >= 0.f) mass[u >> 3] += y;
+                    ex[i] = y;
+                    const uint32_t key = __float_as_uint(y);
+                    if (kCount && key - 1u < kOneBits) {
+                        const uint32_t bin = (kOneBits - key) >> kTopShift;
+                        if (bin < (uint32_t)kBins) atomicAdd(&sh.bins[bin], 1u);
+                        else rest = true;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mass[h] += __shfl_xor_sync(0xffffffffu, mass[h], o);
+            if (lane == 0 && b + h < blocks) atomicAdd(&sh.cum[((b + h) * kBlock) >> g.shift], mass[h]);
+        }
+    }
+    rest = __syncthreads_or(rest) != 0;
+    level = Level{kOneBits + 1u, kTopShift, 0, rest};
+}
+
+__device__ void sample_row(const StepArgs& a, float* scratch, int r) {
+    ExactShared& sh = shared_memory();
+    const int tid = threadIdx.x;
+    const sampler_row_params p = a.rows[r];
+    const uint32_t V = (uint32_t)a.vocab;
+    const float* logits = a.logits + p.logits_row * a.vocab;
+    const bool raw_lp = (p.do_sample & SAMPLER_ROW_RAW_LOG_PROB) != 0;
+    const float raw_lse = raw_lp ? a.out_log_prob[r] : 0.f;   // left there by the first kernel (NaN: no scratch for the raw logits)
+    const bool vec_ok = (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+    const bool top_p_active = p.top_p != 1.0f;
+    const Segs g = segments_of(a.vocab);
+    float* ex = scratch;
+    float* sorted = scratch + sampler_exact_pitch(a.vocab);
+    const float inv_T = __fdiv_rn(1.0f, p.temperature);
+#ifdef SAMPLER_EXACT_PROF
+    __syncthreads();
+    if (tid < kProfN) sh.prof[tid] = 0;
+#endif
+    __syncthreads();
+    PROF_BEGIN;
+    bool has_nan;
+    const float mx = row_maximum(logits, V, vec_ok, &has_nan);
+    PROF_END(kProfMax);
+    const bool plain = !has_nan && fabsf(mx) < CUDART_INF_F && inv_T > 0.f && inv_T < CUDART_INF_F;   // every exponential is between 0 and 1
+    Level level;
+    if (top_p_active) exponentials<true>(logits, V, vec_ok, plain, g, mx, inv_T, ex, level);
+    else exponentials<false>(logits, V, vec_ok, plain, g, mx, inv_T, ex, level);
+    PROF_END(kProfExp);
+    masses_to_sums(g.count);
+    const float norm = index_order_sum(Exponentials{ex, 0}, g, V);
+    const float inv_norm = __fdiv_rn(1.0f, norm);   // the largest probability, that of the maximum, and the shared reciprocal of the divisions
+    const bool any = norm > 0.0f;                   // else every probability is NaN: none is kept
+    const float min_thr = p.min_p > 0.0f ? __fmul_rn((float)(double)p.min_p, inv_norm) : 0.0f;
+    const Row row{ex, sorted, V, norm, inv_norm, min_thr};
+    const Probabilities probs{ex, 0, norm, inv_norm, min_thr};
+    Kept kept{0, 0, 0, 0.f};
+    float total = 0.0f;
+    if (any && top_p_active) {
+        kept = keep_top_p(row, g, level, p.top_p, p.rand_u);
+        total = kept.total;
+    } else if (any) {
+        // approximate sums: those of the exponentials over the norm (min-p drops mass: guesses that do not hold cost time only)
+        __syncthreads();
+        for (int j = tid; j <= g.count; j += kThreads) sh.cum[j] *= inv_norm;
+        total = index_order_sum(probs, g, V);
+    }
+    const bool uniform_fallback = !(total > 0.0f && isfinite(total)) || (top_p_active && kept.n == 0);
+    long long kept_count = kept.n, last_kept = -1;
+    bool looked = top_p_active;   // kept_count and, without top-p, last_kept are known
+    auto look = [&] {
+        if (looked) return;
+        looked = true;
+        uint32_t n = 0;
+        int last = -1;
+        for (uint32_t i = tid; any && i < V; i += kThreads)
+            if (probability(ex[i], norm, inv_norm) >= min_thr) { ++n; last = (int)i; }
+        kept_count = block_sum(n, sh.scan_u);
+        last_kept = block_reduce(last, [](int x, int y) { return max(x, y); }, sh.red_i);
+    };
+    const long long x0 = a.extra_offsets ? a.extra_offsets[r] : 0, x1 = a.extra_offsets ? a.extra_offsets[r + 1] : 0;
+    for (long long k = -1; k < x1 - x0; ++k) {   // the row's own draw, then the further ones (sampler.cpp:1065)
+        const float u = k < 0 ? p.rand_u : a.extra_rand_u[x0 + k];
+        long long pick = -1;
+        float pick_p = 0.f;
+        if (uniform_fallback) look();
+        else {
+            const float rr = __fmul_rn(total, u);
+            if (!top_p_active) {
+                pick = find_draw(probs, g.count, V, nullptr, rr, pick_p);
+                if (pick < 0) {   // rounding left r at or beyond the total: the last kept element
+                    look();
+                    pick = last_kept;
+                    pick_p = probability(ex[pick < 0 ? 0 : pick], norm, inv_norm);
+                }
+            } else {
+                long long rank = find_draw(Sorted{sorted, 0}, kept.segs, kept.n, sorted, rr, pick_p);
+                if (rank < 0) {   // the last of the kept ones
+                    rank = (long long)kept.n - 1;
+                    pick_p = rank < (long long)kept.placed ? sorted[rank] : 0.f;
+                }
+                pick = index_of_rank(row, (uint32_t)rank, pick_p);
+            }
+        }
+        if (tid == 0) {
+            float lp;
+            if (uniform_fallback) {
+                // non-finite or empty mass: the reference draws an index uniformly (sampler.cpp:1047-1059)
+                const long long n = kept_count > 0 ? kept_count : (long long)V;
+                long long q = (long long)(u * (float)n);
+                if (q > n - 1) q = n - 1;
+                pick = q < (long long)V ? q : (long long)V - 1;
+                lp = logf(1.0f / (float)n);
+            } else {
+                lp = logf(pick_p) - logf(total);
+                if (raw_lp) {
+                    float raw = logits[pick];
+                    const long long h0 = a.hist_offsets ? a.hist_offsets[r] : 0, h1 = a.hist_offsets ? a.hist_offsets[r + 1] : 0;
+                    if (a.hist_raw)
+                        for (long long i = h0; i < h1; ++i)
+                            if (a.hist_ids[i] == pick) { raw = a.hist_raw[i]; break; }
+                    lp = raw_lse != raw_lse ? CUDART_NAN_F : raw - raw_lse;
+                }
+            }
+            if (k < 0) { a.out_token[r] = pick; a.out_log_prob[r] = lp; }
+            else { a.extra_out_token[x0 + k] = pick; a.extra_out_log_prob[x0 + k] = lp; }
+        }
+    }
+#ifdef SAMPLER_EXACT_PROF
+    if (tid == 0 && blockIdx.x % 37 == 0)
+        printf("row %d kept %u: max %lld exp %lld | guesses %lld steps %lld walk %lld (misses %lld) | ranks %lld gather %lld same %lld place %lld masses %lld | find %lld index %lld + %lld cycles; walk: tiles %lld in %lld, slots %lld in %lld, serial %lld\n", r, kept.n, sh.prof[kProfMax],
+               sh.prof[kProfExp], sh.prof[kProfGuess], sh.prof[kProfSteps], sh.prof[kProfWalk], sh.prof[kProfMisses], sh.prof[kProfRank], sh.prof[kProfGather], sh.prof[kProfSame],
+               sh.prof[kProfPlace], sh.prof[kProfMass], sh.prof[kProfFind], sh.prof[kProfIndex], sh.prof[kProfIndex2], sh.prof[kProfTiles], sh.prof[kProfTile], sh.prof[kProfSlots], sh.prof[kProfSlot], sh.prof[kProfSerial]);
+#endif
+}
+
+__global__ void __launch_bounds__(kThreads, 1) sampler_exact_kernel(StepArgs a, float* scratch) {
+    ExactShared& sh = shared_memory();
+    const int tid = threadIdx.x;
+    float* own = scratch + (size_t)blockIdx.x * 2 * sampler_exact_pitch(a.vocab);
+    uint32_t seen = 0;   // rows of this kernel among those looked at: they are dealt to the CTAs in turn
+    for (int base = 0; base < a.num_rows; base += kThreads) {
+        bool take = false;
+        if (base + tid < a.num_rows) {
+            const sampler_row_params& p = a.rows[base + tid];
+            const bool top_k = p.top_k > 0 && p.top_k < 0x7fffffffffffffffLL && p.top_k < a.vocab;   // the first kernel's
+            take = (p.do_sample & SAMPLER_ROW_MULTINOMIAL) && !top_k && p.logits_row >= 0 && p.logits_row < a.num_logit_rows;
+        }
+        uint32_t n;
+        const uint32_t at = seen + block_scan_exclusive(take ? 1u : 0u, sh.scan_u, &n);
+        const uint32_t mine = __ballot_sync(0xffffffffu, take && at % gridDim.x == blockIdx.x);
+        if ((tid & 31) == 0) sh.queue[tid >> 5] = mine;
+        __syncthreads();
+        for (int w = 0; w < kWarps; ++w)
+            for (uint32_t rows = sh.queue[w]; rows; rows &= rows - 1) sample_row(a, own, base + 32 * w + __ffs(rows) - 1);
+        seen += n;
+        __syncthreads();
+    }
+}
 
 __global__ void expf_selftest_kernel(const float* in, float* out, long long n) {
-    __shared__ uint64_t tab[32];
-    if (threadIdx.x < 32) tab[threadIdx.x] = fsx::kExp2TabDev[threadIdx.x];
-    __syncthreads();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) out[i] = fsx::expf_libm(in[i], tab);
+    const int lane = threadIdx.x & 31;
+    const uint64_t tab = fsx::kExp2TabDev[lane];
+    for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x - lane; i0 < n; i0 += (long long)gridDim.x * blockDim.x) {
+        const long long i = i0 + lane;
+        const float y = expf_lanes(i < n ? in[i] : 0.f, (uint32_t)tab, (uint32_t)(tab >> 32));
+        if (i < n) out[i] = y;
+    }
 }
 
 }  // namespace
@@ -61,22 +1432,13 @@ cudaError_t launch_expf_selftest(const float* in, float* out, long long n, cudaS
     return cudaGetLastError();
 }
 
-size_t sampler_exact_smem_bytes() { return sizeof(sx512::ExactShared) > sizeof(sx1024::ExactShared) ? sizeof(sx512::ExactShared) : sizeof(sx1024::ExactShared); }
-
-size_t sampler_exact_scratch_bytes(int ctas, long long vocab) { return (size_t)ctas * (size_t)((vocab + 3) & ~3LL) * sizeof(float); }
+size_t sampler_exact_scratch_bytes(int ctas, long long vocab) { return (size_t)ctas * 2 * sampler_exact_pitch(vocab) * sizeof(float); }
 
 cudaError_t launch_sampler_exact(const StepArgs& a, float* scratch, int ctas, cudaStream_t stream) {
     if (a.num_rows <= 0 || ctas <= 0) return cudaSuccess;
-    const int grid = a.num_rows < ctas ? a.num_rows : ctas;
-    if (a.num_rows * 2 <= ctas) {   // at most one row per SM (ctas = 2 per SM): the large CTA
-        cudaError_t e = cudaFuncSetAttribute(sx1024::sampler_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(sx1024::ExactShared));
-        if (e != cudaSuccess) return e;
-        sx1024::sampler_exact_kernel<<<grid, 1024, sizeof(sx1024::ExactShared), stream>>>(a, scratch);
-        return cudaGetLastError();
-    }
-    cudaError_t e = cudaFuncSetAttribute(sx512::sampler_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(sx512::ExactShared));
+    cudaError_t e = cudaFuncSetAttribute(sampler_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ExactShared));
     if (e != cudaSuccess) return e;
-    sx512::sampler_exact_kernel<<<grid, 512, sizeof(sx512::ExactShared), stream>>>(a, scratch);
+    sampler_exact_kernel<<<a.num_rows < ctas ? a.num_rows : ctas, kThreads, sizeof(ExactShared), stream>>>(a, scratch);
     return cudaGetLastError();
 }
 
