@@ -54,10 +54,16 @@ constexpr int kBins = 2048;
 constexpr int kBinsPerThread = kBins / kThreads;
 constexpr int kTopShift = 16;         // first level: 2^16 bit patterns per bin, 128 bins per binade, 16 binades
 constexpr int kFinerBy = 5;           // bits a level is cut finer by where a bin is too full to be sorted
-constexpr int kCap = 47104;           // elements of a chunk in shared memory
+constexpr int kCap = 46720;           // elements of a chunk in shared memory
 constexpr int kSlots = 32;            // segments with the amounts of their lanes at hand, for those in which the sum may change binade
-constexpr int kMaxMisses = 24;        // segments added one by one before the guesses of those behind are made anew
-constexpr float kMargin = 1.0f / 1024, kDrawMargin = 1.0f / 256;   // around the sums at which a segment is sorted ahead
+constexpr int kTwice = 220;           // further ones whose amounts are taken for two binades (of a chunk; of a row in memory: all)
+constexpr uint8_t kInKeys = 255;
+static_assert(kSlots + kTwice < kInKeys, "slot numbers");
+constexpr int kMaxMisses = 10;        // segments added one by one before the guesses of those behind are made anew (3 k cycles each; a new
+                                      // pass over a row takes 35 k)
+// Relative margins around the approximate sums: where the sum may change binade (the second one: or may not have yet, since what
+// rounding took from a sum of small terms adds up), pass the threshold, be drawn
+constexpr float kMargin = 1.0f / 1024, kWideMargin = 1.0f / 64, kDrawMargin = 1.0f / 256;
 constexpr uint32_t kOneBits = 0x3f800000u;
 constexpr uint32_t kNoGuess = 0, kEmpty = 255;
 
@@ -82,11 +88,13 @@ struct ExactShared {
     uint32_t step[kSegCap];              // amounts of a segment's elements for an even and an odd sum (pack_amounts)
     uint8_t E[kSegCap];                  // binade the sum is taken to lie in
     uint8_t sorted[kSegCap];             // 1: the elements are in descending order, 2: they are to be brought into it
-    uint8_t slot[kSegCap];               // 1 + its place in `upto` and `from`; 0: none
+    uint8_t slot[kSegCap];               // 1 + its place in `upto` and `from`, or 1 + kSlots + its place in step_up; kInKeys; 0: none
+    uint32_t step_up[kTwice];            // amounts of such segments under E + 1
     uint16_t bin[kSegCap + 1];           // the segment's first bin
+    uint16_t tile[kSegCap / 2];          // runs of segments that the walk took as a whole: the first, and 2^11 times the others' number
+    int tiles;
     uint32_t upto[kSlots][32];           // amounts of the segment's lanes up to this one under E (pack_amounts)
     uint32_t from[kSlots][32];           // ... from this one on under E + 1
-    int slots;
     alignas(16) float serial[kBlock];    // elements the walking warp adds one by one
     uint32_t queue[kWarps];              // rows of this CTA among the kThreads rows looked at, a bit each
     int stop;                            // first segment of a chunk that is too large to be sorted
@@ -104,6 +112,7 @@ struct ExactShared {
 #endif
 };
 static_assert(sizeof(ExactShared) <= 232448, "shared memory of a CTA");
+static_assert(kSlots * kBlock + kSegCap <= kCap, "room in keys");
 extern __shared__ __align__(16) uint8_t sx_smem[];
 // (by its name and not by an argument: the compiler then knows that it is shared memory)
 __device__ __forceinline__ ExactShared& shared_memory() { return *reinterpret_cast<ExactShared*>(sx_smem); }
@@ -158,10 +167,10 @@ struct Segs {
     int count;   // segments of the row in index order
     __device__ uint32_t len() const { return 1u << shift; }
 };
-__device__ __forceinline__ Segs segments_of(long long V) {
+__device__ __forceinline__ Segs segments_of(uint32_t end) {
     int shift = 8;
-    while (((V - 1) >> shift) >= kMaxSegs) ++shift;
-    return Segs{shift, (int)((V + (1ll << shift) - 1) >> shift)};
+    while (((end - 1) >> shift) >= (uint32_t)kMaxSegs) ++shift;
+    return Segs{shift, (int)((end + (1u << shift) - 1) >> shift)};
 }
 
 // Eight elements from i on (a multiple of eight), those outside lo .. hi - 1 as zero, which leaves a sum as it is.
@@ -333,32 +342,49 @@ __device__ __forceinline__ void sort_in_chunk(Chunk src, int j) {
     __syncwarp();
 }
 
-// Guesses the binade of the sum at the segments c .. c1 - 1 from the approximate sums and the exact one, s, before c.  Where the sum
-// may change binade the segment gets a slot.  Segments of unsorted elements in which the order will matter are marked:
-// those, and where the sum may pass one of two thresholds.
-__device__ void guess_binades(int c, int c1, float s, float thr, float thr2) {
+// Guesses the binade of the sum at the segments c .. c1 - 1 from the approximate sums and the exact one, s, before c.  Where the sum may
+// change binade, or may have, the amounts are taken for two; the first of the former also get a slot each.  Segments of
+// unsorted elements in which the order will matter are marked: those, and where the sum may pass one of two thresholds.
+// `rows`: the elements are a row's in memory, and `keys` has room for every segment's second amounts.
+__device__ void guess_binades(int c, int c1, float s, float thr, float thr2, bool rows) {
     ExactShared& sh = shared_memory();
     __syncthreads();
-    if (threadIdx.x == 0) sh.slots = 0;
-    __syncthreads();
     const float shift = s - sh.cum[c];
-    for (int j = c + (int)threadIdx.x; j < c1; j += kThreads) {
-        const float lo = j == c ? s : sh.cum[j] + shift, hi = sh.cum[j + 1] + shift;
-        const float l = lo * (1.f - kMargin), h = hi * (1.f + kMargin);
-        const uint32_t El = fsx::state_exp(l), Eh = fsx::state_exp(h);
-        uint32_t E = fsx::state_exp(lo);
-        uint8_t slot = 0;
-        const bool empty = sh.start[j] == sh.start[j + 1], usable = lo > 0.f && El >= 24u && Eh < 253u;
-        if (!empty && usable && Eh == El + 1u) {
-            const int at = atomicAdd(&sh.slots, 1);
-            if (at < kSlots) { slot = (uint8_t)(at + 1); E = El; }
+    uint32_t slots = 0, twice = 0;
+    for (int base = c; base < c1; base += kThreads) {
+        const int j = base + (int)threadIdx.x;
+        bool maybe = false, wide = false;
+        uint32_t Ew = 0, El = 0;
+        if (j < c1) {
+            const float lo = j == c ? s : sh.cum[j] + shift, hi = sh.cum[j + 1] + shift;
+            const float l = lo * (1.f - kMargin), h = hi * (1.f + kMargin);
+            const uint32_t Eh = fsx::state_exp(h), Ev = fsx::state_exp(hi * (1.f + kWideMargin));
+            El = fsx::state_exp(l);
+            Ew = fsx::state_exp(lo * (1.f - kWideMargin));
+            const bool empty = sh.start[j] == sh.start[j + 1], usable = lo > 0.f && Ew >= 25u && Ev < 252u;
+            wide = !empty && usable && Ev == Ew + 1u;
+            maybe = wide && El != Eh;
+            sh.E[j] = (uint8_t)(empty ? kEmpty : usable ? fsx::state_exp(lo) : kNoGuess);
+            if (sh.sorted[j] == 0 && (j == 0 || El != Eh || (l <= thr && thr <= h) || (lo * (1.f - kDrawMargin) <= thr2 && thr2 <= hi * (1.f + kDrawMargin))))
+                sh.sorted[j] = 2;
         }
-        sh.slot[j] = slot;
-        sh.E[j] = (uint8_t)(empty ? kEmpty : usable ? E : kNoGuess);
-        if (sh.sorted[j] == 0 && (j == 0 || El != Eh || (l <= thr && thr <= h) || (lo * (1.f - kDrawMargin) <= thr2 && thr2 <= hi * (1.f + kDrawMargin))))
-            sh.sorted[j] = 2;
+        uint32_t n;
+        const uint32_t before = block_scan_exclusive((maybe ? 1u : 0u) | (wide ? 65536u : 0u), sh.scan_u, &n);
+        if (j < c1) {
+            const uint32_t at = slots + (before & 0xffffu), at2 = twice + (before >> 16);
+            const bool lanes = maybe && at < (uint32_t)kSlots, two = wide && (rows || at2 < (uint32_t)kTwice);
+            sh.slot[j] = lanes ? (uint8_t)(at + 1) : !two ? 0 : rows ? kInKeys : (uint8_t)(at2 + 1 + kSlots);
+            if (wide) sh.E[j] = (uint8_t)(lanes || two ? Ew : El);
+        }
+        slots += n & 0xffffu;
+        twice += n >> 16;
     }
     __syncthreads();
+}
+// Where a segment's amounts under E + 1 are (its slot holds none for the lanes).
+__device__ __forceinline__ uint32_t& step_up(int slot, int j) {
+    ExactShared& sh = shared_memory();
+    return slot == kInKeys ? reinterpret_cast<uint32_t*>(sh.keys)[kSlots * kBlock + j] : sh.step_up[slot - 1 - kSlots];
 }
 
 // The amounts for an even and an odd sum differ by one at most: two neighbouring sums stay neighbours or meet.
@@ -389,6 +415,9 @@ __device__ __forceinline__ fsx::Step block_step(const float (&x)[8], uint32_t E,
     }
     return st;
 }
+
+// Does the slot hold the amounts of the segment's lanes (else: those of the whole segment under the next binade)?
+__device__ __forceinline__ bool lanes_at_hand(int slot) { return slot != 0 && slot <= kSlots; }
 
 // A segment with a slot: the amounts of its lanes, each of which takes m * 8 consecutive elements, under E up to every lane and under
 // E + 1 from every lane on.  Elements of rows in memory stay at hand in `keys`, which nothing else uses then (m = 1).
@@ -426,15 +455,17 @@ __device__ __forceinline__ void lane_steps(Src src, int j) {
     }
     sh.upto[slot][lane] = pack_amounts(p);
     sh.from[slot][lane] = pack_amounts(q);
+    if (lane == 31) sh.step[j] = pack_amounts(p);
+    __syncwarp();
 }
 
-// Amounts of the segments' elements under the guesses: rows in memory, a block of each of four segments at a time (a warp's loads are
+// Amounts of the segments' elements under the guesses: rows in memory, a block of each of two segments at a time (a warp's loads are
 // what it waits for: one block at a time 23 k cycles for 152 k elements).
 template <class Src>
 __device__ __forceinline__ void segment_steps(Src src, int c, int c1) {
     ExactShared& sh = shared_memory();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int kAtOnce = 4;
+    constexpr int kAtOnce = 2;
     for (int j = c + warp; j < c1; j += kAtOnce * kWarps) {
         uint32_t lo[kAtOnce], hi[kAtOnce];
         fsx::Step total[kAtOnce];
@@ -463,13 +494,18 @@ __device__ __forceinline__ void segment_steps(Src src, int c, int c1) {
                 src.prepare(x[u]);
                 bool tie;
                 total[u] = fsx::then(total[u], block_step(x[u], E, true, &tie));
+                const int slot = sh.slot[j + u * kWarps];
+                if (slot > kSlots) {
+                    const fsx::Step up = block_step(x[u], E + 1u, true, &tie);
+                    if (lane == 0) step_up(slot, j + u * kWarps) = pack_amounts(at ? fsx::then(unpack_amounts(step_up(slot, j + u * kWarps)), up) : up);
+                }
             }
         }
 #pragma unroll
         for (int u = 0; u < kAtOnce; ++u)
             if (j + u * kWarps < c1) {
                 if (lane == 0) sh.step[j + u * kWarps] = pack_amounts(total[u]);
-                if (sh.slot[j + u * kWarps]) lane_steps(src, j + u * kWarps);
+                if (lanes_at_hand(sh.slot[j + u * kWarps])) lane_steps(src, j + u * kWarps);
             }
     }
     __syncthreads();
@@ -482,19 +518,22 @@ __device__ void segment_steps(Chunk src, int c, int c1) {
         const uint32_t E = sh.E[j];
         if (sh.sorted[j] == 2) sort_in_chunk(src, j);
         if (E == kNoGuess || E == kEmpty) continue;
-        if (sh.slot[j]) { lane_steps(src, j); continue; }   // (sorted now)
+        const int slot = sh.slot[j];
+        if (lanes_at_hand(slot)) { lane_steps(src, j); continue; }   // (sorted now)
         const uint32_t lo = sh.start[j] - src.off, hi = sh.start[j + 1] - src.off;
         for (bool again = true; again;) {
             const bool in_order = sh.sorted[j] == 1;
-            fsx::Step total = fsx::step_identity();
+            fsx::Step total = fsx::step_identity(), total_up = fsx::step_identity();
             again = false;
             for (uint32_t i = lo & ~7u; i < hi && !again; i += kBlock) {
                 float x[8];
                 load8(src.data(), i + 8 * lane, lo, hi, x);
-                bool tie;
+                bool tie, tie_up = false;
                 total = fsx::then(total, block_step(x, E, in_order, &tie));
-                again = tie && !in_order;
+                if (slot) total_up = fsx::then(total_up, block_step(x, E + 1u, in_order, &tie_up));
+                again = (tie || tie_up) && !in_order;
             }
+            if (!again && slot && lane == 0) step_up(slot, j) = pack_amounts(total_up);
             if (again) sort_in_chunk(src, j);
             else if (lane == 0) sh.step[j] = pack_amounts(total);
         }
@@ -518,24 +557,37 @@ __device__ __forceinline__ long long add_segment(Src src, int j, float& s, float
         buf[2 * lane] = make_float4(x[0], x[1], x[2], x[3]);
         buf[2 * lane + 1] = make_float4(x[4], x[5], x[6], x[7]);
         __syncwarp();
-        for (int q = 0; q < kBlock / 4; q += 4) {   // every lane adds the same
-            float4 v[4];
+        float4 v[4], w[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = buf[q + u];
+        for (int u = 0; u < 4; ++u) v[u] = buf[u];
+        for (int q = 0; q < kBlock / 4; q += 16) {   // every lane adds the same, sixteen elements ahead of the additions
             const float before = s;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                s = __fadd_rn(s, v[u].x);
-                s = __fadd_rn(s, v[u].y);
-                s = __fadd_rn(s, v[u].z);
-                s = __fadd_rn(s, v[u].w);
+            for (int h = 0; h < 4; ++h) {
+                float4 (&now)[4] = h & 1 ? w : v;
+                float4 (&next)[4] = h & 1 ? v : w;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) next[u] = buf[(q + 4 * h + 4 + u) & (kBlock / 4 - 1)];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    s = __fadd_rn(s, now[u].x);
+                    s = __fadd_rn(s, now[u].y);
+                    s = __fadd_rn(s, now[u].z);
+                    s = __fadd_rn(s, now[u].w);
+                }
             }
-            if (s > thr) {   // sums only grow: the end of the sixteen tells
+            if (s > thr) {   // sums only grow: the end of the 64 tells
                 s = before;
-                for (int e = 0; e < 16; ++e) {
-                    p = sh.serial[4 * q + e];
-                    s = __fadd_rn(s, p);
-                    if (s > thr) return (long long)src.off + i + 4 * q + e;
+                for (int h = q;; h += 2) {
+                    const float4 a = buf[h], b = buf[h + 1];
+                    float t = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a.x), a.y), a.z), a.w);
+                    t = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(t, b.x), b.y), b.z), b.w);
+                    if (!(t > thr)) { s = t; continue; }
+                    for (int e = 4 * h;; ++e) {
+                        p = sh.serial[e];
+                        s = __fadd_rn(s, p);
+                        if (s > thr) return (long long)src.off + i + e;
+                    }
                 }
             }
         }
@@ -550,43 +602,59 @@ __device__ void walk_segments(Src src, int c, int c1, float s, float thr) {
     ExactShared& sh = shared_memory();
     const int lane = threadIdx.x & 31;
     uint32_t E = fsx::state_exp(s), S = fsx::state_sig(s);
-    int misses = 0;
+    int misses = 0, tiles = 0;
     long long hit = -1;
     PROF_BEGIN;
     while (c < c1) {
         PROF_END(kProfOther);
         PROF_COUNT(kProfTiles);
         const int n = min(32, c1 - c), my = c + lane;
-        fsx::Step st = fsx::step_identity();
-        bool good = true;
-        if (lane < n) {
-            const uint32_t Eg = sh.E[my];
-            good = Eg == kEmpty || (Eg == E && S >= 0x800000u && sh.slot[my] == 0);
-            if (!good) st = fsx::Step{fsx::kSat, fsx::kSat};
-            else if (Eg != kEmpty) st = unpack_amounts(sh.step[my]);
+        const uint32_t Eg = lane < n ? sh.E[my] : kEmpty;
+        uint32_t word = lane < n ? sh.step[my] : 1u;
+        const int own_slot = lane < n ? sh.slot[my] : 0;
+        bool right = Eg == E;
+        if (own_slot && Eg + 1u == E) {   // the sum has changed binade before this one
+            word = own_slot <= kSlots ? sh.from[own_slot - 1][0] : step_up(own_slot, my);
+            right = true;
         }
+        const uint32_t wrong = __ballot_sync(0xffffffffu, !(Eg == kEmpty || (right && S >= 0x800000u)));
+        const int most = wrong ? __ffs(wrong) - 1 : n;   // as far as the guesses hold
+        if (lane == 0) sh.state[c] = fsx::state_float(E, S);
+        if (most > 0) {
+            fsx::Step st = lane < most && Eg != kEmpty ? unpack_amounts(word) : fsx::step_identity();
+            int taken = 0;
+            if (!__any_sync(0xffffffffu, st.a != st.b)) {
+                const uint32_t after = S + __reduce_add_sync(0xffffffffu, st.a);   // 32 x kSat at most
+                if (after < fsx::kOne24 && !(fsx::state_float(E, after) > thr)) {
+                    if (most > 1) {
+                        if (lane == 0) sh.tile[tiles] = (uint16_t)(c | (most - 1) << 11);
+                        ++tiles;
+                        if (lane < most && Eg != kEmpty) sh.step[my] = word;   // (what the sums before them are filled in from)
+                    }
+                    S = after;
+                    taken = most;
+                }
+            }
+            if (taken == 0) {   // a half-way case, or the sum leaves the binade or passes the threshold: one segment after the other
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const fsx::Step up{__shfl_up_sync(0xffffffffu, st.a, o), __shfl_up_sync(0xffffffffu, st.b, o)};
-            if (lane >= o) st = fsx::then(up, st);
-        }
-        const uint32_t after = fsx::apply(st, S);
-        const uint32_t up = __shfl_up_sync(0xffffffffu, after, 1);
-        const uint32_t before = lane > 0 ? up : S;
-        const bool bad = !good || after >= fsx::kOne24 || fsx::state_float(E, after) > thr;
-        const uint32_t mask = __ballot_sync(0xffffffffu, bad);
-        const int first = mask ? __ffs(mask) - 1 : 32;   // below n where any
-        if (lane < n && lane <= first) sh.state[my] = fsx::state_float(E, before);
-        if (first >= n) {
-            S = __shfl_sync(0xffffffffu, after, 31);   // (lanes from n on add nothing)
-            c += n;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const fsx::Step up{__shfl_up_sync(0xffffffffu, st.a, o), __shfl_up_sync(0xffffffffu, st.b, o)};
+                    if (lane >= o) st = fsx::then(up, st);
+                }
+                const uint32_t after = fsx::apply(st, S);
+                const uint32_t up = __shfl_up_sync(0xffffffffu, after, 1);
+                const uint32_t before = lane > 0 ? up : S;
+                const uint32_t mask = __ballot_sync(0xffffffffu, lane < most && (after >= fsx::kOne24 || fsx::state_float(E, after) > thr));
+                taken = mask ? __ffs(mask) - 1 : most;
+                if (lane < n && lane <= taken) sh.state[my] = fsx::state_float(E, before);   // (from `most` on nothing is added)
+                S = taken < 32 ? __shfl_sync(0xffffffffu, before, taken & 31) : __shfl_sync(0xffffffffu, after, 31);
+            }
+            c += taken;
             PROF_END(kProfTile);
-            continue;
+            if (taken == n) continue;
+            if (lane == 0) sh.state[c] = fsx::state_float(E, S);
         }
-        S = __shfl_sync(0xffffffffu, before, first);
-        c += first;
-        PROF_END(kProfTile);
-        if (sh.slot[c] && S >= 0x800000u) {   // the sum may change binade in this one: its lanes' amounts are at hand
+        if (lanes_at_hand(sh.slot[c]) && S >= 0x800000u) {   // the sum may change binade in this one: its lanes' amounts are at hand
             const int slot = sh.slot[c] - 1;
             const uint32_t Eg = sh.E[c];
             uint32_t E2 = E, S2 = fsx::kOne24;
@@ -639,22 +707,42 @@ __device__ void walk_segments(Src src, int c, int c1, float s, float thr) {
         if (hit >= 0) break;
         ++c;
     }
-    if (lane == 0) { sh.bc_s = fsx::state_float(E, S); sh.bc_seg = c; sh.bc_hit = hit; }
+    if (lane == 0) { sh.bc_s = fsx::state_float(E, S); sh.bc_seg = c; sh.bc_hit = hit; sh.tiles = tiles; }
+}
+// The sums before the segments of the runs that the walk took as a whole.
+__device__ void fill_states() {
+    ExactShared& sh = shared_memory();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t = warp; t < sh.tiles; t += kWarps) {
+        const int c = sh.tile[t] & 2047, n = (sh.tile[t] >> 11) + 1;
+        const float s = sh.state[c];
+        uint32_t sum = lane < n && sh.E[c + lane] != kEmpty ? sh.step[c + lane] >> 2 : 0u;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += up;
+        }
+        const uint32_t before = __shfl_up_sync(0xffffffffu, sum, 1);
+        if (lane > 0 && lane < n) sh.state[c + lane] = fsx::state_float(fsx::state_exp(s), fsx::state_sig(s) + before);
+    }
 }
 
-// Adds the segments c .. c1 - 1 to s in order, exactly as `s += x[i]` does, from the approximate sums in sh.cum.  It stops at the
-// first running sum above thr and returns that element, else -1.  sh.state: the sum before every segment it came to.
+// Adds the segments c .. c1 - 1 to s in order, exactly as `s += x[i]` does, from the approximate sums in sh.cum (have_steps: the guesses
+// are made and the amounts known).  It stops at the first running sum above thr and returns that element, else -1.  sh.state: the sum before every segment it came to.
 template <class Src>
-__device__ __noinline__ long long ordered_sum(Src src, int c, int c1, float& s, float thr, float thr2) {
+__device__ __noinline__ long long ordered_sum(Src src, int c, int c1, float& s, float thr, float thr2, bool have_steps = false) {
     ExactShared& sh = shared_memory();
     PROF_BEGIN;
-    for (;;) {
-        guess_binades(c, c1, s, thr, thr2);
-        PROF_END(kProfGuess);
-        segment_steps(src, c, c1);
-        PROF_END(kProfSteps);
+    for (;; have_steps = false) {
+        if (!have_steps) {
+            guess_binades(c, c1, s, thr, thr2, !Src::kSortable);
+            PROF_END(kProfGuess);
+            segment_steps(src, c, c1);
+            PROF_END(kProfSteps);
+        }
         if (threadIdx.x < 32) walk_segments(src, c, c1, s, thr);
         __syncthreads();
+        fill_states();
         PROF_END(kProfWalk);
         s = sh.bc_s; c = sh.bc_seg;
         const long long hit = sh.bc_hit;
@@ -662,17 +750,13 @@ __device__ __noinline__ long long ordered_sum(Src src, int c, int c1, float& s, 
         if (hit >= 0 || c >= c1) return hit;
     }
 }
-// The same over a whole row in index order, from the approximate sums before its segments.
-template <class Src>
-__device__ __noinline__ float index_order_sum(Src src, Segs g, uint32_t V) {
+// The segments of a row in index order: elements lo .. hi - 1.
+__device__ void index_order_segments(Segs g, uint32_t lo, uint32_t hi) {
     ExactShared& sh = shared_memory();
     for (int j = threadIdx.x; j <= g.count; j += kThreads) {
-        sh.start[j] = min(V, (uint32_t)j << g.shift);
+        sh.start[j] = max(lo, min(hi, (uint32_t)j << g.shift));
         if (j < g.count) sh.sorted[j] = 1;
     }
-    float s = 0.f;
-    ordered_sum(src, 0, g.count, s, CUDART_INF_F, -1.f);
-    return s;
 }
 
 // ---- descending order --------------------------------------------------------------------------------------
@@ -699,11 +783,12 @@ __device__ __forceinline__ void put_below(uint32_t addr, float v, uint32_t x, ui
     asm volatile("{ .reg .pred p; setp.lt.u32 p, %2, %3; @p st.shared.f32 [%0], %1; }" ::"r"(addr), "f"(v), "r"(x), "r"(end) : "memory");
 }
 
-// Calls fn(four elements) for the row's exponentials, 16-byte loads, four in flight per thread; zeros beyond the row.
+// Calls fn(four elements) for the exponentials, 16-byte loads, four in flight per thread.  The row begins on a 16-byte boundary, its
+// elements are those from lo to hi - 1, and what the first and the last load bring along are zeros.
 template <class F>
-__device__ __forceinline__ void for_exponentials(const float* ex, uint32_t V, F&& fn) {
+__device__ __forceinline__ void for_exponentials(const float* ex, uint32_t hi, F&& fn) {
     const float4* e4 = reinterpret_cast<const float4*>(ex);
-    const uint32_t n4 = V >> 2;
+    const uint32_t n4 = (hi + 3) >> 2;
     for (uint32_t i = threadIdx.x; i < n4; i += 4 * kThreads) {
         float4 v[4];
 #pragma unroll
@@ -711,23 +796,16 @@ __device__ __forceinline__ void for_exponentials(const float* ex, uint32_t V, F&
 #pragma unroll
         for (int u = 0; u < 4; ++u) fn(v[u]);
     }
-    if (threadIdx.x == 0 && (V & 3)) {
-        float t[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-        for (int e = 0; e < 3; ++e)
-            if (4 * n4 + e < V) t[e] = ex[4 * n4 + e];
-        fn(make_float4(t[0], t[1], t[2], 0.f));
-    }
 }
 
-__device__ __noinline__ void count_level(Level& L, const float* ex, uint32_t V) {
+__device__ __noinline__ void count_level(Level& L, const float* ex, uint32_t hi) {
     ExactShared& sh = shared_memory();
     __syncthreads();
     for (int j = threadIdx.x; j < kBins; j += kThreads) sh.bins[j] = 0;
     __syncthreads();
     bool rest = false;
     const uint32_t bins = (uint32_t)__cvta_generic_to_shared(sh.bins);
-    for_exponentials(ex, V, [&](float4 v) {
+    for_exponentials(ex, hi, [&](float4 v) {
         const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -801,10 +879,10 @@ __device__ __noinline__ int rank_bins(Level& L, Segs g, int c, uint32_t placed, 
 }
 
 struct Row {
-    const float* ex;    // exponentials in index order
+    const float* ex;    // exponentials in index order: elements lo .. hi - 1
     float* sorted;      // the largest probabilities, as far as they were needed: segment by segment in descending order, those within
                         // a segment only where it mattered
-    uint32_t V;
+    uint32_t lo, hi;
     float norm, inv_norm, min_thr;
 };
 
@@ -822,7 +900,7 @@ __device__ __noinline__ uint32_t place_chunk(Row row, Level L, Segs g, int c, in
     const long long below = (long long)L.F - ((long long)j1 << L.shift);
     const uint32_t low = below > 1 ? (uint32_t)below : 1u;
     const uint32_t bins = (uint32_t)__cvta_generic_to_shared(sh.bins), keys = (uint32_t)__cvta_generic_to_shared(sh.keys) - 4 * (off - placed);
-    for_exponentials(row.ex, row.V, [&](float4 v) {
+    for_exponentials(row.ex, row.hi, [&](float4 v) {
         const float e[4] = {v.x, v.y, v.z, v.w};
         uint32_t pos[4];
 #pragma unroll
@@ -923,7 +1001,7 @@ __device__ __noinline__ Kept keep_top_p(Row row, Segs g, Level L, float top_p, f
     while (!last) {
         PROF_BEGIN;
         // room for the segments of all that is left (a row of many levels: one or two extra for each)
-        const uint32_t most = (row.V - placed) >> g.shift;
+        const uint32_t most = (row.hi - placed) >> g.shift;
         while (c > 1 && (uint32_t)c + most + 2 * (most / kBigSegs) + 4 > (uint32_t)kSegCap) c = merge_segments(c);
         int reach;
         const int end = rank_bins(L, g, c, placed, row.inv_norm, s, top_p * (1.0f + 1.0f / 1024), &reach);
@@ -990,12 +1068,12 @@ __device__ __noinline__ Kept keep_top_p(Row row, Segs g, Level L, float top_p, f
             L = Level{(uint32_t)(L.F - span), next_shift, 0, false};
         }
         if (L.F <= 1u) break;
-        count_level(L, row.ex, row.V);
+        count_level(L, row.ex, row.hi);
     }
     // every candidate is in the sum; without a min-p threshold the zeros are candidates too
     uint32_t zeros = 0;
     if (!last && 0.f >= row.min_thr) {
-        for (uint32_t i = tid; i < row.V; i += kThreads) zeros += row.ex[i] == 0.f ? 1u : 0u;
+        for (uint32_t i = row.lo + tid; i < row.hi; i += kThreads) zeros += row.ex[i] == 0.f ? 1u : 0u;
         zeros = block_sum(zeros, sh.scan_u);
     }
     while (c > 0 && sh.start[c - 1] >= placed) --c;   // segments of nothing but zeros
@@ -1026,7 +1104,7 @@ __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p)
     };
     uint32_t same = 0, lowest = 0xffffffffu;
     const float4* e4 = reinterpret_cast<const float4*>(row.ex);
-    const uint32_t n4 = (row.V + 3) >> 2;   // (the row's pitch is a multiple of four; what lies beyond the row is not counted)
+    const uint32_t n4 = (row.hi + 3) >> 2;
     const uint32_t span = key_lo ? key_hi - key_lo : 0xffffffffu;
     for (uint32_t i0 = threadIdx.x; i0 < n4; i0 += 4 * kThreads) {
         float4 v[4];
@@ -1042,16 +1120,16 @@ __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p)
 #pragma unroll 1
         for (int u = 0; u < 16; ++u) {
             const uint32_t i = 4 * (i0 + (u >> 2) * kThreads) + (u & 3);
-            if (i < row.V && equal(row.ex[i])) { ++same; lowest = min(lowest, i); }
+            if (i >= row.lo && i < row.hi && equal(row.ex[i])) { ++same; lowest = min(lowest, i); }
         }
     }
     __syncthreads();
     same = block_sum(same, sh.scan_u);
     lowest = block_reduce(lowest, [](uint32_t a, uint32_t b) { return min(a, b); }, sh.scan_u);
     PROF_END(kProfIndex);
-    if (same <= 1 || same > kMostEqual) return lowest == 0xffffffffu ? 0 : (long long)lowest;
+    if (same <= 1 || same > kMostEqual) return lowest == 0xffffffffu ? row.lo : (long long)lowest;
     // several: the rank among them
-    const uint32_t blocks = (row.V + kBlock - 1) / kBlock, per = (blocks + kWarps - 1) / kWarps;
+    const uint32_t blocks = (row.hi + kBlock - 1) / kBlock, per = (blocks + kWarps - 1) / kWarps;
     const uint32_t b0 = min(blocks, warp * per), b1 = min(blocks, b0 + per);
     uint32_t greater = 0;
     same = 0;
@@ -1059,7 +1137,7 @@ __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p)
         const uint32_t i = b * kBlock + 8 * lane;
 #pragma unroll
         for (int e = 0; e < 8; ++e)
-            if (i + e < row.V) {
+            if (i + e >= row.lo && i + e < row.hi) {
                 const float q = probability(row.ex[i + e], row.norm, row.inv_norm);
                 same += q == p ? 1u : 0u;
                 greater += q > p ? 1u : 0u;
@@ -1079,7 +1157,7 @@ __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p)
             uint32_t mine = 0;   // a bit per element
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-                if (i + e < row.V && probability(row.ex[i + e], row.norm, row.inv_norm) == p) mine |= 1u << e;
+                if (i + e >= row.lo && i + e < row.hi && probability(row.ex[i + e], row.norm, row.inv_norm) == p) mine |= 1u << e;
             uint32_t incl = __popc(mine);
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -1187,92 +1265,160 @@ __device__ __forceinline__ float expf_lanes_nonpositive(float x, uint32_t tab_lo
     return (float)__dmul_rn(y, s);
 }
 
-__device__ float row_maximum(const float* row, uint32_t V, bool vec_ok, bool* has_nan) {
+// The elements of a logits row from an address on a 16-byte boundary on: lo .. hi - 1 of `base`.
+struct Logits {
+    const float* base;
+    uint32_t lo, hi;
+    // i: a multiple of four; -inf beyond the elements.  kLast: the row is not read again, its place in L2 is the exponentials'
+    template <bool kLast = false>
+    __device__ __forceinline__ void load4(uint32_t i, float (&x)[4]) const {
+        if (i >= lo && i + 4 <= hi) {
+            const float4* at = reinterpret_cast<const float4*>(base + i);
+            const float4 q = kLast ? __ldcs(at) : *at;
+            x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] = i + e >= lo && i + e < hi ? base[i + e] : -CUDART_INF_F;
+        }
+    }
+};
+
+// Maximum of the row and, for `masses`, the approximate sums of the exponentials before its segments (of one block each), from the
+// maxima and masses of 1024 elements at a time; *odd: the row holds NaN or +inf.  Bound by HBM.
+__device__ __noinline__ float survey(Logits row, Segs g, float inv_T, bool masses, bool* odd) {
     ExactShared& sh = shared_memory();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr float kLog2e = 1.442695040888963f;
+    const float scale = inv_T * kLog2e;
+    const uint32_t blocks = (row.hi + kBlock - 1) / kBlock;
     float mx = -CUDART_INF_F;
     bool bad = false;
-    auto take = [&](float x) { mx = fmaxf(mx, x); bad |= x != x; };
-    if (vec_ok) {
-        const float4* r4 = reinterpret_cast<const float4*>(row);
-        const uint32_t n4 = V >> 2;
-        for (uint32_t i = threadIdx.x; i < n4; i += 8 * kThreads) {
-            float4 q[8];
+    for (uint32_t b = 4 * warp; b < blocks; b += 4 * kWarps) {
+        float x[8][4];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) q[u] = i + u * kThreads < n4 ? r4[i + u * kThreads] : make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+        for (int u = 0; u < 8; ++u) row.load4(b * kBlock + u * 128 + 4 * lane, x[u]);
+        float top = -CUDART_INF_F;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) { take(q[u].x); take(q[u].y); take(q[u].z); take(q[u].w); }
+        for (int u = 0; u < 8; ++u) top = fmaxf(top, fmaxf(fmaxf(x[u][0], x[u][1]), fmaxf(x[u][2], x[u][3])));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        mx = fmaxf(mx, top);
+        const float ref = top == -CUDART_INF_F ? 0.f : -top * scale;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float m = 0.f;
+#pragma unroll
+            for (int u = 2 * k; u < 2 * k + 2; ++u)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float y;
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaf(x[u][e], scale, ref)));
+                    m += y;   // NaN where the row or the temperature is odd
+                }
+            bad |= !(m < CUDART_INF_F);
+            if (masses) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+                if (lane == 0 && b + k < blocks) { sh.cum[b + k] = m; sh.state[b + k] = top; }
+            }
         }
-        for (uint32_t j = 4 * n4 + threadIdx.x; j < V; j += kThreads) take(row[j]);
-    } else {
-        for (uint32_t i = threadIdx.x; i < V; i += kThreads) take(row[i]);
     }
-    *has_nan = __syncthreads_or(bad) != 0;
-    return block_reduce(mx, [](float a, float b) { return fmaxf(a, b); }, sh.scan_f);
+    *odd = __syncthreads_or(bad) != 0;
+    mx = block_reduce(mx, [](float a, float b) { return fmaxf(a, b); }, sh.scan_f);
+    if (masses && !*odd) {
+        for (int j = threadIdx.x; j < g.count; j += kThreads) sh.cum[j] *= exp2f((sh.state[j] - mx) * scale);   // (-inf: 0)
+        masses_to_sums(g.count);
+    }
+    return mx;
 }
 
-// Exponentials of the row into ex[], the masses of the segments into sh.cum, and with kCount the counts of the first level's bins.
-// Bound by instruction issue (some 30 per element, eight of them in double precision).
+// Exponentials of the row into ex[], with kCount the counts of the first level's bins, and the amounts of the segments (of one block
+// each) under the guesses made.  For rows and temperatures that make every exponential a number from 0 to 1.
+// Bound by instruction issue (some 35 per element, eight of them in double precision).
 template <bool kCount>
-__device__ __noinline__ void exponentials(const float* row, uint32_t V, bool vec_ok, bool plain, Segs g, float mx, float inv_T, float* ex, Level& level) {
+__device__ __noinline__ void exponentials(Logits row, float mx, float inv_T, float* ex, Level& level) {
     ExactShared& sh = shared_memory();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t tab = fsx::kExp2TabDev[lane];
     const uint32_t tab_lo = (uint32_t)tab, tab_hi = (uint32_t)(tab >> 32);
     const uint32_t bins = (uint32_t)__cvta_generic_to_shared(sh.bins);
-    for (int j = tid; j < g.count; j += kThreads) sh.cum[j] = 0.f;
     if (kCount)
         for (int j = tid; j < kBins; j += kThreads) sh.bins[j] = 0;
     __syncthreads();
     bool rest = false;
-    const uint32_t blocks = (V + kBlock - 1) / kBlock;
-    for (uint32_t b = 2 * warp; b < blocks; b += 2 * kWarps) {   // two blocks: four 16-byte loads in flight per lane
-        float mass[2] = {0.f, 0.f};
-        if (plain && vec_ok && (b + 2) * kBlock <= V) {
-            float4 x[4];
+    const uint32_t blocks = (row.hi + kBlock - 1) / kBlock;
+    for (uint32_t b = warp; b < blocks; b += 2 * kWarps) {   // two blocks: four 16-byte loads in flight per lane
+        float x[2][2][4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) x[u] = *reinterpret_cast<const float4*>(row + b * kBlock + u * 128 + 4 * lane);
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                float y[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
+            for (int u = 0; u < 2; ++u) row.load4<true>((b + h * kWarps) * kBlock + 8 * lane + 4 * u, x[h][u]);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) y[e] = expf_lanes_nonpositive(__fmul_rn(__fsub_rn(y[e], mx), inv_T), tab_lo, tab_hi);   // (inv_T 1: as it is)
-                mass[u >> 1] += (y[0] + y[1]) + (y[2] + y[3]);
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t j = b + h * kWarps;
+            if (j >= blocks) break;
+            float y[8];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) y[4 * u + e] = expf_lanes_nonpositive(__fmul_rn(__fsub_rn(x[h][u][e], mx), inv_T), tab_lo, tab_hi);   // (inv_T 1: as it is)
                 if (kCount) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        const uint32_t bin = (kOneBits - __float_as_uint(y[e])) >> kTopShift;
+                        const uint32_t bin = (kOneBits - __float_as_uint(y[4 * u + e])) >> kTopShift;
                         count_below(bins + 4 * bin, bin, (uint32_t)kBins);
                         rest |= bin >= (uint32_t)kBins;   // (zeros too: the next level's counts tell)
                     }
                 }
-                *reinterpret_cast<float4*>(ex + b * kBlock + u * 128 + 4 * lane) = make_float4(y[0], y[1], y[2], y[3]);
+                *reinterpret_cast<float4*>(ex + j * kBlock + 8 * lane + 4 * u) = make_float4(y[4 * u], y[4 * u + 1], y[4 * u + 2], y[4 * u + 3]);
             }
-        } else {
-            for (int u = 0; u < 16; ++u) {
-                const uint32_t i = b * kBlock + u * 32 + lane;
-                const float d = i < V ? __fsub_rn(row[i], mx) : -CUDART_INF_F;
-                const float y = expf_lanes(__fmul_rn(d, inv_T), tab_lo, tab_hi);
-                if (i < V) {
-                    if (y >= 0.f) mass[u >> 3] += y;
-                    ex[i] = y;
-                    const uint32_t key = __float_as_uint(y);
-                    if (kCount && key - 1u < kOneBits) {
-                        const uint32_t bin = (kOneBits - key) >> kTopShift;
-                        if (bin < (uint32_t)kBins) atomicAdd(&sh.bins[bin], 1u);
-                        else rest = true;
-                    }
+            const uint32_t E = sh.E[j];
+            const int slot = sh.slot[j];
+            if (lanes_at_hand(slot)) {
+                __syncwarp();   // the block's exponentials are in memory
+                lane_steps(Exponentials{ex, 0}, (int)j);
+            } else if (E != kNoGuess && E != kEmpty) {
+                bool tie;
+                const fsx::Step st = block_step(y, E, true, &tie);
+                if (lane == 0) sh.step[j] = pack_amounts(st);
+                if (slot) {
+                    const fsx::Step up = block_step(y, E + 1u, true, &tie);
+                    if (lane == 0) step_up(slot, (int)j) = pack_amounts(up);
                 }
             }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mass[h] += __shfl_xor_sync(0xffffffffu, mass[h], o);
-            if (lane == 0 && b + h < blocks) atomicAdd(&sh.cum[((b + h) * kBlock) >> g.shift], mass[h]);
         }
     }
     rest = __syncthreads_or(rest) != 0;
     level = Level{kOneBits + 1u, kTopShift, 0, rest};
+}
+// The same for any row and temperature, and the sums before the segments.
+__device__ __noinline__ void exponentials_any(Logits row, Segs g, float mx, float inv_T, float* ex) {
+    ExactShared& sh = shared_memory();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t tab = fsx::kExp2TabDev[lane];
+    const uint32_t tab_lo = (uint32_t)tab, tab_hi = (uint32_t)(tab >> 32);
+    for (int j = tid; j < g.count; j += kThreads) sh.cum[j] = 0.f;
+    __syncthreads();
+    const uint32_t blocks = (row.hi + kBlock - 1) / kBlock;
+    for (uint32_t b = warp; b < blocks; b += kWarps) {
+        float mass = 0.f;
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t i = b * kBlock + u * 128 + 4 * lane;
+            float x[4];
+            row.load4(i, x);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float y = expf_lanes(__fmul_rn(__fsub_rn(x[e], mx), inv_T), tab_lo, tab_hi);
+                x[e] = i + e >= row.lo && i + e < row.hi ? y : 0.f;
+                if (x[e] >= 0.f) mass += x[e];
+            }
+            *reinterpret_cast<float4*>(ex + i) = make_float4(x[0], x[1], x[2], x[3]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
+        if (lane == 0) atomicAdd(&sh.cum[(b * kBlock) >> g.shift], mass);
+    }
+    masses_to_sums(g.count);
 }
 
 __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
@@ -1283,9 +1429,10 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
     const float* logits = a.logits + p.logits_row * a.vocab;
     const bool raw_lp = (p.do_sample & SAMPLER_ROW_RAW_LOG_PROB) != 0;
     const float raw_lse = raw_lp ? a.out_log_prob[r] : 0.f;   // left there by the first kernel (NaN: no scratch for the raw logits)
-    const bool vec_ok = (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
     const bool top_p_active = p.top_p != 1.0f;
-    const Segs g = segments_of(a.vocab);
+    const uint32_t lo = (uint32_t)(reinterpret_cast<uintptr_t>(logits) & 15) / 4, hi = lo + V;   // (a row may begin anywhere)
+    const Logits in{logits - lo, lo, hi};
+    const Segs g = segments_of(hi);
     float* ex = scratch;
     float* sorted = scratch + sampler_exact_pitch(a.vocab);
     const float inv_T = __fdiv_rn(1.0f, p.temperature);
@@ -1295,20 +1442,30 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
 #endif
     __syncthreads();
     PROF_BEGIN;
-    bool has_nan;
-    const float mx = row_maximum(logits, V, vec_ok, &has_nan);
+    bool odd;
+    const bool one_block = g.shift == 8;
+    const float mx = survey(in, g, inv_T, one_block, &odd);
     PROF_END(kProfMax);
-    const bool plain = !has_nan && fabsf(mx) < CUDART_INF_F && inv_T > 0.f && inv_T < CUDART_INF_F;   // every exponential is between 0 and 1
-    Level level;
-    if (top_p_active) exponentials<true>(logits, V, vec_ok, plain, g, mx, inv_T, ex, level);
-    else exponentials<false>(logits, V, vec_ok, plain, g, mx, inv_T, ex, level);
-    PROF_END(kProfExp);
-    masses_to_sums(g.count);
-    const float norm = index_order_sum(Exponentials{ex, 0}, g, V);
+    const bool plain = !odd && fabsf(mx) < CUDART_INF_F && inv_T > 0.f && inv_T < CUDART_INF_F;   // every exponential is between 0 and 1
+    index_order_segments(g, lo, hi);
+    Level level{kOneBits + 1u, kTopShift, 0, false};
+    float norm = 0.f;
+    if (plain && one_block) {
+        guess_binades(0, g.count, 0.f, CUDART_INF_F, -1.f, true);
+        if (top_p_active) exponentials<true>(in, mx, inv_T, ex, level);
+        else exponentials<false>(in, mx, inv_T, ex, level);
+        PROF_END(kProfExp);
+        ordered_sum(Exponentials{ex, 0}, 0, g.count, norm, CUDART_INF_F, -1.f, true);
+    } else {
+        exponentials_any(in, g, mx, inv_T, ex);
+        if (top_p_active) count_level(level, ex, hi);
+        PROF_END(kProfExp);
+        ordered_sum(Exponentials{ex, 0}, 0, g.count, norm, CUDART_INF_F, -1.f);
+    }
     const float inv_norm = __fdiv_rn(1.0f, norm);   // the largest probability, that of the maximum, and the shared reciprocal of the divisions
     const bool any = norm > 0.0f;                   // else every probability is NaN: none is kept
     const float min_thr = p.min_p > 0.0f ? __fmul_rn((float)(double)p.min_p, inv_norm) : 0.0f;
-    const Row row{ex, sorted, V, norm, inv_norm, min_thr};
+    const Row row{ex, sorted, lo, hi, norm, inv_norm, min_thr};
     const Probabilities probs{ex, 0, norm, inv_norm, min_thr};
     Kept kept{0, 0, 0, 0.f};
     float total = 0.0f;
@@ -1319,7 +1476,7 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
         // approximate sums: those of the exponentials over the norm (min-p drops mass: guesses that do not hold cost time only)
         __syncthreads();
         for (int j = tid; j <= g.count; j += kThreads) sh.cum[j] *= inv_norm;
-        total = index_order_sum(probs, g, V);
+        ordered_sum(probs, 0, g.count, total, CUDART_INF_F, -1.f);
     }
     const bool uniform_fallback = !(total > 0.0f && isfinite(total)) || (top_p_active && kept.n == 0);
     long long kept_count = kept.n, last_kept = -1;
@@ -1329,7 +1486,7 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
         looked = true;
         uint32_t n = 0;
         int last = -1;
-        for (uint32_t i = tid; any && i < V; i += kThreads)
+        for (uint32_t i = lo + tid; any && i < hi; i += kThreads)
             if (probability(ex[i], norm, inv_norm) >= min_thr) { ++n; last = (int)i; }
         kept_count = block_sum(n, sh.scan_u);
         last_kept = block_reduce(last, [](int x, int y) { return max(x, y); }, sh.red_i);
@@ -1343,19 +1500,20 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
         else {
             const float rr = __fmul_rn(total, u);
             if (!top_p_active) {
-                pick = find_draw(probs, g.count, V, nullptr, rr, pick_p);
+                pick = find_draw(probs, g.count, hi, nullptr, rr, pick_p);
                 if (pick < 0) {   // rounding left r at or beyond the total: the last kept element
                     look();
                     pick = last_kept;
-                    pick_p = probability(ex[pick < 0 ? 0 : pick], norm, inv_norm);
+                    pick_p = probability(ex[pick < 0 ? lo : pick], norm, inv_norm);
                 }
+                pick -= lo;
             } else {
                 long long rank = find_draw(Sorted{sorted, 0}, kept.segs, kept.n, sorted, rr, pick_p);
                 if (rank < 0) {   // the last of the kept ones
                     rank = (long long)kept.n - 1;
                     pick_p = rank < (long long)kept.placed ? sorted[rank] : 0.f;
                 }
-                pick = index_of_rank(row, (uint32_t)rank, pick_p);
+                pick = index_of_rank(row, (uint32_t)rank, pick_p) - lo;
             }
         }
         if (tid == 0) {

@@ -43,7 +43,7 @@ size_t sampler_smem_bytes();
 // Full-vocabulary multinomial rows (sampler_exact.cu).  `scratch` holds two rows per CTA of the persistent grid, the exponentials
 // and the kept probabilities in descending order: sampler_exact_scratch_bytes(ctas, vocab) bytes.
 cudaError_t launch_sampler_exact(const StepArgs& a, float* scratch, int ctas, cudaStream_t stream);
-__host__ __device__ inline size_t sampler_exact_pitch(long long vocab) { return (size_t)((vocab + 255) & ~255LL); }   // floats per row
+__host__ __device__ inline size_t sampler_exact_pitch(long long vocab) { return (size_t)((vocab + 3 + 255) & ~255LL); }   // floats per row, which may begin with up to three that are not the row's
 size_t sampler_exact_scratch_bytes(int ctas, long long vocab);
 cudaError_t launch_expf_selftest(const float* in, float* out, long long n, cudaStream_t stream);
 constexpr int kSamplerMaxTopK = 1024;   // heap capacity of the top-k path
