@@ -14,9 +14,8 @@
 //      order of operations.  A step (both launches, no penalties, logits in place) of 256 rows x
 //      151936, K 50: 301 -> 91 us (the serial replay, about 400 replacements of 250 cycles with two
 //      rows per SM, is what a row waits for; reading the rows takes 24 us); 5 rows x 32000: 215 -> 50 us;
-//   4. multinomial rows over the full vocabulary get their penalties here and are finished by
-//      sampler_exact_kernel (sampler_exact.cu), which reproduces the reference's index-order and
-//      sorted-order float sums exactly.
+//   4. multinomial rows over the full vocabulary are left to sampler_exact_kernel (sampler_exact.cu), which reproduces the
+//      reference's index-order and sorted-order float sums exactly and runs beside this kernel where there is room.
 // Greedy rows are bound by reading the row once (HBM from some 100 rows on, latency below); top-k rows by the serial replay;
 // what the whole-vocabulary rows wait for is said in sampler_exact.cu.
 #include <cuda_runtime.h>
@@ -25,6 +24,7 @@
 
 #include "../../include/sampler_b200.h"
 #include "sampler_kernels.h"
+#include "sampler_rows.cuh"
 
 namespace sampler {
 
@@ -389,30 +389,6 @@ __device__ void std_sort(Cand* v, int n) {
 }
 
 // ---- block reductions -------------------------------------------------------------------------------
-template <class T>
-__device__ __forceinline__ T shfl_xor_any(T v, int o) {
-    static_assert(sizeof(T) % 4 == 0, "word-sized types only");
-    union { T t; uint32_t w[sizeof(T) / 4]; } in, out;
-    in.t = v;
-#pragma unroll
-    for (int i = 0; i < (int)(sizeof(T) / 4); ++i) out.w[i] = __shfl_xor_sync(0xffffffffu, in.w[i], o);
-    return out.t;
-}
-
-template <class T, class Op>
-__device__ T block_reduce(T v, T identity, Op op, T* sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = op(v, shfl_xor_any(v, o));
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[w] = v;
-    __syncthreads();
-    v = lane < kWarps ? sh[lane] : identity;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = op(v, shfl_xor_any(v, o));
-    return v;
-}
-
 struct ArgMax {
     float v;
     int i;
@@ -427,35 +403,6 @@ __device__ __forceinline__ ArgMax better(ArgMax a, ArgMax b) {
 __device__ __forceinline__ uint32_t float_key(float x) {
     const uint32_t b = __float_as_uint(x);
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
-// Calls fn(value, index) once for every element of a row, in no particular order. 16-byte loads,
-// four of them in flight per thread: with one 4-byte load per iteration a pass over the row is bound
-// by the latency of that load, not by bandwidth.
-template <class F>
-__device__ __forceinline__ void for_row(const float* row, long long V, int tid, F&& fn) {
-    if ((reinterpret_cast<uintptr_t>(row) & 15) != 0) {
-        for (long long i = tid; i < V; i += kThreads) fn(row[i], i);
-        return;
-    }
-    const float4* r4 = reinterpret_cast<const float4*>(row);
-    const long long n4 = V >> 2;
-    long long i = tid;
-    for (; i + 3 * kThreads < n4; i += 4 * kThreads) {
-        float4 v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = r4[i + u * kThreads];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const long long e = 4 * (i + u * kThreads);
-            fn(v[u].x, e); fn(v[u].y, e + 1); fn(v[u].z, e + 2); fn(v[u].w, e + 3);
-        }
-    }
-    for (; i < n4; i += kThreads) {
-        const float4 v = r4[i];
-        fn(v.x, 4 * i); fn(v.y, 4 * i + 1); fn(v.z, 4 * i + 2); fn(v.w, 4 * i + 3);
-    }
-    for (long long j = 4 * n4 + tid; j < V; j += kThreads) fn(row[j], j);
 }
 
 constexpr int kSortWarp = 128;   // candidates one warp ranks by counting
@@ -476,33 +423,6 @@ struct Shared {
     unsigned long long red_u[kWarps];
     ArgMax red_a[kWarps];
 };
-
-// ---- phase 1: penalties ---------------------------------------------------------------------------------
-__device__ void apply_history(float* row, long long V, const sampler_row_params& p, const int32_t* ids, const uint32_t* meta,
-                              long long n, uint32_t* status, float* raw_out) {
-    const double rep = (double)p.repetition_penalty, pres = (double)p.presence_penalty, freq = (double)p.frequency_penalty;
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-        const int id = ids[i];
-        const uint32_t m = meta[i];
-        if (id < 0 || id >= V) {
-            atomicOr(status, 1u);
-            continue;
-        }
-        float v = row[id];
-        if (raw_out) raw_out[i] = v;   // the raw logit, for rows that report raw log-probabilities
-        if (m & SAMPLER_HIST_STOP_MASK) v = -CUDART_INF_F;
-        if (p.repetition_penalty != 1.0f && (m & (SAMPLER_HIST_IN_PROMPT | SAMPLER_HIST_GENERATED)))
-            v = v >= 0 ? (float)__ddiv_rn((double)v, rep) : (float)__dmul_rn((double)v, rep);
-        if (m & SAMPLER_HIST_GENERATED) {
-            if (p.presence_penalty != 0.0f) v = v >= 0 ? (float)__dsub_rn((double)v, pres) : (float)__dadd_rn((double)v, pres);
-            if (p.frequency_penalty != 0.0f) {
-                const double t = __dmul_rn(freq, (double)(m >> 3));
-                v = v >= 0 ? (float)__dsub_rn((double)v, t) : (float)__dadd_rn((double)v, t);
-            }
-        }
-        row[id] = v;
-    }
-}
 
 // ---- phase 3 tail: softmax / min-p / top-p over the K heap entries, then the draws, one thread -------
 // Mirrors TemperatureLogitTransform, MinPFilter, TopPFilter (logit_transformers.hpp:90-362) and
@@ -917,6 +837,8 @@ __device__ __noinline__ void replay_unordered(Shared& sh, long long V, int K) {
 __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
+    // the next kernel's CTAs may come as soon as every CTA of this one is there (they wait for its end before they leave)
+    asm volatile("griddepcontrol.launch_dependents;");
     const int r = blockIdx.x;
     const sampler_row_params p = a.rows[r];
     const long long V = a.vocab;
@@ -929,57 +851,19 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
 
     const bool multinomial = (p.do_sample & SAMPLER_ROW_MULTINOMIAL) != 0;
     const bool raw_lp = (p.do_sample & SAMPLER_ROW_RAW_LOG_PROB) != 0;
-    const long long h0 = a.hist_offsets ? a.hist_offsets[r] : 0, h1 = a.hist_offsets ? a.hist_offsets[r + 1] : 0;
+    const RowHistory hist = row_history(a, r);
 
-    // ---- 0. log-partition of the raw row (FullVocabLogSumExpTransform, logit_transformers.hpp:264-277) ----
-    // The reference adds the exponentials in single precision in index order; here they are added in
-    // double precision in parallel and rounded once, which is within an ulp or two of any float order.
+    // Whole-vocabulary rows are the next kernel's from the beginning on: it may run beside this one.
+    if (whole_vocabulary_row(p, V)) return;
+
+    // ---- 0. log-partition of the raw row -----------------------------------------------------------
     float raw_lse = 0.f;
     bool raw_ok = true;
-    if (raw_lp) {
-        float mx0 = -CUDART_INF_F;
-        for_row(row, V, tid, [&](float x, long long) { mx0 = fmaxf(mx0, x); });
-        mx0 = block_reduce(mx0, -CUDART_INF_F, [](float x, float y) { return fmaxf(x, y); }, sh.red_f);
-        double s0 = 0.0;
-        for_row(row, V, tid, [&](float x, long long) { s0 += (double)expf(x - mx0); });
-        s0 = block_reduce(s0, 0.0, [](double x, double y) { return x + y; }, sh.red_d);
-        raw_lse = logf((float)s0) + mx0;
-        if (h1 > h0 && !a.hist_raw) {
-            raw_ok = false;
-            if (tid == 0) atomicOr(a.status, 4u);
-        }
-    }
-    // the raw log-probability of the selected token: its logit before the penalties minus the log-partition
-    auto raw_log_prob = [&](long long idx) {
-        if (!raw_ok) return CUDART_NAN_F;
-        float raw = row[idx];
-        for (long long i = h0; i < h1; ++i)
-            if (a.hist_ids[i] == idx) { raw = a.hist_raw[i]; break; }
-        return raw - raw_lse;
-    };
+    if (raw_lp) raw_lse = raw_log_partition<kThreads>(a, row, hist, sh.red_f, sh.red_d, &raw_ok);
+    auto raw_log_prob_of = [&](long long idx) { return raw_log_prob(a, row, hist, idx, raw_lse, raw_ok); };
 
-    // ---- grammar bitmask (logit_processor.hpp:52-57: after the stop-token mask, before the penalties; both only
-    //      write -inf, so their order does not show) ------------------------------------------------
-    if (a.bitmask_index) {
-        const int mi = a.bitmask_index[r];
-        if (mi >= 0) {
-            const uint32_t* mask = reinterpret_cast<const uint32_t*>(a.token_bitmasks) + (long long)mi * a.bitmask_words;
-            for (long long w = tid; w < a.bitmask_words; w += kThreads) {
-                uint32_t denied = ~mask[w];
-                if (w == a.bitmask_words - 1 && (V & 31)) denied &= (1u << (V & 31)) - 1u;   // bits beyond the vocabulary
-                while (denied) {
-                    const int b = __ffs(denied) - 1;
-                    denied &= denied - 1;
-                    row[32 * w + b] = -CUDART_INF_F;
-                }
-            }
-            __syncthreads();
-        }
-    }
-
-    // ---- 1. penalties ------------------------------------------------------------------------------
-    if (h1 > h0) apply_history(row, V, p, a.hist_ids + h0, a.hist_meta + h0, h1 - h0, a.status, raw_lp && raw_ok ? a.hist_raw + h0 : nullptr);
-    __syncthreads();
+    // ---- 1. grammar bitmask, penalties -------------------------------------------------------------
+    mask_and_penalise<kThreads>(a, row, p, r, hist, raw_lp && raw_ok);
 
     // ---- 2. greedy ----------------------------------------------------------------------------------
     if (!multinomial) {
@@ -1013,11 +897,11 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
             const float x = row[i];
             if (x > best.v) { best.v = x; best.i = (int)i; }
         }
-        best = block_reduce(best, ArgMax{-CUDART_INF_F, 0x7fffffff}, better, sh.red_a);
+        best = block_reduce_n<kThreads>(best, ArgMax{-CUDART_INF_F, 0x7fffffff}, better, sh.red_a);
         if (tid == 0) {
             const int chosen = best.i == 0x7fffffff ? 0 : best.i;  // all -inf / NaN: the reference returns index 0
             a.out_token[r] = chosen;
-            a.out_log_prob[r] = raw_lp ? raw_log_prob(chosen) : 0.f;   // sampler.cpp:965-974
+            a.out_log_prob[r] = raw_lp ? raw_log_prob_of(chosen) : 0.f;   // sampler.cpp:965-974
         }
         return;
     }
@@ -1130,7 +1014,7 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
                 float lp;
                 long long idx;
                 draw_top_k(kept, dist, sh.prob, k < 0 ? p.rand_u : a.extra_rand_u[x0 + k], &lp, &idx);
-                if (raw_lp && !dist.uniform) lp = raw_log_prob(idx);   // sampler.cpp:1022-1029, 1076-1081
+                if (raw_lp && !dist.uniform) lp = raw_log_prob_of(idx);   // sampler.cpp:1022-1029, 1076-1081
                 if (k < 0) { a.out_token[r] = idx; a.out_log_prob[r] = lp; }
                 else { a.extra_out_token[x0 + k] = idx; a.extra_out_log_prob[x0 + k] = lp; }
             }
@@ -1138,20 +1022,12 @@ __global__ void __launch_bounds__(kThreads, 2) sampler_kernel(StepArgs a) {
         return;
     }
 
-    // ---- 4. full vocabulary ---------------------------------------------------------------------------
-    if (top_k_active && p.top_k < V) {
-        // a heap larger than the shared-memory capacity: not supported, and said so (status bit 3, token -1)
-        if (tid == 0) {
-            atomicOr(a.status, 8u); a.out_token[r] = -1; a.out_log_prob[r] = 0.f;
-            if (a.extra_offsets)
-                for (long long k = a.extra_offsets[r]; k < a.extra_offsets[r + 1]; ++k) { a.extra_out_token[k] = -1; a.extra_out_log_prob[k] = 0.f; }
-        }
-        return;
+    // a heap larger than the shared-memory capacity: not supported, and said so (status bit 3, token -1)
+    if (tid == 0) {
+        atomicOr(a.status, 8u); a.out_token[r] = -1; a.out_log_prob[r] = 0.f;
+        if (a.extra_offsets)
+            for (long long k = a.extra_offsets[r]; k < a.extra_offsets[r + 1]; ++k) { a.extra_out_token[k] = -1; a.extra_out_log_prob[k] = 0.f; }
     }
-    // The row is finished by sampler_exact_kernel (sampler_exact.cu), launched right after this one: it
-    // needs the penalised row, which is in place now, and for raw log-probabilities the log-partition
-    // of the raw row, parked in the row's output slot (NaN: no scratch for the raw logits).
-    if (tid == 0) a.out_log_prob[r] = raw_lp ? (raw_ok ? raw_lse : CUDART_NAN_F) : 0.f;
 }
 
 }  // namespace

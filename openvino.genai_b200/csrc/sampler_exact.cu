@@ -39,6 +39,7 @@
 #include "../../include/sampler_b200.h"
 #include "fsum_exact.cuh"
 #include "sampler_kernels.h"
+#include "sampler_rows.cuh"
 
 namespace sampler {
 
@@ -54,7 +55,7 @@ constexpr int kBins = 2048;
 constexpr int kBinsPerThread = kBins / kThreads;
 constexpr int kTopShift = 16;         // first level: 2^16 bit patterns per bin, 128 bins per binade, 16 binades
 constexpr int kFinerBy = 5;           // bits a level is cut finer by where a bin is too full to be sorted
-constexpr int kCap = 46720;           // elements of a chunk in shared memory
+constexpr int kCap = 46592;           // elements of a chunk in shared memory
 constexpr int kSlots = 32;            // segments with the amounts of their lanes at hand, for those in which the sum may change binade
 constexpr int kTwice = 220;           // further ones whose amounts are taken for two binades (of a chunk; of a row in memory: all)
 constexpr uint8_t kInKeys = 255;
@@ -101,6 +102,7 @@ struct ExactShared {
     int count;
     uint32_t scan_u[kWarps];
     float scan_f[kWarps];
+    double scan_d[kWarps];
     int red_i[kWarps];
     // results of the walking warp
     float bc_s;
@@ -1426,9 +1428,14 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
     const int tid = threadIdx.x;
     const sampler_row_params p = a.rows[r];
     const uint32_t V = (uint32_t)a.vocab;
-    const float* logits = a.logits + p.logits_row * a.vocab;
+    float* logits = a.logits + p.logits_row * a.vocab;
     const bool raw_lp = (p.do_sample & SAMPLER_ROW_RAW_LOG_PROB) != 0;
-    const float raw_lse = raw_lp ? a.out_log_prob[r] : 0.f;   // left there by the first kernel (NaN: no scratch for the raw logits)
+    const RowHistory hist = row_history(a, r);
+    __syncthreads();
+    float raw_lse = 0.f;
+    bool raw_ok = true;
+    if (raw_lp) raw_lse = raw_log_partition<kThreads>(a, logits, hist, sh.scan_f, sh.scan_d, &raw_ok);
+    mask_and_penalise<kThreads>(a, logits, p, r, hist, raw_lp && raw_ok);
     const bool top_p_active = p.top_p != 1.0f;
     const uint32_t lo = (uint32_t)(reinterpret_cast<uintptr_t>(logits) & 15) / 4, hi = lo + V;   // (a row may begin anywhere)
     const Logits in{logits - lo, lo, hi};
@@ -1527,14 +1534,7 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
                 lp = logf(1.0f / (float)n);
             } else {
                 lp = logf(pick_p) - logf(total);
-                if (raw_lp) {
-                    float raw = logits[pick];
-                    const long long h0 = a.hist_offsets ? a.hist_offsets[r] : 0, h1 = a.hist_offsets ? a.hist_offsets[r + 1] : 0;
-                    if (a.hist_raw)
-                        for (long long i = h0; i < h1; ++i)
-                            if (a.hist_ids[i] == pick) { raw = a.hist_raw[i]; break; }
-                    lp = raw_lse != raw_lse ? CUDART_NAN_F : raw - raw_lse;
-                }
+                if (raw_lp) lp = raw_log_prob(a, logits, hist, pick, raw_lse, raw_ok);
             }
             if (k < 0) { a.out_token[r] = pick; a.out_log_prob[r] = lp; }
             else { a.extra_out_token[x0 + k] = pick; a.extra_out_log_prob[x0 + k] = lp; }
@@ -1557,9 +1557,9 @@ __global__ void __launch_bounds__(kThreads, 1) sampler_exact_kernel(StepArgs a, 
         bool take = false;
         if (base + tid < a.num_rows) {
             const sampler_row_params& p = a.rows[base + tid];
-            const bool top_k = p.top_k > 0 && p.top_k < 0x7fffffffffffffffLL && p.top_k < a.vocab;   // the first kernel's
-            take = (p.do_sample & SAMPLER_ROW_MULTINOMIAL) && !top_k && p.logits_row >= 0 && p.logits_row < a.num_logit_rows;
+            take = whole_vocabulary_row(p, a.vocab) && p.logits_row >= 0 && p.logits_row < a.num_logit_rows;   // (else reported by the first kernel)
         }
+        if (!__syncthreads_or(take)) continue;
         uint32_t n;
         const uint32_t at = seen + block_scan_exclusive(take ? 1u : 0u, sh.scan_u, &n);
         const uint32_t mine = __ballot_sync(0xffffffffu, take && at % gridDim.x == blockIdx.x);
@@ -1570,6 +1570,8 @@ __global__ void __launch_bounds__(kThreads, 1) sampler_exact_kernel(StepArgs a, 
         seen += n;
         __syncthreads();
     }
+    // The step's first kernel has its rows done: what follows in the stream waits for this one only.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 __global__ void expf_selftest_kernel(const float* in, float* out, long long n) {
@@ -1596,7 +1598,20 @@ cudaError_t launch_sampler_exact(const StepArgs& a, float* scratch, int ctas, cu
     if (a.num_rows <= 0 || ctas <= 0) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(sampler_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ExactShared));
     if (e != cudaSuccess) return e;
-    sampler_exact_kernel<<<a.num_rows < ctas ? a.num_rows : ctas, kThreads, sizeof(ExactShared), stream>>>(a, scratch);
+    // Programmatic dependent launch: the rows of the two kernels of a step have nothing to do with one another, so the CTAs of this one
+    // start where the first one's leave room.
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(a.num_rows < ctas ? a.num_rows : ctas));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = sizeof(ExactShared);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, sampler_exact_kernel, a, scratch);
+    if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
 
