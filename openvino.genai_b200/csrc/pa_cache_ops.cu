@@ -325,8 +325,8 @@ __device__ __forceinline__ void write_group(const KernelArgs& a, int group, int 
 template <int D, bool PLAN, bool GROUPS>
 __global__ void __launch_bounds__(256) write_kv_kernel(KernelArgs a) {
     constexpr int PER = D / 32;
-    // No early griddepcontrol.launch_dependents here: decode CTAs placed while blocks of this grid still hold
-    // shared memory do not all fit, and the decode kernel's static slices then run in two waves.
+    grid_wait();
+    grid_release();
     // The plan blocks come first, so that they run beside the writes of a long chunk and not behind them.
     int first_block = 0;
     if constexpr (PLAN) {
@@ -454,6 +454,8 @@ __global__ void __launch_bounds__(256, 4) rotate_kernel(KernelArgs a) {
     constexpr int EL = 8;                  // pairs per lane: an 8-byte (u8) or 16-byte (f16 / bf16) vector per half
     constexpr int LPT = HALF / EL;         // lanes per token: 8 (D = 128) or 4 (D = 64)
     constexpr int UPP = 256 / LPT;         // units per pass
+    grid_wait();
+    grid_release();
     const int l = threadIdx.x % LPT;
     const int r = blockIdx.x;
     const int units = a.g.Hkv * a.g.bs;
@@ -609,25 +611,22 @@ cudaError_t launch_write_kv(const KernelArgs& a, cudaStream_t stream, bool with_
                           reinterpret_cast<uintptr_t>(a.value_cache)) & 15) == 0;
     const long long blocks = groups ? (long long)((a.num_tokens + kWriteTokens - 1) / kWriteTokens) * a.g.Hkv : (warps * 32 + 255) / 256;
     const int grid = (int)blocks + plan_blocks;
-    auto launch = [&](auto kernel) { kernel<<<grid, 256, 0, stream>>>(a); };
+    auto launch = [&](auto kernel) { return launch_dependent(kernel, dim3(grid), dim3(256), 0, stream, a); };
     if (a.g.D == 128) {
-        if (with_plan) groups ? launch(write_kv_kernel<128, true, true>) : launch(write_kv_kernel<128, true, false>);
-        else groups ? launch(write_kv_kernel<128, false, true>) : launch(write_kv_kernel<128, false, false>);
-    } else {
-        if (with_plan) groups ? launch(write_kv_kernel<64, true, true>) : launch(write_kv_kernel<64, true, false>);
-        else groups ? launch(write_kv_kernel<64, false, true>) : launch(write_kv_kernel<64, false, false>);
+        if (with_plan) return groups ? launch(write_kv_kernel<128, true, true>) : launch(write_kv_kernel<128, true, false>);
+        return groups ? launch(write_kv_kernel<128, false, true>) : launch(write_kv_kernel<128, false, false>);
     }
-    return cudaGetLastError();
+    if (with_plan) return groups ? launch(write_kv_kernel<64, true, true>) : launch(write_kv_kernel<64, true, false>);
+    return groups ? launch(write_kv_kernel<64, false, true>) : launch(write_kv_kernel<64, false, false>);
 }
 
 cudaError_t launch_rotate(const KernelArgs& a, cudaStream_t stream) {
     if (a.num_rotated_blocks <= 0) return cudaSuccess;
     const int grid = a.num_rotated_blocks;
     const bool u8 = a.g.cache == PA_DTYPE_U8;
-    auto launch = [&](auto kernel) { kernel<<<grid, 256, 0, stream>>>(a); };
-    if (a.g.D == 128) u8 ? launch(rotate_kernel<128, true>) : launch(rotate_kernel<128, false>);
-    else u8 ? launch(rotate_kernel<64, true>) : launch(rotate_kernel<64, false>);
-    return cudaGetLastError();
+    auto launch = [&](auto kernel) { return launch_dependent(kernel, dim3(grid), dim3(256), 0, stream, a); };
+    if (a.g.D == 128) return u8 ? launch(rotate_kernel<128, true>) : launch(rotate_kernel<128, false>);
+    return u8 ? launch(rotate_kernel<64, true>) : launch(rotate_kernel<64, false>);
 }
 
 cudaError_t launch_copy_blocks(void* key_cache, void* value_cache, long long block_bytes, int num_blocks,

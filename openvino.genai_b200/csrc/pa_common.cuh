@@ -13,6 +13,31 @@ namespace pa {
 
 constexpr int kWarp = 32;
 
+// ---- programmatic dependent launch --------------------------------------------------------------
+// The kernels of a step follow one another through memory only.  Each is launched as a programmatic dependent of the one before it in
+// the stream and waits at its top for that one's end (which by then is the end of all before it): what is left between two
+// kernels is the wait's own microsecond instead of a drain, a launch and a ramp.  No path of a kernel may leave before grid_wait().
+// The short ones (cache write, rotation, scores) also let the next one's CTAs come as soon as all of their own are there.  The
+// decode and prefill kernels do not: CTAs that wait beside theirs cost them more than a ramp (16 chunks of 512 tokens 707 | 733 us
+// with it, 64 decode rows 125 | 128, a mixed step 899 | 944).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class Kernel, class Args>
+inline cudaError_t launch_dependent(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const Args& args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
 // ---- geometry of the paged cache (see pa_cache_layout in pa_b200.h) -------------------------
 struct CacheGeom {
     int Hq, Hkv, D, bs;

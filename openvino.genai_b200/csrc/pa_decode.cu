@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, (HI || PA_DECODE_STAGES > 2
     const bool q_pairs = (reinterpret_cast<uintptr_t>(a.query) & 7) == 0;   // a pair of elements is one aligned load
     bool bad_index = false;
     // everything below reads what the launch before this one wrote (plan, start records, cache)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    grid_wait();
 
     // ---- this worker's slice of the global tile sequence -----------------------------------------
     const int all_workers = gridDim.x * kDecodeWarps;
@@ -809,21 +809,8 @@ cudaError_t launch_decode_t(const KernelArgs& a, cudaStream_t stream, int sm_cou
     if (per_sm < 1) return cudaErrorLaunchOutOfResources;
     const long long ctas = decode_ctas(a, per_sm, sm_count);
     if (ev0) cudaEventRecord(ev0, stream);
-    // Programmatic dependent launch: the launch is queued behind the cache-write kernel without a full
-    // stream serialisation; that kernel never triggers early, so the CTAs start when it has finished, and
-    // they still wait (griddepcontrol.wait) before the first read of anything it writes.  An event record
-    // in between (kernel timing) serialises as usual.
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(kDecodeWarps * 32);
-    cfg.dynamicSmemBytes = Cfg::SMEM;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a);
+    // (An event record in between, for the kernel timing, serialises as usual.)
+    const cudaError_t e = launch_dependent(kern, dim3((unsigned)ctas), dim3(kDecodeWarps * 32), Cfg::SMEM, stream, a);
     if (e != cudaSuccess) return e;
     if (ev1) cudaEventRecord(ev1, stream);
     ++*launches;

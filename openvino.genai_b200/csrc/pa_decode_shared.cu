@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kShMaxWarps * 32, 1) decode_shared_kernel(Kern
     }
     const float sm_scale = a.scale != 0.f ? a.scale : rsqrtf((float)D);
     // everything below reads what the launch before this one wrote (plan, start records, cache)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    grid_wait();
 
     const int cta = blockIdx.x, nctas = gridDim.x;
     // ---- the CTA's slice; thread 0 keeps the walk state in shared memory --------------------------------
@@ -844,17 +844,7 @@ cudaError_t launch_shared_t(const KernelArgs& a, cudaStream_t stream, int sm_cou
         set[sc ? 1 : 0].store(smem, std::memory_order_release);
     }
     if (ev0) cudaEventRecord(ev0, stream);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)decode_shared_ctas(a, sm_count));
-    cfg.blockDim = dim3(Cfg::warps(a.rows_per_tile) * 32);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a);
+    const cudaError_t e = launch_dependent(kern, dim3((unsigned)decode_shared_ctas(a, sm_count)), dim3(Cfg::warps(a.rows_per_tile) * 32), smem, stream, a);
     if (e != cudaSuccess) return e;
     if (ev1) cudaEventRecord(ev1, stream);
     ++*launches;

@@ -22,6 +22,7 @@ __device__ __forceinline__ int find_sequence(const int32_t* begins, int num_seq,
 template <int D>
 __global__ void __launch_bounds__(256) prefill_generic_kernel(KernelArgs a) {
     constexpr int PER = D / 32;
+    grid_wait();
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= (long long)a.num_tokens * a.g.Hq) return;

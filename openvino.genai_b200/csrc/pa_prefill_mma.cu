@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 1) prefill_mma_kernel(KernelAr
     const int g = lane >> 2, c = lane & 3;
     const int Hkv = a.g.Hkv, G = a.g.Hq / Hkv, BS = a.g.bs;
 
+    grid_wait();
     // ---- the work item of this CTA ---------------------------------------------------------------------
     const int item = blockIdx.x >> 1, half = blockIdx.x & 1;
     const int total = a.plan->total_ptiles;
@@ -282,8 +283,7 @@ cudaError_t launch_mma_t(const KernelArgs& a, cudaStream_t stream, long long max
         if (e != cudaSuccess) return e;
         set = true;
     }
-    prefill_mma_kernel<D, BF16><<<(unsigned)(2 * max_items), kMmaWarps * 32, smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(prefill_mma_kernel<D, BF16>, dim3((unsigned)(2 * max_items)), dim3(kMmaWarps * 32), smem, stream, a);
 }
 
 }  // namespace

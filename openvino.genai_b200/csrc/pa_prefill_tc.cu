@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(KernelArgs a) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = a.g.Hq / a.g.Hkv;
     const int Hkv = a.g.Hkv;
+    grid_wait();
     const int total_items = a.plan->total_ptiles * Hkv;
     const float qscale = (a.scale != 0.f ? a.scale : rsqrtf((float)kD)) * kLog2eP;
 
@@ -1209,8 +1210,7 @@ cudaError_t launch_tc_t(const KernelArgs& a, cudaStream_t stream, int grid) {
     const int bytes = (int)sizeof(PrefillSmem<BS, CT, D>) + 1024;
     cudaError_t e = cudaFuncSetAttribute(prefill_tc_kernel<BS, CT, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    prefill_tc_kernel<BS, CT, D><<<grid, kThreads, bytes, stream>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(prefill_tc_kernel<BS, CT, D>, dim3(grid), dim3(kThreads), bytes, stream, a);
 }
 template <int CT, int D>
 cudaError_t launch_tc_bs(const KernelArgs& a, cudaStream_t stream, int grid) {

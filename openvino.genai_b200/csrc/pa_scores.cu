@@ -64,6 +64,8 @@ __global__ void __launch_bounds__(kScoreWarps * 32) score_kernel(KernelArgs a) {
     constexpr int NS = Cfg::NSTAGE;
 
     extern __shared__ __align__(128) uint8_t smem[];
+    grid_wait();
+    grid_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, c = lane & 3;
     uint8_t* ring = smem + warp * Cfg::WARP_SMEM;
@@ -373,6 +375,8 @@ __global__ void __launch_bounds__(kScoreWarps * 32) score_kernel(KernelArgs a) {
 // whose window is 0 (their slots still count toward the offsets,
 // src/cpp/src/continuous_batching/model_runner.hpp:1536-1537).
 __global__ void __launch_bounds__(256) score_reduce_kernel(KernelArgs a) {
+    grid_wait();
+    grid_release();
     const int s = blockIdx.y;
     SeqView sv;
     const bool valid = seq_view(a, s, sv);
@@ -430,8 +434,7 @@ cudaError_t launch_score_t(const KernelArgs& a, cudaStream_t stream, int sm_coun
     const long long max_tiles = (a.scores_len / kTileS + a.num_sequences) * a.g.Hkv;
     long long ctas = (long long)std::min(per_sm, 4) * sm_count;
     ctas = std::max(1LL, std::min(ctas, (max_tiles / 4 + kScoreWarps) / kScoreWarps));
-    kern<<<(unsigned)ctas, kScoreWarps * 32, Cfg::SMEM, stream>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(kern, dim3((unsigned)ctas), dim3(kScoreWarps * 32), Cfg::SMEM, stream, a);
 }
 
 template <int D, int BS>
@@ -456,9 +459,8 @@ cudaError_t launch_scores(const KernelArgs& a, cudaStream_t stream, int sm_count
     if (e != cudaSuccess) return e;
     ++*launches;
     const int gx = (int)std::max<long long>(1, std::min<long long>((a.max_context_len + 255) / 256, 64));
-    score_reduce_kernel<<<dim3(gx, a.num_sequences), 256, 0, stream>>>(a);
     ++*launches;
-    return cudaGetLastError();
+    return launch_dependent(score_reduce_kernel, dim3(gx, a.num_sequences), dim3(256), 0, stream, a);
 }
 
 }  // namespace pa
