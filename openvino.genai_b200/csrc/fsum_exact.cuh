@@ -230,6 +230,9 @@ FSX_HD Step then(Step f, Step g) {
 FSX_HD uint32_t apply(Step f, uint32_t S) { return S + ((S & 1u) ? f.b : f.a); }
 
 
+// (From here on: the sequential statement of the sorted sums over bins and lists that tests/cpp/topp_model.hpp runs on the CPU against a plain
+// loop.  The kernel takes the same sums from whole segments, with the step algebra above.)
+
 // ---- sums over probabilities sorted in descending order --------------------------------------------
 // TopPFilter adds the sorted probabilities one by one until the running float sum exceeds top_p
 // (logit_transformers.hpp:105-125) and the draw walks the same running sums (sampler.cpp:1065-1074).

@@ -12,10 +12,10 @@
 // among them (their relative order after std::sort is not defined; the lowest index comes first here).
 //
 // One CTA of 1024 threads per SM works on one row at a time:
-//   1. maximum;
-//   2. exponentials into a scratch row, with the mass of every 256 elements and, for top-p, the counts of 2048 bins of their
+//   1. maximum, and the mass of every 256 elements from approximate exponentials;
+//   2. exponentials into a scratch row, the amounts that ordered_sum adds and, for top-p, the counts of 2048 bins of their
 //      bit patterns (128 per binade);
-//   3. the index-order sum of the exponentials (ordered_sum);
+//   3. the rest of the index-order sum of the exponentials (ordered_sum);
 //   4. without top-p the same for the probabilities, the exact sum before every 256 elements kept for the draws;
 //      with top-p the elements of the highest bins are brought into shared memory bin by bin (one atomic gives a place)
 //      and ordered_sum runs over them in segments of whole bins until the sum exceeds top_p;
@@ -26,11 +26,15 @@
 // real float additions to the two sums 2^e and 2^e + ulp, which gives its amounts for an even and an odd s for two
 // additions per element; without a half-way case the amounts of a segment add up as integers in any order - the
 // elements of a bin need not be sorted -, with one the segment is sorted and its lanes' amounts are composed in order.  The
-// binade of every segment is guessed from the masses and checked by the walk of one warp over the segments; those in
-// which the sum changes binade, or whose guess was wrong, are added one by one.
+// binade of every segment is guessed from the masses (near a change of binade: both) and checked by the walk of one warp over
+// the segments.  Where the sum changes binade the lanes' amounts tell the lane, whose elements are added one by one; a segment
+// whose guess was wrong is added one by one.
 //
-// What it replaced: one thread walked the bins and lists of sorted elements (most of the 400 - 500 k cycles of a top-p row's
-// sorted part), and the CTA rescanned spans with half-way cases (100 k of the index-order sum).
+// 128 rows x 128256 of N(0, 4), top-p 0.95 (46 k kept): 421 -> 220 us a step; 200 rows x 151936, a quarter each greedy, top-k, top-p and
+// plain: 496 -> 160.  Before, one thread walked the bins and lists of sorted elements (most of the 400 - 500 k cycles of a top-p row's
+// sorted part), and the CTA rescanned spans with half-way cases (100 k of the index-order sum).  A top-p row's cycles now: 1. 38 k (HBM);
+// 2. 70 k (instruction issue); 3. 30 k (the walk, latency); 4. 115 k (ranks of the bins 10, gather 29, probabilities 11, amounts 30, walk 30);
+// 5. 42 k (a pass over the row to find the element's index 34).
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
@@ -69,7 +73,7 @@ constexpr uint32_t kOneBits = 0x3f800000u;
 constexpr uint32_t kNoGuess = 0, kEmpty = 255;
 
 // -DSAMPLER_EXACT_PROF: cycles per part of a row, printed by some of the CTAs
-enum { kProfMax, kProfExp, kProfGuess, kProfSteps, kProfWalk, kProfMisses, kProfRank, kProfGather, kProfSame, kProfPlace, kProfMass, kProfFind, kProfIndex, kProfIndex2, kProfOther, kProfTile, kProfTiles, kProfSlot, kProfSlots, kProfSerial, kProfN };
+enum { kProfMax, kProfExp, kProfGuess, kProfSteps, kProfWalk, kProfMisses, kProfRank, kProfGather, kProfSame, kProfPlace, kProfFind, kProfIndex, kProfIndex2, kProfOther, kProfTile, kProfTiles, kProfSlot, kProfSlots, kProfSerial, kProfN };
 #ifdef SAMPLER_EXACT_PROF
 #define PROF_BEGIN long long prof_t0 = clock64()
 #define PROF_END(slot) do { if (threadIdx.x == 0) sh.prof[slot] += clock64() - prof_t0; prof_t0 = clock64(); } while (0)
@@ -1542,9 +1546,9 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
     }
 #ifdef SAMPLER_EXACT_PROF
     if (tid == 0 && blockIdx.x % 37 == 0)
-        printf("row %d kept %u: max %lld exp %lld | guesses %lld steps %lld walk %lld (misses %lld) | ranks %lld gather %lld same %lld place %lld masses %lld | find %lld index %lld + %lld cycles; walk: tiles %lld in %lld, slots %lld in %lld, serial %lld\n", r, kept.n, sh.prof[kProfMax],
+        printf("row %d kept %u: max %lld exp %lld | guesses %lld steps %lld walk %lld (misses %lld) | ranks %lld gather %lld same %lld place %lld | find %lld index %lld + %lld cycles; walk: tiles %lld in %lld, slots %lld in %lld, serial %lld\n", r, kept.n, sh.prof[kProfMax],
                sh.prof[kProfExp], sh.prof[kProfGuess], sh.prof[kProfSteps], sh.prof[kProfWalk], sh.prof[kProfMisses], sh.prof[kProfRank], sh.prof[kProfGather], sh.prof[kProfSame],
-               sh.prof[kProfPlace], sh.prof[kProfMass], sh.prof[kProfFind], sh.prof[kProfIndex], sh.prof[kProfIndex2], sh.prof[kProfTiles], sh.prof[kProfTile], sh.prof[kProfSlots], sh.prof[kProfSlot], sh.prof[kProfSerial]);
+               sh.prof[kProfPlace], sh.prof[kProfFind], sh.prof[kProfIndex], sh.prof[kProfIndex2], sh.prof[kProfTiles], sh.prof[kProfTile], sh.prof[kProfSlots], sh.prof[kProfSlot], sh.prof[kProfSerial]);
 #endif
 }
 
