@@ -1086,11 +1086,10 @@ __device__ __noinline__ Kept keep_top_p(Row row, Segs g, Level L, float top_p, f
     return Kept{placed + zeros, placed, c, s};
 }
 
-// The vocabulary index of the element of rank `rank` in descending order, whose probability is p: among equal ones the lowest
-// index comes first.  (Of more than 4096 equal ones the first is taken.)
+// The vocabulary index of the element of rank `rank` in descending order, whose probability is p: among equal ones, however many, the
+// lowest index comes first.
 __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p) {
     ExactShared& sh = shared_memory();
-    constexpr uint32_t kMostEqual = 4096;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     PROF_BEGIN;
     // the exponentials with this probability are neighbours: a look around p * norm finds the first and the last of them
@@ -1133,7 +1132,7 @@ __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p)
     same = block_sum(same, sh.scan_u);
     lowest = block_reduce(lowest, [](uint32_t a, uint32_t b) { return min(a, b); }, sh.scan_u);
     PROF_END(kProfIndex);
-    if (same <= 1 || same > kMostEqual) return lowest == 0xffffffffu ? row.lo : (long long)lowest;
+    if (same <= 1) return lowest == 0xffffffffu ? row.lo : (long long)lowest;
     // several: the rank among them
     const uint32_t blocks = (row.hi + kBlock - 1) / kBlock, per = (blocks + kWarps - 1) / kWarps;
     const uint32_t b0 = min(blocks, warp * per), b1 = min(blocks, b0 + per);
@@ -1158,7 +1157,7 @@ __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p)
     __syncthreads();
     if (want >= before && want < before + same) {   // one warp
         uint32_t seen = before;
-        for (uint32_t b = b0; b < b1; ++b) {
+        for (uint32_t b = b0; b < b1 && seen <= want; ++b) {
             const uint32_t i = b * kBlock + 8 * lane;
             uint32_t mine = 0;   // a bit per element
 #pragma unroll
