@@ -1225,50 +1225,29 @@ __device__ __noinline__ long long find_draw(Src src, int segs, uint32_t n, float
     return hit;
 }
 
-// expf with the host libm's bits (fsx::expf_libm), the table of 2^(i / 32) in the lanes' registers: in shared memory, 32
-// different entries of eight bytes cost a warp six to seven passes, two shuffles cost two.
-__device__ __forceinline__ float expf_lanes(float x, uint32_t tab_lo, uint32_t tab_hi) {
-    const double kInvLn2N = 0x1.71547652b82fep+0 * 32.0;
-    const double kShift = 0x1.8p+52;
-    const double kC0 = 0x1.c6af84b912394p-5 / 32768.0, kC1 = 0x1.ebfce50fac4f3p-3 / 1024.0, kC2 = 0x1.62e42ff0c52d6p-1 / 32.0;
+// The table of 2^(i / 32) in the lanes' registers: in shared memory, 32 different entries of eight bytes cost a warp six to seven
+// passes, two shuffles cost two.
+struct LaneTable {
+    uint32_t lo, hi;
+    __device__ explicit LaneTable(int lane) {
+        const uint64_t entry = fsx::kExp2TabDev[lane];
+        lo = (uint32_t)entry;
+        hi = (uint32_t)(entry >> 32);
+    }
+    __device__ __forceinline__ double operator()(uint64_t ki) const {   // (lane ki mod 32)
+        const uint32_t k = (uint32_t)ki, l = __shfl_sync(0xffffffffu, lo, (int)k), h = __shfl_sync(0xffffffffu, hi, (int)k);
+        return __hiloint2double((int)(h + (k << 15)), (int)l);
+    }
+};
+
+// expf with the host libm's bits (fsx::expf_libm), one argument per lane
+__device__ __forceinline__ float expf_lanes(float x, LaneTable tab) {
     const bool in = x >= -103.972076f && !(x > 88.72283f);
-    const double xd = (double)(in ? x : 0.f);
-    double kd = __fma_rn(kInvLn2N, xd, kShift);
-    const uint64_t ki = (uint64_t)__double_as_longlong(kd);
-    kd = __dadd_rn(kd, -kShift);
-    const double r = __fma_rn(kInvLn2N, xd, -kd);
-    const uint32_t lo = __shfl_sync(0xffffffffu, tab_lo, (int)(ki & 31)), hi = __shfl_sync(0xffffffffu, tab_hi, (int)(ki & 31));
-    const double s = __longlong_as_double((long long)((((uint64_t)hi << 32) | lo) + (ki << 47)));
-    const double z = __fma_rn(kC0, r, kC1);
-    const double r2 = __dmul_rn(r, r);
-    double y = __fma_rn(kC2, r, 1.0);
-    y = __fma_rn(z, r2, y);
-    y = __dmul_rn(y, s);
-    const float f = (float)y;
+    const float f = fsx::expf_scaled((double)(in ? x : 0.f), tab);
     return in ? f : x > 0.f ? CUDART_INF_F : x != x ? x : 0.f;
 }
-
-// The same for arguments from -inf to 0, without the selections: below -104.5 the result is zero as it is at -104.5.
-__device__ __forceinline__ float expf_lanes_nonpositive(float x, uint32_t tab_lo, uint32_t tab_hi) {
-    const double kInvLn2N = 0x1.71547652b82fep+0 * 32.0;
-    const double kShift = 0x1.8p+52;
-    const double kC0 = 0x1.c6af84b912394p-5 / 32768.0, kC1 = 0x1.ebfce50fac4f3p-3 / 1024.0, kC2 = 0x1.62e42ff0c52d6p-1 / 32.0;
-    // the conversion to double in integers, for x <= 0 (zeros and denormals as some other number that small): four instructions instead
-    // of one at a quarter of their sixteenth of a warp's lanes per cycle
-    const uint32_t b = __float_as_uint(fmaxf(x, -104.5f));
-    const double xd = __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + 0xb8000000u), (int)(b << 29));
-    double kd = __fma_rn(kInvLn2N, xd, kShift);
-    const uint32_t ki = (uint32_t)__double2loint(kd);
-    kd = __dadd_rn(kd, -kShift);
-    const double r = __fma_rn(kInvLn2N, xd, -kd);
-    const uint32_t lo = __shfl_sync(0xffffffffu, tab_lo, (int)ki), hi = __shfl_sync(0xffffffffu, tab_hi, (int)ki);   // (lane ki mod 32)
-    const double s = __hiloint2double((int)(hi + (ki << 15)), (int)lo);
-    const double z = __fma_rn(kC0, r, kC1);
-    const double r2 = __dmul_rn(r, r);
-    double y = __fma_rn(kC2, r, 1.0);
-    y = __fma_rn(z, r2, y);
-    return (float)__dmul_rn(y, s);
-}
+// The same for arguments from -inf to 0, without the selections.
+__device__ __forceinline__ float expf_lanes_nonpositive(float x, LaneTable tab) { return fsx::expf_scaled(fsx::nonpositive_as_double(x), tab); }
 
 // The elements of a logits row from an address on a 16-byte boundary on: lo .. hi - 1 of `base`.
 struct Logits {
@@ -1344,8 +1323,7 @@ template <bool kCount>
 __device__ __noinline__ void exponentials(Logits row, float mx, float inv_T, float* ex, Level& level) {
     ExactShared& sh = shared_memory();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint64_t tab = fsx::kExp2TabDev[lane];
-    const uint32_t tab_lo = (uint32_t)tab, tab_hi = (uint32_t)(tab >> 32);
+    const LaneTable tab(lane);
     const uint32_t bins = (uint32_t)__cvta_generic_to_shared(sh.bins);
     if (kCount)
         for (int j = tid; j < kBins; j += kThreads) sh.bins[j] = 0;
@@ -1366,7 +1344,7 @@ __device__ __noinline__ void exponentials(Logits row, float mx, float inv_T, flo
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) y[4 * u + e] = expf_lanes_nonpositive(__fmul_rn(__fsub_rn(x[h][u][e], mx), inv_T), tab_lo, tab_hi);   // (inv_T 1: as it is)
+                for (int e = 0; e < 4; ++e) y[4 * u + e] = expf_lanes_nonpositive(__fmul_rn(__fsub_rn(x[h][u][e], mx), inv_T), tab);   // (inv_T 1: as it is)
                 if (kCount) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
@@ -1400,8 +1378,7 @@ __device__ __noinline__ void exponentials(Logits row, float mx, float inv_T, flo
 __device__ __noinline__ void exponentials_any(Logits row, Segs g, float mx, float inv_T, float* ex) {
     ExactShared& sh = shared_memory();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint64_t tab = fsx::kExp2TabDev[lane];
-    const uint32_t tab_lo = (uint32_t)tab, tab_hi = (uint32_t)(tab >> 32);
+    const LaneTable tab(lane);
     for (int j = tid; j < g.count; j += kThreads) sh.cum[j] = 0.f;
     __syncthreads();
     const uint32_t blocks = (row.hi + kBlock - 1) / kBlock;
@@ -1413,7 +1390,7 @@ __device__ __noinline__ void exponentials_any(Logits row, Segs g, float mx, floa
             row.load4(i, x);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const float y = expf_lanes(__fmul_rn(__fsub_rn(x[e], mx), inv_T), tab_lo, tab_hi);
+                const float y = expf_lanes(__fmul_rn(__fsub_rn(x[e], mx), inv_T), tab);
                 x[e] = i + e >= row.lo && i + e < row.hi ? y : 0.f;
                 if (x[e] >= 0.f) mass += x[e];
             }
@@ -1577,13 +1554,15 @@ __global__ void __launch_bounds__(kThreads, 1) sampler_exact_kernel(StepArgs a, 
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Both forms; NaN where they differ.
 __global__ void expf_selftest_kernel(const float* in, float* out, long long n) {
     const int lane = threadIdx.x & 31;
-    const uint64_t tab = fsx::kExp2TabDev[lane];
+    const LaneTable tab(lane);
     for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x - lane; i0 < n; i0 += (long long)gridDim.x * blockDim.x) {
         const long long i = i0 + lane;
-        const float y = expf_lanes(i < n ? in[i] : 0.f, (uint32_t)tab, (uint32_t)(tab >> 32));
-        if (i < n) out[i] = y;
+        const float x = i < n ? in[i] : 0.f;
+        const float y = expf_lanes(x, tab), z = expf_lanes_nonpositive(fminf(x, 0.f), tab);
+        if (i < n) out[i] = x <= 0.f && __float_as_uint(y) != __float_as_uint(z) ? CUDART_NAN_F : y;
     }
 }
 
