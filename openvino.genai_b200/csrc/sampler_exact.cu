@@ -41,9 +41,9 @@
 #include <stdio.h>
 
 #include "../../include/sampler_b200.h"
-#include "fsum_exact.cuh"
 #include "sampler_kernels.h"
 #include "sampler_rows.cuh"
+#include "segment_sum.cuh"
 
 namespace sampler {
 
@@ -66,11 +66,9 @@ constexpr uint8_t kInKeys = 255;
 static_assert(kSlots + kTwice < kInKeys, "slot numbers");
 constexpr int kMaxMisses = 10;        // segments added one by one before the guesses of those behind are made anew (3 k cycles each; a new
                                       // pass over a row takes 35 k)
-// Relative margins around the approximate sums: where the sum may change binade (the second one: or may not have yet, since what
-// rounding took from a sum of small terms adds up), pass the threshold, be drawn
-constexpr float kMargin = 1.0f / 1024, kWideMargin = 1.0f / 64, kDrawMargin = 1.0f / 256;
+using fsx::kEmpty, fsx::kMargin, fsx::kNoGuess;
+constexpr float kDrawMargin = 1.0f / 256;   // relative margin around the approximate sums within which an element may be drawn
 constexpr uint32_t kOneBits = 0x3f800000u;
-constexpr uint32_t kNoGuess = 0, kEmpty = 255;
 
 // -DSAMPLER_EXACT_PROF: cycles per part of a row, printed by some of the CTAs
 enum { kProfMax, kProfExp, kProfGuess, kProfSteps, kProfWalk, kProfMisses, kProfRank, kProfGather, kProfSame, kProfPlace, kProfFind, kProfIndex, kProfIndex2, kProfOther, kProfTile, kProfTiles, kProfSlot, kProfSlots, kProfSerial, kProfN };
@@ -359,28 +357,21 @@ __device__ void guess_binades(int c, int c1, float s, float thr, float thr2, boo
     uint32_t slots = 0, twice = 0;
     for (int base = c; base < c1; base += kThreads) {
         const int j = base + (int)threadIdx.x;
-        bool maybe = false, wide = false;
-        uint32_t Ew = 0, El = 0;
+        fsx::Guess g{kNoGuess, kNoGuess, false, false, false};
         if (j < c1) {
             const float lo = j == c ? s : sh.cum[j] + shift, hi = sh.cum[j + 1] + shift;
-            const float l = lo * (1.f - kMargin), h = hi * (1.f + kMargin);
-            const uint32_t Eh = fsx::state_exp(h), Ev = fsx::state_exp(hi * (1.f + kWideMargin));
-            El = fsx::state_exp(l);
-            Ew = fsx::state_exp(lo * (1.f - kWideMargin));
-            const bool empty = sh.start[j] == sh.start[j + 1], usable = lo > 0.f && Ew >= 25u && Ev < 252u;
-            wide = !empty && usable && Ev == Ew + 1u;
-            maybe = wide && El != Eh;
-            sh.E[j] = (uint8_t)(empty ? kEmpty : usable ? fsx::state_exp(lo) : kNoGuess);
-            if (sh.sorted[j] == 0 && (j == 0 || El != Eh || (l <= thr && thr <= h) || (lo * (1.f - kDrawMargin) <= thr2 && thr2 <= hi * (1.f + kDrawMargin))))
+            g = fsx::guess_binade(lo, hi, sh.start[j] == sh.start[j + 1]);
+            if (sh.sorted[j] == 0 && (j == 0 || g.changes || (lo * (1.f - kMargin) <= thr && thr <= hi * (1.f + kMargin)) ||
+                                      (lo * (1.f - kDrawMargin) <= thr2 && thr2 <= hi * (1.f + kDrawMargin))))
                 sh.sorted[j] = 2;
         }
         uint32_t n;
-        const uint32_t before = block_scan_exclusive((maybe ? 1u : 0u) | (wide ? 65536u : 0u), sh.scan_u, &n);
+        const uint32_t before = block_scan_exclusive((g.edge ? 1u : 0u) | (g.two ? 65536u : 0u), sh.scan_u, &n);
         if (j < c1) {
             const uint32_t at = slots + (before & 0xffffu), at2 = twice + (before >> 16);
-            const bool lanes = maybe && at < (uint32_t)kSlots, two = wide && (rows || at2 < (uint32_t)kTwice);
+            const bool lanes = g.edge && at < (uint32_t)kSlots, two = g.two && (rows || at2 < (uint32_t)kTwice);
             sh.slot[j] = lanes ? (uint8_t)(at + 1) : !two ? 0 : rows ? kInKeys : (uint8_t)(at2 + 1 + kSlots);
-            if (wide) sh.E[j] = (uint8_t)(lanes || two ? Ew : El);
+            sh.E[j] = (uint8_t)(g.two && !lanes && !two ? g.alone : g.E);
         }
         slots += n & 0xffffu;
         twice += n >> 16;
@@ -393,22 +384,14 @@ __device__ __forceinline__ uint32_t& step_up(int slot, int j) {
     return slot == kInKeys ? reinterpret_cast<uint32_t*>(sh.keys)[kSlots * kBlock + j] : sh.step_up[slot - 1 - kSlots];
 }
 
-// The amounts for an even and an odd sum differ by one at most: two neighbouring sums stay neighbours or meet.
-__device__ __forceinline__ uint32_t pack_amounts(fsx::Step st) { return st.a << 2 | (st.b - st.a + 1u); }
-__device__ __forceinline__ fsx::Step unpack_amounts(uint32_t w) { return fsx::Step{w >> 2, (w >> 2) + (w & 3u) - 1u}; }
+using fsx::pack_amounts, fsx::unpack_amounts;
 
 // The amounts of a warp's 256 elements under binade E; *tie: they depend on the order.
 __device__ __forceinline__ fsx::Step block_step(const float (&x)[8], uint32_t E, bool in_order, bool* tie) {
-    const uint32_t even = E << 23, odd = even + 1;
-    float s0 = __uint_as_float(even), s1 = __uint_as_float(odd);
+    fsx::Sums sums = fsx::sums_begin(E);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        s0 = __fadd_rn(s0, x[e]);
-        s1 = __fadd_rn(s1, x[e]);
-    }
-    const uint32_t b0 = __float_as_uint(s0), b1 = __float_as_uint(s1);
-    fsx::Step st{b0 - even, b1 - odd};
-    if (b1 >= even + (1u << 23)) st = fsx::Step{fsx::kSat, fsx::kSat};   // the lane's own sum leaves the binade
+    for (int e = 0; e < 8; ++e) fsx::sums_add(sums, x[e]);
+    fsx::Step st = fsx::sums_amounts(sums, E);
     *tie = __any_sync(0xffffffffu, st.a != st.b);
     if (!*tie) {
         st.a = st.b = min(__reduce_add_sync(0xffffffffu, st.a), fsx::kSat);   // 32 x kSat at most
@@ -432,8 +415,8 @@ __device__ __forceinline__ void lane_steps(Src src, int j) {
     ExactShared& sh = shared_memory();
     const int lane = threadIdx.x & 31, slot = sh.slot[j] - 1;
     const uint32_t lo = sh.start[j] - src.off, hi = sh.start[j + 1] - src.off, lo8 = lo & ~7u, m = (hi - lo8 + kBlock - 1) / kBlock;
-    const uint32_t even = (uint32_t)sh.E[j] << 23, up = 1u << 23;
-    float s[4] = {__uint_as_float(even), __uint_as_float(even + 1), __uint_as_float(even + up), __uint_as_float(even + up + 1)};
+    const uint32_t E = sh.E[j];
+    fsx::Sums here = fsx::sums_begin(E), above = fsx::sums_begin(E + 1u);
     for (uint32_t t = 0; t < m; ++t) {
         float x[8];
         load8(src.data(), lo8 + 8 * (lane * m + t), lo, hi, x);
@@ -443,15 +426,12 @@ __device__ __forceinline__ void lane_steps(Src src, int j) {
             *reinterpret_cast<float4*>(sh.keys + slot * kBlock + 8 * lane + 4) = make_float4(x[4], x[5], x[6], x[7]);
         }
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) s[k] = __fadd_rn(s[k], x[e]);
+        for (int e = 0; e < 8; ++e) {
+            fsx::sums_add(here, x[e]);
+            fsx::sums_add(above, x[e]);
+        }
     }
-    auto amounts = [&](int k, uint32_t base) {
-        const uint32_t b0 = __float_as_uint(s[k]), b1 = __float_as_uint(s[k + 1]);
-        return b1 >= base + up ? fsx::Step{fsx::kSat, fsx::kSat} : fsx::Step{b0 - base, b1 - base - 1};
-    };
-    fsx::Step p = amounts(0, even), q = amounts(2, even + up);
+    fsx::Step p = fsx::sums_amounts(here, E), q = fsx::sums_amounts(above, E + 1u);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const fsx::Step pu{__shfl_up_sync(0xffffffffu, p.a, o), __shfl_up_sync(0xffffffffu, p.b, o)};
@@ -618,12 +598,8 @@ __device__ void walk_segments(Src src, int c, int c1, float s, float thr) {
         const uint32_t Eg = lane < n ? sh.E[my] : kEmpty;
         uint32_t word = lane < n ? sh.step[my] : 1u;
         const int own_slot = lane < n ? sh.slot[my] : 0;
-        bool right = Eg == E;
-        if (own_slot && Eg + 1u == E) {   // the sum has changed binade before this one
-            word = own_slot <= kSlots ? sh.from[own_slot - 1][0] : step_up(own_slot, my);
-            right = true;
-        }
-        const uint32_t wrong = __ballot_sync(0xffffffffu, !(Eg == kEmpty || (right && S >= 0x800000u)));
+        if (own_slot && Eg + 1u == E) word = own_slot <= kSlots ? sh.from[own_slot - 1][0] : step_up(own_slot, my);   // the sum has changed binade before this one
+        const uint32_t wrong = __ballot_sync(0xffffffffu, !fsx::guess_holds(Eg, own_slot != 0, E, S));
         const int most = wrong ? __ffs(wrong) - 1 : n;   // as far as the guesses hold
         if (lane == 0) sh.state[c] = fsx::state_float(E, S);
         if (most > 0) {
