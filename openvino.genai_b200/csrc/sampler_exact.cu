@@ -64,8 +64,8 @@ constexpr int kSlots = 32;            // segments with the amounts of their lane
 constexpr int kTwice = 220;           // further ones whose amounts are taken for two binades (of a chunk; of a row in memory: all)
 constexpr uint8_t kInKeys = 255;
 static_assert(kSlots + kTwice < kInKeys, "slot numbers");
-constexpr int kMaxMisses = 10;        // segments added one by one before the guesses of those behind are made anew (3 k cycles each; a new
-                                      // pass over a row takes 35 k)
+constexpr int kMaxMisses = 10;        // segments with a wrong guess before the guesses of those behind are made anew (each is added one by one, 3 k
+                                      // cycles; a new pass over a row takes 35 k)
 using fsx::kEmpty, fsx::kMargin, fsx::kNoGuess;
 constexpr float kDrawMargin = 1.0f / 256;   // relative margin around the approximate sums within which an element may be drawn
 constexpr uint32_t kOneBits = 0x3f800000u;
@@ -386,7 +386,8 @@ __device__ __forceinline__ uint32_t& step_up(int slot, int j) {
 
 using fsx::pack_amounts, fsx::unpack_amounts;
 
-// The amounts of a warp's 256 elements under binade E; *tie: they depend on the order.
+// The amounts of a warp's 256 elements under binade E, the same on all lanes; *tie (the same too): they depend on the order, and only lane 0
+// has those of all elements.
 __device__ __forceinline__ fsx::Step block_step(const float (&x)[8], uint32_t E, bool in_order, bool* tie) {
     fsx::Sums sums = fsx::sums_begin(E);
 #pragma unroll
@@ -598,8 +599,9 @@ __device__ void walk_segments(Src src, int c, int c1, float s, float thr) {
         const uint32_t Eg = lane < n ? sh.E[my] : kEmpty;
         uint32_t word = lane < n ? sh.step[my] : 1u;
         const int own_slot = lane < n ? sh.slot[my] : 0;
-        if (own_slot && Eg + 1u == E) word = own_slot <= kSlots ? sh.from[own_slot - 1][0] : step_up(own_slot, my);   // the sum has changed binade before this one
-        const uint32_t wrong = __ballot_sync(0xffffffffu, !fsx::guess_holds(Eg, own_slot != 0, E, S));
+        const bool above = own_slot != 0 && Eg + 1u == E;   // the sum has changed binade before this one
+        if (above) word = own_slot <= kSlots ? sh.from[own_slot - 1][0] : step_up(own_slot, my);
+        const uint32_t wrong = __ballot_sync(0xffffffffu, !fsx::guess_holds(Eg, above, E));
         const int most = wrong ? __ffs(wrong) - 1 : n;   // as far as the guesses hold
         if (lane == 0) sh.state[c] = fsx::state_float(E, S);
         if (most > 0) {
@@ -636,7 +638,7 @@ __device__ void walk_segments(Src src, int c, int c1, float s, float thr) {
             if (taken == n) continue;
             if (lane == 0) sh.state[c] = fsx::state_float(E, S);
         }
-        if (lanes_at_hand(sh.slot[c]) && S >= 0x800000u) {   // the sum may change binade in this one: its lanes' amounts are at hand
+        if (lanes_at_hand(sh.slot[c])) {   // the sum may change binade in this one: its lanes' amounts are at hand
             const int slot = sh.slot[c] - 1;
             const uint32_t Eg = sh.E[c];
             uint32_t E2 = E, S2 = fsx::kOne24;
@@ -676,7 +678,8 @@ __device__ void walk_segments(Src src, int c, int c1, float s, float thr) {
                 continue;
             }
         }
-        if (++misses > kMaxMisses && c1 - c > 32) break;
+        const uint32_t guessed = sh.E[c];   // (none or a right one: another would not help)
+        if (guessed != kNoGuess && !fsx::guess_holds(guessed, sh.slot[c] != 0, E) && ++misses > kMaxMisses && c1 - c > 32) break;
         PROF_COUNT(kProfMisses);
         if constexpr (Src::kSortable) {
             if (sh.sorted[c] != 1) sort_in_chunk(src, c);

@@ -2,6 +2,8 @@
 // segments with guessed binades - 32 lanes of eight elements each, as the kernel has them - against `s += x[i]`.
 //
 // usage: segment_sum_test sums SEEDS        every sum before a segment and every crossing of a threshold is the plain loop's
+//        segment_sum_test late SEEDS        rows whose sum begins late or grows in jumps: the walk goes by the amounts, except where the sum
+//                                           changes binade
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -44,11 +46,40 @@ static uint32_t segment_word(const float* x, uint32_t E) {
     return fsx::pack_amounts(st);
 }
 
+// The elements of a segment without amounts made before: all lanes' at once as far as the sum stays in its binade.
+static int add_by_lanes(const float* x, uint32_t& E, uint32_t& S, float thr) {
+    for (int from = 0; from < kLanes; ++from) {
+        if (E < 252u) {
+            fsx::Step st = fsx::step_identity();
+            uint32_t before = S;
+            int l = from;
+            for (; l < kLanes; ++l) {
+                st = fsx::then(st, amounts(x + kPer * l, kPer, E));
+                const uint32_t after = fsx::apply(st, S);
+                if (after >= fsx::kOne24 || fsx::state_float(E, after) > thr) break;
+                before = after;
+            }
+            S = before;
+            if (l == kLanes) break;
+            from = l;
+        }
+        float s = fsx::state_float(E, S);
+        for (int e = 0; e < kPer; ++e) {
+            s += x[kPer * from + e];
+            if (s > thr) { E = fsx::state_exp(s); S = fsx::state_sig(s); return kPer * from + e; }
+        }
+        E = fsx::state_exp(s);
+        S = fsx::state_sig(s);
+    }
+    return -1;
+}
+
 struct Walk {
     std::vector<float> before;   // sum before every segment
     float s = 0.f;
     long long hit = -1;
-    int misses = 0;              // segments that were not taken by their amounts
+    int misses = 0;              // segments that were not taken by their amounts,
+    int wrong = 0;               // of them those whose guess did not hold
 };
 
 static Walk walk(const std::vector<float>& x, const std::vector<float>& cum, float thr) {
@@ -58,8 +89,9 @@ static Walk walk(const std::vector<float>& x, const std::vector<float>& cum, flo
     for (size_t j = 0; j < segs; ++j) {
         const float* at = x.data() + j * kBlock;
         const fsx::Guess g = fsx::guess_binade(cum[j], cum[j + 1], false);
+        const bool holds = g.E != fsx::kNoGuess && fsx::guess_holds(g.E, g.two, E);
         w.before.push_back(fsx::state_float(E, S));
-        if (g.E != fsx::kNoGuess && fsx::guess_holds(g.E, g.two, E, S)) {
+        if (holds) {
             const uint32_t after = g.E == fsx::kEmpty ? S : fsx::apply(fsx::unpack_amounts(segment_word(at, E)), S);
             if (after < fsx::kOne24 && !(fsx::state_float(E, after) > thr)) {
                 S = after;
@@ -67,14 +99,12 @@ static Walk walk(const std::vector<float>& x, const std::vector<float>& cum, flo
             }
         }
         ++w.misses;
-        float s = fsx::state_float(E, S);
-        for (int i = 0; i < kBlock && w.hit < 0; ++i) {
-            s += at[i];
-            if (s > thr) w.hit = (long long)(j * kBlock) + i;
+        w.wrong += holds || g.E == fsx::kNoGuess ? 0 : 1;
+        const int e = add_by_lanes(at, E, S, thr);
+        if (e >= 0) {
+            w.hit = (long long)(j * kBlock) + e;
+            break;
         }
-        E = fsx::state_exp(s);
-        S = fsx::state_sig(s);
-        if (w.hit >= 0) break;
     }
     w.s = fsx::state_float(E, S);
     return w;
@@ -169,6 +199,19 @@ int main(int argc, char** argv) {
                     for (float& c : off) c *= std::exp2((float)(int)(r() % 7u) - 3.f);
                     check_walk(kind, x, off, 0.6f * total);
                 }
+    }
+    if (mode == "late") {
+        for (int seed = 0; seed < seeds; ++seed)
+            for (const char* kind : {"cold_spikes", "freezing", "late", "last_ids", "few_ids", "upper_half"}) {
+                std::mt19937 r(31u + seed);
+                const std::vector<float> x = exponentials(kind, r, 128256), cum = approximate_sums(x, r);
+                const Walk w = walk(x, cum, std::numeric_limits<float>::infinity());
+                int changes = 0;   // segments in which the sum changes binade: those the walk has to open
+                for (size_t j = 0; j < w.before.size(); ++j)
+                    changes += fsx::state_exp(w.before[j]) != fsx::state_exp(j + 1 < w.before.size() ? w.before[j + 1] : w.s);
+                std::printf("%s: %d changes of binade, %d segments not taken by their amounts, %d of them guessed wrong\n", kind, changes, w.misses, w.wrong);
+                CHECK(w.misses <= changes + 4 && w.wrong <= 4, "%s: %d segments are not taken by their amounts, %d wrong guesses", kind, w.misses, w.wrong);
+            }
     }
     std::printf("%ld failures\n", failures);
     return failures != 0;

@@ -27,3 +27,8 @@ def run(exe, *args):
 
 def test_sums_and_crossings_are_those_of_the_plain_loop(exe):
     run(exe, "sums", "3")
+
+
+def test_rows_whose_sum_begins_late_are_walked_by_their_amounts(exe):
+    """Grammar masks, low temperatures, a late peak: a segment that adds nothing, or to a sum that is zero or tiny, is no wrong guess."""
+    run(exe, "late", "3")
