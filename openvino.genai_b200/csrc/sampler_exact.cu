@@ -735,6 +735,29 @@ __device__ __noinline__ long long ordered_sum(Src src, int c, int c1, float& s, 
         if (hit >= 0 || c >= c1) return hit;
     }
 }
+// Sums before the segments of a row in memory from its elements as they are prepared, where those that count as zero would make the sums at
+// hand useless.
+template <class Src>
+__device__ __noinline__ void sums_of(Src src, int n) {
+    ExactShared& sh = shared_memory();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();
+    for (int j = warp; j < n; j += kWarps) {
+        const uint32_t lo = sh.start[j] - src.off, hi = sh.start[j + 1] - src.off;
+        float mass = 0.f;
+        for (uint32_t i = lo & ~7u; i < hi; i += kBlock) {
+            float x[8];
+            load8(src.data(), i + 8 * lane, lo, hi, x);
+            src.prepare(x);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) mass += x[e];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
+        if (lane == 0) sh.cum[j] = mass;
+    }
+    masses_to_sums(n);
+}
 // The segments of a row in index order: elements lo .. hi - 1.
 __device__ void index_order_segments(Segs g, uint32_t lo, uint32_t hi) {
     ExactShared& sh = shared_memory();
@@ -803,24 +826,47 @@ __device__ __noinline__ void count_level(Level& L, const float* ex, uint32_t hi)
     L.rest = __syncthreads_or(rest) != 0;
 }
 
+struct Row {
+    const float* ex;    // exponentials in index order: elements lo .. hi - 1
+    float* sorted;      // the largest probabilities, as far as they were needed: segment by segment in descending order, those within
+                        // a segment only where it mattered
+    uint32_t lo, hi;
+    float norm, inv_norm, min_thr;
+};
+
 // Counts -> ranks of the bins' first elements, and the level's segments from number c on: whole bins, one beginning with the first
 // bin at or after every multiple of the segment length, bins of kBigSegs times that by themselves.  `placed` elements come
-// before the level, `sum` is their sum.  Returns the number after the level's last segment; *reach: the first segment that begins
+// before the level, `sum` is their sum.  Bins of nothing but probabilities below the min-p threshold are left out, and with them what
+// lies below the level.  Returns the number after the level's last segment; *reach: the first segment that begins
 // above target as far as the bins tell (that number: none).
-__device__ __noinline__ int rank_bins(Level& L, Segs g, int c, uint32_t placed, float inv_norm, float sum, float target, int* reach) {
+__device__ __noinline__ int rank_bins(Level& L, Row row, Segs g, int c, uint32_t placed, float sum, float target, int* reach) {
     ExactShared& sh = shared_memory();
     const int tid = threadIdx.x, j0 = tid * kBinsPerThread;
     __syncthreads();
     uint32_t n[kBinsPerThread];
 #pragma unroll
     for (int k = 0; k < kBinsPerThread; ++k) n[k] = sh.bins[j0 + k];
+    int bins = kBins;   // those that count: the bins' largest keys fall
+    if (row.min_thr > 0.f) {
+        int dropped = kBins;
+#pragma unroll
+        for (int k = 0; k < kBinsPerThread; ++k) {
+            const unsigned long long down = ((unsigned long long)(j0 + k) << L.shift) + 1u;
+            if (down >= L.F || !(probability(__uint_as_float(L.F - (uint32_t)down), row.norm, row.inv_norm) >= row.min_thr)) {
+                n[k] = 0;
+                dropped = min(dropped, j0 + k);
+            }
+        }
+        bins = block_reduce(dropped, [](int a, int b) { return min(a, b); }, sh.red_i);
+        if (bins < kBins) L.rest = false;
+    }
     const uint32_t big = (uint32_t)kBigSegs << g.shift;
     float value[kBinsPerThread], mass = 0.f;
     uint32_t count = 0, own_last = 0;
 #pragma unroll
     for (int k = 0; k < kBinsPerThread; ++k) {   // the middle of the bin
         const uint32_t down = ((uint32_t)(j0 + k) << L.shift) + ((1u << L.shift) >> 1) + 1u;
-        value[k] = n[k] && down < L.F ? (float)n[k] * (__uint_as_float(L.F - down) * inv_norm) : 0.f;
+        value[k] = n[k] && down < L.F ? (float)n[k] * (__uint_as_float(L.F - down) * row.inv_norm) : 0.f;
         mass += value[k];
         count += n[k];
         own_last = n[k] ? n[k] : own_last;
@@ -857,19 +903,11 @@ __device__ __noinline__ int rank_bins(Level& L, Segs g, int c, uint32_t placed, 
         cum += value[k];
     }
     const int end = min(c + (int)total, kSegCap);
-    if (tid == kThreads - 1) { sh.start[end] = placed + L.total; sh.bin[end] = (uint16_t)kBins; sh.cum[end] = cum; }
+    if (tid == kThreads - 1) { sh.start[end] = placed + L.total; sh.bin[end] = (uint16_t)bins; sh.cum[end] = cum; }
     far = block_reduce(far, [](int a, int b) { return min(a, b); }, sh.red_i);   // (its barriers cover the tables)
     *reach = min(far, end);
     return end;
 }
-
-struct Row {
-    const float* ex;    // exponentials in index order: elements lo .. hi - 1
-    float* sorted;      // the largest probabilities, as far as they were needed: segment by segment in descending order, those within
-                        // a segment only where it mattered
-    uint32_t lo, hi;
-    float norm, inv_norm, min_thr;
-};
 
 // Brings the segments c .. c1 - 1 (whole bins, at most kCap elements) into shared memory and the row, up to sh.stop, the first one that is
 // too large to be sorted and not all the same; elements below the min-p threshold as zeros.  Returns how many are not.
@@ -989,7 +1027,7 @@ __device__ __noinline__ Kept keep_top_p(Row row, Segs g, Level L, float top_p, f
         const uint32_t most = (row.hi - placed) >> g.shift;
         while (c > 1 && (uint32_t)c + most + 2 * (most / kBigSegs) + 4 > (uint32_t)kSegCap) c = merge_segments(c);
         int reach;
-        const int end = rank_bins(L, g, c, placed, row.inv_norm, s, top_p * (1.0f + 1.0f / 1024), &reach);
+        const int end = rank_bins(L, row, g, c, placed, s, top_p * (1.0f + 1.0f / 1024), &reach);
         PROF_END(kProfRank);
         const uint32_t level_at = placed;
         bool again = false;    // another level takes over before this one's end
@@ -1439,9 +1477,12 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
         kept = keep_top_p(row, g, level, p.top_p, p.rand_u);
         total = kept.total;
     } else if (any) {
-        // approximate sums: those of the exponentials over the norm (min-p drops mass: guesses that do not hold cost time only)
+        // approximate sums: those of the exponentials over the norm, but with min-p, which drops terms, those of what is left (a pass of 15 us over
+        // 128256 elements; with the exponentials' sums most guesses are wrong and a step takes 960 us instead of 150)
         __syncthreads();
-        for (int j = tid; j <= g.count; j += kThreads) sh.cum[j] *= inv_norm;
+        if (min_thr > 0.f) sums_of(probs, g.count);
+        else
+            for (int j = tid; j <= g.count; j += kThreads) sh.cum[j] *= inv_norm;
         ordered_sum(probs, 0, g.count, total, CUDART_INF_F, -1.f);
     }
     const bool uniform_fallback = !(total > 0.0f && isfinite(total)) || (top_p_active && kept.n == 0);
