@@ -37,7 +37,8 @@ struct sampler_handle {
     uint8_t* stage_dev = nullptr;
     uint8_t* stage_host = nullptr;  // pinned
     size_t stage_bytes = 0;
-    float* exact_scratch = nullptr;   // two rows per CTA of the full-vocabulary kernel
+    float* exact_small = nullptr;     // kSmallScratch bytes from the handle's creation on: scratch of small steps
+    float* exact_scratch = nullptr;   // of larger ones: two rows per CTA of the full-vocabulary kernel
     size_t exact_bytes = 0;
     int exact_ctas = 0;               // persistent grid of that kernel: one CTA per SM
     int64_t launches = 0;
@@ -59,17 +60,22 @@ int ensure_stage(sampler_handle* h, size_t bytes) {
     return SAMPLER_OK;
 }
 
-// Scratch of the full-vocabulary kernel: grows (with a stream synchronisation) when a step has a larger vocabulary.
-int ensure_exact_scratch(sampler_handle* h, int32_t rows, int64_t vocab) {
+// Scratch of the full-vocabulary kernel, which every device step needs (its rows are not known on the host).  A few rows use what the handle has:
+// an allocation of more than the driver has at hand takes 330 us, five times such a step (9 rows x 32000: a new handle's first
+// step 400 us, 58 with this).  Beyond that it grows, with a stream synchronisation, when a step is larger.
+constexpr size_t kSmallScratch = size_t(4) << 20;
+int ensure_exact_scratch(sampler_handle* h, int32_t rows, int64_t vocab, float** scratch) {
     const int ctas = std::min<int64_t>(rows, h->exact_ctas);
     const size_t need = sampler::sampler_exact_scratch_bytes(ctas, vocab);
-    if (need <= h->exact_bytes) return SAMPLER_OK;
+    *scratch = need <= kSmallScratch ? h->exact_small : h->exact_scratch;
+    if (need <= std::max(h->exact_bytes, kSmallScratch)) return SAMPLER_OK;
     S_CUDA(cudaStreamSynchronize(h->stream));
     S_CUDA(cudaDeviceSynchronize());
     if (h->exact_scratch) S_CUDA(cudaFree(h->exact_scratch));
     h->exact_scratch = nullptr; h->exact_bytes = 0;
     S_CUDA(cudaMalloc((void**)&h->exact_scratch, need));
     h->exact_bytes = need;
+    *scratch = h->exact_scratch;
     return SAMPLER_OK;
 }
 
@@ -78,9 +84,10 @@ int launch_step(sampler_handle* h, const sampler::StepArgs& k, cudaStream_t stre
     S_CUDA(sampler::launch_sampler(k, stream));
     h->launches += 1;
     if (any_full_vocab) {
-        int rc = ensure_exact_scratch(h, k.num_rows, k.vocab);
+        float* scratch = nullptr;
+        int rc = ensure_exact_scratch(h, k.num_rows, k.vocab, &scratch);
         if (rc != SAMPLER_OK) return rc;
-        S_CUDA(sampler::launch_sampler_exact(k, h->exact_scratch, h->exact_ctas, stream));
+        S_CUDA(sampler::launch_sampler_exact(k, scratch, h->exact_ctas, stream));
         h->launches += 1;
     }
     return SAMPLER_OK;
@@ -136,23 +143,26 @@ int sampler_b200_create(int device, int32_t max_rows, int64_t max_vocab, sampler
     if (!out) return sfail(SAMPLER_ERR_INVALID_ARG, "NULL out pointer");
     int count = 0;
     if (cudaGetDeviceCount(&count) != cudaSuccess || device < 0 || device >= count) return sfail(SAMPLER_ERR_INVALID_ARG, "no such CUDA device");
-    cudaDeviceProp prop;
-    S_CUDA(cudaGetDeviceProperties(&prop, device));
-    if (prop.major != 10) return sfail(SAMPLER_ERR_UNSUPPORTED, "this library is built for sm_100a only");
+    int major = 0, sm_count = 0;   // (single attributes: all properties take 2.8 ms)
+    S_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    S_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+    if (major != 10) return sfail(SAMPLER_ERR_UNSUPPORTED, "this library is built for sm_100a only");
     S_CUDA(cudaSetDevice(device));
     sampler_handle* h = new sampler_handle();
     h->device = device;
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc((void**)&h->status, 256);
     if (e == cudaSuccess) e = cudaMemset(h->status, 0, 256);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&h->exact_small, kSmallScratch);
     if (e != cudaSuccess) {
-        delete h;
+        sampler_b200_destroy(h);
         return sfail(SAMPLER_ERR_CUDA, std::string("sampler_b200_create: ") + cudaGetErrorString(e));
     }
     if (const char* polls = std::getenv("SAMPLER_B200_TEST_WAIT_POLLS")) h->wait_polls = std::max(0, std::atoi(polls));
-    h->exact_ctas = prop.multiProcessorCount;
+    h->exact_ctas = sm_count;
     if (max_rows > 0 && max_vocab > 0) {   // otherwise sized on first use
-        const int rc = ensure_exact_scratch(h, max_rows, max_vocab);
+        float* scratch = nullptr;
+        const int rc = ensure_exact_scratch(h, max_rows, max_vocab, &scratch);
         if (rc != SAMPLER_OK) { sampler_b200_destroy(h); return rc; }
     }
     *out = h;
@@ -166,6 +176,7 @@ int sampler_b200_destroy(sampler_handle* h) {
     if (h->status) cudaFree(h->status);
     if (h->stage_dev) cudaFree(h->stage_dev);
     if (h->stage_host) cudaFreeHost(h->stage_host);
+    if (h->exact_small) cudaFree(h->exact_small);
     if (h->exact_scratch) cudaFree(h->exact_scratch);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
