@@ -129,9 +129,8 @@ int sampler_b200_step_host(sampler_handle* h, const sampler_step_args* args, int
  * range, bit 2 = SAMPLER_ROW_RAW_LOG_PROB on a row with history but no hist_raw scratch, bit 3 = a
  * multinomial row with 1024 < top_k < vocab (the top-k heap lives in shared memory and holds 1024
  * candidates; such a row gets token -1 and sampler_b200_step_host returns SAMPLER_ERR_UNSUPPORTED),
- * bit 4 = internal: the sorted walk of a top-p row did not terminate, bit 5 = internal: a wait between the
- * warps that filter a top-k row and the one that replays its heap ran out (such a row gets token -1;
- * sampler_b200_step_host returns SAMPLER_ERR_CUDA for both). */
+ * bit 4 = not used, bit 5 = internal: a wait between the warps that filter a top-k row and the one that
+ * replays its heap ran out (such a row gets token -1; sampler_b200_step_host returns SAMPLER_ERR_CUDA). */
 int sampler_b200_last_device_status(sampler_handle* h, uint32_t* status_bits);
 
 int64_t sampler_b200_launch_count(const sampler_handle* h);

@@ -308,7 +308,7 @@ SamplerOutput Sampler::sample_device(const std::vector<SequenceGroup*>& sequence
     check(sampler_b200_last_device_status(m_handle, &bits), "sampler_b200_last_device_status");
     if (bits & 1u) throw std::runtime_error("input_ids token out of bounds");
     if (bits & 8u) throw std::runtime_error("top_k above the sampler's heap capacity of 1024 (and below the vocabulary) is not supported");
-    if (bits & (16u | 32u)) throw std::runtime_error("a bounded wait or walk of the sampler kernel ran out (device status " + std::to_string(bits) + ")");
+    if (bits & 32u) throw std::runtime_error("a bounded wait of the sampler kernel ran out (device status " + std::to_string(bits) + ")");
     std::vector<int64_t> tokens(n), extra_tokens(nx);
     std::vector<float> log_probs(n), extra_log_probs(nx);
     std::memcpy(tokens.data(), hp + o_tok, n * 8);

@@ -283,7 +283,7 @@ int sampler_b200_step_host(sampler_handle* h, const sampler_step_args* a, int co
     S_CUDA(cudaStreamSynchronize(stream));
     if (bits) {
         S_CUDA(cudaMemsetAsync(h->status, 0, 4, stream));
-        const int code = (bits & 1u) ? SAMPLER_ERR_BAD_TOKEN_ID : (bits & 8u) ? SAMPLER_ERR_UNSUPPORTED : (bits & (16u | 32u)) ? SAMPLER_ERR_CUDA : SAMPLER_ERR_INVALID_ARG;
+        const int code = (bits & 1u) ? SAMPLER_ERR_BAD_TOKEN_ID : (bits & 8u) ? SAMPLER_ERR_UNSUPPORTED : (bits & 32u) ? SAMPLER_ERR_CUDA : SAMPLER_ERR_INVALID_ARG;
         return sfail(code, "device status word " + std::to_string(bits));
     }
     return SAMPLER_OK;

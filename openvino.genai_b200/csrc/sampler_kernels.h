@@ -21,7 +21,7 @@ struct StepArgs {
     int64_t* out_token;
     float* out_log_prob;
     uint32_t* status;  // bit 0: history id out of range, bit 1: logits_row out of range, bit 2: raw log-prob without scratch,
-                       // bit 3: top_k above the heap capacity (and below the vocabulary), bit 4: no longer set,
+                       // bit 3: top_k above the heap capacity (and below the vocabulary), bit 4: not used,
                        // bit 5: a wait between the warps of a top-k row ran out
     float* hist_raw;   // raw logits of the history entries (rows that report raw log-probabilities), may be null
     // further draws of a row (all null: none): CSR offsets, their uniform numbers, their outputs
