@@ -100,10 +100,9 @@ cudaError_t launch_prefill(const KernelArgs& a, cudaStream_t stream, int* launch
     if (a.num_tokens <= 0) return cudaSuccess;
     const long long warps = (long long)a.num_tokens * a.g.Hq;
     const int grid = (int)((warps * 32 + 255) / 256);
-    if (a.g.D == 128) prefill_generic_kernel<128><<<grid, 256, 0, stream>>>(a);
-    else prefill_generic_kernel<64><<<grid, 256, 0, stream>>>(a);
     ++*launches;
-    return cudaGetLastError();
+    if (a.g.D == 128) return launch_dependent(prefill_generic_kernel<128>, dim3(grid), dim3(256), 0, stream, a);
+    return launch_dependent(prefill_generic_kernel<64>, dim3(grid), dim3(256), 0, stream, a);
 }
 
 }  // namespace pa
