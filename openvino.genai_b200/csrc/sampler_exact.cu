@@ -1124,6 +1124,7 @@ __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p)
         if (key_lo) return __float_as_uint(e) - key_lo <= key_hi - key_lo;
         return probability(e, row.norm, row.inv_norm) == p;
     };
+    auto above = [&](float e) { return key_lo ? e > __uint_as_float(key_hi) : probability(e, row.norm, row.inv_norm) > p; };
     uint32_t same = 0, lowest = 0xffffffffu;
     const float4* e4 = reinterpret_cast<const float4*>(row.ex);
     const uint32_t n4 = (row.hi + 3) >> 2;
@@ -1160,9 +1161,9 @@ __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p)
 #pragma unroll
         for (int e = 0; e < 8; ++e)
             if (i + e >= row.lo && i + e < row.hi) {
-                const float q = probability(row.ex[i + e], row.norm, row.inv_norm);
-                same += q == p ? 1u : 0u;
-                greater += q > p ? 1u : 0u;
+                const float q = row.ex[i + e];
+                same += equal(q) ? 1u : 0u;
+                greater += above(q) ? 1u : 0u;
             }
     }
     same = __reduce_add_sync(0xffffffffu, same);
@@ -1179,7 +1180,7 @@ __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p)
             uint32_t mine = 0;   // a bit per element
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-                if (i + e >= row.lo && i + e < row.hi && probability(row.ex[i + e], row.norm, row.inv_norm) == p) mine |= 1u << e;
+                if (i + e >= row.lo && i + e < row.hi && equal(row.ex[i + e])) mine |= 1u << e;
             uint32_t incl = __popc(mine);
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
