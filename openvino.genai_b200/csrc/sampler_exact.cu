@@ -196,7 +196,7 @@ __device__ __forceinline__ float probability(float e, float norm, float inv_norm
 struct Exponentials {
     const float* v;
     uint32_t off;
-    static constexpr bool kSortable = false;
+    static constexpr bool kSortable = false, kThreshold = false;
     __device__ __forceinline__ const float* data() const { return v; }
     __device__ __forceinline__ void prepare(float (&x)[8]) const {
 #pragma unroll
@@ -207,7 +207,7 @@ struct Probabilities {
     const float* v;
     uint32_t off;
     float norm, inv_norm, min_thr;
-    static constexpr bool kSortable = false;
+    static constexpr bool kSortable = false, kThreshold = true;   // some elements may count as zero
     __device__ __forceinline__ const float* data() const { return v; }
     __device__ __forceinline__ void prepare(float (&x)[8]) const {
 #pragma unroll
@@ -220,14 +220,14 @@ struct Probabilities {
 struct Chunk {   // probabilities in shared memory (keys), and the row that they also are in
     uint32_t off;
     float* out;
-    static constexpr bool kSortable = true;
+    static constexpr bool kSortable = true, kThreshold = false;
     __device__ __forceinline__ const float* data() const { return shared_memory().keys; }
     __device__ __forceinline__ void prepare(float (&)[8]) const {}
 };
 struct Sorted {
     const float* v;
     uint32_t off;
-    static constexpr bool kSortable = false;
+    static constexpr bool kSortable = false, kThreshold = false;
     __device__ __forceinline__ const float* data() const { return v; }
     __device__ __forceinline__ void prepare(float (&)[8]) const {}
 };
@@ -357,21 +357,26 @@ __device__ void guess_binades(int c, int c1, float s, float thr, float thr2, boo
     uint32_t slots = 0, twice = 0;
     for (int base = c; base < c1; base += kThreads) {
         const int j = base + (int)threadIdx.x;
-        fsx::Guess g{kNoGuess, kNoGuess, false, false, false};
+        bool edge = false, twofold = false;
+        uint32_t alone = 0;
         if (j < c1) {
             const float lo = j == c ? s : sh.cum[j] + shift, hi = sh.cum[j + 1] + shift;
-            g = fsx::guess_binade(lo, hi, sh.start[j] == sh.start[j + 1]);
+            const fsx::Guess g = fsx::guess_binade(lo, hi, sh.start[j] == sh.start[j + 1]);
+            edge = g.edge;
+            twofold = g.two;
+            alone = g.alone;
+            sh.E[j] = (uint8_t)g.E;
             if (sh.sorted[j] == 0 && (j == 0 || g.changes || (lo * (1.f - kMargin) <= thr && thr <= hi * (1.f + kMargin)) ||
                                       (lo * (1.f - kDrawMargin) <= thr2 && thr2 <= hi * (1.f + kDrawMargin))))
                 sh.sorted[j] = 2;
         }
         uint32_t n;
-        const uint32_t before = block_scan_exclusive((g.edge ? 1u : 0u) | (g.two ? 65536u : 0u), sh.scan_u, &n);
+        const uint32_t before = block_scan_exclusive((edge ? 1u : 0u) | (twofold ? 65536u : 0u), sh.scan_u, &n);
         if (j < c1) {
             const uint32_t at = slots + (before & 0xffffu), at2 = twice + (before >> 16);
-            const bool lanes = g.edge && at < (uint32_t)kSlots, two = g.two && (rows || at2 < (uint32_t)kTwice);
+            const bool lanes = edge && at < (uint32_t)kSlots, two = twofold && (rows || at2 < (uint32_t)kTwice);
             sh.slot[j] = lanes ? (uint8_t)(at + 1) : !two ? 0 : rows ? kInKeys : (uint8_t)(at2 + 1 + kSlots);
-            sh.E[j] = (uint8_t)(g.two && !lanes && !two ? g.alone : g.E);
+            if (twofold && !lanes && !two) sh.E[j] = (uint8_t)alone;
         }
         slots += n & 0xffffu;
         twice += n >> 16;
@@ -410,9 +415,10 @@ __device__ __forceinline__ fsx::Step block_step(const float (&x)[8], uint32_t E,
 __device__ __forceinline__ bool lanes_at_hand(int slot) { return slot != 0 && slot <= kSlots; }
 
 // A segment with a slot: the amounts of its lanes, each of which takes m * 8 consecutive elements, under E up to every lane and under
-// E + 1 from every lane on.  Elements of rows in memory stay at hand in `keys`, which nothing else uses then (m = 1).
+// E + 1 from every lane on.  Elements of rows in memory stay at hand in `keys`, which nothing else uses then (m = 1).  Out of line: a few segments
+// of a row come here, and without its instructions the passes are 2 - 3 us shorter.
 template <class Src>
-__device__ __forceinline__ void lane_steps(Src src, int j) {
+__device__ __noinline__ void lane_steps(Src src, int j) {
     ExactShared& sh = shared_memory();
     const int lane = threadIdx.x & 31, slot = sh.slot[j] - 1;
     const uint32_t lo = sh.start[j] - src.off, hi = sh.start[j + 1] - src.off, lo8 = lo & ~7u, m = (hi - lo8 + kBlock - 1) / kBlock;
@@ -679,7 +685,7 @@ __device__ void walk_segments(Src src, int c, int c1, float s, float thr) {
             }
         }
         const uint32_t guessed = sh.E[c];   // (none or a right one: another would not help)
-        if (guessed != kNoGuess && !fsx::guess_holds(guessed, sh.slot[c] != 0, E) && ++misses > kMaxMisses && c1 - c > 32) break;
+        if (guessed != kNoGuess && guessed != E && ++misses > kMaxMisses && c1 - c > 32) break;
         PROF_COUNT(kProfMisses);
         if constexpr (Src::kSortable) {
             if (sh.sorted[c] != 1) sort_in_chunk(src, c);
@@ -712,31 +718,8 @@ __device__ void fill_states() {
     }
 }
 
-// Adds the segments c .. c1 - 1 to s in order, exactly as `s += x[i]` does, from the approximate sums in sh.cum (have_steps: the guesses
-// are made and the amounts known).  It stops at the first running sum above thr and returns that element, else -1.  sh.state: the sum before every segment it came to.
-template <class Src>
-__device__ __noinline__ long long ordered_sum(Src src, int c, int c1, float& s, float thr, float thr2, bool have_steps = false) {
-    ExactShared& sh = shared_memory();
-    PROF_BEGIN;
-    for (;; have_steps = false) {
-        if (!have_steps) {
-            guess_binades(c, c1, s, thr, thr2, !Src::kSortable);
-            PROF_END(kProfGuess);
-            segment_steps(src, c, c1);
-            PROF_END(kProfSteps);
-        }
-        if (threadIdx.x < 32) walk_segments(src, c, c1, s, thr);
-        __syncthreads();
-        fill_states();
-        PROF_END(kProfWalk);
-        s = sh.bc_s; c = sh.bc_seg;
-        const long long hit = sh.bc_hit;
-        __syncthreads();
-        if (hit >= 0 || c >= c1) return hit;
-    }
-}
-// Sums before the segments of a row in memory from its elements as they are prepared, where those that count as zero would make the sums at
-// hand useless.
+// Sums before the segments of a row from its elements as they are prepared: with min-p, which drops terms, the sums at hand are of no use.  (A pass
+// of 15 us over 128256 elements; with the sums of all elements most guesses are wrong and a step takes 960 us instead of 150.)
 template <class Src>
 __device__ __noinline__ void sums_of(Src src, int n) {
     ExactShared& sh = shared_memory();
@@ -757,6 +740,32 @@ __device__ __noinline__ void sums_of(Src src, int n) {
         if (lane == 0) sh.cum[j] = mass;
     }
     masses_to_sums(n);
+}
+// Adds the segments c .. c1 - 1 to s in order, exactly as `s += x[i]` does, from the approximate sums in sh.cum (have_steps: the guesses
+// are made and the amounts known).  It stops at the first running sum above thr and returns that element, else -1.  sh.state: the sum before every segment it came to.
+template <class Src>
+__device__ __noinline__ long long ordered_sum(Src src, int c, int c1, float& s, float thr, float thr2, bool have_steps = false) {
+    ExactShared& sh = shared_memory();
+    PROF_BEGIN;
+    if constexpr (Src::kThreshold) {
+        if (src.min_thr > 0.f) sums_of(src, c1);
+    }
+    for (;; have_steps = false) {
+        if (!have_steps) {
+            guess_binades(c, c1, s, thr, thr2, !Src::kSortable);
+            PROF_END(kProfGuess);
+            segment_steps(src, c, c1);
+            PROF_END(kProfSteps);
+        }
+        if (threadIdx.x < 32) walk_segments(src, c, c1, s, thr);
+        __syncthreads();
+        fill_states();
+        PROF_END(kProfWalk);
+        s = sh.bc_s; c = sh.bc_seg;
+        const long long hit = sh.bc_hit;
+        __syncthreads();
+        if (hit >= 0 || c >= c1) return hit;
+    }
 }
 // The segments of a row in index order: elements lo .. hi - 1.
 __device__ void index_order_segments(Segs g, uint32_t lo, uint32_t hi) {
@@ -1478,12 +1487,9 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
         kept = keep_top_p(row, g, level, p.top_p, p.rand_u);
         total = kept.total;
     } else if (any) {
-        // approximate sums: those of the exponentials over the norm, but with min-p, which drops terms, those of what is left (a pass of 15 us over
-        // 128256 elements; with the exponentials' sums most guesses are wrong and a step takes 960 us instead of 150)
+        // approximate sums: those of the exponentials over the norm (with min-p they are taken anew)
         __syncthreads();
-        if (min_thr > 0.f) sums_of(probs, g.count);
-        else
-            for (int j = tid; j <= g.count; j += kThreads) sh.cum[j] *= inv_norm;
+        for (int j = tid; j <= g.count; j += kThreads) sh.cum[j] *= inv_norm;
         ordered_sum(probs, 0, g.count, total, CUDART_INF_F, -1.f);
     }
     const bool uniform_fallback = !(total > 0.0f && isfinite(total)) || (top_p_active && kept.n == 0);

@@ -27,7 +27,9 @@ FSX_HD void sums_add(Sums& s, float x) {
 // What was added since sums_begin(E); saturated where a sum has left the binade.
 FSX_HD Step sums_amounts(const Sums& s, uint32_t E) {
     const uint32_t base = E << 23, even = float_bits(s.even), odd = float_bits(s.odd);
-    return odd >= base + (1u << 23) ? Step{kSat, kSat} : Step{even - base, odd - base - 1u};
+    Step st{even - base, odd - (base + 1u)};
+    if (odd >= base + (1u << 23)) st = Step{kSat, kSat};
+    return st;
 }
 
 // The amounts for an even and an odd sum differ by one at most: without a half-way case they are the same; at the first x = q + 1/2
