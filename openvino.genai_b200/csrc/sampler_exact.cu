@@ -60,6 +60,7 @@ constexpr int kBinsPerThread = kBins / kThreads;
 constexpr int kTopShift = 16;         // first level: 2^16 bit patterns per bin, 128 bins per binade, 16 binades
 constexpr int kFinerBy = 5;           // bits a level is cut finer by where a bin is too full to be sorted
 constexpr int kCap = 46592;           // elements of a chunk in shared memory
+constexpr int kListed = 4096;         // elements that a row with several draws lists with their indices
 constexpr int kSlots = 32;            // segments with the amounts of their lanes at hand, for those in which the sum may change binade
 constexpr int kTwice = 220;           // further ones whose amounts are taken for two binades (of a chunk; of a row in memory: all)
 constexpr uint8_t kInKeys = 255;
@@ -116,7 +117,7 @@ struct ExactShared {
 #endif
 };
 static_assert(sizeof(ExactShared) <= 232448, "shared memory of a CTA");
-static_assert(kSlots * kBlock + kSegCap <= kCap, "room in keys");
+static_assert(kSlots * kBlock + kSegCap <= kCap && 3 * kListed <= kCap, "room in keys");
 extern __shared__ __align__(16) uint8_t sx_smem[];
 // (by its name and not by an argument: the compiler then knows that it is shared memory)
 __device__ __forceinline__ ExactShared& shared_memory() { return *reinterpret_cast<ExactShared*>(sx_smem); }
@@ -1209,6 +1210,74 @@ __device__ __noinline__ long long index_of_rank(Row row, uint32_t rank, float p)
     return idx;
 }
 
+// A row with several draws and few elements kept: their probabilities and indices are listed in one pass, at the end of `keys` (what a draw may
+// sort there has room before it).  Without the list every draw takes a pass of its own: a row of three to eight kept elements with 16 further
+// draws 352 us a step, with it 205.  False: more elements than fit.
+__device__ __forceinline__ uint2* listed() { return reinterpret_cast<uint2*>(shared_memory().keys + kCap - 2 * kListed); }
+__device__ __forceinline__ bool list_kept(Row row, uint32_t placed) {
+    ExactShared& sh = shared_memory();
+    if (placed > (uint32_t)kListed) return false;
+    float least = CUDART_INF_F;   // (zeros are below the min-p threshold)
+    for (uint32_t i = threadIdx.x; i < placed; i += kThreads) {
+        const float p = row.sorted[i];
+        if (p > 0.f) least = fminf(least, p);
+    }
+    least = block_reduce(least, [](float a, float b) { return fminf(a, b); }, sh.scan_f);
+    if (!(least >= 0x1p-100f)) return false;   // (too few bits for `about`)
+    if (threadIdx.x == 0) sh.count = 0;
+    __syncthreads();
+    const float about = least * row.norm * (1.f - 1.f / 1048576);   // (a little below the least exponential: the division tells)
+    const float4* e4 = reinterpret_cast<const float4*>(row.ex);
+    const uint32_t n4 = (row.hi + 3) >> 2;
+    for (uint32_t i0 = threadIdx.x; i0 < n4; i0 += 4 * kThreads) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = i0 + u * kThreads < n4 ? e4[i0 + u * kThreads] : make_float4(0.f, 0.f, 0.f, 0.f);
+        float most = 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) most = fmaxf(most, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)));
+        if (!(most >= about)) continue;
+#pragma unroll 1
+        for (int u = 0; u < 16; ++u) {
+            const uint32_t i = 4 * (i0 + (u >> 2) * kThreads) + (u & 3);
+            if (i < row.lo || i >= row.hi || !(row.ex[i] >= about)) continue;
+            const float p = probability(row.ex[i], row.norm, row.inv_norm);
+            if (!(p >= least)) continue;
+            const int at = atomicAdd(&sh.count, 1);
+            if (at < kListed) listed()[at] = make_uint2(__float_as_uint(p), i);
+        }
+    }
+    __syncthreads();
+    return sh.count <= kListed;
+}
+// index_of_rank from the list (-1: not there, or too many of one value).
+__device__ __noinline__ long long listed_index(uint32_t rank, float p) {
+    ExactShared& sh = shared_memory();
+    const int n = sh.count;
+    uint32_t greater_same = 0;   // 2^16 times those with the same probability
+    for (int i = threadIdx.x; i < n; i += kThreads) {
+        const float q = __uint_as_float(listed()[i].x);
+        greater_same += (q > p ? 1u : 0u) + (q == p ? 65536u : 0u);
+    }
+    greater_same = block_sum(greater_same, sh.scan_u);
+    const uint32_t greater = greater_same & 0xffffu, same = greater_same >> 16;
+    const uint32_t want = rank < greater ? 0u : rank - greater;
+    if (threadIdx.x == 0) sh.bc_hit = -1;
+    __syncthreads();
+    if (same <= 64u)
+        for (int i = threadIdx.x; i < n; i += kThreads) {
+            const uint2 own = listed()[i];
+            if (__uint_as_float(own.x) != p) continue;
+            uint32_t before = 0;
+            for (int k = 0; same > 1u && k < n; ++k) before += listed()[k].x == own.x && listed()[k].y < own.y ? 1u : 0u;
+            if (before == want) sh.bc_hit = own.y;
+        }
+    __syncthreads();
+    const long long at = sh.bc_hit;
+    __syncthreads();
+    return at;
+}
+
 // First element of src, of those below n, whose running sum exceeds r (-1: none), from the sums recorded before the segments
 // 0 .. segs - 1.  `unsorted`: the row in memory whose segment may have to be sorted first.
 template <class Src>
@@ -1506,6 +1575,7 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
         last_kept = block_reduce(last, [](int x, int y) { return max(x, y); }, sh.red_i);
     };
     const long long x0 = a.extra_offsets ? a.extra_offsets[r] : 0, x1 = a.extra_offsets ? a.extra_offsets[r + 1] : 0;
+    const bool list = x1 > x0 && top_p_active && !uniform_fallback && list_kept(row, kept.placed);
     for (long long k = -1; k < x1 - x0; ++k) {   // the row's own draw, then the further ones (sampler.cpp:1065)
         const float u = k < 0 ? p.rand_u : a.extra_rand_u[x0 + k];
         long long pick = -1;
@@ -1527,7 +1597,9 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
                     rank = (long long)kept.n - 1;
                     pick_p = rank < (long long)kept.placed ? sorted[rank] : 0.f;
                 }
-                pick = index_of_rank(row, (uint32_t)rank, pick_p) - lo;
+                pick = list && pick_p > 0.f ? listed_index((uint32_t)rank, pick_p) : -1;
+                if (pick < 0) pick = index_of_rank(row, (uint32_t)rank, pick_p);
+                pick -= lo;
             }
         }
         if (tid == 0) {

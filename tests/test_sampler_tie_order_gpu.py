@@ -1,6 +1,8 @@
 """The token a top-p draw gives when it falls among equal probabilities: the reference's std::sort leaves their order open, the kernel takes
 them in index order.  So every row has exactly one right answer: a stable descending sort, float32 sums one by one, the first sum above
 total * u.  Also in runs of many thousands, which other tests accept any element of."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -71,3 +73,36 @@ def test_draws_among_equal_probabilities_follow_the_index(kind, v):
     p, _, _ = sampler_oracle.transform(0, x[0], 1.0)
     want = np.concatenate([expected_tokens(p, kw["top_p"], kw.get("min_p", 0.0), DRAWS) for kw in OPTIONS])
     assert np.array_equal(tok, want), [(i // len(DRAWS), float(DRAWS[i % len(DRAWS)]), int(tok[i]), int(want[i])) for i in np.flatnonzero(tok != want)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("v", [300, 4096, 50257, 128256])
+@pytest.mark.parametrize("kind", KINDS + ["peaks", "steps"])
+def test_further_draws_of_a_row_follow_the_index_too(kind, v):
+    """Several draws of one row, which find their elements in a list where few are kept: as many as fit, one more, runs of equal ones in it."""
+    rng = np.random.default_rng(v + 1)
+    if kind == "peaks":
+        x = (rng.standard_normal(v) * 2).astype(np.float32)
+        x[rng.choice(v, size=min(v, 40), replace=False)] += 15
+    elif kind == "steps":      # 100 values, each a run of v / 100 elements
+        x = (rng.permutation(v) % 100 * 0.125).astype(np.float32)
+    else:
+        x = logits_of(kind, rng, v)
+    x = np.ascontiguousarray(np.tile(x, (len(OPTIONS), 1)))
+    rows = np.concatenate([H.make_rows(1, logits_rows=np.array([i], np.int64), **kw) for i, kw in enumerate(OPTIONS)])
+    us = rng.random((len(rows), 24)).astype(np.float32)
+    rows["rand_u"] = us[:, 0]
+    offs = np.arange(len(rows) + 1, dtype=np.int64) * (us.shape[1] - 1)
+    extra_u = np.ascontiguousarray(us[:, 1:]).ravel()
+    tok, lp = np.full(len(rows), -7, np.int64), np.zeros(len(rows), np.float32)
+    xtok, xlp = np.full(len(extra_u), -7, np.int64), np.zeros(len(extra_u), np.float32)
+    a = H.step_args(x, rows, None, tok, lp)
+    a.extra_offsets, a.extra_rand_u = offs.ctypes.data, extra_u.ctypes.data
+    a.extra_out_token, a.extra_out_log_prob = xtok.ctypes.data, xlp.ctypes.data
+    gpu = H.GpuSampler()
+    assert gpu.lib.sampler_b200_step_host(gpu.h, ctypes.byref(a), 0) == 0
+    p, _, _ = sampler_oracle.transform(0, x[0], 1.0)
+    for i, kw in enumerate(OPTIONS):
+        want = expected_tokens(p, kw["top_p"], kw.get("min_p", 0.0), us[i])
+        got = np.concatenate([tok[i:i + 1], xtok[offs[i]:offs[i + 1]]])
+        assert np.array_equal(got, want), (kw, np.flatnonzero(got != want), got[got != want], want[got != want])
