@@ -1253,25 +1253,27 @@ __device__ __forceinline__ bool list_kept(Row row, uint32_t placed) {
 // index_of_rank from the list (-1: not there, or too many of one value).
 __device__ __noinline__ long long listed_index(uint32_t rank, float p) {
     ExactShared& sh = shared_memory();
-    const int n = sh.count;
-    uint32_t greater_same = 0;   // 2^16 times those with the same probability
-    for (int i = threadIdx.x; i < n; i += kThreads) {
-        const float q = __uint_as_float(listed()[i].x);
-        greater_same += (q > p ? 1u : 0u) + (q == p ? 65536u : 0u);
-    }
-    greater_same = block_sum(greater_same, sh.scan_u);
-    const uint32_t greater = greater_same & 0xffffu, same = greater_same >> 16;
-    const uint32_t want = rank < greater ? 0u : rank - greater;
-    if (threadIdx.x == 0) sh.bc_hit = -1;
+    const int n = sh.count, tid = threadIdx.x;
+    uint32_t* equal = reinterpret_cast<uint32_t*>(sh.serial);   // the indices of those with this probability
+    if (tid == 0) { sh.stop = 0; sh.bc_hit = -1; }
     __syncthreads();
-    if (same <= 64u)
-        for (int i = threadIdx.x; i < n; i += kThreads) {
-            const uint2 own = listed()[i];
-            if (__uint_as_float(own.x) != p) continue;
-            uint32_t before = 0;
-            for (int k = 0; same > 1u && k < n; ++k) before += listed()[k].x == own.x && listed()[k].y < own.y ? 1u : 0u;
-            if (before == want) sh.bc_hit = own.y;
+    uint32_t greater = 0;
+    for (int i = tid; i < n; i += kThreads) {
+        const uint2 e = listed()[i];
+        const float q = __uint_as_float(e.x);
+        greater += q > p ? 1u : 0u;
+        if (q == p) {
+            const int at = atomicAdd(&sh.stop, 1);
+            if (at < kBlock) equal[at] = e.y;
         }
+    }
+    greater = block_sum(greater, sh.scan_u);   // (its barriers cover the list)
+    const int same = sh.stop;
+    if (same <= kBlock && tid < same) {
+        uint32_t before = 0;
+        for (int k = 0; k < same; ++k) before += equal[k] < equal[tid] ? 1u : 0u;
+        if (before == (rank < greater ? 0u : rank - greater)) sh.bc_hit = equal[tid];
+    }
     __syncthreads();
     const long long at = sh.bc_hit;
     __syncthreads();
