@@ -53,6 +53,7 @@ constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
 constexpr int kBlock = 256;           // consecutive elements a warp takes at a time, eight per lane
 constexpr int kMaxSegs = 640;         // segments of a row in index order; longer rows have segments of several blocks
+constexpr int kFusedBlocks = 4;       // segments of more (rows of more than 655360 elements) are summed in passes of their own
 constexpr int kBigSegs = 4;           // a bin of so many segments' elements is a segment by itself
 constexpr int kSegCap = kMaxSegs + 2 * kMaxSegs / kBigSegs + 192;   // in descending order: those, two boundaries per such bin, some per level
 constexpr int kBins = 2048;
@@ -1395,8 +1396,9 @@ struct Logits {
     }
 };
 
-// Maximum of the row and, for `masses`, the approximate sums of the exponentials before its segments (of one block each), from the
-// maxima and masses of 1024 elements at a time; *odd: the row holds NaN or +inf.  Bound by HBM.
+// Maximum of the row and, for `masses`, the approximate sums of the exponentials before its segments (of one block each; kLong: of up to
+// kFusedBlocks), from the maxima and masses of 1024 elements at a time; *odd: the row holds NaN or +inf.  Bound by HBM.
+template <bool kLong>
 __device__ __noinline__ float survey(Logits row, Segs g, float inv_T, bool masses, bool* odd) {
     ExactShared& sh = shared_memory();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1416,6 +1418,7 @@ __device__ __noinline__ float survey(Logits row, Segs g, float inv_T, bool masse
         for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
         mx = fmaxf(mx, top);
         const float ref = top == -CUDART_INF_F ? 0.f : -top * scale;
+        float whole = 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             float m = 0.f;
@@ -1431,7 +1434,15 @@ __device__ __noinline__ float survey(Logits row, Segs g, float inv_T, bool masse
             if (masses) {
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
-                if (lane == 0 && b + k < blocks) { sh.cum[b + k] = m; sh.state[b + k] = top; }
+                if (kLong) {   // (b is a multiple of four)
+                    const int per = g.shift - 8;
+                    const uint32_t j = (b + k) >> per;
+                    whole += m;
+                    if (((k + 1) & ((1 << per) - 1)) == 0) {
+                        if (lane == 0 && j < (uint32_t)g.count) { sh.cum[j] = whole; sh.state[j] = top; }
+                        whole = 0.f;
+                    }
+                } else if (lane == 0 && b + k < blocks) { sh.cum[b + k] = m; sh.state[b + k] = top; }
             }
         }
     }
@@ -1502,6 +1513,64 @@ __device__ __noinline__ void exponentials(Logits row, float mx, float inv_T, flo
     rest = __syncthreads_or(rest) != 0;
     level = Level{kOneBits + 1u, kTopShift, 0, rest};
 }
+// The same for segments of two or four blocks.
+template <bool kCount>
+__device__ __noinline__ void exponentials_long(Logits row, Segs g, float mx, float inv_T, float* ex, Level& level) {
+    ExactShared& sh = shared_memory();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const LaneTable tab(lane);
+    const uint32_t bins = (uint32_t)__cvta_generic_to_shared(sh.bins);
+    if (kCount)
+        for (int j = tid; j < kBins; j += kThreads) sh.bins[j] = 0;
+    __syncthreads();
+    bool rest = false;
+    const uint32_t blocks = (row.hi + kBlock - 1) / kBlock, per = 1u << (g.shift - 8);
+    for (int j = warp; j < g.count; j += kWarps) {
+        const uint32_t E = sh.E[j];
+        const int slot = sh.slot[j];
+        const bool lanes = lanes_at_hand(slot), amounts = !lanes && E != kNoGuess && E != kEmpty;
+        fsx::Step total = fsx::step_identity(), total_up = fsx::step_identity();
+        for (uint32_t b = j * per; b < min(blocks, (j + 1) * per); b += 2) {
+            float x[2][2][4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) row.load4<true>((b + h) * kBlock + 8 * lane + 4 * u, x[h][u]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (b + h >= blocks) break;
+                float y[8];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) y[4 * u + e] = expf_lanes_nonpositive(__fmul_rn(__fsub_rn(x[h][u][e], mx), inv_T), tab);
+                    if (kCount) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const uint32_t bin = (kOneBits - __float_as_uint(y[4 * u + e])) >> kTopShift;
+                            count_below(bins + 4 * bin, bin, (uint32_t)kBins);
+                            rest |= bin >= (uint32_t)kBins;
+                        }
+                    }
+                    *reinterpret_cast<float4*>(ex + (b + h) * kBlock + 8 * lane + 4 * u) = make_float4(y[4 * u], y[4 * u + 1], y[4 * u + 2], y[4 * u + 3]);
+                }
+                if (!amounts) continue;
+                bool tie;
+                total = fsx::then(total, block_step(y, E, true, &tie));
+                if (slot) total_up = fsx::then(total_up, block_step(y, E + 1u, true, &tie));
+            }
+        }
+        if (lanes) {
+            __syncwarp();   // the segment's exponentials are in memory
+            lane_steps(Exponentials{ex, 0}, j);
+        } else if (amounts && lane == 0) {
+            sh.step[j] = pack_amounts(total);
+            if (slot) step_up(slot, j) = pack_amounts(total_up);
+        }
+    }
+    rest = __syncthreads_or(rest) != 0;
+    level = Level{kOneBits + 1u, kTopShift, 0, rest};
+}
 // The same for any row and temperature, and the sums before the segments.
 __device__ __noinline__ void exponentials_any(Logits row, Segs g, float mx, float inv_T, float* ex) {
     ExactShared& sh = shared_memory();
@@ -1559,15 +1628,17 @@ __device__ void sample_row(const StepArgs& a, float* scratch, int r) {
     PROF_BEGIN;
     bool odd;
     const bool one_block = g.shift == 8;
-    const float mx = survey(in, g, inv_T, one_block, &odd);
+    const bool fused = g.len() <= (uint32_t)(kFusedBlocks * kBlock);
+    const float mx = one_block ? survey<false>(in, g, inv_T, true, &odd) : survey<true>(in, g, inv_T, fused, &odd);
     PROF_END(kProfMax);
     const bool plain = !odd && fabsf(mx) < CUDART_INF_F && inv_T > 0.f && inv_T < CUDART_INF_F;   // every exponential is between 0 and 1
     index_order_segments(g, lo, hi);
     Level level{kOneBits + 1u, kTopShift, 0, false};
     float norm = 0.f;
-    if (plain && one_block) {
+    if (plain && fused) {
         guess_binades(0, g.count, 0.f, CUDART_INF_F, -1.f, true);
-        if (top_p_active) exponentials<true>(in, mx, inv_T, ex, level);
+        if (!one_block) top_p_active ? exponentials_long<true>(in, g, mx, inv_T, ex, level) : exponentials_long<false>(in, g, mx, inv_T, ex, level);
+        else if (top_p_active) exponentials<true>(in, mx, inv_T, ex, level);
         else exponentials<false>(in, mx, inv_T, ex, level);
         PROF_END(kProfExp);
         ordered_sum(Exponentials{ex, 0}, 0, g.count, norm, CUDART_INF_F, -1.f, true);

@@ -76,6 +76,14 @@ def test_draws_among_equal_probabilities_follow_the_index(kind, v):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("v", [163838, 262144, 327677, 327681, 400001, 655357, 700001])
+@pytest.mark.parametrize("kind", ["bf16", "masked", "two_values"])
+def test_segments_of_several_blocks(kind, v):
+    """Vocabularies around those from which a segment has two, four and more blocks of 256 elements."""
+    test_draws_among_equal_probabilities_follow_the_index(kind, v)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("v", [300, 4096, 50257, 128256])
 @pytest.mark.parametrize("kind", KINDS + ["peaks", "steps"])
 def test_further_draws_of_a_row_follow_the_index_too(kind, v):
