@@ -219,6 +219,10 @@ int run_forward(pa_handle* h, const pa_forward_args* a, cudaStream_t stream) {
     // go to the warp-per-slice kernel, whose fixed slices cost nothing per chapter and balance well when every warp has hundreds of
     // tiles
     const bool shared_decode = pa::decode_shared_supported(h->g) && k.max_tiles <= (long long)h->sm_count * pa::decode_shared_chapter_tiles(h->g) * pa::decode_shared_max_chapters();
+    // One CTA per SM can wait beside the cache write's blocks.  Of decode_kernel's two or three per SM some find no room then, and come
+    // late where the write's blocks were: its equal slices end unequally (8 kv heads of 64, 4 sequences of 20000: 65 us, without 56;
+    // decode_shared_kernel on 40 heads, 10 of 5000: 50 us, without 55).
+    k.release_early = shared_decode ? 1 : 0;
     if (shared_decode) {   // one CTA per SM is the worker; its warps share the slice
         k.decode_phantom = pa::decode_shared_phantom();
         k.max_tiles += (long long)a->num_sequences * h->g.Hkv * k.decode_phantom;

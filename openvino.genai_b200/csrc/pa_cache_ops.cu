@@ -326,7 +326,7 @@ template <int D, bool PLAN, bool GROUPS>
 __global__ void __launch_bounds__(256) write_kv_kernel(KernelArgs a) {
     constexpr int PER = D / 32;
     grid_wait();
-    grid_release();
+    if (a.release_early) grid_release();
     // The plan blocks come first, so that they run beside the writes of a long chunk and not behind them.
     int first_block = 0;
     if constexpr (PLAN) {

@@ -17,9 +17,9 @@ constexpr int kWarp = 32;
 // The kernels of a step follow one another through memory only.  Each is launched as a programmatic dependent of the one before it in
 // the stream and waits at its top for that one's end (which by then is the end of all before it): what is left between two
 // kernels is the wait's own microsecond instead of a drain, a launch and a ramp.  No path of a kernel may leave before grid_wait().
-// The short ones (cache write, rotation, scores) also let the next one's CTAs come as soon as all of their own are there.  The
-// decode and prefill kernels do not: CTAs that wait beside theirs cost them more than a ramp (16 chunks of 512 tokens 707 | 733 us
-// with it, 64 decode rows 125 | 128, a mixed step 899 | 944).
+// The short ones (rotation, scores, and the cache write in front of one decode CTA per SM) also let the next one's CTAs come as soon as all of
+// their own are there.  The decode and prefill kernels do not: CTAs that wait beside theirs cost them more than a ramp (16 chunks of 512 tokens
+// 707 | 733 us with it, 64 decode rows 125 | 128, a mixed step 899 | 944).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

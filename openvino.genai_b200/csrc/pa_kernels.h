@@ -100,6 +100,7 @@ struct KernelArgs {
     int* pitem_order;      // [kPrefillSortCap] q tiles, longest context first (valid when plan->pitems_sorted); may be null
     int decode_all_workers;      // workers (warps of decode_kernel, CTAs of decode_shared_kernel) the decode launch will have (0: the plan prepares no start records)
     int decode_phantom;          // tiles added to every stream in the sequence the slices are cut in (SM-shared decode: a stream costs a CTA time beyond its tiles)
+    int release_early;           // the cache write lets the decode kernel's CTAs come before its own have ended
     int test_drop_copy;          // test hook: worker 0 issues no copy for its first tile and polls 2^10 times only
     WorkerStart* worker_start;   // [decode_all_workers], may be null
     long long max_tiles;   // upper bound of total_tiles known on the host

@@ -31,3 +31,13 @@ def test_dependents_wait_and_waiting_kernels_are_dependents():
                 assert "return" not in body[:body.index("grid_wait()")], f"{name}: {kernel} may leave before it has waited"
                 checked += 1
     assert checked >= 7
+
+
+def test_the_cache_write_releases_early_only_in_front_of_one_cta_per_sm():
+    """Two or three waiting CTAs per SM do not all fit beside the cache write's blocks, and those that come late end late."""
+    write = _kernels(SOURCES["pa_cache_ops.cu"])["write_kv_kernel"]
+    assert re.search(r"if \(a\.release_early\)\s*grid_release\(\)", write) and write.count("grid_release()") == 1
+    assert re.search(r"release_early = shared_decode\b", SOURCES["pa_api.cu"])
+    shared, sliced = (SOURCES[n] for n in ("pa_decode_shared.cu", "pa_decode.cu"))
+    assert re.search(r"__launch_bounds__\(kShMaxWarps \* 32, 1\) decode_shared_kernel", shared)
+    assert not re.search(r"__launch_bounds__\([^;{]*?, 1\) decode_kernel", sliced)
