@@ -19,7 +19,8 @@
 //   4. without top-p the same for the probabilities, the exact sum before every 256 elements kept for the draws;
 //      with top-p the elements of the highest bins are brought into shared memory bin by bin (one atomic gives a place)
 //      and ordered_sum runs over them in segments of whole bins until the sum exceeds top_p;
-//   5. a draw looks its segment up in the recorded sums and adds that segment's elements one by one.
+//   5. a draw looks its segment up in the recorded sums and adds that segment's elements one by one; with top-p a pass over the row, or the
+//      list that a row with several draws makes, gives the element's index.
 //
 // ordered_sum: while a float sum s stays in one binade, adding x to it is adding a whole number of ulps that depends on s
 // through its parity only, and not even on that unless x lies half-way between two.  So a lane adds its eight elements with
@@ -28,13 +29,14 @@
 // elements of a bin need not be sorted -, with one the segment is sorted and its lanes' amounts are composed in order.  The
 // binade of every segment is guessed from the masses (near a change of binade: both) and checked by the walk of one warp over
 // the segments.  Where the sum changes binade the lanes' amounts tell the lane, whose elements are added one by one; a segment
-// whose guess was wrong is added one by one.
+// whose guess was wrong, or in which the sum goes through binades, is added one by one.  (The rules: segment_sum.cuh.)
 //
-// 128 rows x 128256 of N(0, 4), top-p 0.95 (46 k kept): 421 -> 220 us a step; 200 rows x 151936, a quarter each greedy, top-k, top-p and
-// plain: 496 -> 160.  Before, one thread walked the bins and lists of sorted elements (most of the 400 - 500 k cycles of a top-p row's
+// 128 rows x 128256 of N(0, 4), top-p 0.95 (46 k kept): 421 -> 195 - 217 us a step; 200 rows x 151936, a quarter each greedy, top-k, top-p and
+// plain: 495 -> 160.  Before, one thread walked the bins and lists of sorted elements (most of the 400 - 500 k cycles of a top-p row's
 // sorted part), and the CTA rescanned spans with half-way cases (100 k of the index-order sum).  A top-p row's cycles now: 1. 38 k (HBM);
-// 2. 70 k (instruction issue); 3. 30 k (the walk, latency); 4. 115 k (ranks of the bins 10, gather 29, probabilities 11, amounts 30, walk 30);
-// 5. 42 k (a pass over the row to find the element's index 34).
+// 2. 72 k (instruction issue); 3. 30 k (the walk, latency); 4. 130 k (ranks of the bins 8, gather 39, probabilities 12, amounts 40, walk 30);
+// 5. 27 k (a pass over the row to find the element's index 21).  Some registers spill (64 for each of 1024 threads: 1.1 % of the instructions
+// are loads from local memory).
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
