@@ -31,7 +31,7 @@
 // the segments.  Where the sum changes binade the lanes' amounts tell the lane, whose elements are added one by one; a segment
 // whose guess was wrong, or in which the sum goes through binades, is added one by one.  (The rules: segment_sum.cuh.)
 //
-// 128 rows x 128256 of N(0, 4), top-p 0.95 (46 k kept): 421 -> 195 - 217 us a step; 200 rows x 151936, a quarter each greedy, top-k, top-p and
+// 128 rows x 128256 of N(0, 4), top-p 0.95 (46 k kept): 417 - 436 -> 195 - 222 us a step (by box); 200 rows x 151936, a quarter each greedy, top-k, top-p and
 // plain: 495 -> 160.  Before, one thread walked the bins and lists of sorted elements (most of the 400 - 500 k cycles of a top-p row's
 // sorted part), and the CTA rescanned spans with half-way cases (100 k of the index-order sum).  A top-p row's cycles now: 1. 38 k (HBM);
 // 2. 72 k (instruction issue); 3. 30 k (the walk, latency); 4. 130 k (ranks of the bins 8, gather 39, probabilities 12, amounts 40, walk 30);
